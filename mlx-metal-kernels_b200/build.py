@@ -1,4 +1,5 @@
-"""Builds ``lib/libb200q.so`` from ``csrc/*.cu`` with nvcc for sm_100a.
+"""Builds ``lib/libb200q.so`` from ``csrc/*.cu`` with nvcc for sm_100a, and the extension module ``lib/_b200q_host.so``
+(the operators' native call path, ``csrc/host_ops.cpp``) with the host compiler.
 
     python build.py            # from this directory, or
     build.build()              # from Python
@@ -13,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -20,6 +22,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 LIB = HERE / "lib" / "libb200q.so"
+HOST_SRC = CSRC / "host_ops.cpp"
+HOST_LIB = HERE / "lib" / "_b200q_host.so"
 HEADER = HERE.parent / "include" / "b200q.h"
 
 NVCC_FLAGS = [
@@ -44,6 +48,26 @@ def _newer(target: Path, deps) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _build_host(verbose: bool, force: bool) -> None:
+    """The call path needs the headers and libraries of the installed torch; the CUDA library does not."""
+    if not force and not _newer(HOST_LIB, [HOST_SRC]):
+        return
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda_include = Path(_nvcc()).resolve().parents[1] / "include"
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-isystem{d}" for d in (sysconfig.get_paths()["include"], root / "include",
+                                      root / "include" / "torch" / "csrc" / "api" / "include", cuda_include)),
+           str(HOST_SRC), "-o", str(HOST_LIB), f"-L{root / 'lib'}", f"-Wl,-rpath,{root / 'lib'}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {HOST_SRC.name}:\n{res.stdout}\n{res.stderr}")
+
+
 def build(verbose: bool = False, force: bool = False) -> Path:
     sources = sorted(CSRC.glob("*.cu"))
     headers = sorted(CSRC.glob("*.cuh")) + [HEADER]
@@ -63,7 +87,9 @@ def build(verbose: bool = False, force: bool = False) -> Path:
         return obj
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        host = pool.submit(_build_host, verbose, force)
         objs = list(pool.map(compile_one, sources))
+        host.result()
     if force or _newer(LIB, objs):
         cmd = [nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-gencode", "arch=compute_100a,code=sm_100a"]
         if verbose:

@@ -3,6 +3,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -15,7 +16,8 @@ namespace b200q {
 // ------------------------------------------------------------------------------------------------
 namespace {
 std::mutex g_mu;
-std::unordered_map<std::string, int> g_tuning;
+std::unordered_map<std::string, int> g_tuning;      // keys with a value other than 0 (unset)
+std::atomic<int> g_tuned{0};                        // their number
 struct DevProps { int sms = 0; int smem_optin = 0; };
 DevProps g_props[64];
 
@@ -52,6 +54,7 @@ void tp_take(int* in_slot, int* out_slot) {
 void tp_discard() { g_tp_next_in = g_tp_next_out = -1; }
 
 int tuning_get(const char* key) {
+    if (g_tuned.load(std::memory_order_acquire) == 0) return 0;      // nothing is set: a dozen look-ups per launch cost nothing
     std::lock_guard<std::mutex> lock(g_mu);
     auto it = g_tuning.find(key);
     return it == g_tuning.end() ? 0 : it->second;
@@ -343,7 +346,9 @@ int b200q_tp_next(int in_slot, int out_slot) {
 int b200q_set_tuning(const char* key, int value) {
     if (key == nullptr) return B200Q_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lock(g_mu);
-    g_tuning[key] = value;
+    if (value != 0) g_tuning[key] = value;
+    else g_tuning.erase(key);
+    g_tuned.store((int)g_tuning.size(), std::memory_order_release);
     return B200Q_OK;
 }
 

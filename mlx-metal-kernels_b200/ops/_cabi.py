@@ -7,6 +7,7 @@ exception is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import re
 from pathlib import Path
@@ -16,6 +17,7 @@ import torch
 F16, BF16, F32 = 0, 1, 2
 _PKG = Path(__file__).resolve().parents[1]
 LIB_PATH = _PKG / "lib" / "libb200q.so"
+HOST_LIB_PATH = _PKG / "lib" / "_b200q_host.so"
 HEADER_PATH = _PKG.parent / "include" / "b200q.h"
 
 _c = ctypes
@@ -64,6 +66,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class B200QError(RuntimeError):
@@ -105,6 +108,22 @@ def load():
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def host():
+    """The native call path of the operators (extension module built beside the library), bound to the loaded library.
+    Its functions return None for a call that is not the ordinary one; the Python body of the operator then takes it."""
+    global _host
+    if _host is None:
+        if not HOST_LIB_PATH.exists():
+            raise B200QError(f"{HOST_LIB_PATH} not found: build it with `python {_PKG / 'build.py'}`")
+        lib = load()
+        spec = importlib.util.spec_from_file_location("_b200q_host", HOST_LIB_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in SIGNATURES})
+        _host = module
+    return _host
 
 
 def check(rc: int, what: str) -> None:

@@ -141,6 +141,11 @@ def quantized_mlp_block(x, residual, norm_weight, gate_w, gate_scales, up_w, up_
     """z = x + residual; n = rmsnorm(z); g,u = Wg n, Wu n; m = silu(g)*u; d = Wd m; out = z + d, every
     stage rounded to x.dtype (ops/mlp_block_ops.py:301-364).  With ``return_intermediates`` also
     returns ``{"z","normed","gate","up","mlp","down"}``."""
+    if backend_preset == "cuda" and not return_intermediates:
+        out = _cabi.host().mlp_block(x, residual, norm_weight, gate_w, gate_scales, gate_zeros, up_w, up_scales, up_zeros, down_w,
+                                     down_scales, down_zeros, bits, group_size, eps)
+        if out is not None:
+            return out
     if x.shape != residual.shape:
         raise ValueError(f"x and residual must have identical shapes, got {tuple(x.shape)}, {tuple(residual.shape)}")
     if x.ndim != 3:

@@ -328,6 +328,10 @@ def paged_quantized_kv_gqa_decode_attention(q, paged_qkv: PagedQuantizedKVCache,
     or the reference's ``"metal_q8"`` / ``"metal_q4"`` with their bits precondition; the default
     ``"reference"`` names the pure-MLX path and raises here
     (ops/paged_quantized_kv_ops.py:632-661)."""
+    if backend == "cuda":
+        out = _cabi.host().paged_attention(q, paged_qkv, scale, 0, 0)
+        if out is not None:
+            return out
     B, MAX_S, PAGE_SIZE, MAX_BLOCKS, Hq, Hkv, D, NUM_PAGES = _validate_paged_quantized_decode_inputs(q, paged_qkv)
     if scale is None:
         scale = 1.0 / math.sqrt(D)
@@ -363,6 +367,10 @@ def sparse_paged_quantized_kv_gqa_decode_attention(q, paged_qkv: PagedQuantizedK
         raise TypeError("pattern must be a SparseAttentionPattern")
     block_sparse = pattern.validate().pattern == "block_sparse"
     sink_tokens, window_size = (0, 0) if block_sparse else decode_window(pattern)
+    if backend == "cuda" and not block_sparse:
+        out = _cabi.host().paged_attention(q, paged_qkv, scale, sink_tokens, window_size)
+        if out is not None:
+            return out
     B, MAX_S, PAGE_SIZE, MAX_BLOCKS, Hq, Hkv, D, NUM_PAGES = _validate_paged_quantized_decode_inputs(q, paged_qkv)
     if scale is None:
         scale = 1.0 / math.sqrt(D)

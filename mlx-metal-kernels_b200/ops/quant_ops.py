@@ -203,6 +203,9 @@ def reference_q8_matvec_decode(x, q_w, scales, zeros=None, *, group_size: int = 
 
 def q4_matvec_decode(x, packed_w, scales, zeros=None, *, group_size: int = 32, backend: str = "auto"):
     """x [B,K] or [B,1,K] -> [B,N] in x.dtype (ops/quant_ops.py:529-571)."""
+    y = _cabi.host().matvec(4, x, packed_w, scales, zeros, group_size, backend)
+    if y is not None:
+        return y
     x2d, B, K = _normalize_x_2d(x)
     _validate_matvec_input_dtype(x2d)
     if packed_w.ndim != 2:
@@ -217,6 +220,9 @@ def q4_matvec_decode(x, packed_w, scales, zeros=None, *, group_size: int = 32, b
 
 def q8_matvec_decode(x, q_w, scales, zeros=None, *, group_size: int = 32, backend: str = "auto"):
     """ops/quant_ops.py:591-631."""
+    y = _cabi.host().matvec(8, x, q_w, scales, zeros, group_size, backend)
+    if y is not None:
+        return y
     x2d, B, K = _normalize_x_2d(x)
     _validate_matvec_input_dtype(x2d)
     if q_w.ndim != 2 or q_w.shape[1] != K:
