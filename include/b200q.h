@@ -280,6 +280,15 @@ int b200q_attention_stage_launches(int B, int Hkv, int with_append);
 int b200q_quantize_kv(int bits, const void* values, uint8_t* codes, void* scales, int64_t rows, int D, int group_size,
                       int in_dtype, void* stream);
 
+/* K and V rows of one shape quantised in one launch (quantize_kv_pages, ops/paged_quantized_kv_ops.py:194-292), and the
+ * inverse (dequantize_kv_pages, :295-341): out = fp16((code - 128 | 8) * |scale|) with fp16 scales.  The inverse takes
+ * groups of 8, 16, ... 256 values that divide D and 16-byte aligned rows, else B200Q_ERR_UNSUPPORTED (b200q_dequant with
+ * zero points 128 | 8 and |scale| gives the same bits for every shape). */
+int b200q_quantize_kv_pair(int bits, const void* k, const void* v, uint8_t* k_codes, uint8_t* v_codes, void* k_scales,
+                           void* v_scales, int64_t rows, int D, int group_size, int in_dtype, void* stream);
+int b200q_dequantize_kv_pair(int bits, const uint8_t* k_codes, const uint8_t* v_codes, const void* k_scales,
+                             const void* v_scales, void* k, void* v, int64_t rows, int D, int group_size, void* stream);
+
 /* Tensor-parallel glue (no counterpart in the reference, which is single-device): all-gather of an
  * activation shard over NVLink peer memory.  `local` [rows, row_bytes_local] is this rank's shard;
  * peer_full[r] / peer_flags[r] are HOST arrays of `world` device pointers: rank r's full buffer

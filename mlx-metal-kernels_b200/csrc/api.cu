@@ -67,8 +67,10 @@ int gemv_read_status(int reset, cudaStream_t stream);
 int attn_read_status(int reset, cudaStream_t stream);
 int peer_read_status(int reset, cudaStream_t stream);
 int stack_read_status(int reset, cudaStream_t stream);
-int quantize_kv_impl(int bits, const void* values, uint8_t* codes, void* scales, int64_t rows, int D, int group_size,
-                     int in_dtype, cudaStream_t stream);
+int quantize_kv_pair_impl(int bits, const void* k, const void* v, uint8_t* k_codes, uint8_t* v_codes, void* k_scales, void* v_scales,
+                          int64_t rows, int D, int group_size, int in_dtype, cudaStream_t stream);
+int dequantize_kv_pair_impl(int bits, const uint8_t* k_codes, const uint8_t* v_codes, const void* k_scales, const void* v_scales, void* k,
+                            void* v, int64_t rows, int D, int group_size, cudaStream_t stream);
 int peer_allgather_impl(const void* local, void* const* peer_full, uint32_t* const* peer_flags, uint32_t* epoch,
                         int rank, int world, int rows, int64_t row_bytes_local, cudaStream_t stream);
 int wait_expiry_selftest_impl(uint32_t limit, uint32_t* probes_out, cudaStream_t stream);
@@ -512,7 +514,22 @@ int b200q_paged_fp16_gqa_decode(const void* q, const void* k_pages, const void* 
 int b200q_quantize_kv(int bits, const void* values, uint8_t* codes, void* scales, int64_t rows, int D, int group_size,
                       int in_dtype, void* stream) {
     tp_discard();
-    return quantize_kv_impl(bits, values, codes, scales, rows, D, group_size, in_dtype, (cudaStream_t)stream);
+    return quantize_kv_pair_impl(bits, values, nullptr, codes, nullptr, scales, nullptr, rows, D, group_size, in_dtype,
+                                 (cudaStream_t)stream);
+}
+
+int b200q_quantize_kv_pair(int bits, const void* k, const void* v, uint8_t* k_codes, uint8_t* v_codes, void* k_scales, void* v_scales,
+                           int64_t rows, int D, int group_size, int in_dtype, void* stream) {
+    tp_discard();
+    if (v == nullptr) return B200Q_ERR_BAD_ARG;
+    return quantize_kv_pair_impl(bits, k, v, k_codes, v_codes, k_scales, v_scales, rows, D, group_size, in_dtype, (cudaStream_t)stream);
+}
+
+int b200q_dequantize_kv_pair(int bits, const uint8_t* k_codes, const uint8_t* v_codes, const void* k_scales, const void* v_scales, void* k,
+                             void* v, int64_t rows, int D, int group_size, void* stream) {
+    tp_discard();
+    if (v_codes == nullptr) return B200Q_ERR_BAD_ARG;
+    return dequantize_kv_pair_impl(bits, k_codes, v_codes, k_scales, v_scales, k, v, rows, D, group_size, (cudaStream_t)stream);
 }
 
 int b200q_rope_append_paged_gqa_decode(const void* qkv, const float* cos_table, const float* sin_table,

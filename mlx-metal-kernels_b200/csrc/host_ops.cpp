@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <vector>
 
 namespace {
 
@@ -36,6 +37,9 @@ int (*p_attn)(int, const void*, const uint8_t*, const uint8_t*, const void*, con
               void*, size_t, int, int, int, int, int, int64_t, int, int, float, int, int, void*) = nullptr;
 int (*p_attn_window)(int, const void*, const uint8_t*, const uint8_t*, const void*, const void*, const int32_t*, const int32_t*,
                      void*, void*, size_t, int, int, int, int, int, int64_t, int, int, float, int, int, int, int, void*) = nullptr;
+
+int (*p_quant_pair)(int, const void*, const void*, uint8_t*, uint8_t*, void*, void*, int64_t, int, int, int, void*) = nullptr;
+int (*p_dequant_pair)(int, const uint8_t*, const uint8_t*, const void*, const void*, void*, void*, int64_t, int, int, void*) = nullptr;
 
 constexpr int kMinNormRows = 5;      // from this many rows on the library runs the rmsnorm as a launch of its own
 
@@ -225,12 +229,69 @@ PyObject* paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     return rc == 0 ? THPVariable_Wrap(std::move(out)) : none();
 }
 
+PyObject* tuple_of(std::initializer_list<Tensor*> ts) {
+    PyObject* out = PyTuple_New((Py_ssize_t)ts.size());
+    Py_ssize_t i = 0;
+    for (Tensor* t : ts) PyTuple_SET_ITEM(out, i++, THPVariable_Wrap(std::move(*t)));
+    return out;
+}
+
+// quantize_kv(K, V, bits, group_size) -> (k codes, v codes, k scales, v scales) or None; K, V [..., D] of one shape
+PyObject* quantize_kv(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    int64_t bits, group;
+    if (p_quant_pair == nullptr || n_args != 4 || !as_int(a[2], &bits) || !as_int(a[3], &group) || (bits != 4 && bits != 8) || group <= 0)
+        return none();
+    const Tensor *k = as_tensor(a[0]), *v = as_tensor(a[1]);
+    const int dev = current_device_of(k);
+    if (dev < 0 || v == nullptr || k->dim() < 1 || k->sizes() != v->sizes() || !on(*k, dev) || !on(*v, dev) || !act_dtype(k->scalar_type()) ||
+        v->scalar_type() != k->scalar_type() || k->numel() == 0)
+        return none();
+    const int64_t D = k->size(-1);
+    if (D > INT32_MAX || group > INT32_MAX) return none();
+    std::vector<int64_t> shape(k->sizes().begin(), k->sizes().end());
+    shape.back() = bits == 4 ? (D + 1) / 2 : D;
+    Tensor kc = empty(shape, at::kByte, dev), vc = empty(shape, at::kByte, dev);
+    shape.back() = (D + group - 1) / group;
+    Tensor ks = empty(shape, at::kHalf, dev), vs = empty(shape, at::kHalf, dev);
+    const auto u8 = [](Tensor& t) { return static_cast<uint8_t*>(t.mutable_data_ptr()); };
+    const int rc = p_quant_pair((int)bits, k->const_data_ptr(), v->const_data_ptr(), u8(kc), u8(vc), ks.mutable_data_ptr(),
+                                vs.mutable_data_ptr(), k->numel() / D, (int)D, (int)group, dtype_code(k->scalar_type()), stream_of(dev));
+    return rc == 0 ? tuple_of({&kc, &vc, &ks, &vs}) : none();
+}
+
+// dequantize_kv(k codes, v codes, k scales, v scales, bits, group_size, shape) -> (K, V) fp16 of `shape`, or None
+PyObject* dequantize_kv(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    int64_t bits, group;
+    if (p_dequant_pair == nullptr || n_args != 7 || !as_int(a[4], &bits) || !as_int(a[5], &group) || (bits != 4 && bits != 8) ||
+        group <= 0 || !PyTuple_Check(a[6]))
+        return none();
+    const Tensor *kc = as_tensor(a[0]), *vc = as_tensor(a[1]), *ks = as_tensor(a[2]), *vs = as_tensor(a[3]);
+    const int dev = current_device_of(kc);
+    if (dev < 0 || !vc || !ks || !vs || !on(*kc, dev) || !on(*vc, dev) || !on(*ks, dev) || !on(*vs, dev) || kc->scalar_type() != at::kByte ||
+        vc->scalar_type() != at::kByte || ks->scalar_type() != at::kHalf || vs->scalar_type() != at::kHalf)
+        return none();
+    std::vector<int64_t> shape((size_t)PyTuple_GET_SIZE(a[6]));
+    int64_t n = 1;
+    for (size_t i = 0; i < shape.size(); ++i) {
+        if (!as_int(PyTuple_GET_ITEM(a[6], i), &shape[i]) || shape[i] <= 0) return none();
+        n *= shape[i];
+    }
+    if (shape.empty() || shape.back() > INT32_MAX || group > INT32_MAX) return none();
+    const int64_t D = shape.back(), rows = n / D, dp = bits == 4 ? (D + 1) / 2 : D, gd = (D + group - 1) / group;
+    if (kc->numel() != rows * dp || vc->numel() != rows * dp || ks->numel() != rows * gd || vs->numel() != rows * gd) return none();
+    Tensor k = empty(shape, at::kHalf, dev), v = empty(shape, at::kHalf, dev);
+    const int rc = p_dequant_pair((int)bits, codes(kc), codes(vc), ptr(ks), ptr(vs), k.mutable_data_ptr(), v.mutable_data_ptr(), rows, (int)D,
+                                  (int)group, stream_of(dev));
+    return rc == 0 ? tuple_of({&k, &v}) : none();
+}
+
 // bind({symbol: address}): the C ABI functions to call
 PyObject* bind(PyObject*, PyObject* table) {
     const struct { const char* name; void** slot; } want[] = {
         {"b200q_qmatvec", (void**)&p_qmatvec}, {"b200q_gate_up_swiglu", (void**)&p_gate_up},
         {"b200q_paged_gqa_workspace_bytes", (void**)&p_attn_ws}, {"b200q_attention_stage_launches", (void**)&p_attn_launches},
         {"b200q_paged_gqa_decode", (void**)&p_attn}, {"b200q_paged_gqa_decode_window", (void**)&p_attn_window},
+        {"b200q_quantize_kv_pair", (void**)&p_quant_pair}, {"b200q_dequantize_kv_pair", (void**)&p_dequant_pair},
     };
     for (const auto& w : want) {
         PyObject* v = PyDict_GetItemString(table, w.name);
@@ -257,6 +318,8 @@ PyMethodDef methods[] = {
     {"bind", bind, METH_O, "bind({symbol: address})"},
     {"matvec", FAST(matvec), METH_FASTCALL, nullptr},
     {"mlp_block", FAST(mlp_block), METH_FASTCALL, nullptr},
+    {"quantize_kv", FAST(quantize_kv), METH_FASTCALL, nullptr},
+    {"dequantize_kv", FAST(dequantize_kv), METH_FASTCALL, nullptr},
     {"paged_attention", FAST(paged_attention), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

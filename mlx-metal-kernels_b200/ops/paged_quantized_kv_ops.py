@@ -148,11 +148,13 @@ def quantize_kv_pages(K_pages, V_pages, block_table, lengths, config: PagedQuant
     if K_pages.ndim != 4:
         raise ValueError(f"K_pages must be 4-D [NUM_PAGES,PAGE_SIZE,Hkv,D], got {tuple(K_pages.shape)}")
     NUM_PAGES, PAGE_SIZE, Hkv, D = K_pages.shape
-    out = []
-    for pages in (K_pages, V_pages):
-        out.append(_quantize_groups(pages, config.bits, config.group_size))
+    out = _cabi.host().quantize_kv(K_pages, V_pages, config.bits, config.group_size)
+    if out is None:
+        (kq, ks), (vq, vs) = (_quantize_groups(pages, config.bits, config.group_size) for pages in (K_pages, V_pages))
+    else:
+        kq, vq, ks, vs = out
     return PagedQuantizedKVCache(
-        k_pages_q=out[0][0], v_pages_q=out[1][0], k_scales=out[0][1], v_scales=out[1][1],
+        k_pages_q=kq, v_pages_q=vq, k_scales=ks, v_scales=vs,
         block_table=block_table, lengths=lengths, bits=config.bits, page_size=config.page_size,
         group_size=config.group_size, original_page_shape=tuple(K_pages.shape),
     )
@@ -165,6 +167,10 @@ def dequantize_kv_pages(paged_qkv: PagedQuantizedKVCache):
     orig = paged_qkv.original_page_shape
     if orig is None:
         raise ValueError("original_page_shape is required for dequantization")
+    out = _cabi.host().dequantize_kv(paged_qkv.k_pages_q, paged_qkv.v_pages_q, paged_qkv.k_scales, paged_qkv.v_scales, paged_qkv.bits,
+                                     paged_qkv.group_size, orig)
+    if out is not None:
+        return out
     NUM_PAGES, PAGE_SIZE, Hkv, D = orig
     rows = NUM_PAGES * PAGE_SIZE * Hkv
     groups = (D + paged_qkv.group_size - 1) // paged_qkv.group_size

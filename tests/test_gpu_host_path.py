@@ -50,3 +50,29 @@ def test_paged_attention_equals_python_body(cuda, batch, window):
     assert got is not None and torch.equal(got.reshape(want.shape), want)
     cache.lengths = cache.lengths.to(torch.int64)
     assert cabi.host().paged_attention(q, cache, None, 4, window) is None
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("pages,D,G,dtype", [(1, 128, 32, torch.float16), (5, 128, 64, torch.bfloat16), (67, 64, 8, torch.float16),
+                                             (3, 512, 256, torch.float16), (2, 24, 8, torch.bfloat16), (2, 48, 32, torch.float16)])
+def test_quantised_pages_equal_python_body(cuda, bits, pages, D, G, dtype):
+    """K and V pages through the 16-byte kernels and back: codes and scales of the oracle's rule bit for bit, for values on
+    and next to the ties of the rounding, zero groups and outliers; the last shape (a short last group) takes the general ones."""
+    k, v = (synth.activations((pages, 16, 3, D), s, "cpu", dtype) for s in (21, 22))
+    k.view(-1)[:G] = 0.0
+    limit = 127 if bits == 8 else 7
+    v.view(-1)[:G] = ((torch.arange(G) % (2 * limit)).float() - limit + 0.5).to(dtype)      # scale near 1: quotients at ties
+    v.view(-1)[0] = float(limit)
+    v.view(-1)[-1] = 3.0e4
+    bt, ln = torch.zeros((1, 1), dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+    got = pq_ops.quantize_kv_pages(k.to(cuda), v.to(cuda), bt, ln, pq_ops.PagedQuantizedKVConfig(bits=bits, group_size=G))
+    for pages_t, codes, scales in ((k, got.k_pages_q, got.k_scales), (v, got.v_pages_q, got.v_scales)):
+        oc, osc = synth.quantize_kv_symmetric(pages_t, bits, G)
+        assert torch.equal(codes.cpu(), oc) and torch.equal(scales.cpu(), osc)
+    kd, vd = pq_ops.dequantize_kv_pages(got)
+    off = 128.0 if bits == 8 else 8.0
+    for out, codes, scales in ((kd, got.k_pages_q, got.k_scales), (vd, got.v_pages_q, got.v_scales)):
+        rows = out.numel() // D
+        s = scales.reshape(rows, -1).abs()
+        ref = quant_ops.dequant_codes(bits, codes.reshape(rows, -1), s, torch.full_like(s, off), rows, D, G, torch.float16)
+        assert torch.equal(out.reshape(rows, D), ref)
