@@ -2,9 +2,10 @@
 //
 //   y[b, n] = sum_k x[b, k] * (code[n, k] - zero[n, k/G]) * scale[n, k/G]
 //
-// The tensor-core kernel (gemv_fast.cuh) serves group sizes 32 / 64 / 128 with 16-byte aligned rows
-// and up to 16 batch rows per launch.  Everything else runs the general kernel below, which follows
-// the reference arithmetic literally.
+// Group sizes 32 / 64 / 128 with 16-byte aligned rows run on tensor cores: one to four batch rows on integer products of the raw
+// codes (gemv_i8.cuh), five and more on tcgen05 (qgemm_ts.cu), what neither takes - scales that are not fp16, bf16 rows from
+// batch 5 on - on fp16 mma.sync (gemv_fast.cuh, up to 16 batch rows per launch).  Everything else runs the general kernel
+// below, which follows the reference arithmetic literally.
 #include "gemv_params.cuh"
 
 #include <algorithm>
@@ -20,7 +21,11 @@ int gemv_read_status(int reset, cudaStream_t stream) {
     const int a = gemv_q4_read_status(reset, stream);
     const int b = gemv_q8_read_status(reset, stream);
     const int c = qgemm_ts_read_status(reset, stream);
-    return a != 0 ? a : (b != 0 ? b : c);
+    const int d = gemv_i8_q4_read_status(reset, stream);
+    const int e = gemv_i8_q8_read_status(reset, stream);
+    for (int v : {a, b, c, d})
+        if (v != 0) return v;
+    return e;
 }
 
 namespace {
@@ -123,7 +128,7 @@ bool fast_path_ok(const GemvParams& p) {
 
 // Which kernel takes a launch: "gemv.ts" = 1 sends everything the tcgen05 kernel supports to it, -1 nothing,
 // 0 (default) the batches of gemv.ts_min_batch rows and more (default 5: measured crossover at the Llama-3-8B
-// shapes, where the mma.sync kernel pays its per-group affine step once per batch row tile).
+// shapes; the integer kernel's work grows with every batch row, this one's does not).
 bool prefer_ts(const GemvParams& p) {
     const int mode = tuning_get("gemv.ts");
     if (mode < 0) return false;
@@ -150,6 +155,16 @@ int dispatch_fast(int bits, GemvParams& p, bool gate_up, cudaStream_t stream) {
     if (prefer_ts(p)) {
         const int rc = qgemm_ts(bits, p, gate_up, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
+    }
+    if (p.B <= 4 && tuning_get("gemv.i8") >= 0) {
+        int rc = bits == 4 ? gemv_i8_q4(p, gate_up, stream) : gemv_i8_q8(p, gate_up, stream);
+        if (rc != B200Q_ERR_UNSUPPORTED) return rc;
+        // three or four long rows do not fit into its shared memory: there the tcgen05 kernel comes next (4096 x 14336, four
+        // rows: 17 us against 23 us of the fp16 mma.sync kernel)
+        if (p.B >= 3 && tuning_get("gemv.ts") == 0) {
+            rc = qgemm_ts(bits, p, gate_up, stream);
+            if (rc != B200Q_ERR_UNSUPPORTED) return rc;
+        }
     }
     if (p.B > 16) return B200Q_ERR_UNSUPPORTED;
     return bits == 4 ? gemv_fast_q4(p, gate_up, stream) : gemv_fast_q8(p, gate_up, stream);

@@ -1,0 +1,656 @@
+// Weight-streaming quantized matvec for one to four batch rows (sm_100a): integer tensor-core products of raw codes.
+//
+//   y[b, n] = sum_k x[b, k] * (code[n, k] - zero[n, k/G]) * scale[n, k/G]
+//
+// What bounds it: HBM.  At 6.5 TB/s an SM receives 23 bytes, i.e. 46 q4 codes, per clock, so the code path has to stay
+// well below 4 issue slots per 46 codes.  The kernel it replaces for these batches (gemv_fast.cuh) turns every code pair into
+// fp16 (5 logic instructions and 2 mma.sync per 512 codes and row half) and needed 2.2 slots per clock at 0.49 of the
+// copy rate (2 x 14336 x 4096 q4, one row: 20.7 us; here 14.8 us, 0.69; 6144 x 4096: 6.8 -> 5.5 us).
+//   * mma.sync.m16n8k32 u8 x s8: a q4 word gives its even codes with one mask and its odd ones with a shift and a mask, a
+//     q8 word is the operand as it lies.  512 codes per instruction, exact in int32.
+//   * the activations become integers.  Per quantisation group they are scaled by a power of two to 22-bit fixed point
+//     (an element below 2^-11 of its group's largest is rounded at 2^-23 of that, the size of an fp32 sum's own rounding; all
+//     others are exact) and cut into three signed bytes.  The three digits of a row are three columns of the 8-wide B
+//     operand, which a matvec leaves empty anyway; digit sums meet in int32 and fp32.
+//   * per group, in fp32: y += scale * ((c2 2^16 + c1 2^8 + c0) 2^-e - zero * X), X = sum of the group's activations.  With
+//     one batch row two neighbouring groups sit side by side in the 8 columns and share this step.
+// The weights are not rounded at all.
+//
+// Work: rows are dealt evenly to the CTAs (one per SM), cut into tiles of at most 16 rows; a unit is a tile x 256 bytes of every
+// row (512 q4 or 256 q8 codes), units are dealt to the 16 warps in order.  A warp is on its own: every lane copies 16-byte pieces
+// with cp.async into a private ring (4 KB of codes per warp in flight, 64 KB per SM, started before griddepcontrol.wait since
+// weights do not depend on the previous kernel): no producer warps and no barriers in the stream.  While piece c of a unit is
+// consumed, piece c of the warp's next unit takes its place, so all shared-memory addresses are constants.  For one or two rows the
+// CTA stays below half of an SM, so that the next kernel of a dependent chain can be resident and loading while this one drains.
+// The units' sums meet in shared memory and are added in k order: the order does not depend on the CTA, the tile or the
+// number of rows, so a tensor-parallel shard reproduces the unsharded rows bit for bit.
+//
+// Compiled into one translation unit per code width.
+#pragma once
+
+#include "gemv_params.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+namespace b200q {
+namespace {
+
+constexpr int kI8Warps = 16;
+constexpr int kI8Threads = kI8Warps * 32;
+constexpr int kI8UnitBytes = 256;             // bytes of a unit in one row: four 64-byte pieces
+constexpr int kI8MaxRes = 1024;               // residual values kept in shared memory
+
+struct I8Params {
+    const void* x;          // [B, K]
+    const void* res_in;     // norm prologue: rows = rmsnorm(x + res_in); may be null
+    const void* norm_w;     // [K]; null = no prologue
+    void* z_out;            // [B, K] or null
+    void* normed_out;       // [B, K] or null
+    const uint8_t* w[2];
+    const __half* s[2];
+    const __half* z[2];
+    const void* residual;
+    void* y;
+    void* gate_out;
+    void* up_out;
+    void* act_out;
+    float eps;
+    int B, N, K, Gn, mats;
+    int act_dtype, norm_w_dtype, row_bytes;
+    int rows_lo, rem;       // CTA c owns rows_lo (+1 if c < rem) rows
+    int units;              // units per (tile, matrix)
+    int batch;              // tiles whose sums fit into shared memory at once
+    int meta_vec;           // a row's groups fill whole units: the scales of a unit are aligned pieces
+    TpOut tp_out;
+    TpIn tp_in;
+    uint32_t off_zero, off_xd, off_cst, off_res, off_part, off_meta, off_ring;
+    uint32_t xstride, meta_slot;
+};
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+template <int BYTES>
+__device__ __forceinline__ void cp_small(uint32_t dst, const void* src) {      // 4 or 8 bytes
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void cp16_part(uint32_t dst, const void* src, uint32_t bytes) {      // the rest is zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ float i8_warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ float i8_round_act(float v, int dtype) {
+    return dtype == B200Q_F16 ? __half2float(__float2half_rn(v)) : __bfloat162float(__float2bfloat16_rn(v));
+}
+__device__ __forceinline__ void i8_words_to_f32(const uint32_t (&w)[4], int dtype, float (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (dtype == B200Q_F16) {
+            const __half2 h = *reinterpret_cast<const __half2*>(&w[i]);
+            v[2 * i] = __low2float(h);
+            v[2 * i + 1] = __high2float(h);
+        } else {
+            v[2 * i] = __uint_as_float(w[i] << 16);
+            v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+        }
+    }
+}
+__device__ __forceinline__ void i8_pack(uint32_t (&w)[4], int dtype, const float (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (dtype == B200Q_F16) {
+            const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        } else {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+    }
+}
+__device__ __forceinline__ void i8_ldg(uint32_t (&w)[4], const void* base, int64_t idx) {
+    const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + idx);
+    w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+}
+__device__ __forceinline__ void i8_stg(void* base, int64_t idx, const uint32_t (&w)[4]) {
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(base) + idx) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+// Eight values of an input row, packed: x, or cast(x + res).  Plain rows, or packets of a tensor-parallel exchange, polled
+// until they carry the expected sequence number (a template parameter: kernels that read plain rows are compiled without it).
+struct I8Source { uint32_t seq16, limit; };
+template <bool PACKETS>
+__device__ __forceinline__ void i8_load_z(const I8Params& p, int64_t idx, I8Source& xs, uint32_t (&w)[4]) {
+    if constexpr (!PACKETS) {
+        i8_ldg(w, p.x, idx);
+    } else if (!tp_load8_packets(p.x, idx, xs.seq16, xs.limit, w)) {
+        atomicMax(&g_device_status, (int)EV_PEER_WAIT);
+        xs.limit = 64u;
+    }
+    if (p.res_in != nullptr) {
+        uint32_t rw[4];
+        float v[8], r[8];
+        i8_ldg(rw, p.res_in, idx);
+        i8_words_to_f32(w, p.act_dtype, v);
+        i8_words_to_f32(rw, p.act_dtype, r);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] += r[i];
+        i8_pack(w, p.act_dtype, v);
+    }
+}
+
+__device__ __forceinline__ uint32_t s_ld32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void s_ld64(uint32_t a, uint32_t& x, uint32_t& y) {
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(a));
+}
+__device__ __forceinline__ float s_ldh(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return __half2float(__ushort_as_half(v));
+}
+template <int NW>
+__device__ __forceinline__ void s_ldw(uint32_t a, uint32_t (&w)[NW]) {
+    if constexpr (NW == 1) {
+        w[0] = s_ld32(a);
+    } else if constexpr (NW == 2) {
+        s_ld64(a, w[0], w[1]);
+    } else {
+        static_assert(NW == 4, "one 16-byte piece at most");
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(a));
+    }
+}
+// D(16x8, s32) (+)= A(16x32, u8, row) * B(32x8, s8, col)
+template <bool FIRST>
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (FIRST) {
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+    } else {
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    }
+}
+
+// One group of 16 rows against every column tile: rows g and g + 8 at `a_addr` (+ 512), digits at bx + bofs.
+template <int BITS, int LOGG, int NT, bool FIRST>
+__device__ __forceinline__ void i8_group_mma(int (&acc)[NT][4], uint32_t a_addr, const uint32_t (&bx)[NT], uint32_t bofs) {
+    constexpr int GB = (1 << LOGG) * BITS / 8;
+    constexpr int NW = (GB / 4 > 16 ? 16 : GB / 4) / 4;
+    constexpr int MI = BITS == 4 ? NW : NW / 2;
+#pragma unroll
+    for (int h = 0; h < (GB == 128 ? 2 : 1); ++h) {
+        uint32_t wa[NW], wb[NW];
+        s_ldw<NW>(a_addr + h * 1024, wa);
+        s_ldw<NW>(a_addr + h * 1024 + 512, wb);
+#pragma unroll
+        for (int i = 0; i < MI; ++i) {
+            uint32_t a0, a1, a2, a3;
+            if constexpr (BITS == 4) {
+                a0 = wa[i] & 0x0F0F0F0Fu; a1 = wb[i] & 0x0F0F0F0Fu;
+                a2 = (wa[i] >> 4) & 0x0F0F0F0Fu; a3 = (wb[i] >> 4) & 0x0F0F0F0Fu;
+            } else {
+                a0 = wa[2 * i]; a1 = wb[2 * i]; a2 = wa[2 * i + 1]; a3 = wb[2 * i + 1];
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                uint32_t b0, b1;
+                s_ld64(bx[nt] + bofs + (h * MI + i) * 96, b0, b1);
+                if (FIRST && h == 0 && i == 0) mma_u8s8<true>(acc[nt], a0, a1, a2, a3, b0, b1);
+                else mma_u8s8<false>(acc[nt], a0, a1, a2, a3, b0, b1);
+            }
+        }
+    }
+}
+
+struct I8Pos { int tile, m, i; };             // a unit: tile, matrix, position in the row
+__device__ __forceinline__ void i8_advance(I8Pos& u, int by, int U, int mats) {
+    u.i += by;
+    while (u.i >= U) {
+        u.i -= U;
+        if (++u.m == mats) { u.m = 0; ++u.tile; }
+    }
+}
+
+// BITS: code width.  LOGG: log2(group size), 5..7.  NB: batch columns, 1, 2 or 4.
+template <int BITS, int LOGG> struct I8Shape {
+    static constexpr int G = 1 << LOGG;
+    static constexpr int GB = G * BITS / 8;                  // bytes of a group in one row: 16 .. 128
+    static constexpr int NM = G / 32;                        // mma per group
+    static constexpr int GU = kI8UnitBytes / GB;             // groups per unit: 16 .. 2
+    static constexpr int CP = GB > 64 ? GB / 64 : 1;         // 64-byte pieces per chunk (a chunk holds whole groups)
+    static constexpr int CH = 4 / CP;                        // chunks per unit
+    static constexpr int CG = CP * 64 / GB;                  // groups per chunk: 4, 2 or 1
+    static constexpr int MB = GU * 2;                        // bytes of a unit's scales in one row: 32 .. 4
+    static constexpr int WIN = MB > 16 ? 3 : 2;              // 16-byte pieces of an aligned window around them
+    static constexpr int XG = 96 * NM;                       // digit bytes of one group: [mma][digit][lane t] 8 bytes
+    static constexpr int XU = GU * XG;                       // ... of a unit: 1536 (q4) or 768 (q8)
+};
+
+template <int BITS, int LOGG, int NB, bool PACKETS>
+__global__ void __launch_bounds__(kI8Threads, NB <= 2 ? 2 : 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    using S = I8Shape<BITS, LOGG>;
+    constexpr int G = S::G, GB = S::GB, NM = S::NM, GU = S::GU, CP = S::CP, CH = S::CH, CG = S::CG, MB = S::MB, WIN = S::WIN;
+    constexpr uint32_t XG = S::XG;
+    constexpr int NT = NB <= 2 ? 1 : NB / 2;          // 8-column tiles: one batch row takes 4 columns (3 digits)
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2;
+    const int t = lane & 3;
+    const uint32_t smem0 = smem_u32(smem);
+    float* red = reinterpret_cast<float*>(smem);                   // sums of squares of the norm prologue, one per 32 pieces
+    float* part = reinterpret_cast<float*>(smem + p.off_part);     // [tiles of a batch][mats][units][16 rows][NB]
+    uint16_t* resid = reinterpret_cast<uint16_t*>(smem + p.off_res);
+
+    const int cta = blockIdx.x;
+    const int r_lo = cta * p.rows_lo + min(cta, p.rem);
+    const int r_cnt = p.rows_lo + (cta < p.rem ? 1 : 0);
+    const int n_tiles = (r_cnt + 15) >> 4;
+    const int tile_rows = (r_cnt + n_tiles - 1) / n_tiles;
+    const int U = p.units, mats = p.mats, B = p.B, Gn = p.Gn;
+
+    if (threadIdx.x < S::XU / 16) *reinterpret_cast<uint4*>(smem + p.off_zero + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
+    pdl_launch_dependents();
+
+    // ---------------- the warp's stream: the chunks of its units, in order ----------------
+    const uint32_t ring = smem0 + p.off_ring + (uint32_t)warp * 4096u;
+    const uint32_t meta0 = smem0 + p.off_meta + (uint32_t)warp * (2u * p.meta_slot);
+    const uint32_t sw = (uint32_t)(((g >> 1) & 1) << 1 | ((g >> 2) & 1)) << 4;      // 16-byte pieces of a row are XORed with this: no bank conflicts
+    const uint32_t dst_lane = ring + (uint32_t)g * 64 + ((uint32_t)(t << 4) ^ sw);
+    I8Pos nu = {0, 0, 0};                              // the unit being copied
+    i8_advance(nu, warp, U, mats);
+    const uint8_t *srcA = nullptr, *srcM = nullptr;    // this lane's first 16 bytes of row g of that unit; its scales / zero points
+    int leftA = 0, leftB = 0;                          // bytes from there to the end of row g, of row g + 8 (0: no such row)
+    int leftM = 0;                                     // bytes of scales to copy (-1: there are no zero points)
+    const int row8 = 8 * p.row_bytes;
+    const int lane_w = g * p.row_bytes + t * 16;
+    const int m_row = g + 8 * (t & 1);                 // lanes t = 0, 1 copy scales of rows g, g + 8, lanes t = 2, 3 zero points
+    auto locate = [&]() {
+        leftA = leftB = leftM = 0;
+        if (nu.tile < n_tiles) {
+            const int row0 = r_lo + nu.tile * tile_rows;
+            const int rows = min(tile_rows, r_lo + r_cnt - row0);
+            const int left = p.row_bytes - nu.i * kI8UnitBytes - t * 16;
+            srcA = p.w[nu.m] + ((int64_t)row0 * p.row_bytes + (nu.i * kI8UnitBytes + lane_w));
+            leftA = g < rows ? left : 0;
+            leftB = g + 8 < rows ? left : 0;
+            const __half* mb = t < 2 ? p.s[nu.m] : p.z[nu.m];
+            if (m_row < rows) {
+                const int64_t first = (int64_t)(row0 + m_row) * Gn;
+                const int64_t at = (first + nu.i * GU) * 2;
+                leftM = MB;
+                if (!p.meta_vec) leftM = (int)min((int64_t)(WIN * 16), (first + Gn) * 2 - (at & ~(int64_t)15));
+                srcM = reinterpret_cast<const uint8_t*>(mb) + (p.meta_vec ? at : at & ~(int64_t)15);
+                if (mb == nullptr) leftM = -1;
+            }
+        }
+    };
+    auto issue = [&](int c, uint32_t meta) {           // chunk c of that unit; its scales ride on the first
+        if (c == 0 && leftM > 0) {
+            if (p.meta_vec) {
+                const uint32_t dst = meta + (uint32_t)(t * 8 + g) * MB;
+                if constexpr (MB == 32) { cp16(dst, srcM); cp16(dst + 16, srcM + 16); }
+                else if constexpr (MB == 16) cp16(dst, srcM);
+                else cp_small<MB>(dst, srcM);
+            } else {
+                // the aligned window that holds the row's values, zeros past the end of the row
+                const uint32_t dst = meta + (uint32_t)(t * 8 + g) * (WIN * 16);
+#pragma unroll
+                for (int q = 0; q < WIN; ++q) cp16_part(dst + q * 16, srcM + (leftM > q * 16 ? q * 16 : 0), (uint32_t)max(0, min(16, leftM - q * 16)));
+            }
+        } else if (c == 0 && leftM < 0) {
+            const uint32_t stride = p.meta_vec ? MB : WIN * 16;
+            for (uint32_t q = 0; q < stride; q += 4) asm volatile("st.shared.u32 [%0], %1;" ::"r"(meta + (uint32_t)(t * 8 + g) * stride + q), "r"(0) : "memory");
+        }
+#pragma unroll
+        for (int q = 0; q < CP; ++q) {
+            const int off = (c * CP + q) * 64;
+            if (leftA > off) cp16(dst_lane + (c * CP + q) * 1024, srcA + off);
+            if (leftB > off) cp16(dst_lane + (c * CP + q) * 1024 + 512, srcA + row8 + off);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    locate();
+#pragma unroll
+    for (int c = 0; c < CH; ++c) issue(c, meta0);
+
+    // ---------------- activations: everything from here on depends on the previous kernel ----------------
+    pdl_wait();
+    I8Source xsrc = {0u, p.tp_in.spin_limit ? p.tp_in.spin_limit : kTpSpinLimit};
+    if (PACKETS) {
+        xsrc.seq16 = tp_seq16(*reinterpret_cast<const volatile uint32_t*>(p.tp_in.epoch));
+    } else if (p.tp_in.world > 0) {
+        if ((int)threadIdx.x < p.tp_in.world && !tp_wait_source(p.tp_in, threadIdx.x)) atomicMax(&g_device_status, (int)EV_PEER_WAIT);
+        __syncthreads();
+    }
+    const bool res_smem = p.residual != nullptr && r_cnt * B <= kI8MaxRes;
+    if (res_smem)
+        for (int i = threadIdx.x; i < r_cnt * B; i += kI8Threads) {
+            const int b = i / r_cnt;
+            resid[i] = reinterpret_cast<const uint16_t*>(p.residual)[(size_t)b * p.N + r_lo + (i - b * r_cnt)];
+        }
+    // Items: 8-value pieces of the padded rows.  A warp's 32 pieces lie in one row (a padded row is a multiple of 32 pieces).
+    // The loop stays small on purpose: hoisting four loads per thread made every launch 0.4 us longer (instruction fetch)
+    // and gained nothing on rows of 14336.
+    const int pieces = U * GU * (G / 8);
+    const int total = B * pieces;
+    auto load_item = [&](int it, uint32_t (&w)[4]) -> bool {
+        const int b = it / pieces, k = (it - b * pieces) * 8;
+        w[0] = w[1] = w[2] = w[3] = 0u;
+        if (k < p.K) i8_load_z<PACKETS>(p, (int64_t)b * p.K + k, xsrc, w);
+        return k < p.K;
+    };
+    if (p.norm_w != nullptr) {
+        // sums of squares per 32 pieces, added per row in order: the same bits whatever the rows and the CTAs
+#pragma unroll 1
+        for (int it = threadIdx.x; it < total; it += kI8Threads) {
+            uint32_t w[4];
+            float v[8], ss = 0.0f;
+            load_item(it, w);
+            i8_words_to_f32(w, p.act_dtype, v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+            ss = i8_warp_sum(ss);
+            if (lane == 0) red[it / 32] = ss;
+        }
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int it = threadIdx.x; it < total; it += kI8Threads) {      // whole warps (shuffles below)
+        const int b = it / pieces, pc = it - b * pieces;
+        const int k = pc * 8;
+        const int64_t idx = (int64_t)b * p.K + k;
+        uint32_t w[4];
+        const bool live = load_item(it, w);
+        float v[8];
+        i8_words_to_f32(w, p.act_dtype, v);
+        if (p.norm_w != nullptr && live) {
+            float tot = 0.0f;
+            for (int q = 0; q < pieces / 32; ++q) tot += red[b * (pieces / 32) + q];
+            const float inv = rsqrtf(tot / (float)p.K + p.eps);
+            if (cta == 0 && p.z_out != nullptr) i8_stg(p.z_out, idx, w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] *= inv * load_as_f32(p.norm_w, p.norm_w_dtype, k + i);
+            i8_pack(w, p.act_dtype, v);
+            i8_words_to_f32(w, p.act_dtype, v);
+            if (cta == 0 && p.normed_out != nullptr) i8_stg(p.normed_out, idx, w);
+        }
+        float mx = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
+        float X = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+#pragma unroll
+        for (int o = 1; o < G / 8; o <<= 1) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            X += __shfl_xor_sync(0xffffffffu, X, o);
+        }
+        // 2^e brings the group's largest magnitude to [2^21, 2^22)
+        const int e = min(120, 148 - (int)(__float_as_uint(mx) >> 23));
+        const float up = __uint_as_float((uint32_t)(e + 127) << 23);
+        uint32_t u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[i] = (uint32_t)(__float2int_rn(v[i] * up) + 0x808080);      // three digits, each + 128
+        const int in = pc & (G / 8 - 1), grp = pc / (G / 8);
+        int tt, ii;                                    // lane and mma that meet these 8 values
+        if (GB == 128) { tt = (in & 7) >> 1; ii = ((in >> 3) << 1) | (in & 1); }      // two 16-byte pieces per lane
+        else { tt = in / NM; ii = in & (NM - 1); }
+        uint8_t* dst = smem + p.off_xd + (size_t)b * p.xstride + (uint32_t)grp * XG + ii * 96 + tt * 8;
+        uint32_t d[3][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            // q4: even codes of the word, then odd ones; q8: its first four bytes, then the next
+            const uint32_t a = u[BITS == 4 ? h : 4 * h], b2 = u[BITS == 4 ? 2 + h : 4 * h + 1];
+            const uint32_t c = u[BITS == 4 ? 4 + h : 4 * h + 2], d2 = u[BITS == 4 ? 6 + h : 4 * h + 3];
+            const uint32_t lo0 = prmt(a, b2, 0x5140), lo1 = prmt(c, d2, 0x5140);
+            d[2][h] = prmt(lo0, lo1, 0x5410) ^ 0x80808080u;
+            d[1][h] = prmt(lo0, lo1, 0x7632) ^ 0x80808080u;
+            d[0][h] = prmt(prmt(a, b2, 0x0062), prmt(c, d2, 0x0062), 0x5410) ^ 0x80808080u;
+        }
+#pragma unroll
+        for (int s = 0; s < 3; ++s) *reinterpret_cast<uint2*>(dst + s * 32) = make_uint2(d[s][0], d[s][1]);
+        if (in == 0) {
+            const float down = mx < INFINITY ? __uint_as_float((uint32_t)(127 + 8 - e) << 23) : NAN;     // 2^(8 - e)
+            // even lanes own the two high digits (c2 2^8 + c1), odd lanes the low one and the zero-point term
+            reinterpret_cast<float4*>(smem + p.off_cst)[b * U * GU + grp] = make_float4(down, 0.0f, down * 1.52587890625e-05f, X);
+        }
+    }
+    __syncthreads();
+
+    // ---------------- per-lane constants of the consumer ----------------
+    const int col_b = g >> 2;                          // batch row of this lane's B column inside a tile; one batch row: parity of the group
+    const bool digit = (g & 3) < 3;
+    const uint32_t zaddr = smem0 + p.off_zero + t * 8;
+    const uint32_t xlane = smem0 + p.off_xd + (uint32_t)(g & 3) * 32 + t * 8;
+    const uint32_t cbase = smem0 + p.off_cst + (uint32_t)(t & 1) * 8 + (NB == 1 ? (t >> 1) * 16 : 0);
+    constexpr int LPP = GB >= 64 ? 16 : GB / 4;        // lane pitch in a row
+    const uint32_t a_lane = (((uint32_t)(t * LPP) & ~15u) ^ sw) + ((uint32_t)(t * LPP) & 15u);
+    uint32_t a_grp[CG];                                // this lane's bytes of the chunk's groups (first chunk)
+#pragma unroll
+    for (int q = 0; q < CG; ++q) a_grp[q] = ring + (uint32_t)g * 64 + (a_lane ^ (uint32_t)(q * GB));
+    const uint32_t m_stride = p.meta_vec ? MB : WIN * 16;
+    const uint32_t m_lane = (uint32_t)g * m_stride + (NB == 1 ? (t >> 1) * 2 : 0);
+
+    I8Pos cu = nu;
+    uint32_t cmeta = 0;                                // scale buffer of the unit being consumed
+#pragma unroll 1
+    for (int t0 = 0; t0 < n_tiles; t0 += p.batch) {
+        const int t1 = min(n_tiles, t0 + p.batch);
+#pragma unroll 1
+        while (cu.tile < t1) {
+            uint32_t m_s0 = meta0 + cmeta + m_lane, m_s1 = m_s0 + 8 * m_stride;
+            if (!p.meta_vec) {
+                const uint32_t e = (uint32_t)(r_lo + cu.tile * tile_rows + g) * (uint32_t)Gn + cu.i * GU;      // low bits are enough
+                m_s0 += (e * 2) & 15u;
+                m_s1 += ((e + 8u * Gn) * 2) & 15u;
+            }
+            const uint32_t m_z0 = m_s0 + 16 * m_stride, m_z1 = m_s1 + 16 * m_stride;
+            float y[NT][2];
+            // B operand addresses: a lane without a digit (or with the other group's column) reads zeros
+            uint32_t xb[NT], xo[NT], cc[NT];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                y[nt][0] = y[nt][1] = 0.0f;
+                const int b = NB == 1 ? 0 : 2 * nt + col_b;
+                const uint32_t a = xlane + (uint32_t)b * p.xstride + (uint32_t)cu.i * S::XU;
+                xb[nt] = digit && (NB == 1 ? col_b == 0 : b < B) ? a : zaddr;
+                xo[nt] = digit && col_b == 1 ? a : zaddr;
+                const int cb = NB == 1 ? 0 : min(2 * nt + (t >> 1), B - 1);
+                cc[nt] = cbase + (uint32_t)(cb * U + cu.i) * (GU * 16);
+            }
+
+            i8_advance(nu, kI8Warps, U, mats);
+            locate();
+            int acc[NT][4];
+            // affine step of group `gl` of the unit (one batch row: of groups gl and gl + 1 at once)
+            auto flush = [&](int gl) {
+                const float s0 = s_ldh(m_s0 + gl * 2), s1 = s_ldh(m_s1 + gl * 2), z0 = s_ldh(m_z0 + gl * 2), z1 = s_ldh(m_z1 + gl * 2);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    uint32_t wq, xq;
+                    s_ld64(cc[nt] + gl * 16, wq, xq);
+                    const float wf = __uint_as_float(wq), xf = __uint_as_float(xq);
+                    const float f0 = (float)((acc[nt][0] << 8) + acc[nt][1]) * wf, f1 = (float)((acc[nt][2] << 8) + acc[nt][3]) * wf;
+                    y[nt][0] = fmaf(s0, fmaf(-z0, xf, f0), y[nt][0]);
+                    y[nt][1] = fmaf(s1, fmaf(-z1, xf, f1), y[nt][1]);
+                }
+            };
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(CH - 1) : "memory");
+                __syncwarp();
+                // groups past the end of the row have zero digits: whatever their codes are, they add nothing
+#pragma unroll
+                for (int q = 0; q < CG; ++q) {
+                    const int gl = c * CG + q;
+                    if constexpr (NB == 1) {
+                        if (gl % 2 == 0) i8_group_mma<BITS, LOGG, NT, true>(acc, a_grp[q] + c * CP * 1024, xb, gl * XG);
+                        else i8_group_mma<BITS, LOGG, NT, false>(acc, a_grp[q] + c * CP * 1024, xo, gl * XG);
+                        if (gl % 2 == 1) flush(gl - 1);
+                    } else {
+                        i8_group_mma<BITS, LOGG, NT, true>(acc, a_grp[q] + c * CP * 1024, xb, gl * XG);
+                        flush(gl);
+                    }
+                }
+                __syncwarp();
+                issue(c, meta0 + (cmeta ^ p.meta_slot));
+            }
+            // ---- the unit's sums into their place ----
+            float* dst = part + ((size_t)((cu.tile - t0) * mats + cu.m) * U + cu.i) * (16 * NB);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float v = y[nt][h];
+                    v += __shfl_xor_sync(0xffffffffu, v, 1);
+                    if (NB == 1) v += __shfl_xor_sync(0xffffffffu, v, 2);
+                    if ((NB == 1 ? t == 0 : (t & 1) == 0)) dst[(g + 8 * h) * NB + (NB == 1 ? 0 : 2 * nt + (t >> 1))] = v;
+                }
+            cu = nu;
+            cmeta ^= p.meta_slot;
+        }
+        __syncthreads();
+        // ---- rows of these tiles: units added in k order, clamp, round, residual add or SwiGLU, store ----
+        const float fmax_act = p.act_dtype == B200Q_F16 ? 65504.0f : 3.3895313892515355e38f;
+        const int rb0 = t0 * tile_rows, n_rows = min(r_cnt, t1 * tile_rows) - rb0;
+        for (int it = threadIdx.x; it < n_rows * B; it += kI8Threads) {
+            const int b = it / n_rows, rr = it - b * n_rows;
+            const int tl = rr / tile_rows, r = rr - tl * tile_rows;
+            const float* src = part + (size_t)tl * mats * U * (16 * NB) + r * NB + b;
+            float val[2] = {0.0f, 0.0f};
+            for (int m = 0; m < mats; ++m) {
+                float sum = 0.0f;
+#pragma unroll 4
+                for (int i = 0; i < U; ++i) sum += src[(m * U + i) * (16 * NB)];
+                val[m] = i8_round_act(fminf(fmaxf(sum, -fmax_act), fmax_act), p.act_dtype);
+            }
+            const int row = r_lo + rb0 + rr;
+            const int64_t o = (int64_t)b * p.N + row;
+            auto bits_of = [&](float v) {
+                return p.act_dtype == B200Q_F16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
+            };
+            float v = val[0];
+            if (mats == 2) {
+                if (p.gate_out != nullptr) reinterpret_cast<unsigned short*>(p.gate_out)[o] = bits_of(val[0]);
+                if (p.up_out != nullptr) reinterpret_cast<unsigned short*>(p.up_out)[o] = bits_of(val[1]);
+                v = (val[0] / (1.0f + expf(-val[0]))) * val[1];
+                if (p.act_out != nullptr) reinterpret_cast<unsigned short*>(p.act_out)[o] = bits_of(v);
+            } else {
+                if (p.residual != nullptr) {
+                    const uint16_t rb = res_smem ? resid[b * r_cnt + rb0 + rr] : reinterpret_cast<const uint16_t*>(p.residual)[o];
+                    v = load_as_f32(&rb, p.act_dtype, 0) + v;
+                }
+                if (p.y != nullptr) reinterpret_cast<unsigned short*>(p.y)[o] = bits_of(v);
+            }
+            if (p.tp_out.world > 0) {
+                // tensor-parallel exchange: the value goes to column block `rank` of every rank's full rows
+                const int64_t of = (int64_t)b * p.N * p.tp_out.world + (int64_t)p.tp_out.rank * p.N + row;
+                const unsigned short bits16 = bits_of(v);
+                const uint32_t pk = p.tp_out.packets ? tp_packet(bits16, tp_seq16(tp_writer_seq(p.tp_out))) : 0u;
+#pragma unroll 1
+                for (int peer = 0; peer < p.tp_out.world; ++peer) {
+                    if (p.tp_out.packets) st_volatile_u32(reinterpret_cast<uint32_t*>(p.tp_out.full[peer]) + of, pk);
+                    else reinterpret_cast<unsigned short*>(p.tp_out.full[peer])[of] = bits16;
+                }
+            }
+        }
+        if (t1 < n_tiles || p.tp_out.world > 0) __syncthreads();      // the sums have been read / all peer stores are issued
+    }
+    if (p.tp_out.world > 0 && warp == 0) {
+        if (p.tp_out.packets) tp_finish_writer_packets(p.tp_out, lane);
+        else tp_finish_writer(p.tp_out, lane);
+    }
+}
+
+inline bool i8_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline uint32_t i8_align(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
+
+template <int BITS, int LOGG, int NB>
+int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
+    using S = I8Shape<BITS, LOGG>;
+    I8Params p = {};
+    p.x = q.x; p.res_in = q.res_in; p.norm_w = q.norm_w; p.z_out = q.z_out; p.normed_out = q.normed_out;
+    p.mats = gate_up ? 2 : 1;
+    for (int m = 0; m < p.mats; ++m) {
+        p.w[m] = q.w[m];
+        p.s[m] = (const __half*)q.s[m];
+        p.z[m] = (const __half*)q.z[m];
+    }
+    p.residual = q.residual; p.y = q.y; p.gate_out = q.gate_out; p.up_out = q.up_out; p.act_out = q.act_out;
+    p.eps = q.eps; p.B = q.B; p.N = q.N; p.K = q.K; p.Gn = q.Gn; p.act_dtype = q.act_dtype; p.norm_w_dtype = q.norm_w_dtype;
+    p.row_bytes = q.row_bytes; p.tp_out = q.tp_out; p.tp_in = q.tp_in;
+    p.units = (p.row_bytes + kI8UnitBytes - 1) / kI8UnitBytes;
+    p.meta_vec = p.Gn % S::GU == 0;
+    p.meta_slot = 32u * (p.meta_vec ? S::MB : S::WIN * 16);
+    // a CTA per SM, fewer only when a CTA would own less than four rows
+    const int grid = std::max(1, std::min(sm_count(), (p.N + 3) / 4));
+    p.rows_lo = p.N / grid;
+    p.rem = p.N % grid;
+    const int r_max = p.rows_lo + (p.rem ? 1 : 0);
+    const int tile_bytes = p.mats * p.units * 16 * NB * 4;
+    p.batch = std::min((r_max + 15) / 16, std::max(1, 24 * 1024 / tile_bytes));
+    p.xstride = (uint32_t)p.units * S::GU * S::XG + 32;      // + 32: the two batch rows of a B operand fall into different banks
+    uint32_t off = i8_align((uint32_t)q.B * p.units * S::GU * (S::G / 8) / 32 * 4, 128);
+    p.off_zero = off;  off += S::XU;
+    p.off_xd = off;    off += i8_align((uint32_t)q.B * p.xstride, 128);
+    p.off_cst = off;   off += (uint32_t)q.B * p.units * S::GU * 16;
+    p.off_res = off;   off += p.residual != nullptr ? i8_align((uint32_t)std::min(r_max * q.B, kI8MaxRes) * 2, 128) : 0;
+    off = i8_align(off, 128);
+    p.off_part = off;  off += i8_align((uint32_t)(p.batch * tile_bytes), 128);
+    p.off_meta = off;  off += kI8Warps * 2 * p.meta_slot;
+    off = i8_align(off, 1024);
+    p.off_ring = off;  off += kI8Warps * 4096;
+    if (off > (uint32_t)max_smem_optin()) return B200Q_ERR_UNSUPPORTED;
+
+    const bool packets = p.tp_in.world > 0 && p.tp_in.packets;
+    auto kernel = qgemv_i8_kernel<BITS, LOGG, NB, false>;
+    if (packets) kernel = qgemv_i8_kernel<BITS, LOGG, NB, true>;
+    static bool configured[2][64] = {};   // per instantiation and device; a race only repeats the call
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!configured[packets][dev & 63]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()) != cudaSuccess)
+            return B200Q_ERR_LAUNCH;
+        configured[packets][dev & 63] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kI8Threads);
+    cfg.dynamicSmemBytes = off;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return B200Q_ERR_LAUNCH;
+    return finish_launch();
+}
+
+template <int BITS, int LOGG>
+int dispatch_i8_cols(const GemvParams& p, bool gate_up, cudaStream_t stream) {
+    if (p.B <= 1) return launch_i8<BITS, LOGG, 1>(p, gate_up, stream);
+    if (p.B <= 2) return launch_i8<BITS, LOGG, 2>(p, gate_up, stream);
+    return launch_i8<BITS, LOGG, 4>(p, gate_up, stream);
+}
+
+template <int BITS>
+int dispatch_i8(const GemvParams& p, bool gate_up, cudaStream_t stream) {
+    if (p.B > 4 || p.scale_dtype != B200Q_F16) return B200Q_ERR_UNSUPPORTED;
+    for (int m = 0; m < (gate_up ? 2 : 1); ++m)
+        if (!i8_aligned16(p.s[m]) || !i8_aligned16(p.z[m])) return B200Q_ERR_UNSUPPORTED;
+    if (p.G == 32) return dispatch_i8_cols<BITS, 5>(p, gate_up, stream);
+    if (p.G == 64) return dispatch_i8_cols<BITS, 6>(p, gate_up, stream);
+    return dispatch_i8_cols<BITS, 7>(p, gate_up, stream);
+}
+
+}  // namespace
+}  // namespace b200q

@@ -75,6 +75,13 @@ int gemv_fast_q8(GemvParams& p, bool gate_up, cudaStream_t stream);
 int gemv_q4_read_status(int reset, cudaStream_t stream);
 int gemv_q8_read_status(int reset, cudaStream_t stream);
 
+// Integer tensor-core kernel for up to 4 batch rows (gemv_i8.cuh), one translation unit per code width; B200Q_ERR_UNSUPPORTED
+// outside its plan (scales that are not fp16, activations that do not fit into shared memory).
+int gemv_i8_q4(const GemvParams& p, bool gate_up, cudaStream_t stream);
+int gemv_i8_q8(const GemvParams& p, bool gate_up, cudaStream_t stream);
+int gemv_i8_q4_read_status(int reset, cudaStream_t stream);
+int gemv_i8_q8_read_status(int reset, cudaStream_t stream);
+
 // tcgen05 kernel (qgemm_ts.cu): weights through tensor memory, any batch up to 64 rows per launch.  Returns
 // B200Q_ERR_UNSUPPORTED when the problem is outside its plan.
 int qgemm_ts(int bits, const GemvParams& p, bool gate_up, cudaStream_t stream);

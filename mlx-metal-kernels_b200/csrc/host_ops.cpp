@@ -12,11 +12,13 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -38,9 +40,13 @@ int (*p_attn)(int, const void*, const uint8_t*, const uint8_t*, const void*, con
 int (*p_attn_window)(int, const void*, const uint8_t*, const uint8_t*, const void*, const void*, const int32_t*, const int32_t*,
                      void*, void*, size_t, int, int, int, int, int, int64_t, int, int, float, int, int, int, int, void*) = nullptr;
 
+size_t (*p_plain_ws)(int, int, int, int) = nullptr;
+int (*p_plain_attn)(const void*, const void*, const void*, const int32_t*, const int32_t*, void*, void*, size_t, int, int, int, int, int,
+                    int64_t, int, float, int, void*) = nullptr;
 int (*p_quant_pair)(int, const void*, const void*, uint8_t*, uint8_t*, void*, void*, int64_t, int, int, int, void*) = nullptr;
 int (*p_dequant_pair)(int, const uint8_t*, const uint8_t*, const void*, const void*, void*, void*, int64_t, int, int, void*) = nullptr;
 
+constexpr int kMaxDevices = 64;
 constexpr int kMinNormRows = 5;      // from this many rows on the library runs the rmsnorm as a launch of its own
 
 PyObject* none() { Py_RETURN_NONE; }
@@ -229,6 +235,56 @@ PyObject* paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     return rc == 0 ? THPVariable_Wrap(std::move(out)) : none();
 }
 
+// plain_attention(q, K, V, block_table, lengths, scale or None) -> out or None: fp16 / bf16 pages.  The lengths are
+// range-checked on the host, as the operator promises; they are copied out ahead of the kernels on the same stream, the
+// kernels are enqueued (they clamp what they read), and only then the host waits for that copy - the GPU goes on meanwhile.
+PyObject* plain_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    if (p_plain_attn == nullptr || n_args != 6 || safe_mode()) return none();
+    const Tensor *q = as_tensor(a[0]), *k = as_tensor(a[1]), *v = as_tensor(a[2]), *bt = as_tensor(a[3]), *len = as_tensor(a[4]);
+    const int dev = current_device_of(q);
+    if (dev < 0 || dev >= kMaxDevices || !k || !v || !bt || !len || q->dim() != 4 || q->size(1) != 1 || !q->is_contiguous() ||
+        !act_dtype(q->scalar_type()))
+        return none();
+    const int64_t B = q->size(0), Hq = q->size(2), D = q->size(3);
+    if (!on(*k, dev) || !on(*v, dev) || !on(*bt, dev) || !on(*len, dev) || k->dim() != 4 || k->sizes() != v->sizes() ||
+        k->scalar_type() != q->scalar_type() || v->scalar_type() != q->scalar_type() || k->size(3) != D || bt->dim() != 2 ||
+        bt->size(0) != B || bt->scalar_type() != at::kInt || len->scalar_type() != at::kInt || len->dim() != 1 || len->size(0) != B)
+        return none();
+    const int64_t pages = k->size(0), P = k->size(1), Hkv = k->size(2), mb = bt->size(1);
+    if (B <= 0 || Hq <= 0 || D <= 0 || D > 128 || pages <= 0 || P <= 0 || Hkv <= 0 || mb <= 0 || Hq % Hkv != 0 || B > INT32_MAX ||
+        Hq > INT32_MAX || P * mb > INT32_MAX)
+        return none();
+    double scale = 1.0 / std::sqrt((double)D);
+    if (a[5] != Py_None) {
+        if (!PyFloat_Check(a[5])) return none();
+        scale = PyFloat_AS_DOUBLE(a[5]);
+    }
+    cudaStream_t st = (cudaStream_t)stream_of(dev);
+    cudaStreamCaptureStatus capture;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return none();
+    static thread_local cudaEvent_t copied[kMaxDevices] = {};      // one per thread and device that ever calls this
+    if (copied[dev] == nullptr && cudaEventCreateWithFlags(&copied[dev], cudaEventDisableTiming) != cudaSuccess) return none();
+    Tensor host = at::detail::empty_cpu({B}, at::kInt, std::nullopt, std::nullopt, /*pin_memory=*/true, std::nullopt);
+    if (cudaMemcpyAsync(host.mutable_data_ptr(), len->const_data_ptr(), (size_t)B * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaEventRecord(copied[dev], st) != cudaSuccess)
+        return none();
+    Tensor out = empty(q->sizes(), q->scalar_type(), dev);
+    const size_t ws_bytes = p_plain_ws((int)B, (int)Hq, (int)Hkv, (int)mb);
+    Tensor ws = empty({(int64_t)std::max<size_t>(ws_bytes, 16)}, at::kByte, dev);
+    const int rc = p_plain_attn(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), static_cast<const int32_t*>(bt->const_data_ptr()),
+                                static_cast<const int32_t*>(len->const_data_ptr()), out.mutable_data_ptr(), ws.mutable_data_ptr(), ws_bytes,
+                                (int)B, (int)Hq, (int)Hkv, (int)D, (int)P, pages, (int)mb, (float)scale, dtype_code(q->scalar_type()), st);
+    cudaError_t err;
+    Py_BEGIN_ALLOW_THREADS
+    err = cudaEventSynchronize(copied[dev]);
+    Py_END_ALLOW_THREADS
+    if (rc != 0 || err != cudaSuccess) return none();
+    const int32_t* n = static_cast<const int32_t*>(host.const_data_ptr());
+    for (int64_t b = 0; b < B; ++b)
+        if (n[b] < 0 || n[b] > mb * P) return none();              // the Python body raises
+    return THPVariable_Wrap(std::move(out));
+}
+
 PyObject* tuple_of(std::initializer_list<Tensor*> ts) {
     PyObject* out = PyTuple_New((Py_ssize_t)ts.size());
     Py_ssize_t i = 0;
@@ -291,6 +347,7 @@ PyObject* bind(PyObject*, PyObject* table) {
         {"b200q_qmatvec", (void**)&p_qmatvec}, {"b200q_gate_up_swiglu", (void**)&p_gate_up},
         {"b200q_paged_gqa_workspace_bytes", (void**)&p_attn_ws}, {"b200q_attention_stage_launches", (void**)&p_attn_launches},
         {"b200q_paged_gqa_decode", (void**)&p_attn}, {"b200q_paged_gqa_decode_window", (void**)&p_attn_window},
+        {"b200q_paged_fp16_gqa_workspace_bytes", (void**)&p_plain_ws}, {"b200q_paged_fp16_gqa_decode", (void**)&p_plain_attn},
         {"b200q_quantize_kv_pair", (void**)&p_quant_pair}, {"b200q_dequantize_kv_pair", (void**)&p_dequant_pair},
     };
     for (const auto& w : want) {
@@ -320,6 +377,7 @@ PyMethodDef methods[] = {
     {"mlp_block", FAST(mlp_block), METH_FASTCALL, nullptr},
     {"quantize_kv", FAST(quantize_kv), METH_FASTCALL, nullptr},
     {"dequantize_kv", FAST(dequantize_kv), METH_FASTCALL, nullptr},
+    {"plain_attention", FAST(plain_attention), METH_FASTCALL, nullptr},
     {"paged_attention", FAST(paged_attention), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

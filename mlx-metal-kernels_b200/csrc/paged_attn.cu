@@ -3,31 +3,21 @@
 //   out[b, hq] = softmax_j( scale * q[b, hq] . Khat[j, hkv] ) . Vhat[j, hkv],  hkv = hq / (Hq/Hkv)
 //   Khat = fp16((code - 8|128) * |k_scale|)   over the valid tokens j of sequence b.
 //
-// Fast kernel (head_dim 128, page size 16, q in fp16, fp16 scales, group size 32 or 64, at most 8
-// query heads per kv head, at most 8 kv heads):
+// Fast kernels (head_dim 128, page size 16, q in fp16 or bf16, at most 8 query heads per kv head; quantised pages with fp16 scales in
+// groups of 32 or 64, or plain pages in the dtype of q):
 //   * the (sequence, page) pairs of the whole batch form one flattened list that is cut into
 //     equal contiguous ranges, one per CTA ("stream-K" over ragged lengths: every CTA streams the
 //     same number of pages whatever the length distribution).  A CTA writes one partial
 //     (max, sum, accumulator) per sequence it touches; a second small kernel merges them.
 //   * warp w of a CTA owns kv head w % Hkv (and, when there are fewer than 8 kv heads, every
-//     (8/Hkv)-th page of the range).  It is self-contained: it looks up its page ids 32 at a time,
-//     and every lane copies exactly the bytes IT will consume (16 bytes of two K token rows,
-//     8 bytes of four V token rows) with cp.async into a private ring in shared memory, several
-//     pages ahead.  No CTA-wide barrier, no bank conflicts (the ring is laid out [piece][lane]).
-//     Measured on B200: the bulk-copy (TMA) engine needs >= 2 KB per copy to reach HBM speed,
-//     and a token row of one page is 512 B, so per-lane asynchronous copies are the faster route.
-//   * scores S[token, head] = K Q^T on mma.sync.m16n8k16 with the 16 tokens of a page as rows (in-register
-//     dequantised K is the A operand) and the up to 8 query heads of the group as columns: no padding rows and
-//     no zero operand registers.  Online softmax in fp32 (a lane holds two heads of tokens g and g + 8; the row
-//     maximum is a butterfly over the 8 token lanes, the sums stay per lane until a partial is written).  One
-//     movmatrix per 8 tokens turns the probabilities into the B operand of O^T[d, head] += V^T P, where V^T is
-//     the A operand built from the four token rows with one byte-permute per word pair.  KV bytes are read once
-//     per kv head, not once per query head; Khat / Vhat are bit-identical to the reference's fp16 dequantised
-//     cache.
+//     (8/Hkv)-th page of the range; more than 8 kv heads are cut into chunks of 8, grid.y).  It is self-contained: it looks up
+//     its page ids 32 at a time and copies its pages with cp.async into a private ring in shared memory, several pages
+//     ahead.  No CTA-wide barrier.
+//   * what a warp does with a page is in paged_attn_page.cuh.
 //
-// Everything else (other head dims, bf16 queries, other group sizes) runs the simple kernel: one
+// Everything else (other head dims, other group sizes) runs the simple kernel: one
 // warp per (sequence, query head), the reference's streaming-softmax loop.
-#include "common.cuh"
+#include "paged_attn_page.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -45,11 +35,12 @@ constexpr int kAttnThreads = kAttnWarps * 32;
 #define B200Q_ATTN_CTAS 2                    // resident CTAs per SM of the fast kernel's dense shape
 #endif
 constexpr int kMaxGrid = 152 * B200Q_ATTN_CTAS;   // upper bound on CTAs of the fast kernel (sizes the workspace)
+constexpr int kMaxRanges = 4 * kMaxGrid;  // upper bound on page ranges: a CTA holds several when there are fewer than 8 kv heads
 constexpr int kMaxBatchFast = 2048;       // prefix sums of page counts live in shared memory
-constexpr float kLog2e = 1.4426950408889634f;
+using namespace attn;
 
 struct AttnParams {
-    const __half* q;            // [B, Hq, D]
+    const void* q;              // [B, Hq, D]
     const uint8_t* k_codes;
     const uint8_t* v_codes;
     const __half* k_scales;
@@ -64,7 +55,8 @@ struct AttnParams {
     int q_dtype;
     int bits;
     int stages;                 // pages in flight per warp
-    int subs;                   // ranges per CTA (8 / Hkv)
+    int subs;                   // ranges per CTA (8 / hc)
+    int hc;                     // kv heads per CTA: Hkv, at most 8
     int row_bytes;              // bytes of one token row of codes, all kv heads
     int scale_row_halves;       // halves of one token row of scales, all kv heads
     uint32_t off_prefix, off_ring, slot_bytes;
@@ -99,20 +91,6 @@ __device__ __forceinline__ uint32_t page_mask16(int pg, int L, int sink, int win
         m &= recent | sinks;
     }
     return m;
-}
-
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // Prefix sums of per-sequence page counts into shared memory; returns the total.
@@ -150,270 +128,15 @@ __device__ __forceinline__ int find_sequence(const int* prefix, int B, int f) {
     return lo;
 }
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// ------------------------------------------------------------------------------------------------
-// Per-warp building blocks shared by the split-KV kernel and the cluster kernel: a warp owns one kv head and
-// walks pages of it; every lane copies exactly the bytes IT will consume into a private ring slot.
-// ------------------------------------------------------------------------------------------------
-struct WarpAcc {
-    uint32_t qb[8][2];          // Q^T as B operand: [mma][b0b1, b2b3], column g = query head g of the group
-    float o[8][4];              // O^T tiles: rows d, cols heads
-    float m_run[2];             // running max of query heads 2t, 2t+1 of the group
-    float l_run[2];             // this lane's share (tokens g, g + 8 of every page) of their running sums
-};
-__device__ __forceinline__ void acc_reset(WarpAcc& a) {
-    a.m_run[0] = a.m_run[1] = -INFINITY;
-    a.l_run[0] = a.l_run[1] = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) a.o[i][e] = 0.0f;
-}
-// Q fragments of one kv head's group: row r of `qrows` (D halves apart) is query head r of the group (r < group <= 8).
-// qrows may point to global or shared memory.
-template <int BITS>
-__device__ __forceinline__ void load_q_frags(WarpAcc& a, const __half* qrows, int group, int g, int t) {
-    constexpr int D = 128;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        uint4 u = make_uint4(0, 0, 0, 0);
-        int d0;
-        if (BITS == 4) d0 = 32 * t + 8 * c;
-        else d0 = (c < 2 ? 16 * t + 8 * c : 64 + 16 * t + 8 * (c - 2));
-        if (g < group) u = *reinterpret_cast<const uint4*>(qrows + (size_t)g * D + d0);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};   // halves d0..d0+7
-        if (BITS == 4) {
-            // mma 2c: pairs (0,4) (1,5); mma 2c+1: pairs (2,6) (3,7)
-            a.qb[2 * c][0] = prmt(w[0], w[2], 0x5410);     a.qb[2 * c][1] = prmt(w[0], w[2], 0x7632);
-            a.qb[2 * c + 1][0] = prmt(w[1], w[3], 0x5410); a.qb[2 * c + 1][1] = prmt(w[1], w[3], 0x7632);
-        } else {
-            // mma 2c: codes 0..3 -> pairs (0,1) (2,3); mma 2c+1: codes 4..7
-            a.qb[2 * c][0] = w[0];     a.qb[2 * c][1] = w[1];
-            a.qb[2 * c + 1][0] = w[2]; a.qb[2 * c + 1][1] = w[3];
-        }
-    }
-}
-// Per-lane source offsets inside a page for kv head h.
-struct PageLanes {
-    uint32_t k_src0, k_src1, v_src[4], sc_src, sc_dst;
-    const __half* sc_base;      // lanes 0-15 copy K scales, lanes 16-31 V scales
-};
-template <int BITS>
-__device__ __forceinline__ PageLanes page_lanes(int lane, int h, uint32_t row_bytes, int scale_row_halves, int Gd,
-                                                const __half* k_scales, const __half* v_scales) {
-    constexpr int DP = BITS == 4 ? 64 : 128;
-    constexpr int K_BYTES = BITS == 4 ? 1024 : 2048;
-    const int g = lane >> 2, t = lane & 3;
-    PageLanes L;
-    L.k_src0 = (uint32_t)g * row_bytes + h * DP + 16 * t;            // token g
-    L.k_src1 = L.k_src0 + 8 * row_bytes;                             // token g + 8
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        L.v_src[i] = (uint32_t)(2 * t + (i & 1) + 8 * (i >> 1)) * row_bytes + h * DP + (BITS == 4 ? 8 : 16) * g;
-    L.sc_src = (uint32_t)(lane & 15) * scale_row_halves + h * Gd;    // halves
-    L.sc_dst = 2 * K_BYTES + (lane < 16 ? 0 : 128) + (lane & 15) * 8;
-    L.sc_base = lane < 16 ? k_scales : v_scales;
-    return L;
-}
-// Asynchronous copies of one page of kv head h into a ring slot (one commit group, also for a missing page).
-template <int BITS, int LOGG>
-__device__ __forceinline__ void issue_page(uint8_t* slot, const PageLanes& L, int lane, int page, int valid, const uint8_t* k_codes,
-                                           const uint8_t* v_codes, size_t page_code_bytes, size_t page_scale_halves) {
-    constexpr int K_BYTES = BITS == 4 ? 1024 : 2048;
-    const int g = lane >> 2, t = lane & 3;
-    if (page >= 0) {
-        const uint8_t* kbase = k_codes + (size_t)page * page_code_bytes;
-        const uint8_t* vbase = v_codes + (size_t)page * page_code_bytes;
-        if (BITS == 4) {
-            // K: 16 bytes of token g and of token g + 8 ; V: 8 bytes of tokens 2t, 2t+1, 2t+8, 2t+9
-            if (g < valid) cp_async_16(slot + lane * 16, kbase + L.k_src0);
-            if (g + 8 < valid) cp_async_16(slot + 512 + lane * 16, kbase + L.k_src1);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int tok = 2 * t + (i & 1) + 8 * (i >> 1);
-                if (tok < valid) cp_async_8(slot + K_BYTES + i * 256 + lane * 8, vbase + L.v_src[i]);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int tok = g + 8 * (i >> 1);
-                if (tok < valid)
-                    cp_async_16(slot + i * 512 + lane * 16, kbase + (i >> 1 ? L.k_src1 : L.k_src0) + 64 * (i & 1));
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int tok = 2 * t + (i & 1) + 8 * (i >> 1);
-                if (tok < valid) cp_async_16(slot + K_BYTES + i * 512 + lane * 16, vbase + L.v_src[i]);
-            }
-        }
-        // scales of the 16 tokens for this head: lanes 0-15 K, lanes 16-31 V
-        if ((lane & 15) < valid) {
-            const __half* src = L.sc_base + (size_t)page * page_scale_halves + L.sc_src;
-            if (LOGG == 5) cp_async_8(slot + L.sc_dst, src);
-            else cp_async_4(slot + L.sc_dst, src);
-        }
-    }
-    cp_async_commit();
-}
-
-// One page of kv head h against the group's query heads: S = K Q^T on the tensor cores with the page's 16 tokens as
-// rows, online softmax in fp32, O^T += V^T P.  `valid` = tokens of the page below the length (what was copied),
-// `attended` = bit mask of the slots that take part.
-template <int BITS, int LOGG>
-__device__ __forceinline__ void process_page(WarpAcc& a, const uint8_t* slot, int valid, uint32_t attended, float sm_scale,
-                                             int lane) {
-    constexpr int K_BYTES = BITS == 4 ? 1024 : 2048;
-    constexpr int V_BYTES = K_BYTES;
-    const int g = lane >> 2;
-    const int t = lane & 3;
-                const __half* ksc = reinterpret_cast<const __half*>(slot + K_BYTES + V_BYTES);         // [16][4]
-        const __half* vsc = ksc + 64;                                                             // [16][4]
-
-        // ---------------- S = K Q^T : rows = tokens g and g + 8, columns = query heads 2t, 2t+1 ----------
-        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (BITS == 4) {
-            const uint4 ua = *reinterpret_cast<const uint4*>(slot + lane * 16);          // token g
-            const uint4 ub = *reinterpret_cast<const uint4*>(slot + 512 + lane * 16);    // token g + 8
-            const uint32_t wa[4] = {ua.x, ua.y, ua.z, ua.w}, wb[4] = {ub.x, ub.y, ub.z, ub.w};
-            const uint32_t sa = half_dup(__habs(ksc[g * 4 + ((32 * t) >> LOGG)]));
-            const uint32_t sb = half_dup(__habs(ksc[(g + 8) * 4 + ((32 * t) >> LOGG)]));
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const uint32_t wa2 = wa[c] >> 8, wb2 = wb[c] >> 8;
-                // exact (code - 8), then one rounding in the multiply: fp16((code-8)*s)
-                const uint32_t a0 = hmul2_u32(hsub2_u32(lop3_and_or(wa[c], 0x000F000Fu, 0x64006400u), 0x64086408u), sa);
-                const uint32_t a1 = hmul2_u32(hsub2_u32(lop3_and_or(wb[c], 0x000F000Fu, 0x64006400u), 0x64086408u), sb);
-                const uint32_t a2 = hmul2_u32(hsub2_u32(lop3_and_or(wa[c], 0x00F000F0u, 0x54005400u), 0x54805480u), sa);
-                const uint32_t a3 = hmul2_u32(hsub2_u32(lop3_and_or(wb[c], 0x00F000F0u, 0x54005400u), 0x54805480u), sb);
-                mma_m16n8k16(s, a0, a1, a2, a3, a.qb[2 * c][0], a.qb[2 * c][1]);
-                const uint32_t c0 = hmul2_u32(hsub2_u32(lop3_and_or(wa2, 0x000F000Fu, 0x64006400u), 0x64086408u), sa);
-                const uint32_t c1 = hmul2_u32(hsub2_u32(lop3_and_or(wb2, 0x000F000Fu, 0x64006400u), 0x64086408u), sb);
-                const uint32_t c2 = hmul2_u32(hsub2_u32(lop3_and_or(wa2, 0x00F000F0u, 0x54005400u), 0x54805480u), sa);
-                const uint32_t c3 = hmul2_u32(hsub2_u32(lop3_and_or(wb2, 0x00F000F0u, 0x54005400u), 0x54805480u), sb);
-                mma_m16n8k16(s, c0, c1, c2, c3, a.qb[2 * c + 1][0], a.qb[2 * c + 1][1]);
-            }
-        } else {
-#pragma unroll
-            for (int hb = 0; hb < 2; ++hb) {
-                const uint4 ua = *reinterpret_cast<const uint4*>(slot + hb * 512 + lane * 16);          // token g
-                const uint4 ub = *reinterpret_cast<const uint4*>(slot + (2 + hb) * 512 + lane * 16);    // token g + 8
-                const uint32_t wa[4] = {ua.x, ua.y, ua.z, ua.w}, wb[4] = {ub.x, ub.y, ub.z, ub.w};
-                const uint32_t sa = half_dup(__habs(ksc[g * 4 + ((64 * hb + 16 * t) >> LOGG)]));
-                const uint32_t sb = half_dup(__habs(ksc[(g + 8) * 4 + ((64 * hb + 16 * t) >> LOGG)]));
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint32_t a0 = hmul2_u32(hsub2_u32(prmt(wa[c], 0x64646464u, 0x4140u), 0x64806480u), sa);
-                    const uint32_t a1 = hmul2_u32(hsub2_u32(prmt(wb[c], 0x64646464u, 0x4140u), 0x64806480u), sb);
-                    const uint32_t a2 = hmul2_u32(hsub2_u32(prmt(wa[c], 0x64646464u, 0x4342u), 0x64806480u), sa);
-                    const uint32_t a3 = hmul2_u32(hsub2_u32(prmt(wb[c], 0x64646464u, 0x4342u), 0x64806480u), sb);
-                    const int mi = 4 * hb + c;
-                    mma_m16n8k16(s, a0, a1, a2, a3, a.qb[mi][0], a.qb[mi][1]);
-                }
-            }
-        }
-        // ---------------- online softmax: this lane holds heads 2t, 2t+1 of tokens g and g + 8 ----------
-        float alpha[2];
-        uint32_t pb0, pb1;      // P[token][head] as the B operand of O^T += V^T P
-        {
-            // also discards whatever stale bytes sit in unused slots
-            const bool in0 = (attended >> g) & 1u, in1 = (attended >> (g + 8)) & 1u;
-            s[0] = in0 ? s[0] * sm_scale : -INFINITY;
-            s[1] = in0 ? s[1] * sm_scale : -INFINITY;
-            s[2] = in1 ? s[2] * sm_scale : -INFINITY;
-            s[3] = in1 ? s[3] * sm_scale : -INFINITY;
-            float mx0 = fmaxf(s[0], s[2]), mx1 = fmaxf(s[1], s[3]);
-#pragma unroll
-            for (int o2 = 4; o2 < 32; o2 <<= 1) {
-                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o2));
-                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o2));
-            }
-            const float mn0 = fmaxf(a.m_run[0], mx0), mn1 = fmaxf(a.m_run[1], mx1);   // finite: every staged page has a valid token
-            alpha[0] = fast_exp2((a.m_run[0] - mn0) * kLog2e);                       // exp(-inf) = 0 on the first page
-            alpha[1] = fast_exp2((a.m_run[1] - mn1) * kLog2e);
-            const float p0 = fast_exp2((s[0] - mn0) * kLog2e), p1 = fast_exp2((s[1] - mn1) * kLog2e);
-            const float p2 = fast_exp2((s[2] - mn0) * kLog2e), p3 = fast_exp2((s[3] - mn1) * kLog2e);
-            // per-lane share of the sums (tokens g, g + 8); the 8 shares of a head are added when a partial is written
-            a.l_run[0] = a.l_run[0] * alpha[0] + (p0 + p2);
-            a.l_run[1] = a.l_run[1] * alpha[1] + (p1 + p3);
-            a.m_run[0] = mn0;
-            a.m_run[1] = mn1;
-            // transpose (token g, heads 2t, 2t+1) into (tokens 2t, 2t+1, head g): b0b1 tokens 0..7, b2b3 tokens 8..15
-            const __half2 x0 = __floats2half2_rn(p0, p1);
-            const __half2 x1 = __floats2half2_rn(p2, p3);
-            pb0 = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&x0));
-            pb1 = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&x1));
-        }
-        // ---------------- rescale O^T columns (heads 2t, 2t+1) ----------------------------------------------
-        if (__any_sync(0xffffffffu, (alpha[0] != 1.0f) || (alpha[1] != 1.0f))) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                a.o[i][0] *= alpha[0]; a.o[i][1] *= alpha[1]; a.o[i][2] *= alpha[0]; a.o[i][3] *= alpha[1];
-            }
-        }
-        // ---------------- O^T += V^T P ---------------------------------------------------------
-        const int vgrp = (16 * g) >> LOGG;
-        uint32_t vreg[2][16];   // [token pair][j]: (Vhat[tokA][16g + j], Vhat[tokB][16g + j])
-#pragma unroll
-        for (int tp = 0; tp < 2; ++tp) {
-            const int tokA = 2 * t + 8 * tp, tokB = tokA + 1;
-            // slots past the end of the sequence may hold anything: their weight is 0, make the value 0 too
-            const __half sA = tokA < valid ? __habs(vsc[tokA * 4 + vgrp]) : __ushort_as_half(0);
-            const __half sB = tokB < valid ? __habs(vsc[tokB * 4 + vgrp]) : __ushort_as_half(0);
-            const uint32_t s2 = (uint32_t)__half_as_ushort(sA) | ((uint32_t)__half_as_ushort(sB) << 16);
-            if (BITS == 4) {
-                const uint2 ua = *reinterpret_cast<const uint2*>(slot + K_BYTES + (2 * tp) * 256 + lane * 8);
-                const uint2 ub = *reinterpret_cast<const uint2*>(slot + K_BYTES + (2 * tp + 1) * 256 + lane * 8);
-                const uint32_t wa[2] = {ua.x, ua.y}, wb[2] = {ub.x, ub.y};
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    const uint32_t r0 = prmt(wa[w], wb[w], 0x5410);   // nibbles 0..3 of A | of B
-                    const uint32_t r1 = prmt(wa[w], wb[w], 0x7632);   // nibbles 4..7
-                    const uint32_t r0s = r0 >> 8, r1s = r1 >> 8;
-                    vreg[tp][8 * w + 0] = hmul2_u32(hsub2_u32(lop3_and_or(r0, 0x000F000Fu, 0x64006400u), 0x64086408u), s2);
-                    vreg[tp][8 * w + 1] = hmul2_u32(hsub2_u32(lop3_and_or(r0, 0x00F000F0u, 0x54005400u), 0x54805480u), s2);
-                    vreg[tp][8 * w + 2] = hmul2_u32(hsub2_u32(lop3_and_or(r0s, 0x000F000Fu, 0x64006400u), 0x64086408u), s2);
-                    vreg[tp][8 * w + 3] = hmul2_u32(hsub2_u32(lop3_and_or(r0s, 0x00F000F0u, 0x54005400u), 0x54805480u), s2);
-                    vreg[tp][8 * w + 4] = hmul2_u32(hsub2_u32(lop3_and_or(r1, 0x000F000Fu, 0x64006400u), 0x64086408u), s2);
-                    vreg[tp][8 * w + 5] = hmul2_u32(hsub2_u32(lop3_and_or(r1, 0x00F000F0u, 0x54005400u), 0x54805480u), s2);
-                    vreg[tp][8 * w + 6] = hmul2_u32(hsub2_u32(lop3_and_or(r1s, 0x000F000Fu, 0x64006400u), 0x64086408u), s2);
-                    vreg[tp][8 * w + 7] = hmul2_u32(hsub2_u32(lop3_and_or(r1s, 0x00F000F0u, 0x54005400u), 0x54805480u), s2);
-                }
-            } else {
-                const uint4 ua = *reinterpret_cast<const uint4*>(slot + K_BYTES + (2 * tp) * 512 + lane * 16);
-                const uint4 ub = *reinterpret_cast<const uint4*>(slot + K_BYTES + (2 * tp + 1) * 512 + lane * 16);
-                const uint32_t wa[4] = {ua.x, ua.y, ua.z, ua.w}, wb[4] = {ub.x, ub.y, ub.z, ub.w};
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const uint32_t e = prmt(wa[w], wb[w], 0x5140);   // A.b0 B.b0 A.b1 B.b1
-                    const uint32_t f2 = prmt(wa[w], wb[w], 0x7362);  // A.b2 B.b2 A.b3 B.b3
-                    vreg[tp][4 * w + 0] = hmul2_u32(hsub2_u32(prmt(e, 0x64646464u, 0x4140u), 0x64806480u), s2);
-                    vreg[tp][4 * w + 1] = hmul2_u32(hsub2_u32(prmt(e, 0x64646464u, 0x4342u), 0x64806480u), s2);
-                    vreg[tp][4 * w + 2] = hmul2_u32(hsub2_u32(prmt(f2, 0x64646464u, 0x4140u), 0x64806480u), s2);
-                    vreg[tp][4 * w + 3] = hmul2_u32(hsub2_u32(prmt(f2, 0x64646464u, 0x4342u), 0x64806480u), s2);
-                }
-            }
-        }
-        // tile i: row g <-> d = 16g + 2i, row g+8 <-> d = 16g + 2i + 1
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            mma_m16n8k16(a.o[i], vreg[0][2 * i], vreg[0][2 * i + 1], vreg[1][2 * i], vreg[1][2 * i + 1], pb0, pb1);
-}
-
-// Two shapes of the same kernel.  TWO = true: two CTAs per SM (16 warps hide more of the dequantisation
-// latency: 41 us against 45 us on the batch-16 q4 case) with the ring depth that still fits twice into shared
-// memory.  TWO = false: one CTA per SM with a deeper ring, for grids that do not fill the SMs twice anyway.
-constexpr int ring_depth(int bits, bool two) { return bits == 4 ? (two ? 4 : 8) : (two ? 2 : 5); }
-template <int BITS, int LOGG, bool TWO>
+// Two shapes of the same kernel.  TWO = true: two CTAs per SM (16 warps hide more latency) with the ring depth that still
+// fits twice into shared memory.  TWO = false: one CTA per SM with a deeper ring, for grids that do not fill the SMs twice
+// anyway, and for plain pages (8 KB per page and head).
+constexpr int ring_depth(int bits, bool two) { return bits == 4 ? (two ? 5 : 10) : bits == 8 ? (two ? 3 : 6) : 3; }
+template <int BITS, int LOGG, bool TWO, bool WIDE>
 __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged_attn_kernel(const __grid_constant__ AttnParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int D = 128;
-    constexpr int K_BYTES = BITS == 4 ? 1024 : 2048;  // per page and head
-    constexpr int V_BYTES = K_BYTES;
+    constexpr int D = kHeadDim;
+    constexpr int SLOT = PageShape<BITS>::SLOT;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     int* prefix = reinterpret_cast<int*>(smem + p.off_prefix);   // [B + 1]
@@ -422,35 +145,29 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
     pdl_wait();   // lengths / block table / q / the cache itself may be produced by the previous kernel
 
     // The flattened page list is cut into p.grid equal ranges.  A CTA has 8 warps = 8 (range, kv head) pairs:
-    // with 8 kv heads one range, with fewer heads several consecutive ranges (subs of them).  The cut depends
-    // only on the batch and the device, not on the number of heads, so a head's partial results (and the
-    // merged output) are the same bits whether all heads or a tensor-parallel shard of them are computed.
+    // with 8 kv heads one range, with fewer heads several consecutive ranges (subs of them).
     const int total = build_prefix(p, prefix);
     const int ppc = (total + p.grid - 1) / p.grid;               // pages per range
     const int subs = p.subs;
-    const int h = warp % p.Hkv;                                  // kv head of this warp
-    const int sub = warp / p.Hkv;
+    const int h = blockIdx.y * p.hc + warp % p.hc;               // kv head of this warp
+    const int sub = warp / p.hc;
     const int vc = (int)blockIdx.x * subs + sub;                 // range of this warp
     const int lo = min(total, vc * ppc);
     const int hi = min(total, lo + ppc);
-    if (lo >= hi || sub >= subs || vc >= p.grid) return;
+    if (lo >= hi || sub >= subs || vc >= p.grid || h >= p.Hkv) return;
 
-    const int g = lane >> 2;
-    const int t = lane & 3;
     const int group = p.group;
-    const float sm_scale = p.scale;
     constexpr int NS = ring_depth(BITS, TWO);                     // pages in flight per warp
-    constexpr int SLOT = K_BYTES + V_BYTES + 256;                // bytes of one ring slot
-    uint8_t* my_ring = smem + p.off_ring + (size_t)warp * NS * SLOT;
+    const uint32_t my_ring = smem_u32(smem) + p.off_ring + (uint32_t)warp * (NS * SLOT);
     const int n_my = hi - lo;                                     // pages this warp walks: f = lo + j
 
-    WarpAcc acc;
-    acc_reset(acc);
+    WarpState<BITS, WIDE> acc;
+    state_reset(acc);
     int cur_b = -1;
 
     // Page descriptors (page id, sequence, valid tokens) of 32 consecutive pages of this warp, one per
     // lane.  Two windows: one for the page being consumed, one for the page being issued ahead.
-    struct Desc { int page, b, valid; };      // valid: token count | attended-slot mask << 16
+    struct Desc { int page, b, attended; };   // attended: bit mask of the page's slots
     auto lookup = [&](int base) -> Desc {
         const int j = base + lane;
         Desc d = {-1, 0, 0};
@@ -464,8 +181,7 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
             if (page < 0 || page >= p.num_pages) page = -1;
             d.page = page;
             d.b = b;
-            // low half: tokens of the page below the length (what is copied); high half: attended slots
-            d.valid = min(p.P, sp.L - pg * p.P) | (int)(page_mask16(pg, sp.L, p.sink, p.window) << 16);
+            d.attended = (int)page_mask16(pg, sp.L, p.sink, p.window);
         }
         return d;
     };
@@ -480,40 +196,14 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
         if (j > 0 && (j & 31) == 0) win_i = lookup(j);
         const int src_lane = j & 31;
         const int page = __shfl_sync(0xffffffffu, win_i.page, src_lane);
-        const int valid = __shfl_sync(0xffffffffu, win_i.valid, src_lane) & 0xFFFF;
-        issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, L, lane, page, valid, p.k_codes, p.v_codes, page_code_bytes,
-                               page_scale_halves);
+        issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, L, page, p.k_codes, p.v_codes, page_code_bytes, page_scale_halves);
         slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1;
     };
 
     auto flush = [&](int b) {
-        float* dst = p.partial + ((size_t)(vc + b) * p.Hq) * (D + 2);
-        float l0 = acc.l_run[0], l1 = acc.l_run[1];
-#pragma unroll
-        for (int o2 = 4; o2 < 32; o2 <<= 1) {
-            l0 += __shfl_xor_sync(0xffffffffu, l0, o2);
-            l1 += __shfl_xor_sync(0xffffffffu, l1, o2);
-        }
-        // O^T[d][head]: thread (g,t) holds d = 16g + 2i (+1), heads 2t, 2t+1
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int head = 2 * t + (e & 1);
-                const int d = 16 * g + 2 * i + (e >> 1);
-                if (head < group) dst[(size_t)(h * group + head) * (D + 2) + d] = acc.o[i][e];
-            }
-        }
-        if (g == 0) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int head = 2 * t + e;
-                if (head < group) {
-                    dst[(size_t)(h * group + head) * (D + 2) + D] = acc.m_run[e];
-                    dst[(size_t)(h * group + head) * (D + 2) + D + 1] = e ? l1 : l0;
-                }
-            }
-        }
+        float* dst = p.partial + ((size_t)(vc + b) * p.Hq + h * group) * (D + 2);
+        emit(acc, group, lane, [&](int head, int d, float v) { dst[head * (D + 2) + d] = v; },
+             [&](int head, float m, float l) { dst[head * (D + 2) + D] = m; dst[head * (D + 2) + D + 1] = l; });
     };
 
     // prologue: copies of the first NS - 1 pages
@@ -527,9 +217,7 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
         if (j > 0 && (j & 31) == 0) win_c = lookup(j);
         const int page = __shfl_sync(0xffffffffu, win_c.page, j & 31);
         const int b = __shfl_sync(0xffffffffu, win_c.b, j & 31);
-        const uint32_t valid_mask = (uint32_t)__shfl_sync(0xffffffffu, win_c.valid, j & 31);
-        const int valid = (int)(valid_mask & 0xFFFFu);
-        const uint32_t attended = valid_mask >> 16;
+        const uint32_t attended = (uint32_t)__shfl_sync(0xffffffffu, win_c.attended, j & 31);
         // look-ahead: copies of page j + NS - 1 (an empty group keeps the count uniform at the end)
         if (j + NS - 1 < n_my) issue(j + NS - 1);
         else cp_async_commit();
@@ -539,10 +227,11 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
         if (b != cur_b) {
             if (cur_b >= 0) flush(cur_b);
             cur_b = b;
-            acc_reset(acc);
-            load_q_frags<BITS>(acc, p.q + ((size_t)b * p.Hq + h * group) * D, group, g, t);
+            state_reset(acc);
+            load_queries<BITS, LOGG>(acc, reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D, group, p.q_dtype,
+                                     p.scale, lane);
         }
-        if (page >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, valid, attended, sm_scale, lane);
+        if (page >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, L, attended, lane);
         __syncwarp();   // every lane is done with this slot before it is refilled
         slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
     }
@@ -560,7 +249,7 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
 // new position appends kv head h itself before it reads that page, every CTA rotates its own copy of q.
 // ------------------------------------------------------------------------------------------------
 struct ClusterAttnParams {
-    const __half* q;            // [B, Hq, D] rotated queries (fused == 0)
+    const void* q;              // [B, Hq, D] rotated queries (fused == 0)
     const __half* qkv;          // fused: [B, (Hq + 2 Hkv) * D]
     const float* cos_table;     // fused: [table_len, D/2]
     const float* sin_table;
@@ -572,7 +261,7 @@ struct ClusterAttnParams {
     const int32_t* block_table;
     const int32_t* lengths;
     void* out;                  // [B, Hq, D]
-    int B, Hq, Hkv, P, max_blocks, G, Gd, group, bits, table_len, fused, S;
+    int B, Hq, Hkv, P, max_blocks, G, Gd, group, bits, q_dtype, table_len, fused, S;
     int64_t num_pages;
     float scale;
     int row_bytes, scale_row_halves;
@@ -586,18 +275,15 @@ __device__ __forceinline__ uint32_t cluster_rank_x() {
     return r;
 }
 
-template <int BITS, int LOGG>
+template <int BITS, int LOGG, bool WIDE>
 __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterAttnParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int D = 128;
-    constexpr int K_BYTES = BITS == 4 ? 1024 : 2048;
-    constexpr int V_BYTES = K_BYTES;
-    constexpr int NS = BITS == 4 ? 8 : 5;                         // pages in flight per warp
-    constexpr int SLOT = K_BYTES + V_BYTES + 256;
+    constexpr int D = kHeadDim;
+    constexpr int NS = ring_depth(BITS, false) - (WIDE ? 2 : 1);  // pages in flight per warp (room for the partial results)
+    constexpr int SLOT = PageShape<BITS>::SLOT;
     constexpr int PW = D + 2;                                     // floats of one partial: accumulator, max, sum
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int g = lane >> 2, t = lane & 3;
     const uint32_t rank = cluster_rank_x();
     const int h = blockIdx.y;
     const int b = blockIdx.z;
@@ -693,69 +379,42 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     }
 
     // ---- this warp's pages ----
-    WarpAcc acc;
-    acc_reset(acc);
+    WarpState<BITS, WIDE> acc;
+    state_reset(acc);
     const int n_my = hi - lo;
     if (n_my > 0) {
-        const __half* qrows = p.fused ? qs : p.q + ((size_t)b * p.Hq + h * group) * D;
-        load_q_frags<BITS>(acc, qrows, group, g, t);
+        const void* qrows = p.fused ? (const void*)qs : (const void*)(reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D);
         const PageLanes Lp = page_lanes<BITS>(lane, h, (uint32_t)p.row_bytes, p.scale_row_halves, p.Gd, p.k_scales, p.v_scales);
         const size_t page_code_bytes = (size_t)p.P * p.row_bytes;
         const size_t page_scale_halves = (size_t)p.P * p.scale_row_halves;
-        uint8_t* my_ring = smem + p.off_ring + (size_t)warp * NS * SLOT;
+        const uint32_t my_ring = smem_u32(smem) + p.off_ring + (uint32_t)warp * (NS * SLOT);
         auto page_of = [&](int j) -> int {
             int page = p.block_table[(size_t)b * p.max_blocks + lo + j];
             return (page < 0 || page >= p.num_pages) ? -1 : page;
         };
-        auto valid_of = [&](int j) -> int { return min(p.P, L - (lo + j) * p.P); };
         int slot_i = 0, slot_c = 0;
-        for (int j = 0; j < NS - 1; ++j) {
-            if (j < n_my) issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, Lp, lane, page_of(j), valid_of(j), p.k_codes, p.v_codes,
-                                                 page_code_bytes, page_scale_halves);
+        auto issue = [&](int j) {
+            if (j < n_my) issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, Lp, page_of(j), p.k_codes, p.v_codes, page_code_bytes, page_scale_halves);
             else cp_async_commit();
             slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1;
-        }
+        };
+        for (int j = 0; j < NS - 1; ++j) issue(j);
+        load_queries<BITS, LOGG>(acc, qrows, group, p.fused ? B200Q_F16 : p.q_dtype, p.scale, lane);
         for (int j = 0; j < n_my; ++j) {
-            if (j + NS - 1 < n_my)
-                issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, Lp, lane, page_of(j + NS - 1), valid_of(j + NS - 1), p.k_codes,
-                                       p.v_codes, page_code_bytes, page_scale_halves);
-            else cp_async_commit();
-            slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1;
+            issue(j + NS - 1);
             cp_async_wait<NS - 1>();
             __syncwarp();
-            const int valid = valid_of(j);
+            const int valid = min(p.P, L - (lo + j) * p.P);
             const uint32_t attended = valid >= 16 ? 0xFFFFu : ((1u << max(valid, 0)) - 1u);
-            if (page_of(j) >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, valid, attended, p.scale, lane);
+            if (page_of(j) >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, Lp, attended, lane);
             __syncwarp();
             slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
         }
     }
-    // ---- the warp's partial: O^T[d][head] with thread (g,t) holding d = 16g + 2i (+1), heads 2t, 2t+1 ----
     {
-        float l0 = acc.l_run[0], l1 = acc.l_run[1];
-#pragma unroll
-        for (int o2 = 4; o2 < 32; o2 <<= 1) {
-            l0 += __shfl_xor_sync(0xffffffffu, l0, o2);
-            l1 += __shfl_xor_sync(0xffffffffu, l1, o2);
-        }
         float* dst = wpart + (size_t)warp * group * PW;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int head = 2 * t + (e & 1);
-                if (head < group) dst[head * PW + 16 * g + 2 * i + (e >> 1)] = acc.o[i][e];
-            }
-        if (g == 0) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int head = 2 * t + e;
-                if (head < group) {
-                    dst[head * PW + D] = acc.m_run[e];
-                    dst[head * PW + D + 1] = e ? l1 : l0;
-                }
-            }
-        }
+        emit(acc, group, lane, [&](int head, int d, float v) { dst[head * PW + d] = v; },
+             [&](int head, float m, float l) { dst[head * PW + D] = m; dst[head * PW + D + 1] = l; });
     }
     __syncthreads();
     // ---- merge the 8 warps (fixed order) into this CTA's partial; thread -> (head, d) ----
@@ -767,7 +426,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
         for (int i = 0; i < n; ++i) {
             const float* ps = src + ((size_t)i * group + head) * PW;
             const float m = ps[D];
-            const float w = m == -INFINITY ? 0.0f : exp2f((m - m_tot) * kLog2e);
+            const float w = m == -INFINITY ? 0.0f : exp2f(m - m_tot);      // the maxima are in log2 units
             accv = fmaf(w, ps[d], accv);
             l_tot = fmaf(w, ps[D + 1], l_tot);
         }
@@ -796,7 +455,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
             float m_tot, l_tot;
             const float v = merge(cpart, S, head, d, m_tot, l_tot);
             const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
-            const unsigned short bits16 = __half_as_ushort(__float2half_rn(v * inv));
+            const unsigned short bits16 = p.fused || p.q_dtype == B200Q_F16 ? __half_as_ushort(__float2half_rn(v * inv))
+                                                                            : __bfloat16_as_ushort(__float2bfloat16_rn(v * inv));
             const int hq = h * group + head;
             if (p.out != nullptr) reinterpret_cast<unsigned short*>(p.out)[((size_t)b * p.Hq + hq) * D + d] = bits16;
             if (p.tp_out.world > 0) {
@@ -835,8 +495,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) paged_attn_merge_kernel(cons
     __shared__ float red[kMergeWarps][128];
     __shared__ float red_s[2][kMergeWarps];
     __shared__ int red_i[2][kMergeWarps];
-    __shared__ int cand_off[kMaxGrid];            // candidates: page ranges of the main kernel that touch this sequence
-    __shared__ float cand_m[kMaxGrid];
+    __shared__ int cand_off[kMaxRanges];            // candidates: page ranges of the main kernel that touch this sequence
+    __shared__ float cand_m[kMaxRanges];
     const int D = p.D;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -896,7 +556,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) paged_attn_merge_kernel(cons
             const float m = cand_m[i];
             const bool ok = off >= 0 && m != -INFINITY;
             const float* src = p.partial + (ok ? off : 0);
-            const float w = ok ? exp2f((m - m_tot) * kLog2e) : 0.0f;
+            const float w = ok ? exp2f(m - m_tot) : 0.0f;      // the maxima are in log2 units
             const float l = ok ? src[D + 1] : 0.0f;
             l_part = fmaf(w, l, l_part);
 #pragma unroll
@@ -1033,7 +693,9 @@ __global__ void __launch_bounds__(128) paged_attn_simple_kernel(const __grid_con
 }
 
 inline uint32_t align_up_u32(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
-inline int subs_for(int Hkv) { return (Hkv <= kAttnWarps && kAttnWarps % Hkv == 0) ? kAttnWarps / Hkv : 1; }
+inline int subs_for(int hc) { return kAttnWarps % hc == 0 ? kAttnWarps / hc : 1; }
+
+inline bool heads_ok(int Hkv) { return Hkv <= kAttnWarps || Hkv % kAttnWarps == 0; }
 
 // ---- cluster kernel: host side ----
 int cluster_size_for(int B, int Hkv) {
@@ -1054,9 +716,9 @@ int cluster_size_for(int B, int Hkv) {
 }
 
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
-    const bool g32 = p.G == 32;
-    const int slot = (p.bits == 4 ? 2048 : 4096) + 256;
-    const int ns = p.bits == 4 ? 8 : 5;
+    const bool g32 = p.G == 32, wide = p.group > 4;
+    const int slot = p.bits == 4 ? PageShape<4>::SLOT : PageShape<8>::SLOT;
+    const int ns = ring_depth(p.bits, false) - (wide ? 2 : 1);
     uint32_t off = 0;
     p.off_q = off;      off += align_up_u32((uint32_t)p.group * 128 * 2, 128);
     p.off_wpart = off;  off += align_up_u32((uint32_t)kAttnWarps * p.group * 130 * 4, 128);
@@ -1065,16 +727,19 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     const uint32_t cap = (uint32_t)max_smem_optin();
     if (off > cap) return B200Q_ERR_UNSUPPORTED;
     using KernelFn = void (*)(ClusterAttnParams);
-    KernelFn kernel = p.bits == 4 ? (g32 ? paged_attn_cluster_kernel<4, 5> : paged_attn_cluster_kernel<4, 6>)
-                                  : (g32 ? paged_attn_cluster_kernel<8, 5> : paged_attn_cluster_kernel<8, 6>);
-    static bool configured[2][2][64] = {};
+    static const KernelFn kernels[2][2][2] = {{{paged_attn_cluster_kernel<8, 6, false>, paged_attn_cluster_kernel<8, 6, true>},
+                                               {paged_attn_cluster_kernel<8, 5, false>, paged_attn_cluster_kernel<8, 5, true>}},
+                                              {{paged_attn_cluster_kernel<4, 6, false>, paged_attn_cluster_kernel<4, 6, true>},
+                                               {paged_attn_cluster_kernel<4, 5, false>, paged_attn_cluster_kernel<4, 5, true>}}};
+    KernelFn kernel = kernels[p.bits == 4][g32][wide];
+    static bool configured[2][2][2][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!configured[p.bits == 4][g32][dev & 63]) {
+    if (!configured[p.bits == 4][g32][wide][dev & 63]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess ||
             cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
             return B200Q_ERR_LAUNCH;
-        configured[p.bits == 4][g32][dev & 63] = true;
+        configured[p.bits == 4][g32][wide][dev & 63] = true;
     }
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -1099,6 +764,84 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     return finish_launch();
 }
 
+int launch_split_attention(AttnParams& p, cudaStream_t stream) {
+    const int bits = p.bits;
+    p.hc = std::min(p.Hkv, kAttnWarps);
+    p.subs = subs_for(p.hc);
+    const int chunks = p.Hkv / p.hc;
+    p.slot_bytes = bits == 4 ? PageShape<4>::SLOT : bits == 8 ? PageShape<8>::SLOT : PageShape<16>::SLOT;
+    int ctas_per_sm = tuning_get("attn.ctas_per_sm");
+    if (ctas_per_sm <= 0) ctas_per_sm = bits == 16 ? 1 : B200Q_ATTN_CTAS;
+    // At least three pages per range (by the block table's capacity; the lengths live on the device): short
+    // batches otherwise pay for partial results and their merge more than for the KV bytes (measured on the
+    // 32-layer stack at batch 1, context 4096: 2 -> 2.32-2.35, 3 -> 2.26, 4 -> 2.30, 8 -> 2.46 ms per step).
+    const int64_t pages_cap = (int64_t)p.B * p.max_blocks;
+    int min_pages = tuning_get("attn.min_pages");
+    if (min_pages <= 0) min_pages = 3;
+    // Ranges for every warp of the resident CTAs.  The cut follows the kv heads of the UNSHARDED cache ("ts.tp_world" equal head
+    // shards), so that a head's partial results do not depend on the sharding.
+    const int full_subs = subs_for(std::min(p.Hkv * std::max(1, tuning_get("ts.tp_world")), kAttnWarps));
+    const int want = std::max(1, sm_count() * ctas_per_sm / chunks) * full_subs;
+    p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(std::min({kMaxRanges, kMaxGrid * full_subs, want}), (pages_cap + min_pages - 1) / min_pages));
+    const int launch_grid = (p.grid + p.subs - 1) / p.subs;   // CTAs: each covers `subs` ranges
+    const bool two = bits != 16 && launch_grid * chunks > sm_count();
+    const int stages = ring_depth(bits, two);
+
+    uint32_t off = 0;
+    p.off_prefix = off; off += align_up_u32((p.B + 1) * sizeof(int), 16);
+    off = align_up_u32(off, 128);
+    p.off_ring = off;
+    const uint32_t cap = (uint32_t)max_smem_optin();
+    const uint32_t total_smem = off + stages * kAttnWarps * p.slot_bytes;
+    if (total_smem > cap) return B200Q_ERR_UNSUPPORTED;
+    p.stages = stages;
+
+    const bool g32 = p.G == 32, wide_group = p.group > 4, bf = p.q_dtype == B200Q_BF16;
+    using KernelFn = void (*)(AttnParams);
+#define B200Q_ATTN_PAIR(BITS, LOGG, TWO) {paged_attn_kernel<BITS, LOGG, TWO, false>, paged_attn_kernel<BITS, LOGG, TWO, true>}
+    static const KernelFn quantised[2][2][2][2] = {      // [q4][group 32][two][wide]
+        {{B200Q_ATTN_PAIR(8, 6, false), B200Q_ATTN_PAIR(8, 6, true)}, {B200Q_ATTN_PAIR(8, 5, false), B200Q_ATTN_PAIR(8, 5, true)}},
+        {{B200Q_ATTN_PAIR(4, 6, false), B200Q_ATTN_PAIR(4, 6, true)}, {B200Q_ATTN_PAIR(4, 5, false), B200Q_ATTN_PAIR(4, 5, true)}}};
+    static const KernelFn plain[2][2] = {B200Q_ATTN_PAIR(16, 0, false), B200Q_ATTN_PAIR(16, 1, false)};
+#undef B200Q_ATTN_PAIR
+    KernelFn kernel = bits == 16 ? plain[bf][wide_group] : quantised[bits == 4][g32][two][wide_group];
+    static bool configured[32][64] = {};
+    const int slot = bits == 16 ? 16 + bf * 2 + wide_group : (bits == 4) * 8 + g32 * 4 + two * 2 + wide_group;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!configured[slot][dev & 63]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess)
+            return B200Q_ERR_LAUNCH;
+        configured[slot][dev & 63] = true;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(launch_grid, chunks);
+        cfg.blockDim = dim3(kAttnThreads);
+        cfg.dynamicSmemBytes = total_smem;
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
+        if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return B200Q_ERR_LAUNCH;
+    }
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(p.B * p.Hq);
+        const bool wide = p.B * p.Hq < 2 * sm_count();
+        cfg.blockDim = dim3((wide ? 32 : 8) * 32);
+        cfg.dynamicSmemBytes = 0;
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
+        if (cudaLaunchKernelEx(&cfg, wide ? paged_attn_merge_kernel<32> : paged_attn_merge_kernel<8>, p) != cudaSuccess)
+            return B200Q_ERR_LAUNCH;
+    }
+    return finish_launch();
+}
+
 }  // namespace
 
 int attention_stage_launches_impl(int B, int Hkv, int with_append) {
@@ -1109,8 +852,8 @@ int attention_stage_launches_impl(int B, int Hkv, int with_append) {
 
 size_t paged_gqa_workspace_bytes_impl(int B, int Hq, int Hkv, int D) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || D <= 0) return 0;
-    (void)Hkv;
-    return (size_t)(kMaxGrid + B) * Hq * (D + 2) * sizeof(float);
+    const int ranges = std::min(kMaxRanges, kMaxGrid * subs_for(std::min(Hkv, kAttnWarps)));
+    return (size_t)(ranges + B) * Hq * (D + 2) * sizeof(float);
 }
 
 int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const uint8_t* v_codes, const void* k_scales,
@@ -1132,9 +875,9 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     const int group = Hq / Hkv;
     const int dp = bits == 4 ? D / 2 : D;
 
-    const bool fast_ok = tuning_get("attn.force_simple") == 0 && D == 128 && q_dtype == B200Q_F16 &&
+    const bool fast_ok = tuning_get("attn.force_simple") == 0 && D == kHeadDim &&
                          scale_dtype == B200Q_F16 && (group_size == 32 || group_size == 64) && group <= 8 &&
-                         Hkv <= kAttnWarps && page_size == 16 && B <= kMaxBatchFast &&
+                         heads_ok(Hkv) && page_size == 16 && B <= kMaxBatchFast &&
                          ((uintptr_t)q % 16 == 0) && ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) &&
                          ((uintptr_t)k_scales % 8 == 0) && ((uintptr_t)v_scales % 8 == 0);
     if (!fast_ok && tp_out_slot >= 0) return B200Q_ERR_UNSUPPORTED;   // the exchange exists only in the split-KV kernels
@@ -1151,7 +894,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     if (cluster > 0) {
         ClusterAttnParams c = {};
         if (tp_out_slot >= 0) c.tp_out = tp_slot(tp_out_slot)->out;
-        c.q = (const __half*)q;
+        c.q = q; c.q_dtype = q_dtype;
         c.k_codes = const_cast<uint8_t*>(k_codes); c.v_codes = const_cast<uint8_t*>(v_codes);
         c.k_scales = (__half*)const_cast<void*>(k_scales); c.v_scales = (__half*)const_cast<void*>(v_scales);
         c.block_table = block_table; c.lengths = lengths; c.out = out;
@@ -1165,83 +908,33 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
 
     AttnParams p = {};
     if (tp_out_slot >= 0) p.tp_out = tp_slot(tp_out_slot)->out;
-    p.q = (const __half*)q; p.k_codes = k_codes; p.v_codes = v_codes;
+    p.q = q; p.k_codes = k_codes; p.v_codes = v_codes;
     p.k_scales = (const __half*)k_scales; p.v_scales = (const __half*)v_scales;
     p.block_table = block_table; p.lengths = lengths; p.partial = (float*)workspace; p.out = out;
     p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.P = page_size; p.max_blocks = max_blocks; p.G = group_size; p.Gd = Gd;
     p.group = group; p.num_pages = num_pages; p.scale = scale; p.q_dtype = q_dtype; p.bits = bits;
-    p.subs = subs_for(Hkv);
     p.sink = sink_tokens;
     p.window = window_size;
     p.row_bytes = Hkv * dp;
     p.scale_row_halves = Hkv * Gd;
-    p.slot_bytes = (bits == 4 ? 2048 : 4096) + 256;
-    int ctas_per_sm = tuning_get("attn.ctas_per_sm");
-    if (ctas_per_sm <= 0) ctas_per_sm = B200Q_ATTN_CTAS;
-    // At least three pages per range (by the block table's capacity; the lengths live on the device): short
-    // batches otherwise pay for partial results and their merge more than for the KV bytes (measured on the
-    // 32-layer stack at batch 1, context 4096: 2 -> 2.32-2.35, 3 -> 2.26, 4 -> 2.30, 8 -> 2.46 ms per step).
-    const int64_t pages_cap = (int64_t)B * max_blocks;
-    int min_pages = tuning_get("attn.min_pages");
-    if (min_pages <= 0) min_pages = 3;
-    p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(kMaxGrid, sm_count() * ctas_per_sm),
-                                                         (pages_cap + min_pages - 1) / min_pages));
-    const int launch_grid = (p.grid + p.subs - 1) / p.subs;   // CTAs: each covers `subs` ranges
-    const bool two = launch_grid > sm_count();
-    const int stages = ring_depth(bits, two);
+    return launch_split_attention(p, stream);
+}
 
-    uint32_t off = 0;
-    p.off_prefix = off; off += align_up_u32((B + 1) * sizeof(int), 16);
-    off = align_up_u32(off, 128);
-    p.off_ring = off;
-    const uint32_t cap = (uint32_t)max_smem_optin();
-    if (off + (uint64_t)stages * kAttnWarps * p.slot_bytes > cap) return B200Q_ERR_UNSUPPORTED;
-    p.stages = stages;
-    const uint32_t total_smem = off + stages * kAttnWarps * p.slot_bytes;
-
-    const bool g32 = group_size == 32;
-    using KernelFn = void (*)(AttnParams);
-    KernelFn kernel;
-    if (two)
-        kernel = bits == 4 ? (g32 ? paged_attn_kernel<4, 5, true> : paged_attn_kernel<4, 6, true>)
-                           : (g32 ? paged_attn_kernel<8, 5, true> : paged_attn_kernel<8, 6, true>);
-    else
-        kernel = bits == 4 ? (g32 ? paged_attn_kernel<4, 5, false> : paged_attn_kernel<4, 6, false>)
-                           : (g32 ? paged_attn_kernel<8, 5, false> : paged_attn_kernel<8, 6, false>);
-    static bool configured[2][2][2][64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!configured[two][bits == 4][g32][dev & 63]) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess)
-            return B200Q_ERR_LAUNCH;
-        configured[two][bits == 4][g32][dev & 63] = true;
-    }
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(launch_grid);
-        cfg.blockDim = dim3(kAttnThreads);
-        cfg.dynamicSmemBytes = total_smem;
-        cfg.stream = stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
-        if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return B200Q_ERR_LAUNCH;
-    }
-    {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(B * Hq);
-        const bool wide = B * Hq < 2 * sm_count();
-        cfg.blockDim = dim3((wide ? 32 : 8) * 32);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
-        if (cudaLaunchKernelEx(&cfg, wide ? paged_attn_merge_kernel<32> : paged_attn_merge_kernel<8>, p) != cudaSuccess)
-            return B200Q_ERR_LAUNCH;
-    }
-    return finish_launch();
+// Plain fp16 / bf16 pages on the split-KV kernels; B200Q_ERR_UNSUPPORTED outside their shapes.
+int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table, const int32_t* lengths,
+                               void* out, void* workspace, size_t workspace_bytes, int B, int Hq, int Hkv, int D, int page_size,
+                               int64_t num_pages, int max_blocks, float scale, int dtype, cudaStream_t stream) {
+    if (tuning_get("attn.force_simple") || D != kHeadDim || page_size != 16 || Hq / Hkv > 8 || !heads_ok(Hkv) || B > kMaxBatchFast ||
+        ((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) % 16 != 0)
+        return B200Q_ERR_UNSUPPORTED;
+    if (workspace == nullptr || workspace_bytes < paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D)) return B200Q_ERR_WORKSPACE;
+    AttnParams p = {};
+    p.q = q; p.k_codes = (const uint8_t*)k_pages; p.v_codes = (const uint8_t*)v_pages;
+    p.block_table = block_table; p.lengths = lengths; p.partial = (float*)workspace; p.out = out;
+    p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.P = page_size; p.max_blocks = max_blocks;
+    p.group = Hq / Hkv; p.num_pages = num_pages; p.scale = scale; p.q_dtype = dtype; p.bits = 16;
+    p.row_bytes = Hkv * kHeadDim * 2;
+    return launch_split_attention(p, stream);
 }
 
 // Decode-layer attention in one call: split + rotate + append (as rope_kv_append_impl) followed by the attention over
@@ -1271,7 +964,7 @@ int rope_append_attention_impl(const void* qkv, const float* cos_table, const fl
     const int Gd = (D + group_size - 1) / group_size;
     const int dp = bits == 4 ? D / 2 : D;
     const bool fast_ok = tuning_get("attn.force_simple") == 0 && D == 128 && (group_size == 32 || group_size == 64) &&
-                         group <= 8 && Hkv <= kAttnWarps && page_size == 16 && B <= 65535 && ((uintptr_t)qkv % 16 == 0) &&
+                         group <= 8 && heads_ok(Hkv) && page_size == 16 && B <= 65535 && ((uintptr_t)qkv % 16 == 0) &&
                          ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) && ((uintptr_t)k_scales % 8 == 0) &&
                          ((uintptr_t)v_scales % 8 == 0);
     const int cluster = fast_ok ? cluster_size_for(B, Hkv) : 0;

@@ -1,0 +1,477 @@
+// One warp, one kv head, one page of 16 tokens of head_dim 128: the building blocks of the paged decode attention kernels, for
+// quantised pages (q4 / q8 codes, symmetric fp16 scales per token and group) and for plain fp16 / bf16 pages.
+//
+// A page of q4 codes is 2.3 KB per kv head and an SM receives one every 100 clocks at the HBM rate, so the instructions per page
+// decide.  (The form before this one dequantised K and V to fp16 with three operations per pair and took 591 warp
+// instructions per page and kv head; it ran at 58 % issue and 0.27 of the DRAM rate.)
+//   * copies: every lane moves 16-byte pieces with cp.async, rows whole, into a ring slot laid out chunk-major
+//     ([16-byte chunk of a row][16 tokens], positions XORed so that neither the copies nor ldmatrix meet bank conflicts).
+//   * S = K Q^T: ldmatrix hands every lane the word of its token row; raw codes go into mma.sync.m16n8k32 u8 x s8 (a q4 word costs
+//     two masks and a shift, a q8 word nothing).  The queries are 16-bit fixed point relative to the head's largest
+//     element, as two signed bytes = two columns of the B operand; the offset of the codes is the accumulator's start value.
+//     The scale is applied once per token and group in fp32, so K is not rounded at all.
+//   * softmax: a lane holds one head (two when there are more than four query heads per kv head) of tokens g and g + 8.  The
+//     reference maximum only moves when a score exceeds it by 2^8, decided by one vote per page; no shuffles otherwise.
+//   * O^T += V^T P: ldmatrix.trans delivers the codes of two tokens side by side, exact fp16 code - offset takes two operations per
+//     pair, and the scales are folded into the probabilities, (p * scale) rounded once to fp16 as an operand column
+//     per scale group.  Plain pages need no arithmetic; there the spare columns carry the rounding remainder of p.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200q {
+namespace attn {
+
+constexpr int kHeadDim = 128;
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kQLevels = 32639.0f;          // largest 16-bit value whose high digit still fits a signed byte
+
+// BITS: 4, 8 (codes) or 16 (plain).  LOGG: log2 of the scale group, 5 or 6; for plain pages 0 = fp16, 1 = bf16.
+template <int BITS> struct PageShape {
+    static constexpr int ROW = kHeadDim * BITS / 8;        // bytes of one token row of one kv head
+    static constexpr int TILE = 16 * ROW;                  // K (or V) bytes of a page
+    static constexpr int SLOT = 2 * TILE + (BITS == 16 ? 0 : 256);   // ring slot: K, V, scales of K, scales of V
+    static constexpr int NCH = ROW / 16;                   // 16-byte chunks of a row
+};
+
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+template <int BYTES>
+__device__ __forceinline__ void cp_async_small(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void lds64(uint32_t (&r)[2], uint32_t a) {
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool BF>
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (BF) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    } else {
+        mma_m16n8k16(d, a0, a1, a2, a3, b0, b1);
+    }
+}
+__device__ __forceinline__ float half_lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xFFFFu))); }
+__device__ __forceinline__ float half_hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+__device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// WIDE: five to eight query heads per kv head.  ST: heads ("streams") a lane holds: head t, and head 4 + t when WIDE.
+template <int BITS, bool WIDE> struct WarpState {
+    static constexpr int ST = WIDE ? 2 : 1;
+    uint32_t qb[BITS == 16 ? 1 : ST][BITS == 16 ? 8 : 4][2];      // queries as B operand, per mma
+    int c0[BITS == 16 ? 1 : ST][BITS == 16 ? 1 : 4][2];           // -offset * (sum of the group's query digits): accumulator start
+    float qs[ST];               // factor of the integer scores: digit step * softmax scale * log2(e)
+    float m[ST], l[ST];         // reference maximum (log2 units), this lane's share of the sum
+    float vk;                   // power of two on the V scales inside the probabilities
+    float o[8][4];              // O^T tiles; see out_value()
+};
+template <int BITS, bool WIDE>
+__device__ __forceinline__ void state_reset(WarpState<BITS, WIDE>& a) {
+#pragma unroll
+    for (int s = 0; s < WarpState<BITS, WIDE>::ST; ++s) { a.m[s] = -INFINITY; a.l[s] = 0.0f; }
+    a.vk = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a.o[i][e] = 0.0f;
+}
+
+// Queries of one kv head's group: row r of `rows` (128 values apart) is query head r (r < group <= 8).  Shared or global memory.
+template <int BITS, int LOGG, bool WIDE>
+__device__ __forceinline__ void load_queries(WarpState<BITS, WIDE>& a, const void* rows, int group, int dtype, float sm_scale, int lane) {
+    constexpr int ST = WarpState<BITS, WIDE>::ST;
+    const int g = lane >> 2, t = lane & 3;
+    const uint16_t* q = reinterpret_cast<const uint16_t*>(rows);
+    if constexpr (BITS == 16) {
+        // column 2h is head h, column 2h + 1 head 4 + h (when WIDE): this lane feeds column g
+        const int head = (g >> 1) + ((g & 1) ? 4 : 0);
+        const bool live = ((g & 1) == 0 || WIDE) && head < group;
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                a.qb[0][s][h] = live ? *reinterpret_cast<const uint32_t*>(q + (size_t)head * kHeadDim + 16 * s + 8 * h + 2 * t) : 0u;
+#pragma unroll
+        for (int s = 0; s < ST; ++s) a.qs[s] = sm_scale * kLog2e;
+    } else {
+#pragma unroll
+        for (int s = 0; s < ST; ++s) {
+            // column 2h is the high digit of head h (+ 4), column 2h + 1 its low digit: this lane feeds column g
+            const int head = (g >> 1) + 4 * s;
+            float v[4][8], mx = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t w[4] = {0u, 0u, 0u, 0u};
+                if (head < group) {
+                    const uint16_t* row = q + (size_t)head * kHeadDim + 32 * i;
+                    if (BITS == 4) {      // d = 8t .. 8t + 7 of the 32
+                        const uint4 u = *reinterpret_cast<const uint4*>(row + 8 * t);
+                        w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+                    } else {              // d = 4t .. 4t + 3 and 16 + 4t ..
+                        const uint2 u0 = *reinterpret_cast<const uint2*>(row + 4 * t), u1 = *reinterpret_cast<const uint2*>(row + 16 + 4 * t);
+                        w[0] = u0.x; w[1] = u0.y; w[2] = u1.x; w[3] = u1.y;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[i][2 * j] = dtype == B200Q_F16 ? half_lo(w[j]) : __uint_as_float(w[j] << 16);
+                    v[i][2 * j + 1] = dtype == B200Q_F16 ? half_hi(w[j]) : __uint_as_float(w[j] & 0xFFFF0000u);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) mx = v[i][j] == v[i][j] ? fmaxf(mx, fabsf(v[i][j])) : INFINITY;
+            }
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float up = mx > 0.0f ? kQLevels / mx : 0.0f;
+            int sum[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t dig[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int x = __float2int_rn(fminf(fmaxf(v[i][j] * up, -kQLevels), kQLevels));
+                    const int hi = (x + 128) >> 8;
+                    dig[j] = (uint32_t)((g & 1) ? x - (hi << 8) : hi) & 0xFFu;
+                }
+                // q4: even elements, then odd ones (low and high nibbles of the code word); q8: the two runs of four
+                constexpr int E = BITS == 4 ? 2 : 1, O = BITS == 4 ? 1 : 4;
+                a.qb[s][i][0] = dig[0] | (dig[E] << 8) | (dig[2 * E] << 16) | (dig[3 * E] << 24);
+                a.qb[s][i][1] = dig[O] | (dig[O + E] << 8) | (dig[O + 2 * E] << 16) | (dig[O + 3 * E] << 24);
+                sum[i] = __dp4a((int)a.qb[s][i][0], 0x01010101, __dp4a((int)a.qb[s][i][1], 0x01010101, 0));
+                sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 1);
+                sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 2);
+            }
+            if (LOGG == 6) { sum[0] += sum[1]; sum[2] += sum[3]; }
+            // as accumulator owner this lane holds columns 2t, 2t + 1: head t (+ 4)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) a.c0[s][i][e] = (BITS == 4 ? -8 : -128) * __shfl_sync(0xffffffffu, sum[i], (2 * t + e) * 4);
+            a.qs[s] = __shfl_sync(0xffffffffu, mx, 2 * t * 4) / kQLevels * (sm_scale * kLog2e);
+        }
+    }
+}
+
+// Per-lane source and ring offsets of a page copy for kv head h.
+struct PageLanes {
+    uint32_t src, dst;                // first 16-byte piece of this lane
+    uint32_t step;                    // source distance of its next piece (another token row)
+    uint32_t sc_src, sc_dst;          // scales: lanes 0-15 copy K's, lanes 16-31 V's (halves / bytes)
+    const __half* sc_base;
+    uint32_t rd;                      // ldmatrix row address inside a tile, first pair of chunks
+};
+template <int BITS>
+__device__ __forceinline__ PageLanes page_lanes(int lane, int h, uint32_t row_bytes, int scale_row_halves, int Gd, const __half* k_scales,
+                                                const __half* v_scales) {
+    using P = PageShape<BITS>;
+    constexpr int LPR = P::NCH;                            // lanes that share a token row: 4, 8, 16
+    const int row = lane / LPR, ch = lane % LPR;
+    PageLanes L;
+    L.src = (uint32_t)row * row_bytes + (uint32_t)h * P::ROW + 16u * ch;
+    L.step = (uint32_t)(32 / LPR) * row_bytes;
+    L.dst = (uint32_t)ch * 256 + (uint32_t)(((row & 7) ^ ((BITS == 4 ? 2 * ch : ch) & 7)) << 4);
+    L.sc_src = (uint32_t)(lane & 15) * scale_row_halves + h * Gd;
+    L.sc_dst = 2 * P::TILE + (lane < 16 ? 0 : 128) + (lane & 15) * 8;
+    L.sc_base = lane < 16 ? k_scales : v_scales;
+    // matrices of an x4 load: chunk c tokens 0-7, chunk c tokens 8-15, chunk c + 1 tokens 0-7, chunk c + 1 tokens 8-15
+    const int up = lane >> 4;
+    L.rd = (uint32_t)up * 256 + (uint32_t)((lane >> 3) & 1) * 128 + (uint32_t)(((lane & 7) ^ (BITS == 4 ? 2 * up : up)) << 4);
+    return L;
+}
+// Asynchronous copies of one page into a ring slot: one commit group, empty for a missing page.  Whole pages are copied; slots
+// past the length are masked where they are used.
+template <int BITS, int LOGG>
+__device__ __forceinline__ void issue_page(uint32_t slot, const PageLanes& L, int page, const uint8_t* k, const uint8_t* v, size_t page_bytes,
+                                           size_t page_scale_halves) {
+    using P = PageShape<BITS>;
+    if (page >= 0) {
+        const uint8_t* kb = k + (size_t)page * page_bytes + L.src;
+        const uint8_t* vb = v + (size_t)page * page_bytes + L.src;
+        constexpr int N = P::TILE / 512;                   // pieces per lane
+        constexpr int RPS = 32 / P::NCH;                   // token rows per step: 8, 4, 2
+#pragma unroll
+        for (int s = 0; s < N; ++s) {
+            // row = lane row + s * RPS: bits of the row below 8 toggle the position, the others move by half a chunk
+            const uint32_t d = (L.dst ^ (uint32_t)(((s * RPS) & 7) << 4)) + (uint32_t)((s * RPS) >> 3) * 128;
+            cp_async_16(slot + d, kb + (size_t)s * L.step);
+            cp_async_16(slot + P::TILE + d, vb + (size_t)s * L.step);
+        }
+        if constexpr (BITS != 16) cp_async_small<LOGG == 5 ? 8 : 4>(slot + L.sc_dst, L.sc_base + (size_t)page * page_scale_halves + L.sc_src);
+    }
+    cp_async_commit();
+}
+
+// One page: `attended` = bit mask of the token slots that take part (at least one).
+template <int BITS, int LOGG, bool WIDE>
+__device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t slot, const PageLanes& L, uint32_t attended, int lane) {
+    using P = PageShape<BITS>;
+    constexpr int ST = WarpState<BITS, WIDE>::ST;
+    constexpr bool BF = BITS == 16 && LOGG == 1;
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t kr = slot + L.rd, vr = kr + P::TILE;
+    const bool in0 = (attended >> g) & 1u, in1 = (attended >> (g + 8)) & 1u;
+
+    // ---------------- scores of tokens g, g + 8 ----------------
+    float s[ST][2];
+    float vs[2][4];                                        // V scales of the two tokens, per 32 dims
+    if constexpr (BITS == 16) {
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            uint32_t r[4];
+            ldsm4(r, (kr ^ (uint32_t)(((2 * i) & 7) << 4)) + 2 * i * 256);
+            mma_f16<BF>(c, r[0], r[1], r[2], r[3], a.qb[0][i][0], a.qb[0][i][1]);
+        }
+        s[0][0] = c[0] * a.qs[0];
+        s[0][1] = c[2] * a.qs[0];
+        if constexpr (WIDE) { s[ST - 1][0] = c[1] * a.qs[0]; s[ST - 1][1] = c[3] * a.qs[0]; }
+    } else {
+        uint32_t ks0[2], ks1[2], vs0[2], vs1[2];
+        const uint32_t sc = slot + 2 * P::TILE + g * 8;
+        lds64(ks0, sc); lds64(ks1, sc + 64); lds64(vs0, sc + 128); lds64(vs1, sc + 192);
+        float acc[ST][2];
+#pragma unroll
+        for (int x = 0; x < ST; ++x) acc[x][0] = acc[x][1] = 0.0f;
+        int c[ST][4];
+        uint32_t r[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t w[4];
+            if constexpr (BITS == 4) {
+                if (i % 2 == 0) ldsm4(r, (kr ^ (uint32_t)((2 * i) << 4)) + i * 256);
+                const uint32_t w0 = r[(i & 1) * 2], w1 = r[(i & 1) * 2 + 1];
+                w[0] = w0 & 0x0F0F0F0Fu; w[1] = w1 & 0x0F0F0F0Fu;
+                w[2] = (w0 >> 4) & 0x0F0F0F0Fu; w[3] = (w1 >> 4) & 0x0F0F0F0Fu;
+            } else {
+                ldsm4(w, (kr ^ (uint32_t)((2 * i) << 4)) + 2 * i * 256);
+            }
+#pragma unroll
+            for (int x = 0; x < ST; ++x) {
+                if (LOGG == 5 || i % 2 == 0) {
+                    c[x][0] = c[x][2] = a.c0[x][i][0];
+                    c[x][1] = c[x][3] = a.c0[x][i][1];
+                }
+                mma_u8s8(c[x], w, a.qb[x][i][0], a.qb[x][i][1]);
+                if (LOGG == 5 || i % 2 == 1) {
+                    const int gi = LOGG == 5 ? i : i / 2;
+                    const uint32_t k0 = ks0[gi / 2] & 0x7FFF7FFFu, k1 = ks1[gi / 2] & 0x7FFF7FFFu;
+                    acc[x][0] = fmaf((gi & 1) ? half_hi(k0) : half_lo(k0), (float)((c[x][0] << 8) + c[x][1]), acc[x][0]);
+                    acc[x][1] = fmaf((gi & 1) ? half_hi(k1) : half_lo(k1), (float)((c[x][2] << 8) + c[x][3]), acc[x][1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < ST; ++x) { s[x][0] = acc[x][0] * a.qs[x]; s[x][1] = acc[x][1] * a.qs[x]; }
+        if (attended != 0xFFFFu) {                         // masked slots may hold anything
+            if (!in0) vs0[0] = vs0[1] = 0u;
+            if (!in1) vs1[0] = vs1[1] = 0u;
+        }
+#pragma unroll
+        for (int w = 0; w < (LOGG == 5 ? 2 : 1); ++w) {
+            vs0[w] &= 0x7FFF7FFFu; vs1[w] &= 0x7FFF7FFFu;
+            constexpr int R = LOGG == 5 ? 1 : 2;           // 32-dim blocks per scale
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                vs[0][2 * w * R + q] = half_lo(vs0[w]); vs[0][(2 * w + 1) * R + q] = half_hi(vs0[w]);
+                vs[1][2 * w * R + q] = half_lo(vs1[w]); vs[1][(2 * w + 1) * R + q] = half_hi(vs1[w]);
+            }
+        }
+    }
+    if (attended != 0xFFFFu) {
+#pragma unroll
+        for (int x = 0; x < ST; ++x) {
+            s[x][0] = in0 ? s[x][0] : -INFINITY;
+            s[x][1] = in1 ? s[x][1] : -INFINITY;
+        }
+    }
+    // ---------------- reference maximum: moves only when a score passes it by 2^8 (or a V scale its range) ----------------
+    bool move = false;
+#pragma unroll
+    for (int x = 0; x < ST; ++x) move = move || fmaxf(s[x][0], s[x][1]) > a.m[x] + 8.0f;
+    float vmax = 0.0f;
+    if constexpr (BITS != 16) {
+        vmax = fmaxf(fmaxf(fmaxf(vs[0][0], vs[0][1]), fmaxf(vs[0][2], vs[0][3])), fmaxf(fmaxf(vs[1][0], vs[1][1]), fmaxf(vs[1][2], vs[1][3])));
+        move = move || vmax * a.vk > 128.0f;
+    }
+    if (__any_sync(0xffffffffu, move)) {
+        float f[ST];
+#pragma unroll
+        for (int x = 0; x < ST; ++x) {
+            float mx = fmaxf(s[x][0], s[x][1]);
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float mn = fmaxf(a.m[x], mx);
+            f[x] = ex2(a.m[x] - mn);                       // 0 on the first page
+            a.l[x] *= f[x];
+            a.m[x] = mn;
+        }
+        if constexpr (BITS != 16) {
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+            // the page's largest scale to [16, 32): the products p * scale (p <= 2^8) stay inside fp16, small ones stay normal
+            const float vk = fminf(a.vk == 0.0f ? INFINITY : a.vk, __uint_as_float((uint32_t)(258 - max(32, (int)(__float_as_uint(vmax) >> 23))) << 23));
+            const float fv = a.vk == 0.0f ? 0.0f : vk / a.vk;
+            a.vk = vk;
+#pragma unroll
+            for (int x = 0; x < ST; ++x) f[x] *= fv;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            a.o[i][0] *= f[0]; a.o[i][2] *= f[0];
+            a.o[i][1] *= f[ST - 1]; a.o[i][3] *= f[ST - 1];
+        }
+    }
+    float p[ST][2];
+#pragma unroll
+    for (int x = 0; x < ST; ++x) {
+        p[x][0] = ex2(s[x][0] - a.m[x]);
+        p[x][1] = ex2(s[x][1] - a.m[x]);
+        a.l[x] += p[x][0] + p[x][1];
+    }
+    // ---------------- O^T += V^T P ----------------
+    if constexpr (BITS == 16) {
+        // columns 2t, 2t + 1: p rounded and its remainder (one head per lane), or two heads and a second pass with the remainders
+        auto split = [&](float x, float& hi, float& lo) {
+            hi = BF ? __bfloat162float(__float2bfloat16_rn(x)) : __half2float(__float2half_rn(x));
+            lo = x - hi;
+        };
+        auto pack = [&](float x, float y) -> uint32_t {
+            if constexpr (BF) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+                return *reinterpret_cast<const uint32_t*>(&h);
+            } else {
+                return pack_h2(x, y);
+            }
+        };
+        float hi[ST][2], lo[ST][2];
+#pragma unroll
+        for (int x = 0; x < ST; ++x)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) split(p[x][e], hi[x][e], lo[x][e]);
+        uint32_t b[2][2];
+        if constexpr (WIDE) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                b[0][e] = movmatrix_trans(pack(hi[0][e], hi[ST - 1][e]));
+                b[1][e] = movmatrix_trans(pack(lo[0][e], lo[ST - 1][e]));
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) b[0][e] = movmatrix_trans(pack(hi[0][e], lo[0][e]));
+        }
+        const uint32_t two = attended >> (2 * t);
+        const uint32_t mask0 = ((two & 1u) ? 0xFFFFu : 0u) | ((two & 2u) ? 0xFFFF0000u : 0u);            // tokens 2t, 2t + 1
+        const uint32_t mask1 = ((two & 0x100u) ? 0xFFFFu : 0u) | ((two & 0x200u) ? 0xFFFF0000u : 0u);    // tokens 2t + 8, 2t + 9
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            uint32_t r[4];
+            ldsm4_trans(r, (vr ^ (uint32_t)(((2 * i) & 7) << 4)) + 2 * i * 256);
+            if (attended != 0xFFFFu) { r[0] &= mask0; r[2] &= mask0; r[1] &= mask1; r[3] &= mask1; }
+            mma_f16<BF>(a.o[i], r[0], r[2], r[1], r[3], b[0][0], b[0][1]);
+            if constexpr (WIDE) mma_f16<BF>(a.o[i], r[0], r[2], r[1], r[3], b[1][0], b[1][1]);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) vs[e][q] *= a.vk;
+        // operand columns 2t, 2t + 1: one head with the scales of 32-dim blocks 2c and 2c + 1, or (WIDE) two heads with one block's
+#pragma unroll
+        for (int cp = 0; cp < 2; ++cp) {                   // 64 dims
+            uint32_t b[2][2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if constexpr (WIDE) {
+                    b[0][e] = movmatrix_trans(pack_h2(p[0][e] * vs[e][2 * cp], p[ST - 1][e] * vs[e][2 * cp]));
+                    b[1][e] = LOGG == 6 ? b[0][e] : movmatrix_trans(pack_h2(p[0][e] * vs[e][2 * cp + 1], p[ST - 1][e] * vs[e][2 * cp + 1]));
+                } else {
+                    b[0][e] = movmatrix_trans(pack_h2(p[0][e] * vs[e][2 * cp], p[0][e] * vs[e][2 * cp + 1]));
+                    b[1][e] = b[0][e];
+                }
+            }
+            if constexpr (BITS == 4) {
+                uint32_t r[4];
+                ldsm4_trans(r, (vr ^ (uint32_t)((4 * cp) << 4)) + 2 * cp * 256);
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc) {           // 32 dims: this lane's 4 codes of two token pairs
+                    const uint32_t x = r[2 * cc], y = r[2 * cc + 1], x8 = x >> 8, y8 = y >> 8;
+                    mma_m16n8k16(a.o[4 * cp + 2 * cc], hsub2_u32(lop3_and_or(x, 0x000F000Fu, 0x64006400u), 0x64086408u),
+                                 hsub2_u32(lop3_and_or(x, 0x00F000F0u, 0x54005400u), 0x54805480u),
+                                 hsub2_u32(lop3_and_or(y, 0x000F000Fu, 0x64006400u), 0x64086408u),
+                                 hsub2_u32(lop3_and_or(y, 0x00F000F0u, 0x54005400u), 0x54805480u), b[cc][0], b[cc][1]);
+                    mma_m16n8k16(a.o[4 * cp + 2 * cc + 1], hsub2_u32(lop3_and_or(x8, 0x000F000Fu, 0x64006400u), 0x64086408u),
+                                 hsub2_u32(lop3_and_or(x8, 0x00F000F0u, 0x54005400u), 0x54805480u),
+                                 hsub2_u32(lop3_and_or(y8, 0x000F000Fu, 0x64006400u), 0x64086408u),
+                                 hsub2_u32(lop3_and_or(y8, 0x00F000F0u, 0x54005400u), 0x54805480u), b[cc][0], b[cc][1]);
+                }
+            } else {
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc) {           // 32 dims = chunks 4cp + 2cc and the next
+                    uint32_t r[4];
+                    ldsm4_trans(r, (vr ^ (uint32_t)((4 * cp + 2 * cc) << 4)) + (4 * cp + 2 * cc) * 256);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const uint32_t x = r[2 * q], y = r[2 * q + 1];
+                        mma_m16n8k16(a.o[4 * cp + 2 * cc + q], hsub2_u32(prmt(x, 0x64646464u, 0x4240u), 0x64806480u),
+                                     hsub2_u32(prmt(x, 0x64646464u, 0x4341u), 0x64806480u), hsub2_u32(prmt(y, 0x64646464u, 0x4240u), 0x64806480u),
+                                     hsub2_u32(prmt(y, 0x64646464u, 0x4341u), 0x64806480u), b[cc][0], b[cc][1]);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// The warp's result: for every (head of the group, dim) this lane owns, put(head, dim, weighted sum); then the statistics
+// of the heads lane g == 0 owns, stat(head, max in log2 units, sum).
+template <int BITS, bool WIDE, typename Put, typename Stat>
+__device__ __forceinline__ void emit(WarpState<BITS, WIDE>& a, int group, int lane, Put put, Stat stat) {
+    constexpr int ST = WarpState<BITS, WIDE>::ST;
+    const int g = lane >> 2, t = lane & 3;
+    const float inv = BITS == 16 ? 1.0f : (a.vk > 0.0f ? 1.0f / a.vk : 0.0f);
+#pragma unroll
+    for (int x = 0; x < ST; ++x) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) a.l[x] += __shfl_xor_sync(0xffffffffu, a.l[x], o);
+        const int head = t + 4 * x;
+        if (head >= group) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int d = BITS == 4 ? 32 * (i >> 1) + 4 * g + 2 * (i & 1) + e : BITS == 8 ? 16 * i + 2 * g + e : 16 * i + 8 * e + g;
+                float v;
+                if (WIDE) v = a.o[i][2 * e + x];
+                else if (BITS == 16) v = a.o[i][2 * e] + a.o[i][2 * e + 1];
+                else v = a.o[i][2 * e + ((i >> 1) & 1)];      // column of the block's own scales
+                put(head, d, v * inv);
+            }
+        if (g == 0) stat(head, a.m[x], a.l[x]);
+    }
+}
+
+}  // namespace attn
+}  // namespace b200q

@@ -2,7 +2,8 @@
 //
 // K_pages / V_pages [num_pages, page_size, Hkv, D], block_table [B, max_blocks], lengths [B], q [B, Hq, D]:
 // out[b, hq] = softmax(scale * q . K[b, :len_b, hq / group]) V[b, :len_b, hq / group], scores and sums in fp32.
-// The cache is four (q4: eight) times the bytes of the quantised one, so the kernel is a plain HBM streamer:
+// The general kernel: any head_dim up to 128, any page size and group (head_dim 128 on pages of 16 runs on the tensor-core
+// kernels of paged_attn.cu).  The cache is four (q4: eight) times the bytes of the quantised one, so the kernel is a plain HBM streamer:
 // grid (splits, Hkv, B); a warp takes four tokens per pass, eight lanes per token, each lane 16 consecutive
 // dimensions of the K and of the V row (two 16-byte loads each) and the running softmax state of up to four query
 // heads of the group; lanes, warps and finally the splits are merged with the usual (max, sum, weighted rows) rule.
@@ -209,10 +210,16 @@ int splits_for(int B, int Hkv, int max_blocks) {
 
 }  // namespace
 
+// paged_attn.cu: the tensor-core kernels on plain pages (head_dim 128, pages of 16)
+size_t paged_gqa_workspace_bytes_impl(int B, int Hq, int Hkv, int D);
+int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table, const int32_t* lengths,
+                               void* out, void* workspace, size_t workspace_bytes, int B, int Hq, int Hkv, int D, int page_size,
+                               int64_t num_pages, int max_blocks, float scale, int dtype, cudaStream_t stream);
+
 size_t paged_fp16_workspace_bytes_impl(int B, int Hq, int Hkv, int max_blocks) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || max_blocks <= 0) return 0;
     const int s = splits_for(B, Hkv, max_blocks);
-    return s == 1 ? 0 : (size_t)s * B * Hq * kPartStride * sizeof(float);
+    return std::max((size_t)s * B * Hq * kPartStride * sizeof(float), paged_gqa_workspace_bytes_impl(B, Hq, Hkv, 128));
 }
 
 int paged_fp16_gqa_decode_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table,
@@ -225,13 +232,17 @@ int paged_fp16_gqa_decode_impl(const void* q, const void* k_pages, const void* v
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || D <= 0 || page_size <= 0 || num_pages <= 0 || max_blocks <= 0)
         return B200Q_ERR_BAD_ARG;
     if (D > 128 || (dtype != B200Q_F16 && dtype != B200Q_BF16) || Hkv > 65535 || B > 65535) return B200Q_ERR_UNSUPPORTED;
+    // a workspace too small for the split-KV kernels (a caller that knows this kernel's own need) stays here
+    const int rc0 = paged_plain_attention_impl(q, k_pages, v_pages, block_table, lengths, out, workspace, workspace_bytes, B, Hq, Hkv, D,
+                                               page_size, num_pages, max_blocks, scale, dtype, stream);
+    if (rc0 != B200Q_ERR_UNSUPPORTED && rc0 != B200Q_ERR_WORKSPACE) return rc0;
     Fp16AttnParams p = {};
     p.q = q; p.k_pages = k_pages; p.v_pages = v_pages; p.block_table = block_table; p.lengths = lengths; p.out = out;
     p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.P = page_size; p.max_blocks = max_blocks; p.dtype = dtype;
     p.num_pages = num_pages; p.scale = scale;
     p.splits = splits_for(B, Hkv, max_blocks);
     if (p.splits > 1) {
-        const size_t need = paged_fp16_workspace_bytes_impl(B, Hq, Hkv, max_blocks);
+        const size_t need = (size_t)p.splits * B * Hq * kPartStride * sizeof(float);
         if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0)
             return B200Q_ERR_WORKSPACE;
         p.workspace = reinterpret_cast<float*>(workspace);

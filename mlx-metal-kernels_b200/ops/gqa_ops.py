@@ -43,6 +43,10 @@ def paged_gqa_decode_attention(q, K_pages, V_pages, block_table, lengths=None, s
     import torch
 
     from . import _cabi, paged_kv_ops
+    if backend == "cuda" and lengths is not None:
+        out = _cabi.host().plain_attention(q, K_pages, V_pages, block_table, lengths, scale)
+        if out is not None:
+            return out
     if K_pages.ndim != 4 or V_pages.ndim != 4 or K_pages.shape != V_pages.shape:
         raise ValueError(f"K_pages and V_pages must match [NUM_PAGES,PAGE_SIZE,Hkv,D], got {tuple(K_pages.shape)}, {tuple(V_pages.shape)}")
     if block_table.ndim != 2:

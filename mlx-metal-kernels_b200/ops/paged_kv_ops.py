@@ -130,6 +130,10 @@ def paged_decode_attention(q, K_pages, V_pages, block_table, lengths, *, scale=N
     """Decode attention over an fp16 / bf16 paged cache, q [B,1,H,D] with as many query as kv heads
     (ops/paged_kv_ops.py:307-360 of the reference; for Hq != Hkv see ``paged_gqa_decode_attention``).  Every Metal
     backend name selects the one CUDA kernel."""
+    if backend == "cuda" and lengths is not None and q.ndim == 4 and K_pages.ndim == 4 and q.shape[2] == K_pages.shape[2]:
+        out = _cabi.host().plain_attention(q, K_pages, V_pages, block_table, lengths, scale)
+        if out is not None:
+            return out
     NUM_PAGES, PAGE_SIZE, H, D, B, MAX_BLOCKS = _validate_page_tensors(K_pages, V_pages, block_table)
     if q.ndim != 4 or tuple(q.shape) != (B, 1, H, D):
         raise ValueError(

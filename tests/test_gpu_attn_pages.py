@@ -1,0 +1,94 @@
+"""Decode attention through the page building blocks (quantised and plain pages) where they can go wrong: both layouts of the
+query heads, bf16 queries, chunks of kv heads, a maximum that keeps moving, V scales far apart, and slots past the length
+that hold anything at all."""
+import pytest
+import torch
+
+from helpers import cabi, pq_ops, synth
+import importlib
+
+gqa_ops = importlib.import_module("mlx_metal_kernels_b200.ops.gqa_ops")
+pytestmark = pytest.mark.gpu
+
+
+def _expected(q, k, v, table, lengths):
+    """softmax(q k / sqrt(D)) v in fp64 over the first lengths[b] tokens, from dequantised pages [pages, 16, Hkv, D]."""
+    B, _, Hq, D = q.shape
+    Hkv = k.shape[2]
+    out = torch.zeros(B, 1, Hq, D, dtype=torch.float64)
+    for b in range(B):
+        L = int(lengths[b])
+        if L == 0:
+            continue
+        pages = table[b, :(L + 15) // 16].long()
+        kb, vb = (t[pages].reshape(-1, Hkv, D)[:L].double().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+        p = torch.softmax(torch.einsum("hd,lhd->hl", q[b, 0].double(), kb) / D ** 0.5, -1)
+        out[b, 0] = torch.einsum("hl,lhd->hd", p, vb)
+    return out
+
+
+def _table(lengths, pages, seed):
+    g = torch.Generator().manual_seed(seed)
+    perm = torch.randperm(pages, generator=g).to(torch.int32)
+    table = torch.full((len(lengths), max(1, (max(lengths) + 15) // 16)), -1, dtype=torch.int32)
+    at = 0
+    for b, n in enumerate(lengths):
+        m = (n + 15) // 16
+        table[b, :m] = perm[at:at + m]
+        at += m
+    return table
+
+
+@pytest.mark.parametrize("bits,G", [(4, 32), (4, 64), (8, 32), (8, 64)])
+@pytest.mark.parametrize("Hq,Hkv,lengths", [(8, 1, [1, 300, 17]), (16, 2, [16, 33]), (12, 2, [700]), (6, 3, [129, 5]), (32, 16, [40, 0, 250]),
+                                            (32, 8, [2000] * 9)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_quantised_pages(cuda, bits, G, Hq, Hkv, lengths, dtype):
+    pages = sum((n + 15) // 16 for n in lengths) + 3
+    table, ln = _table(lengths, pages, 1), torch.tensor(lengths, dtype=torch.int32)
+    k, v = (synth.activations((pages, 16, Hkv, 128), s) for s in (11, 12))
+    # scores that grow along the sequence: the reference maximum moves again and again; V of one page far larger than the rest
+    for b, n in enumerate(lengths):
+        m = (n + 15) // 16
+        k[table[b, :m].long()] *= torch.linspace(0.2, 3.0, max(m, 1))[:m].half().reshape(-1, 1, 1, 1)
+        if m > 2:
+            v[table[b, 2].long()] *= 200.0
+    q = synth.activations((len(lengths), 1, Hq, 128), 13, "cpu", dtype)
+    cache = pq_ops.quantize_kv_pages(k.to(cuda), v.to(cuda), table.to(cuda), ln.to(cuda), pq_ops.PagedQuantizedKVConfig(bits=bits, group_size=G))
+    kd, vd = (t.cpu() for t in pq_ops.dequantize_kv_pages(cache))
+    for b, n in enumerate(lengths):                       # scales of slots past the length: anything
+        if n % 16:
+            for t in (cache.k_scales, cache.v_scales):
+                t[int(table[b, n // 16]), n % 16:] = float("nan")
+    want = _expected(q, kd, vd, table, ln)
+    tol = 2e-3 if dtype == torch.float16 else 8e-3
+    for cluster in (-1, 1):
+        cabi.set_tuning("attn.cluster", cluster)
+        try:
+            got = pq_ops.paged_quantized_kv_gqa_decode_attention(q.to(cuda), cache, backend="cuda").cpu().double()
+        finally:
+            cabi.set_tuning("attn.cluster", 0)
+        assert (got - want).abs().max() <= tol * max(1.0, want.abs().max())
+    assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Hq,Hkv,lengths", [(8, 8, [1, 300, 17]), (16, 2, [16, 33]), (4, 1, [700, 0]), (6, 3, [129, 5]), (40, 8, [513]), (64, 16, [31] * 5)])
+def test_plain_pages(cuda, dtype, Hq, Hkv, lengths):
+    pages = sum((n + 15) // 16 for n in lengths) + 3
+    table, ln = _table(lengths, pages, 2), torch.tensor(lengths, dtype=torch.int32)
+    k, v = (synth.activations((pages, 16, Hkv, 128), s, "cpu", dtype) for s in (21, 22))
+    q = synth.activations((len(lengths), 1, Hq, 128), 23, "cpu", dtype)
+    want = _expected(q, k, v, table, ln)
+    for b, n in enumerate(lengths):                       # slots past the length may hold anything
+        if n % 16:
+            for t in (k, v):
+                t[int(table[b, n // 16]), n % 16:] = float("nan")
+    args = [t.to(cuda) for t in (q, k, v, table, ln)]
+    got = gqa_ops.paged_gqa_decode_attention(*args).cpu().double()
+    assert (got - want).abs().max() <= (2e-3 if dtype == torch.float16 else 1.6e-2)
+    assert cabi.host().plain_attention(*args, None) is not None
+    bad = args[4].clone()
+    bad[0] = 10 ** 6
+    with pytest.raises(ValueError, match="positions must be in"):
+        gqa_ops.paged_gqa_decode_attention(*args[:4], bad)

@@ -1,0 +1,49 @@
+"""The integer tensor-core matvec (one to four rows) against the oracle: unit, tile and group remainders, both row types, zero
+points absent, the fused norm and residual, values that stress its fixed-point activations, and row shards bit for bit."""
+import pytest
+import torch
+
+from helpers import cabi, mlp_ops, quant_ops, rel_l2, synth, to_dev
+from oracle import quant_ops as oq
+
+pytestmark = pytest.mark.gpu
+
+
+def _ref(bits):
+    return oq.reference_q4_matvec_decode if bits == 4 else oq.reference_q8_matvec_decode
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("B,N,K,G", [(1, 1, 64, 32), (2, 17, 64, 64), (3, 333, 2592, 32), (4, 150, 640, 64), (1, 4097, 1024, 128),
+                                     (2, 600, 4096, 64), (4, 260, 4096, 32), (1, 64, 14336, 64), (1, 40000, 128, 64), (3, 2000, 384, 128)])
+def test_shapes(cuda, bits, B, N, K, G):
+    w, s, z = synth.quantized_weight(N, K, bits, G, seed=N + K)
+    for dtype, tol in ((torch.float16, 1e-3), (torch.bfloat16, 6e-3)):
+        x = synth.activations((B, K), 7, "cpu", dtype)
+        for zeros in (z, None):
+            want = _ref(bits)(x, w, s, zeros, group_size=G)
+            got = quant_ops.matvec_rows(bits, *to_dev(cuda, x, w, s, zeros), G)
+            assert rel_l2(got, want) <= tol
+    assert cabi.device_status() == 0
+
+
+def test_outliers_and_empty_groups(cuda):
+    """Groups of zeros, an outlier of 2^14 beside small values, and the smallest normal halves."""
+    w, s, z = synth.quantized_weight(256, 1024, 4, 64, seed=3)
+    x = synth.activations((2, 1024), 9)
+    x[0, :64] = 0
+    x[0, 70] = 16384.0
+    x[1] *= 2.0 ** -14
+    want = _ref(4)(x, w, s, z, group_size=64)
+    got = quant_ops.matvec_rows(4, *to_dev(cuda, x, w, s, z), 64)
+    assert rel_l2(got[:1], want[:1]) <= 1e-3 and rel_l2(got[1:], want[1:]) <= 6e-3      # the second row's results are subnormal halves
+
+
+@pytest.mark.parametrize("rows", [1, 2, 4])
+@pytest.mark.parametrize("lo,hi", [(0, 96), (96, 333), (5, 6)])
+def test_row_shards_reproduce_the_unsharded_rows(cuda, rows, lo, hi):
+    w, s, z = (t.to(cuda) for t in synth.quantized_weight(333, 1024, 4, 64, seed=5))
+    x = synth.activations((rows, 1024), 6, cuda)
+    full = quant_ops.matvec_rows(4, x, w, s, z, 64)
+    part = quant_ops.matvec_rows(4, x, w[lo:hi].contiguous(), s[lo:hi].contiguous(), z[lo:hi].contiguous(), 64)
+    assert torch.equal(part, full[:, lo:hi])
