@@ -20,8 +20,10 @@
 // row (512 q4 or 256 q8 codes), units are dealt to the 16 warps in order.  A warp is on its own: every lane copies 16-byte pieces
 // with cp.async into a private ring (4 KB of codes per warp in flight, 64 KB per SM, started before griddepcontrol.wait since
 // weights do not depend on the previous kernel): no producer warps and no barriers in the stream.  While piece c of a unit is
-// consumed, piece c of the warp's next unit takes its place, so all shared-memory addresses are constants.  For one or two rows the
-// CTA stays below half of an SM, so that the next kernel of a dependent chain can be resident and loading while this one drains.
+// consumed, piece c of the warp's next unit takes its place, so all shared-memory addresses are constants.  (Twice the
+// ring in flight gained nothing: 2 x 14336 x 4096 15.7 against 14.9 us, the decode step 1.80 against 1.73 ms.)
+// One CTA per SM, by its shared memory: with room for two, the CTAs of the next kernel of a dependent chain start beside this
+// one's, and later ones then share an SM while another SM has none (gate/up and down of one row in turn: 36 us against 26.8).
 // The units' sums meet in shared memory and are added in k order: the order does not depend on the CTA, the tile or the
 // number of rows, so a tensor-parallel shard reproduces the unsharded rows bit for bit.
 //
@@ -39,6 +41,7 @@ namespace {
 constexpr int kI8Warps = 16;
 constexpr int kI8Threads = kI8Warps * 32;
 constexpr int kI8UnitBytes = 256;             // bytes of a unit in one row: four 64-byte pieces
+constexpr uint32_t kI8OnePerSm = 116 * 1024;  // shared memory that keeps a second CTA off the SM
 constexpr int kI8MaxRes = 1024;               // residual values kept in shared memory
 
 struct I8Params {
@@ -235,7 +238,7 @@ template <int BITS, int LOGG> struct I8Shape {
 };
 
 template <int BITS, int LOGG, int NB, bool PACKETS>
-__global__ void __launch_bounds__(kI8Threads, NB <= 2 ? 2 : 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
+__global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
     using S = I8Shape<BITS, LOGG>;
     constexpr int G = S::G, GB = S::GB, NM = S::NM, GU = S::GU, CP = S::CP, CH = S::CH, CG = S::CG, MB = S::MB, WIN = S::WIN;
@@ -607,7 +610,7 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
     p.off_part = off;  off += i8_align((uint32_t)(p.batch * tile_bytes), 128);
     p.off_meta = off;  off += kI8Warps * 2 * p.meta_slot;
     off = i8_align(off, 1024);
-    p.off_ring = off;  off += kI8Warps * 4096;
+    p.off_ring = off;  off = std::max<uint32_t>(off + kI8Warps * 4096, kI8OnePerSm);
     if (off > (uint32_t)max_smem_optin()) return B200Q_ERR_UNSUPPORTED;
 
     const bool packets = p.tp_in.world > 0 && p.tp_in.packets;

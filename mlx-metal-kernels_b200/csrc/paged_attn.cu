@@ -141,12 +141,32 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
     const int lane = threadIdx.x & 31;
     int* prefix = reinterpret_cast<int*>(smem + p.off_prefix);   // [B + 1]
 
-    pdl_launch_dependents();
     pdl_wait();   // lengths / block table / q / the cache itself may be produced by the previous kernel
+    pdl_launch_dependents();      // after the wait: the merge kernel may read the lengths before this kernel ends
 
     // The flattened page list is cut into p.grid equal ranges.  A CTA has 8 warps = 8 (range, kv head) pairs:
-    // with 8 kv heads one range, with fewer heads several consecutive ranges (subs of them).
-    const int total = build_prefix(p, prefix);
+    // with 8 kv heads one range, with fewer heads several consecutive ranges (subs of them).  Up to 32 sequences, every warp
+    // keeps their lengths and page counts in its lanes: one load and a scan, no shared memory and no barrier.
+    const bool small = p.B <= 32;
+    const int cap = p.max_blocks * p.P;
+    int len_l = 0, pre_l = 0, total;                             // lane b: length of sequence b, pages before it
+    if (small) {
+        int n = 0;
+        if (lane < p.B) {
+            len_l = p.lengths[lane];
+            n = seq_pages(len_l, cap, p.P, p.sink, p.window).n;
+        }
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        pre_l = incl - n;
+        total = __shfl_sync(0xffffffffu, incl, 31);
+    } else {
+        total = build_prefix(p, prefix);
+    }
     const int ppc = (total + p.grid - 1) / p.grid;               // pages per range
     const int subs = p.subs;
     const int h = blockIdx.y * p.hc + warp % p.hc;               // kv head of this warp
@@ -163,24 +183,34 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
 
     WarpState<BITS, WIDE> acc;
     state_reset(acc);
-    int cur_b = -1;
 
     // Page descriptors (page id, sequence, valid tokens) of 32 consecutive pages of this warp, one per
     // lane.  Two windows: one for the page being consumed, one for the page being issued ahead.
     struct Desc { int page, b, attended; };   // attended: bit mask of the page's slots
     auto lookup = [&](int base) -> Desc {
         const int j = base + lane;
-        Desc d = {-1, 0, 0};
+        const int f = min(lo + j, hi - 1);
+        int b = 0, len, before;
+        if (small) {                           // largest b with pages before it <= f
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const int v = __shfl_sync(0xffffffffu, pre_l, b + step);
+                if (b + step < p.B && v <= f) b += step;
+            }
+            len = __shfl_sync(0xffffffffu, len_l, b);
+            before = __shfl_sync(0xffffffffu, pre_l, b);
+        } else {
+            b = find_sequence(prefix, p.B, f);
+            len = p.lengths[b];
+            before = prefix[b];
+        }
+        Desc d = {-1, b, 0};
         if (j < n_my) {
-            const int f = lo + j;
-            const int b = find_sequence(prefix, p.B, f);
-            const SeqPages sp = seq_pages(p.lengths[b], p.max_blocks * p.P, p.P, p.sink, p.window);
-            const int idx = f - prefix[b];
+            const SeqPages sp = seq_pages(len, cap, p.P, p.sink, p.window);
+            const int idx = f - before;
             const int pg = idx < sp.sink_pages ? idx : sp.first_recent + (idx - sp.sink_pages);
-            int page = p.block_table[(int64_t)b * p.max_blocks + pg];
-            if (page < 0 || page >= p.num_pages) page = -1;
-            d.page = page;
-            d.b = b;
+            const int page = p.block_table[(int64_t)b * p.max_blocks + pg];
+            d.page = (page < 0 || page >= p.num_pages) ? -1 : page;
             d.attended = (int)page_mask16(pg, sp.L, p.sink, p.window);
         }
         return d;
@@ -212,6 +242,13 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
         else { cp_async_commit(); slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1; }
     }
 
+    // the first sequence's queries, while the copies are in flight
+    auto queries = [&](int b) {
+        load_queries<BITS, LOGG>(acc, reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D, group, p.q_dtype, p.scale, lane);
+    };
+    int cur_b = __shfl_sync(0xffffffffu, win_c.b, 0);
+    queries(cur_b);
+
     int slot_c = 0;     // ring slot of the page being consumed
     for (int j = 0; j < n_my; ++j) {
         if (j > 0 && (j & 31) == 0) win_c = lookup(j);
@@ -225,17 +262,16 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
         __syncwarp();
 
         if (b != cur_b) {
-            if (cur_b >= 0) flush(cur_b);
+            flush(cur_b);
             cur_b = b;
             state_reset(acc);
-            load_queries<BITS, LOGG>(acc, reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D, group, p.q_dtype,
-                                     p.scale, lane);
+            queries(b);
         }
         if (page >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, L, attended, lane);
         __syncwarp();   // every lane is done with this slot before it is refilled
         slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
     }
-    if (cur_b >= 0) flush(cur_b);
+    flush(cur_b);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -302,6 +338,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     const int c_lo = min(n_pages, (int)rank * ppc), c_hi = min(n_pages, c_lo + ppc);
     const int ppw = (c_hi - c_lo + kAttnWarps - 1) / kAttnWarps;         // pages per warp
     const int lo = min(c_hi, c_lo + warp * ppw), hi = min(c_hi, lo + ppw);
+
+    const int n_my = hi - lo;
+    auto page_ids = [&](int base) -> int {
+        const int j = base + lane;
+        const int page = j < n_my ? p.block_table[(size_t)b * p.max_blocks + lo + j] : -1;
+        return page >= p.num_pages ? -1 : page;
+    };
 
     if (p.fused) {
         const int heads = p.Hq + 2 * p.Hkv;
@@ -381,32 +424,34 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     // ---- this warp's pages ----
     WarpState<BITS, WIDE> acc;
     state_reset(acc);
-    const int n_my = hi - lo;
     if (n_my > 0) {
         const void* qrows = p.fused ? (const void*)qs : (const void*)(reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D);
         const PageLanes Lp = page_lanes<BITS>(lane, h, (uint32_t)p.row_bytes, p.scale_row_halves, p.Gd, p.k_scales, p.v_scales);
         const size_t page_code_bytes = (size_t)p.P * p.row_bytes;
         const size_t page_scale_halves = (size_t)p.P * p.scale_row_halves;
         const uint32_t my_ring = smem_u32(smem) + p.off_ring + (uint32_t)warp * (NS * SLOT);
-        auto page_of = [&](int j) -> int {
-            int page = p.block_table[(size_t)b * p.max_blocks + lo + j];
-            return (page < 0 || page >= p.num_pages) ? -1 : page;
-        };
+        int ids_c = page_ids(0), ids_i = ids_c;                  // page ids of 32 consecutive pages, one per lane: consumed / issued window
         int slot_i = 0, slot_c = 0;
         auto issue = [&](int j) {
-            if (j < n_my) issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, Lp, page_of(j), p.k_codes, p.v_codes, page_code_bytes, page_scale_halves);
-            else cp_async_commit();
+            if (j < n_my) {
+                if (j > 0 && (j & 31) == 0) ids_i = page_ids(j);
+                issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, Lp, __shfl_sync(0xffffffffu, ids_i, j & 31), p.k_codes, p.v_codes,
+                                       page_code_bytes, page_scale_halves);
+            } else {
+                cp_async_commit();
+            }
             slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1;
         };
         for (int j = 0; j < NS - 1; ++j) issue(j);
         load_queries<BITS, LOGG>(acc, qrows, group, p.fused ? B200Q_F16 : p.q_dtype, p.scale, lane);
         for (int j = 0; j < n_my; ++j) {
+            if (j > 0 && (j & 31) == 0) ids_c = page_ids(j);
             issue(j + NS - 1);
             cp_async_wait<NS - 1>();
             __syncwarp();
             const int valid = min(p.P, L - (lo + j) * p.P);
             const uint32_t attended = valid >= 16 ? 0xFFFFu : ((1u << max(valid, 0)) - 1u);
-            if (page_of(j) >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, Lp, attended, lane);
+            if (__shfl_sync(0xffffffffu, ids_c, j & 31) >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, Lp, attended, lane);
             __syncwarp();
             slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
         }
@@ -485,96 +530,72 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
 
 // Merges the partials of every (sequence, query head): one warp each, lanes over d.
 
-// One CTA per (sequence, query head).  The partials of a sequence may sit in every CTA slot of the
-// main kernel (a single long sequence is cut over the whole grid), so the slots are spread over the
-// CTA's warps and their loads are independent of one another; lanes cover the head dimension.
-// kMergeWarps: 32 for short batches (few CTAs, up to ~300 candidates each: four loads in flight per warp cover
-// them in one or two rounds), 8 for long batches (many CTAs with a dozen candidates each).
+// One CTA per (sequence, query head).  The partials of a sequence may sit in every range of the
+// main kernel (a single long sequence is cut over the whole grid), so the ranges are spread over the
+// CTA's warps; lanes cover the head dimension.  The lengths are known before the main kernel ends, so everything but the
+// partials themselves is worked out ahead of griddepcontrol.wait; a warp then loads maximum, sum and row of its ranges
+// at once and rescales as it goes (16 ragged sequences of 32 heads: 7 -> 4.9 us after the main kernel's end).
+// kMergeWarps: 32 for short batches (few CTAs, up to ~300 ranges each), 8 for long batches (many CTAs with a dozen each).
 template <int kMergeWarps>
 __global__ void __launch_bounds__(kMergeWarps * 32) paged_attn_merge_kernel(const __grid_constant__ AttnParams p) {
     __shared__ float red[kMergeWarps][128];
     __shared__ float red_s[2][kMergeWarps];
-    __shared__ int red_i[2][kMergeWarps];
-    __shared__ int cand_off[kMaxRanges];            // candidates: page ranges of the main kernel that touch this sequence
-    __shared__ float cand_m[kMaxRanges];
     const int D = p.D;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int b = blockIdx.x / p.Hq;
     const int hq = blockIdx.x - b * p.Hq;
-    pdl_wait();
 
-    // pages before sequence b and in total (the flattened page list of the main kernel)
+    // pages before sequence b and in total (the flattened page list of the main kernel); every warp for itself
     const int cap = p.max_blocks * p.P;
-    int below = 0, all = 0;
-    for (int i = threadIdx.x; i < p.B; i += kMergeWarps * 32) {
-        const int n = seq_pages(p.lengths[i], cap, p.P, p.sink, p.window).n;
+    int below = 0, all = 0, mine = 0;
+    for (int i = lane; i < p.B; i += 32) {
+        const int n = seq_pages(__ldcg(p.lengths + i), cap, p.P, p.sink, p.window).n;
         all += n;
         if (i < b) below += n;
+        if (i == b) mine = n;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        below += __shfl_xor_sync(0xffffffffu, below, o);
-        all += __shfl_xor_sync(0xffffffffu, all, o);
-    }
-    if (lane == 0) { red_i[0][warp] = below; red_i[1][warp] = all; }
-    __syncthreads();
-    below = 0; all = 0;
-#pragma unroll
-    for (int w = 0; w < kMergeWarps; ++w) { below += red_i[0][w]; all += red_i[1][w]; }
-    const int total = all;
-    const int s_lo = below;
-    const int s_hi = below + seq_pages(p.lengths[b], cap, p.P, p.sink, p.window).n;
-    const int ppc = (total + p.grid - 1) / p.grid;
+    below = __reduce_add_sync(0xffffffffu, below);
+    all = __reduce_add_sync(0xffffffffu, all);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    const int ppc = (all + p.grid - 1) / p.grid;
+    pdl_wait();
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float l_part = 0.0f;
-    if (s_hi > s_lo) {
-        const int c_first = s_lo / ppc, c_last = (s_hi - 1) / ppc;
-        const int n_cand = c_last - c_first + 1;
-        // Every range c_first..c_last holds at least one page of b, i.e. wrote a partial into slot c + b.
-        // Pass 1 (one candidate per thread): the offset of the partial and its running maximum, kept in shared
-        // memory so that pass 2 is free of index arithmetic.
-        float m_tot = -INFINITY;
-        for (int i = threadIdx.x; i < n_cand; i += kMergeWarps * 32) {
-            const int off = ((c_first + i + b) * p.Hq + hq) * (D + 2);
-            const float m = p.partial[(size_t)off + D];
-            cand_off[i] = off;
-            cand_m[i] = m;
-            m_tot = fmaxf(m_tot, m);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m_tot = fmaxf(m_tot, __shfl_xor_sync(0xffffffffu, m_tot, o));
-        if (lane == 0) red_s[0][warp] = m_tot;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < kMergeWarps; ++w) m_tot = fmaxf(m_tot, red_s[0][w]);
-
+    float l_part = 0.0f, m_run = -INFINITY;
+    if (mine > 0) {
+        // every range c_first..c_last holds at least one page of b, i.e. wrote a partial into slot c + b
+        const int c_first = below / ppc, c_last = (below + mine - 1) / ppc;
 #pragma unroll 4
-        for (int i = warp; i < n_cand; i += kMergeWarps) {
-            const int off = cand_off[i];
-            const float m = cand_m[i];
-            const bool ok = off >= 0 && m != -INFINITY;
-            const float* src = p.partial + (ok ? off : 0);
-            const float w = ok ? exp2f(m - m_tot) : 0.0f;      // the maxima are in log2 units
-            const float l = ok ? src[D + 1] : 0.0f;
-            l_part = fmaf(w, l, l_part);
+        for (int c = c_first + warp; c <= c_last; c += kMergeWarps) {
+            const float* src = p.partial + ((size_t)(c + b) * p.Hq + hq) * (D + 2);
+            const float m = src[D], l = src[D + 1];
+            float v[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int d = lane + 32 * j;
-                const float v = (ok && d < D) ? src[d] : 0.0f;
-                acc[j] = fmaf(w, v, acc[j]);
-            }
+            for (int j = 0; j < 4; ++j) v[j] = lane + 32 * j < D ? src[lane + 32 * j] : 0.0f;
+            if (m == -INFINITY) continue;
+            const float mn = fmaxf(m_run, m);                    // the maxima are in log2 units
+            const float f = exp2f(m_run - mn), w = exp2f(m - mn);
+            m_run = mn;
+            l_part = fmaf(w, l, l_part * f);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[j] = fmaf(w, v[j], acc[j] * f);
         }
     }
+    if (lane == 0) { red_s[0][warp] = m_run; red_s[1][warp] = l_part; }
 #pragma unroll
     for (int j = 0; j < 4; ++j) red[warp][lane + 32 * j] = acc[j];
-    if (lane == 0) red_s[1][warp] = l_part;
     __syncthreads();
     if (threadIdx.x < D) {
-        float sum = 0.0f, l_tot = 0.0f;
+        float m_tot = -INFINITY, sum = 0.0f, l_tot = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kMergeWarps; ++w) { sum += red[w][threadIdx.x]; l_tot += red_s[1][w]; }
+        for (int w = 0; w < kMergeWarps; ++w) m_tot = fmaxf(m_tot, red_s[0][w]);
+#pragma unroll
+        for (int w = 0; w < kMergeWarps; ++w) {
+            const float f = red_s[0][w] == -INFINITY ? 0.0f : exp2f(red_s[0][w] - m_tot);
+            sum = fmaf(f, red[w][threadIdx.x], sum);
+            l_tot = fmaf(f, red_s[1][w], l_tot);
+        }
         const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
         const size_t o = ((size_t)b * p.Hq + hq) * D + threadIdx.x;
         const unsigned short bits16 = p.q_dtype == B200Q_F16 ? __half_as_ushort(__float2half_rn(sum * inv))

@@ -24,7 +24,7 @@ namespace attn {
 
 constexpr int kHeadDim = 128;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kQLevels = 32639.0f;          // largest 16-bit value whose high digit still fits a signed byte
+constexpr float kQLevels = 32638.0f;          // the largest 16-bit value whose high digit still fits a signed byte, less one for the product's rounding
 
 // BITS: 4, 8 (codes) or 16 (plain).  LOGG: log2 of the scale group, 5 or 6; for plain pages 0 = fp16, 1 = bf16.
 template <int BITS> struct PageShape {
@@ -56,6 +56,11 @@ __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+__device__ __forceinline__ void mma_u8s8_start(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0, int c1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1));
 }
 __device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -152,7 +157,7 @@ __device__ __forceinline__ void load_queries(WarpState<BITS, WIDE>& a, const voi
                 uint32_t dig[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const int x = __float2int_rn(fminf(fmaxf(v[i][j] * up, -kQLevels), kQLevels));
+                    const int x = __float2int_rn(v[i][j] * up);
                     const int hi = (x + 128) >> 8;
                     dig[j] = (uint32_t)((g & 1) ? x - (hi << 8) : hi) & 0xFFu;
                 }
@@ -270,11 +275,8 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
             }
 #pragma unroll
             for (int x = 0; x < ST; ++x) {
-                if (LOGG == 5 || i % 2 == 0) {
-                    c[x][0] = c[x][2] = a.c0[x][i][0];
-                    c[x][1] = c[x][3] = a.c0[x][i][1];
-                }
-                mma_u8s8(c[x], w, a.qb[x][i][0], a.qb[x][i][1]);
+                if (LOGG == 5 || i % 2 == 0) mma_u8s8_start(c[x], w, a.qb[x][i][0], a.qb[x][i][1], a.c0[x][i][0], a.c0[x][i][1]);
+                else mma_u8s8(c[x], w, a.qb[x][i][0], a.qb[x][i][1]);
                 if (LOGG == 5 || i % 2 == 1) {
                     const int gi = LOGG == 5 ? i : i / 2;
                     const uint32_t k0 = ks0[gi / 2] & 0x7FFF7FFFu, k1 = ks1[gi / 2] & 0x7FFF7FFFu;

@@ -218,6 +218,7 @@ int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v
 
 size_t paged_fp16_workspace_bytes_impl(int B, int Hq, int Hkv, int max_blocks) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || max_blocks <= 0) return 0;
+    if (max_blocks == 1) return 0;      // one page per sequence: the general kernel in one CTA per kv head
     const int s = splits_for(B, Hkv, max_blocks);
     return std::max((size_t)s * B * Hq * kPartStride * sizeof(float), paged_gqa_workspace_bytes_impl(B, Hq, Hkv, 128));
 }

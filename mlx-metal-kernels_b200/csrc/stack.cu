@@ -172,15 +172,6 @@ struct KvPair {
     void* scales[2];      // written by the quantiser, read by the dequantiser
 };
 
-// rint(v / scale) through the reciprocal.  The product differs from the correctly rounded quotient by less than
-// 2^-15 at magnitudes up to 128, so it rounds to the same integer unless it lies that close to a tie; there the quotient is taken.
-__device__ __forceinline__ float rint_quotient(float v, float scale, float inv) {
-    const float t = v * inv;
-    const float n = rintf(t);
-    if (fabsf(fabsf(t - n) - 0.5f) < 1e-3f) return rintf(__fdiv_rn(v, scale));
-    return n;
-}
-
 template <typename T, int BITS>
 __global__ void __launch_bounds__(256) quantize_kv_vec_kernel(const __grid_constant__ KvPair p, int64_t pieces, int log_lanes) {
     const T* in = reinterpret_cast<const T*>(p.in[blockIdx.y]);
@@ -207,9 +198,23 @@ __global__ void __launch_bounds__(256) quantize_kv_vec_kernel(const __grid_const
         for (int o = 1; o < (1 << log_lanes); o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float scale = __fdiv_rn(fmaxf(mx, 1e-8f), limit);
         const float inv = __fdiv_rn(1.0f, scale);
+        // rint(v / scale) through the reciprocal: v * inv differs from the correctly rounded quotient by less than 2^-15 (|quotients|
+        // stay below 128), so it rounds to the same integer unless it lies that close to a tie.  Adding 1.5 2^23 + offset rounds to
+        // nearest even and leaves the code in the low byte.  Pieces with a value near a tie, or not finite, are done over by division.
         uint32_t c[8];
+        float far = 0.0f, odd = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) c[k] = (uint32_t)(int)(fminf(fmaxf(rint_quotient(v[k], scale, inv), -limit), limit) + offset);
+        for (int k = 0; k < 8; ++k) {
+            const float t = v[k] * inv;
+            const float r = t + (12582912.0f + offset);
+            far = fmaxf(far, fabsf(t - (r - (12582912.0f + offset))));
+            odd = fmaf(t, 0.0f, odd);                      // NaN when t is not finite
+            c[k] = __float_as_uint(r) & 0xFFu;
+        }
+        if (far > 0.4999f || odd != 0.0f) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c[k] = (uint32_t)(int)(fminf(fmaxf(rintf(__fdiv_rn(v[k], scale)), -limit), limit) + offset);
+        }
         if (i >= pieces) continue;
         if (BITS == 8) {
             reinterpret_cast<uint2*>(p.out[blockIdx.y])[i] = make_uint2(c[0] | (c[1] << 8) | (c[2] << 16) | (c[3] << 24),
