@@ -57,13 +57,11 @@ int b200q_device_status(int reset, void* stream);
  *   "gemv.ts"            1 = every matvec the tcgen05 kernel supports goes to it, -1 = none, 0 = by batch
  *   "gemv.ts_min_batch"  smallest batch the tcgen05 kernel takes when "gemv.ts" is 0
  *   "gemv.i8"            -1 = batches of one to four rows do not use the integer tensor-core kernel
- *   "gemv.fuse_norm"     1 = the tcgen05 kernel computes a requested rmsnorm in its own prologue even when the caller
- *                        gave a buffer for the normalised rows (default: a launch of the row kernel in front of it)
  *   "gemv.force_generic" 1 = always the one-warp-per-row kernel that follows the reference arithmetic literally
  *   "gemv.stage_k", "gemv.stages", "gemv.smem_kb", "gemv.interleave"   ring geometry, shared-memory budget and row
  *                        dealing of the mma.sync kernel
- *   "ts.stages", "ts.smem_kb", "ts.split", "ts.big"     ring depth, shared-memory budget, K split, shape of the tcgen05 kernel
- *   "ts.slow_reduce"     1 = the partial sums of a K split always travel through the first CTA's weight ring
+ *   "ts.stages", "ts.split"     ring depth and K split (1, 2, 4, 8) of the tcgen05 kernel
+ *   "ts.slow_reduce"     1 = the partial sums of a K split always travel through the first CTA's rings
  *   "ts.tp_world"        number of equal row shards the matrices of this process are split into (tensor parallelism):
  *                        the tcgen05 kernel then splits K, and the attention picks its kernel, as the unsharded call
  *                        would, which keeps a shard's rows bit-identical to the unsharded result
@@ -75,6 +73,13 @@ int b200q_device_status(int reset, void* stream);
  *                        into a kernel gives up and records event 5 (default 2^22; tests shorten it)
  *   "no_pdl"             1 = launch without programmatic dependent launch */
 int b200q_set_tuning(const char* key, int value);
+
+/* Scratch for the NEXT b200q_qmatvec / b200q_norm_qmatvec / b200q_gate_up_swiglu call of this thread (device memory, 16-byte
+ * aligned, stream-ordered like the other buffers; NULL = none).  b200q_scratch_bytes(rows, K, act_dtype) is what such a call on
+ * rows [rows, K] can use: bf16 rows from batch 5 on (0 otherwise).  With it they run on the tcgen05 kernel - as fp16 with a
+ * power of two per row - instead of 16 rows per launch. */
+int b200q_scratch_next(void* ptr, size_t bytes);
+size_t b200q_scratch_bytes(int rows, int64_t K, int act_dtype);
 
 /* Group-wise dequantisation, bit-exact: out = cast(fp32(code - zero) * scale) with two
  * separately rounded fp32 operations.  Replaces kernels/dequant_q4.metal, dequant_q8.metal as

@@ -3,8 +3,8 @@
 //   y[b, n] = sum_k x[b, k] * (code[n, k] - zero[n, k/G]) * scale[n, k/G]
 //
 // Group sizes 32 / 64 / 128 with 16-byte aligned rows run on tensor cores: one to four batch rows on integer products of the raw
-// codes (gemv_i8.cuh), five and more on tcgen05 (qgemm_ts.cu), what neither takes - scales that are not fp16, bf16 rows from
-// batch 5 on - on fp16 mma.sync (gemv_fast.cuh, up to 16 batch rows per launch).  Everything else runs the general kernel
+// codes (gemv_i8.cuh), five and more on tcgen05 (qgemm_ts.cu; bf16 rows when the caller gives scratch for their fp16 form), what
+// neither takes - scales that are not fp16 - on fp16 mma.sync (gemv_fast.cuh, up to 16 batch rows per launch).  Everything else runs the general kernel
 // below, which follows the reference arithmetic literally.
 #include "gemv_params.cuh"
 
@@ -138,24 +138,55 @@ bool prefer_ts(const GemvParams& p) {
     return p.B >= min_b;
 }
 
-// The rmsnorm prologue costs the tcgen05 kernel's activation warps more than a launch of the row kernel (measured,
-// 4096 -> 2 x 14336: at batch 32 56 us fused against 33 + 3 us, at batch 8 40 us against 30 + 3 us), so when the caller
-// provides the buffer for the normalised rows they are materialised first.
-int split_norm_prologue(GemvParams& p, cudaStream_t stream) {
-    if (p.norm_w == nullptr || p.normed_out == nullptr || !prefer_ts(p) || tuning_get("gemv.fuse_norm") > 0) return B200Q_OK;
-    const int rc = rmsnorm_residual_launch(p.x, p.res_in, p.norm_w, p.normed_out, p.z_out, p.B, p.K, p.eps, p.act_dtype,
-                                           p.norm_w_dtype, stream);
-    if (rc != B200Q_OK) return rc;
-    p.x = p.normed_out;
-    p.norm_w = nullptr; p.res_in = nullptr; p.z_out = nullptr; p.normed_out = nullptr;
-    return B200Q_OK;
+// bf16 rows in fp16 for the tcgen05 kernel: one power of two per row brings the largest element to [2^13, 2^14); bf16 has 8
+// significant bits, so everything down to 2^-20 of the largest element is exact.  One CTA per row.
+__global__ void __launch_bounds__(256) rows_to_fp16_kernel(const uint16_t* __restrict__ x, __half* __restrict__ out, float* __restrict__ scale, int K) {
+    __shared__ float part[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t row = (size_t)blockIdx.x * K;
+    float mx = 0.0f;
+    for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
+        const uint4 u = *reinterpret_cast<const uint4*>(x + row + k);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mx = fmaxf(mx, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xFFFF0000u))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, part[i]);
+    int ex = 0;
+    if (mx > 0.0f && mx < INFINITY) frexpf(mx, &ex);
+    ex = max(-100, min(114, ex - 14));
+    const float sc = exp2f((float)ex), down = exp2f((float)-ex);
+    if (threadIdx.x == 0) scale[blockIdx.x] = sc;
+    for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {
+        const uint4 u = *reinterpret_cast<const uint4*>(x + row + k);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        __half2 h[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(__uint_as_float(w[i] << 16) * down, __uint_as_float(w[i] & 0xFFFF0000u) * down);
+        *reinterpret_cast<uint4*>(out + row + k) = *reinterpret_cast<const uint4*>(h);
+    }
+}
+int rows_to_fp16(const void* x, void* out, float* scale, int rows, int K, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
+    if (cudaLaunchKernelEx(&cfg, rows_to_fp16_kernel, (const uint16_t*)x, (__half*)out, scale, K) != cudaSuccess) return B200Q_ERR_LAUNCH;
+    return finish_launch();
 }
 
 int dispatch_fast(int bits, GemvParams& p, bool gate_up, cudaStream_t stream) {
-    if (prefer_ts(p)) {
-        const int rc = qgemm_ts(bits, p, gate_up, stream);
-        if (rc != B200Q_ERR_UNSUPPORTED) return rc;
-    }
     if (p.B <= 4 && tuning_get("gemv.i8") >= 0) {
         int rc = bits == 4 ? gemv_i8_q4(p, gate_up, stream) : gemv_i8_q8(p, gate_up, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
@@ -170,13 +201,123 @@ int dispatch_fast(int bits, GemvParams& p, bool gate_up, cudaStream_t stream) {
     return bits == 4 ? gemv_fast_q4(p, gate_up, stream) : gemv_fast_q8(p, gate_up, stream);
 }
 
+thread_local void* t_scratch = nullptr;          // b200q_scratch_next: for the next matvec / gate-up call of this thread
+thread_local size_t t_scratch_bytes = 0;
+struct ScratchGuard {                            // a call that ends early must not leave its scratch to the next one
+    ~ScratchGuard() { t_scratch = nullptr; t_scratch_bytes = 0; }
+};
+
+// rows b0 .. b0 + bn of a problem
+GemvParams slice(const GemvParams& a, int b0, int bn) {
+    GemvParams p = a;
+    auto in = [&](const void* base, size_t width) -> const void* { return base ? static_cast<const uint8_t*>(base) + (size_t)b0 * width * 2 : nullptr; };
+    auto out = [&](void* base, size_t width) -> void* { return base ? static_cast<uint8_t*>(base) + (size_t)b0 * width * 2 : nullptr; };
+    p.x = in(a.x, a.K); p.res_in = in(a.res_in, a.K);
+    p.z_out = out(a.z_out, a.K); p.normed_out = out(a.normed_out, a.K);
+    p.residual = in(a.residual, a.N);
+    p.y = out(a.y, a.N); p.gate_out = out(a.gate_out, a.N); p.up_out = out(a.up_out, a.N); p.act_out = out(a.act_out, a.N);
+    p.B = bn;
+    return p;
+}
+
+// All rows of a problem (all.B of them) through the kernels.
+int run_rows(int bits, GemvParams all, bool gate_up, cudaStream_t stream) {
+    void* scratch = t_scratch;
+    const size_t scratch_bytes = t_scratch_bytes;
+    const bool tp_used = all.tp_in.world > 0 || all.tp_out.world > 0;
+    const bool tensor_cores = !tuning_get("gemv.force_generic");
+    // From five rows on the norm is a launch of its own where the caller gives the buffer: inside the matvec kernels every CTA would
+    // repeat it (fp16 mma.sync kernel, 4096 -> 2 x 14336 at batch 8: 40 us fused against 30 + 3).
+    auto norm_first = [&]() -> int {
+        if (all.norm_w == nullptr || all.normed_out == nullptr) return B200Q_OK;
+        const int rc = rmsnorm_residual_launch(all.x, all.res_in, all.norm_w, all.normed_out, all.z_out, all.B, all.K, all.eps, all.act_dtype,
+                                               all.norm_w_dtype, stream);
+        all.x = all.normed_out;
+        all.norm_w = nullptr; all.res_in = nullptr; all.z_out = nullptr; all.normed_out = nullptr;
+        return rc;
+    };
+    if (!tp_used && tensor_cores && prefer_ts(all)) {
+        const bool bf = all.act_dtype == B200Q_BF16;
+        const size_t rows_bytes = ((size_t)all.B * all.K * 2 + 255) / 256 * 256;
+        const bool room = !bf || (scratch != nullptr && (reinterpret_cast<uintptr_t>(scratch) & 15u) == 0 && scratch_bytes >= rows_bytes + (size_t)all.B * 4);
+        GemvParams probe = all;
+        if (bf) probe.col_scale = reinterpret_cast<const float*>(scratch);
+        if (probe.norm_w != nullptr) probe.x = probe.normed_out;
+        if (room && probe.x != nullptr && qgemm_ts_applies(probe, gate_up)) {
+            int rc = norm_first();
+            if (rc != B200Q_OK) return rc;
+            GemvParams p = all;
+            if (bf) {
+                float* cs = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + rows_bytes);
+                rc = rows_to_fp16(all.x, scratch, cs, all.B, all.K, stream);
+                if (rc != B200Q_OK) return rc;
+                p.x = scratch;
+                p.col_scale = cs;
+            }
+            rc = qgemm_ts(bits, p, gate_up, stream);
+            if (rc != B200Q_ERR_UNSUPPORTED) return rc;
+        }
+        if (fast_path_ok(slice(all, 0, std::min(all.B, 16)))) {
+            const int rc = norm_first();
+            if (rc != B200Q_OK) return rc;
+        }
+    }
+    int chunk = 16;      // batch rows per launch; halved when a kernel's shared-memory plan does not fit
+    for (int b0 = 0; b0 < all.B;) {
+        GemvParams p = slice(all, b0, std::min(chunk, all.B - b0));
+        const bool fast = fast_path_ok(p);
+        int rc = fast ? dispatch_fast(bits, p, gate_up, stream) : B200Q_ERR_UNSUPPORTED;
+        if (rc == B200Q_ERR_UNSUPPORTED && tp_used) return rc;      // exchanges exist only in the tensor-core kernels
+        if (rc == B200Q_ERR_UNSUPPORTED && p.B > 1 && fast) {
+            chunk = (p.B + 1) / 2;
+            continue;
+        }
+        if (rc == B200Q_ERR_UNSUPPORTED) {
+            if (!fast) p = slice(all, b0, all.B - b0);              // the general kernel takes all rows at once
+            if (p.norm_w != nullptr) {
+                // generic route: materialise the normalised rows first (normed_out is required as the buffer)
+                if (p.normed_out == nullptr) return B200Q_ERR_UNSUPPORTED;
+                rc = rmsnorm_residual_launch(p.x, p.res_in, p.norm_w, p.normed_out, p.z_out, p.B, p.K, p.eps, p.act_dtype, p.norm_w_dtype, stream);
+                if (rc != B200Q_OK) return rc;
+                p.x = p.normed_out;
+                p.norm_w = nullptr; p.res_in = nullptr; p.z_out = nullptr; p.normed_out = nullptr;
+            }
+            rc = gate_up ? launch_generic<true>(p, bits, stream) : launch_generic<false>(p, bits, stream);
+        }
+        if (rc != B200Q_OK) return rc;
+        b0 += p.B;
+    }
+    return B200Q_OK;
+}
+
+void set_tp(GemvParams& p, int in_slot, int out_slot) {
+    if (out_slot >= 0) p.tp_out = tp_slot(out_slot)->out;
+    if (in_slot >= 0) {
+        const TpOut& src = tp_slot(in_slot)->out;
+        p.tp_in.flags = src.flags[src.rank];
+        p.tp_in.epoch = src.epoch;
+        p.tp_in.world = src.world;
+        p.tp_in.spin_limit = (uint32_t)std::max(0, tuning_get("tp.spin_limit"));
+        p.tp_in.packets = src.packets;
+    }
+}
+
 }  // namespace
 
+void scratch_next(void* ptr, size_t bytes) {
+    t_scratch = ptr;
+    t_scratch_bytes = ptr != nullptr ? bytes : 0;
+}
+size_t scratch_bytes_impl(int rows, int64_t K, int act_dtype) {
+    if (K <= 0 || act_dtype != B200Q_BF16 || rows < 5) return 0;
+    return ((size_t)rows * K * 2 + 255) / 256 * 256 + ((size_t)rows * 4 + 255) / 256 * 256;
+}
 
 int qmatvec_impl(int bits, const void* x, const uint8_t* codes, const void* scales, const void* zeros,
                  const void* residual, void* y, int B, int64_t N, int64_t K, int group_size, int act_dtype,
                  int scale_dtype, const void* residual_in, const void* norm_weight, int norm_w_dtype, float eps,
                  void* z_out, void* normed_out, cudaStream_t stream) {
+    const ScratchGuard guard;
     int tp_in_slot = -1, tp_out_slot = -1;
     tp_take(&tp_in_slot, &tp_out_slot);
     if ((bits != 4 && bits != 8) || x == nullptr || codes == nullptr || scales == nullptr ||
@@ -189,64 +330,16 @@ int qmatvec_impl(int bits, const void* x, const uint8_t* codes, const void* scal
     if (norm_weight == nullptr && (residual_in != nullptr || z_out != nullptr || normed_out != nullptr))
         return B200Q_ERR_BAD_ARG;
     if (N > INT32_MAX || K > INT32_MAX) return B200Q_ERR_UNSUPPORTED;
-    const int esz = 2;
-    auto off = [&](const void* base, size_t elems) -> const uint8_t* {
-        return base ? reinterpret_cast<const uint8_t*>(base) + elems * esz : nullptr;
-    };
-    auto offw = [&](void* base, size_t elems) -> uint8_t* {
-        return base ? reinterpret_cast<uint8_t*>(base) + elems * esz : nullptr;
-    };
-    int chunk = 64;      // batch rows per launch; halved when the kernels' shared-memory plans do not fit
-    for (int b0 = 0; b0 < B;) {
-        GemvParams p = {};
-        const int bn = std::min(chunk, B - b0);
-        p.x = off(x, (size_t)b0 * K);
-        p.res_in = off(residual_in, (size_t)b0 * K);
-        p.norm_w = norm_weight; p.eps = eps; p.norm_w_dtype = norm_w_dtype;
-        p.z_out = offw(z_out, (size_t)b0 * K);
-        p.normed_out = offw(normed_out, (size_t)b0 * K);
-        p.w[0] = codes; p.s[0] = scales; p.z[0] = zeros;
-        p.residual = off(residual, (size_t)b0 * N);
-        p.y = offw(y, (size_t)b0 * N);
-        p.B = bn; p.N = (int)N; p.K = (int)K; p.G = group_size; p.Gn = (int)((K + group_size - 1) / group_size);
-        p.act_dtype = act_dtype; p.scale_dtype = scale_dtype;
-        p.row_bytes = bits == 4 ? (int)((K + 1) / 2) : (int)K;
-        if (tp_out_slot >= 0) p.tp_out = tp_slot(tp_out_slot)->out;
-        if (tp_in_slot >= 0) {
-            const TpOut& src = tp_slot(tp_in_slot)->out;
-            p.tp_in.flags = src.flags[src.rank];
-            p.tp_in.epoch = src.epoch;
-            p.tp_in.world = src.world;
-            p.tp_in.spin_limit = (uint32_t)std::max(0, tuning_get("tp.spin_limit"));
-            p.tp_in.packets = src.packets;
-        }
-        const bool tp_used = tp_in_slot >= 0 || tp_out_slot >= 0;
-        if (!tp_used && fast_path_ok(p)) {
-            const int nrc = split_norm_prologue(p, stream);
-            if (nrc != B200Q_OK) return nrc;
-        }
-        int rc = fast_path_ok(p) ? dispatch_fast(bits, p, false, stream) : B200Q_ERR_UNSUPPORTED;
-        if (rc == B200Q_ERR_UNSUPPORTED && tp_used) return rc;      // exchanges exist only in the tensor-core kernel
-        if (rc == B200Q_ERR_UNSUPPORTED && bn > 1 && fast_path_ok(p)) {
-            chunk = (bn + 1) / 2;
-            continue;
-        }
-        if (rc == B200Q_ERR_UNSUPPORTED) {
-            if (norm_weight != nullptr) {
-                // generic route: materialise the normalised rows first (normed_out is required as the buffer)
-                if (p.normed_out == nullptr) return B200Q_ERR_UNSUPPORTED;
-                rc = rmsnorm_residual_launch(p.x, p.res_in, norm_weight, p.normed_out, p.z_out, bn, K, eps, act_dtype,
-                                             norm_w_dtype, stream);
-                if (rc != B200Q_OK) return rc;
-                p.x = p.normed_out;
-                p.norm_w = nullptr; p.res_in = nullptr; p.z_out = nullptr; p.normed_out = nullptr;
-            }
-            rc = launch_generic<false>(p, bits, stream);
-        }
-        if (rc != B200Q_OK) return rc;
-        b0 += bn;
-    }
-    return B200Q_OK;
+    GemvParams p = {};
+    p.x = x; p.res_in = residual_in; p.norm_w = norm_weight; p.eps = eps; p.norm_w_dtype = norm_w_dtype;
+    p.z_out = z_out; p.normed_out = normed_out;
+    p.w[0] = codes; p.s[0] = scales; p.z[0] = zeros;
+    p.residual = residual; p.y = y;
+    p.B = B; p.N = (int)N; p.K = (int)K; p.G = group_size; p.Gn = (int)((K + group_size - 1) / group_size);
+    p.act_dtype = act_dtype; p.scale_dtype = scale_dtype;
+    p.row_bytes = bits == 4 ? (int)((K + 1) / 2) : (int)K;
+    set_tp(p, tp_in_slot, tp_out_slot);
+    return run_rows(bits, p, false, stream);
 }
 
 int gate_up_impl(int bits, const void* x, const uint8_t* gate_codes, const uint8_t* up_codes, const void* gate_scales,
@@ -254,6 +347,7 @@ int gate_up_impl(int bits, const void* x, const uint8_t* gate_codes, const uint8
                  void* act_out, const void* residual_in, const void* norm_weight, float eps, void* z_out,
                  void* normed_out, int rows, int64_t N, int64_t K, int group_size, int act_dtype, int scale_dtype,
                  int norm_w_dtype, cudaStream_t stream) {
+    const ScratchGuard guard;
     int tp_in_slot = -1, tp_out_slot = -1;
     tp_take(&tp_in_slot, &tp_out_slot);
     if ((bits != 4 && bits != 8) || x == nullptr || gate_codes == nullptr || up_codes == nullptr ||
@@ -266,68 +360,18 @@ int gate_up_impl(int bits, const void* x, const uint8_t* gate_codes, const uint8
     if (norm_weight == nullptr && (residual_in != nullptr || z_out != nullptr || normed_out != nullptr))
         return B200Q_ERR_BAD_ARG;
     if (N > INT32_MAX || K > INT32_MAX) return B200Q_ERR_UNSUPPORTED;
-    const int esz = 2;
-    auto off = [&](const void* base, size_t elems) -> const uint8_t* {
-        return base ? reinterpret_cast<const uint8_t*>(base) + elems * esz : nullptr;
-    };
-    auto offw = [&](void* base, size_t elems) -> uint8_t* {
-        return base ? reinterpret_cast<uint8_t*>(base) + elems * esz : nullptr;
-    };
-    int chunk = 64;      // batch rows per launch; halved when the kernels' shared-memory plans do not fit
-    for (int b0 = 0; b0 < rows;) {
-        GemvParams p = {};
-        const int bn = std::min(chunk, rows - b0);
-        p.x = off(x, (size_t)b0 * K);
-        p.res_in = off(residual_in, (size_t)b0 * K);
-        p.norm_w = norm_weight; p.eps = eps; p.norm_w_dtype = norm_w_dtype;
-        p.z_out = offw(z_out, (size_t)b0 * K);
-        p.normed_out = offw(normed_out, (size_t)b0 * K);
-        p.w[0] = gate_codes; p.w[1] = up_codes;
-        p.s[0] = gate_scales; p.s[1] = up_scales;
-        p.z[0] = gate_zeros; p.z[1] = up_zeros;
-        p.gate_out = offw(gate_out, (size_t)b0 * N);
-        p.up_out = offw(up_out, (size_t)b0 * N);
-        p.act_out = offw(act_out, (size_t)b0 * N);
-        p.B = bn; p.N = (int)N; p.K = (int)K; p.G = group_size; p.Gn = (int)((K + group_size - 1) / group_size);
-        p.act_dtype = act_dtype; p.scale_dtype = scale_dtype;
-        p.row_bytes = bits == 4 ? (int)((K + 1) / 2) : (int)K;
-        if (tp_out_slot >= 0) p.tp_out = tp_slot(tp_out_slot)->out;
-        if (tp_in_slot >= 0) {
-            const TpOut& src = tp_slot(tp_in_slot)->out;
-            p.tp_in.flags = src.flags[src.rank];
-            p.tp_in.epoch = src.epoch;
-            p.tp_in.world = src.world;
-            p.tp_in.spin_limit = (uint32_t)std::max(0, tuning_get("tp.spin_limit"));
-            p.tp_in.packets = src.packets;
-        }
-        const bool tp_used = tp_in_slot >= 0 || tp_out_slot >= 0;
-        if (!tp_used && fast_path_ok(p)) {
-            const int nrc = split_norm_prologue(p, stream);
-            if (nrc != B200Q_OK) return nrc;
-        }
-        int rc;
-        rc = fast_path_ok(p) ? dispatch_fast(bits, p, true, stream) : B200Q_ERR_UNSUPPORTED;
-        if (rc == B200Q_ERR_UNSUPPORTED && tp_used) return rc;      // exchanges exist only in the tensor-core kernel
-        if (rc == B200Q_ERR_UNSUPPORTED && bn > 1 && fast_path_ok(p)) {
-            chunk = (bn + 1) / 2;
-            continue;
-        }
-        if (rc == B200Q_ERR_UNSUPPORTED) {
-            if (norm_weight != nullptr) {
-                // generic route: materialise the normalised rows first (normed_out is required as the buffer)
-                if (p.normed_out == nullptr) return B200Q_ERR_UNSUPPORTED;
-                rc = rmsnorm_residual_launch(p.x, p.res_in, norm_weight, p.normed_out, p.z_out, bn, K, eps, act_dtype,
-                                             norm_w_dtype, stream);
-                if (rc != B200Q_OK) return rc;
-                p.x = p.normed_out;
-                p.norm_w = nullptr; p.res_in = nullptr; p.z_out = nullptr; p.normed_out = nullptr;
-            }
-            rc = launch_generic<true>(p, bits, stream);
-        }
-        if (rc != B200Q_OK) return rc;
-        b0 += bn;
-    }
-    return B200Q_OK;
+    GemvParams p = {};
+    p.x = x; p.res_in = residual_in; p.norm_w = norm_weight; p.eps = eps; p.norm_w_dtype = norm_w_dtype;
+    p.z_out = z_out; p.normed_out = normed_out;
+    p.w[0] = gate_codes; p.w[1] = up_codes;
+    p.s[0] = gate_scales; p.s[1] = up_scales;
+    p.z[0] = gate_zeros; p.z[1] = up_zeros;
+    p.gate_out = gate_out; p.up_out = up_out; p.act_out = act_out;
+    p.B = rows; p.N = (int)N; p.K = (int)K; p.G = group_size; p.Gn = (int)((K + group_size - 1) / group_size);
+    p.act_dtype = act_dtype; p.scale_dtype = scale_dtype;
+    p.row_bytes = bits == 4 ? (int)((K + 1) / 2) : (int)K;
+    set_tp(p, tp_in_slot, tp_out_slot);
+    return run_rows(bits, p, true, stream);
 }
 
 }  // namespace b200q

@@ -62,6 +62,7 @@ struct GemvParams {
     int meta_vec;           // scales / zeros are fp16, 16-byte aligned, Gn % 8 == 0: vector loads
     int interleave;         // 1: CTA c takes tiles c, c + grid, ... instead of a contiguous row range
     int rows_lo, rem;       // CTA c owns rows_lo (+1 if c < rem) rows
+    const float* col_scale; // [B] or null: x holds the rows as fp16, divided by these powers of two (act_dtype is that of the outputs)
     TpOut tp_out;           // tensor-parallel exchange: outputs go to every rank's full buffer (world == 0: off)
     TpIn tp_in;             // ... the activations are another exchange's full buffer: wait for its flags first
     uint32_t off_xs, off_xzero, off_xmx, off_xscale, off_part, off_meta, off_ring;
@@ -82,8 +83,9 @@ int gemv_i8_q8(const GemvParams& p, bool gate_up, cudaStream_t stream);
 int gemv_i8_q4_read_status(int reset, cudaStream_t stream);
 int gemv_i8_q8_read_status(int reset, cudaStream_t stream);
 
-// tcgen05 kernel (qgemm_ts.cu): weights through tensor memory, any batch up to 64 rows per launch.  Returns
+// tcgen05 kernel (qgemm_ts.cu): weights through tensor memory, any number of rows per launch.  qgemm_ts returns
 // B200Q_ERR_UNSUPPORTED when the problem is outside its plan.
+bool qgemm_ts_applies(const GemvParams& p, bool gate_up);
 int qgemm_ts(int bits, const GemvParams& p, bool gate_up, cudaStream_t stream);
 int qgemm_ts_read_status(int reset, cudaStream_t stream);
 

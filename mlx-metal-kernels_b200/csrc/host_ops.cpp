@@ -33,6 +33,8 @@ int (*p_qmatvec)(int, const void*, const uint8_t*, const void*, const void*, con
                  int, void*) = nullptr;
 int (*p_gate_up)(int, const void*, const uint8_t*, const uint8_t*, const void*, const void*, const void*, const void*, void*, void*,
                  void*, const void*, const void*, int, float, void*, void*, int, int64_t, int64_t, int, int, int, void*) = nullptr;
+int (*p_scratch_next)(void*, size_t) = nullptr;
+size_t (*p_scratch_bytes)(int, int64_t, int) = nullptr;
 size_t (*p_attn_ws)(int, int, int, int) = nullptr;
 int (*p_attn_launches)(int, int, int) = nullptr;
 int (*p_attn)(int, const void*, const uint8_t*, const uint8_t*, const void*, const void*, const int32_t*, const int32_t*, void*,
@@ -122,7 +124,11 @@ PyObject* matvec(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const int64_t B = x->size(0), K = x->size(x->dim() - 1);
     Matrix m;
     if (B <= 0 || B > INT32_MAX || K <= 0 || !matrix(m, a[2], a[3], a[4], (int)bits, K, group, dev)) return none();
-    Tensor y = empty({B, m.n}, x->scalar_type(), dev);
+    Tensor y = empty({B, m.n}, x->scalar_type(), dev), scratch;
+    if (const size_t n = p_scratch_bytes((int)B, K, dtype_code(x->scalar_type()))) {
+        scratch = empty({(int64_t)n}, at::kByte, dev);
+        p_scratch_next(scratch.mutable_data_ptr(), n);
+    }
     const int rc = p_qmatvec((int)bits, x->const_data_ptr(), codes(m.w), ptr(m.s), ptr(m.z), nullptr, y.mutable_data_ptr(), (int)B, m.n,
                              K, (int)group, dtype_code(x->scalar_type()), dtype_code(m.s->scalar_type()), stream_of(dev));
     return rc == 0 ? THPVariable_Wrap(std::move(y)) : none();
@@ -152,15 +158,19 @@ PyObject* mlp_block(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     // one scratch block: z [rows, D], the SwiGLU rows [rows, inter], and the normalised rows where the library wants them
     const int64_t zb = (rows * D * 2 + 255) / 256 * 256, mb = (rows * g.n * 2 + 255) / 256 * 256;
     const bool want_normed = rows >= kMinNormRows;
-    Tensor scratch = empty({zb + mb + (want_normed ? zb : 0)}, at::kByte, dev);
+    const size_t xb = std::max(p_scratch_bytes((int)rows, D, act), p_scratch_bytes((int)rows, g.n, act));
+    Tensor scratch = empty({zb + mb + (want_normed ? zb : 0) + (int64_t)xb}, at::kByte, dev);
     uint8_t* z = static_cast<uint8_t*>(scratch.mutable_data_ptr());
     uint8_t *mlp = z + zb, *normed = want_normed ? mlp + mb : nullptr;
     Tensor out = empty(x->sizes(), x->scalar_type(), dev);
+    void* xs = xb ? z + zb + mb + (want_normed ? zb : 0) : nullptr;
     const float eps = (float)PyFloat_AS_DOUBLE(a[14]);
+    p_scratch_next(xs, xb);
     int rc = p_gate_up((int)bits, x->const_data_ptr(), codes(g.w), codes(u.w), ptr(g.s), ptr(u.s), ptr(g.z), ptr(u.z), nullptr, nullptr,
                        mlp, res->const_data_ptr(), nw->const_data_ptr(), dtype_code(nw->scalar_type()), eps, z, normed, (int)rows, g.n,
                        D, (int)group, act, dtype_code(g.s->scalar_type()), st);
     if (rc != 0) return none();
+    p_scratch_next(xs, xb);
     rc = p_qmatvec((int)bits, mlp, codes(d.w), ptr(d.s), ptr(d.z), z, out.mutable_data_ptr(), (int)rows, D, g.n, (int)group, act,
                    dtype_code(d.s->scalar_type()), st);
     return rc == 0 ? THPVariable_Wrap(std::move(out)) : none();
@@ -345,6 +355,7 @@ PyObject* dequantize_kv(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 PyObject* bind(PyObject*, PyObject* table) {
     const struct { const char* name; void** slot; } want[] = {
         {"b200q_qmatvec", (void**)&p_qmatvec}, {"b200q_gate_up_swiglu", (void**)&p_gate_up},
+        {"b200q_scratch_next", (void**)&p_scratch_next}, {"b200q_scratch_bytes", (void**)&p_scratch_bytes},
         {"b200q_paged_gqa_workspace_bytes", (void**)&p_attn_ws}, {"b200q_attention_stage_launches", (void**)&p_attn_launches},
         {"b200q_paged_gqa_decode", (void**)&p_attn}, {"b200q_paged_gqa_decode_window", (void**)&p_attn_window},
         {"b200q_paged_fp16_gqa_workspace_bytes", (void**)&p_plain_ws}, {"b200q_paged_fp16_gqa_decode", (void**)&p_plain_attn},

@@ -1,35 +1,32 @@
-// Quantized skinny GEMM for decode on the 5th-generation tensor cores (tcgen05, sm_100a):
+// Quantized GEMM for batches of rows on the 5th-generation tensor cores (tcgen05, sm_100a):
 //
-//   y[b, n] = sum_k x[b, k] * (code[n, k] - zero[n, k/G]) * scale[n, k/G]          b < B <= 32 per launch
+//   y[b, n] = sum_k x[b, k] * (code[n, k] - zero[n, k/G]) * scale[n, k/G]
 //
 // The weights are the A operand and live in TENSOR MEMORY, the activations are the B operand in
-// shared memory, the accumulator D[128 weight rows, batch columns] stays in tensor memory:
+// shared memory, the accumulator D[128 weight rows, up to 128 batch columns] stays in tensor memory:
 //
-//   TMA (one elected thread)      2-D tiled copies, 128-byte swizzle: 128 rows x 128 bytes of codes per
-//                                 stage and matrix, plus the rows' scales / zero points of the stage
-//   dequantise warps (8)          thread = weight row.  Codes come out of shared memory 16 bytes at a time
-//                                 (conflict-free through the swizzle), become fp16 weights in registers,
-//                                     w = ((1024+q) - (1024+rint(z))) * s + (rint(z) - z) * s
-//                                 (exact subtraction, then one fused multiply-add), and go to tensor memory
-//                                 with tcgen05.st, 128 k (64 columns) per chunk.  No loop-carried dependency:
-//                                 the work is a pure stream.
-//   activation warps (2 or 4)     each owns every n-th stage: one TMA copy per 64 k lands the stage's rows in the
-//                                 operand tile (the copy's 128-byte swizzle is the K-major operand layout), then
-//                                 the warp rewrites them in place where needed (order of the q4 codes inside a
-//                                 32-bit word, x := rmsnorm(x + residual))
-//   MMA (one warp, one elected    tcgen05.mma.kind::f16, M = 128, N = batch rounded up to 16, K = 16, A from
-//        lane issues)             tensor memory, B through a shared-memory descriptor; tcgen05.commit releases
-//                                 the chunk / the operand tile / the accumulator
-//   epilogue (warps 0-3)          tcgen05.ld of D, clamp, round, residual add or SwiGLU, store
+//   weight producer (one lane)    2-D TMA, 128-byte swizzle: 128 rows x 128 bytes of codes per stage and matrix; scales / zero
+//                                 points 16 groups at a time where their rows allow it
+//   row producer (one lane)       2-D TMA of the activations: 128 k x the block's columns straight into the operand layout (the
+//                                 128-byte swizzle of the copy is the K-major layout of the MMA); rows past the batch are zero-filled
+//   dequantise warps (16)         thread = weight row, four groups of four warps take the chunks (128 k) in turn.  Codes come out of
+//                                 shared memory 16 bytes at a time (conflict-free through the swizzle), become fp16 weights in
+//                                     w = ((base+q) - (base+rint(z))) * s + (rint(z) - z) * s
+//                                 (exact subtraction, then one fused multiply-add) and go to tensor memory with tcgen05.st
+//   MMA (one warp, one elected    tcgen05.mma.kind::f16, M = 128, N = block columns, K = 16, A from tensor memory; tcgen05.commit
+//        lane issues)             releases the chunk / the operand slot / the accumulator
+//   epilogue (dequantise warps)   tcgen05.ld of D, clamp, round, residual add or SwiGLU, store
 //
-// Measured on B200: one tcgen05.mma of this shape occupies the tensor pipe for about 86 cycles whatever N <= 128,
-// i.e. 128 rows x 16 k of weights per 86 cycles and SM.  That bounds q4 at about half of the HBM rate and q8 at
-// about the full rate, for every batch up to 128 rows alike; the mma.sync kernel (gemv_fast.cuh) stays ahead for
-// batches of a few rows.
+// What bounds it: a chunk (128 x 128 weights) costs the dequantisation 4 x 260 warp instructions, i.e. about 300 clocks on the SM's four
+// schedulers, and the tensor pipe 8 x 22 clocks up to 32 columns, 8 x 65 at 128.  So small batches run at the dequantisation's rate,
+// large ones at the tensor pipe's, and one block of 128 columns shares each dequantised weight.
+// Codes are unpacked in k order (one byte permute per pair): the activations need no rearrangement, and nothing but TMA touches
+// them.  (The form before this one permuted the rows in shared memory with four warps, recomputed the group constants per 32 k and
+// kept 32 columns per launch: 1800 warp instructions per chunk; a 256-row prompt chunk re-streamed its weights eight times.)
 //
-// A CTA owns row tiles of 128 rows.  When there are fewer tiles than SMs the K range of a tile is split
-// over the CTAs of a thread-block cluster; the partial accumulators are summed in rank order through
-// distributed shared memory by the cluster's first CTA (deterministic, no global scratch).
+// Work items are (row tile, column block) pairs.  When there are fewer than SMs, the K range of an item is split over the CTAs of a
+// thread-block cluster; the partial accumulators are summed in rank order through distributed shared memory by the cluster's first
+// CTA (deterministic, no global scratch).
 // Every wait is bounded; a wait that runs out records an event in the status word and the kernel
 // carries on without the data so that it always terminates and frees its tensor memory.
 #include "gemv_params.cuh"
@@ -53,54 +50,50 @@ constexpr int kChunkK = 128;                   // k per chunk of A in tensor mem
 constexpr int kChunkCols = kChunkK / 2;
 constexpr int kRowBytes = 128;                 // bytes of one weight row per stage = the swizzle span
 constexpr int kWTile = kRows * kRowBytes;      // 16 KB of codes per stage and matrix
-constexpr int kMetaTile = kRows * 16;          // 2 KB: 8 fp16 scales (or zero points) per row
+constexpr int kMetaGroups = 16;                // groups per scale tile: 32 bytes of a row (one sector), several stages' worth
+constexpr int kMetaTile = kRows * kMetaGroups * 2;   // 4 KB of scales (or zero points)
+constexpr int kMaxMetaBufs = 4;
 constexpr int kMaxStages = 8;
 constexpr int kMaxASlots = 8;
-constexpr int kMaxXTiles = 6;
+constexpr int kMaxXSlots = 8;
+constexpr int kMaxCols = 128;                  // batch columns per item
 constexpr uint32_t kTsWaitLimit = 1u << 20;
-// Warp roles: [0, 8) dequantise (two groups of four: one warp per 32-lane quarter of tensor memory), 8 the TMA
-// producer (also owns the tensor-memory allocation), 9 the MMA issuer, then the activation warps.  Two shapes:
-// the compact one (2 activation warps) stays below half of an SM's shared memory, registers and tensor memory, so
-// that two kernels of a dependent chain can be resident together; the whole-SM one (4 activation warps, deeper
-// rings, all of tensor memory) is for large matrices (16 MB of codes and up) and for whatever the compact one cannot hold.
-constexpr int kDeqWarps = 8;
-constexpr int ts_xwarps(bool whole) { return whole ? 4 : 2; }
-constexpr int ts_threads(bool whole) { return (kDeqWarps + 2 + ts_xwarps(whole)) * 32; }
+constexpr int kDeqWarps = 16;
+constexpr int kGroups = kDeqWarps / 4;         // a group = four warps = one per 32-lane quarter of tensor memory
+constexpr int kTmaWarp = kDeqWarps, kMmaWarp = kDeqWarps + 1, kRowWarp = kDeqWarps + 2;
+constexpr int kTsThreads = (kDeqWarps + 3) * 32;
 
 struct alignas(64) TsParams {
     CUtensorMap wmap[2];        // codes [N, row_bytes] u8, box 128 B x 128 rows, 128-byte swizzle
-    CUtensorMap smap[2];        // scales [N, Gn] fp16 as bytes, box 16 B x 128 rows
+    CUtensorMap smap[2];        // scales [N, Gn] fp16 as bytes, box 32 B x 128 rows, 32-byte swizzle
     CUtensorMap zmap[2];        // zero points, same
-    CUtensorMap xmap;           // activations [B, K] fp16 as bytes, box 128 B (64 k) x B rows, 128-byte swizzle (= the operand layout)
-    CUtensorMap rmap;           // residual rows of the norm prologue, box 64 k x B rows, no swizzle
-    const __half* x;            // [B, K]
-    const __half* res_in;       // norm prologue: rows = rmsnorm(x + res_in); may be null
-    const void* norm_w;         // [K]; null = no prologue
-    __half* z_out;              // [B, K] or null
-    __half* normed_out;         // [B, K] or null
-    const __half* residual;     // plain: out = cast(residual + cast(y)); may be null
-    __half* y;
-    __half* gate_out;
-    __half* up_out;
-    __half* act_out;
-    float eps;
-    int norm_w_dtype;
-    int B, N, K;
+    CUtensorMap xmap;           // activations [B, K] fp16 as bytes, box 128 B (64 k) x block columns, 128-byte swizzle
+    const void* x;              // activations (host side: the map depends on the block's columns)
+    const uint16_t* s[2];       // scales / zero points where a row is no multiple of 16 bytes: read by the dequantise warps
+    const uint16_t* z[2];
+    const float* col_scale;     // [B] factor of the result columns (rows that were scaled into fp16), or null
+    const uint16_t* residual;   // plain: out = cast(residual + cast(y)); may be null
+    uint16_t* y;
+    uint16_t* gate_out;
+    uint16_t* up_out;
+    uint16_t* act_out;
+    int B, N, Gn;
     int has_z;
-    int ncols;                  // MMA N: batch rows rounded up to a multiple of 16
-    int tiles;                  // row tiles of 128
+    int bf16;                   // outputs and residual are bf16
+    int ncols;                  // columns of a block: MMA N, a multiple of 16
+    int nblk;                   // column blocks
+    int items;                  // row tiles x column blocks
     int split;                  // CTAs per cluster = parts of the K range
-    int n_stage_total;          // K / (k per stage)
+    int n_stage_total;          // stages over the whole K (the last may be short: TMA fills zeros)
     int stages;                 // depth of the ring of weight stages
     int a_slots;                // chunks of A in tensor memory
     int a_col0;                 // first column of the A ring (the accumulators sit below it)
-    int tmem_cols;              // columns allocated (power of two)
-    int x_tiles;                // depth of the ring of activation operand tiles
-    uint32_t stage_bytes;       // one weight stage: [codes x MATS][scales, zeros x MATS]
-    uint32_t off_meta;          // scales inside a stage
-    uint32_t off_xt, xt_bytes;  // ring of operand tiles [ncols rows, k of a stage], K-major, 128-byte swizzle
-    uint32_t off_res, res_bytes;  // residual rows of the norm prologue, one slot per operand tile (16-byte pieces, compact)
-    uint32_t off_red;           // dedicated buffer for the cluster's partial sums (0: the weight ring is reused instead)
+    int x_slots;                // depth of the ring of activation chunks
+    int meta_bufs;              // depth of the ring of scale tiles
+    uint32_t stage_bytes;       // one weight stage: codes x MATS
+    uint32_t off_meta;          // ring of scale tiles, each [scales, zeros] x MATS
+    uint32_t off_x, x_bytes;    // ring of activation chunks [2 x 64 k][columns], K-major, 128-byte swizzle
+    uint32_t off_red;           // dedicated buffer for the cluster's partial sums (0: the rings are reused instead)
 };
 
 // ---- PTX wrappers specific to this kernel ---------------------------------------------------------------------
@@ -228,152 +221,124 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int eve
 }
 
 // Per-group constants of the dequantisation, each duplicated into both halves of a register:
-//   w = ((base + q) + c_base) * s + r,   c_base = -(base + zi),  zi = rint(z),  r = (zi - z) * s
-struct GroupConst { uint32_t s2, r2, c1024, c64; };
+//   w = ((base + q) + c) * s + r,   c = -(base + zi),  zi = rint(z),  r = (zi - z) * s
+// base: 1024 in both halves (q8), or 1024 / 64 for the low / high nibble of a byte (q4).
+struct GroupConst { uint32_t s2, r2, c; };
+template <int BITS>
 __device__ __forceinline__ GroupConst group_const(uint32_t s_bits, uint32_t z_bits) {
     GroupConst c;
-    c.s2 = (s_bits & 0xFFFFu) | (s_bits << 16);
-    const uint32_t z2 = (z_bits & 0xFFFFu) | (z_bits << 16);
+    c.s2 = prmt(s_bits, s_bits, 0x1010);
+    const uint32_t z2 = prmt(z_bits, z_bits, 0x1010);
     const __half2 zi = h2rint(*reinterpret_cast<const __half2*>(&z2));
     const uint32_t zi2 = *reinterpret_cast<const uint32_t*>(&zi);
     c.r2 = hmul2_u32(hsub2_u32(zi2, z2), c.s2);
-    c.c1024 = hsub2_u32(0xE400E400u, zi2);        // -1024 - zi (exact: integers below 2048)
-    c.c64 = hsub2_u32(0xD400D400u, zi2);          // -64 - zi
+    c.c = hsub2_u32(BITS == 4 ? 0xD400E400u : 0xE400E400u, zi2);        // exact: integers below 2048
     return c;
 }
 
-// The residual values of output row n for all batch columns, fetched before the accumulators are waited for and before
-// the first store: y may alias the residual rows as far as the compiler knows, so a load placed after a store would
-// wait for it - one global-memory latency per column.
-template <int MATS>
-__device__ __forceinline__ void ts_load_residual(const TsParams& p, int n, float (&res)[32]) {
-    if (MATS == 1 && p.residual != nullptr && n < p.N) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) res[j] = j < p.B ? __half2float(p.residual[(size_t)j * p.N + n]) : 0.0f;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) res[j] = 0.0f;
-    }
+__device__ __forceinline__ float ts_round(const TsParams& p, float v) {
+    return p.bf16 ? __bfloat162float(__float2bfloat16_rn(v)) : __half2float(__float2half_rn(v));
 }
-// The epilogue of one 16-column slice: clamp, round, residual add or SwiGLU, store.
-template <int MATS, int C0>
-__device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&acc)[MATS][16], int n, const float (&res)[32]) {
+__device__ __forceinline__ uint16_t ts_bits(const TsParams& p, float v) {
+    return p.bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+}
+__device__ __forceinline__ float ts_float(const TsParams& p, uint16_t u) {
+    return p.bf16 ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
+}
+// The residual values of output row n for 16 columns, fetched before the accumulators are waited for and before the first
+// store (y may alias the residual rows as far as the compiler knows).
+template <int MATS>
+__device__ __forceinline__ void ts_load_residual(const TsParams& p, int n, int b0, int nb, uint16_t (&res)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        const int b = C0 + j;
-        if (b >= p.B) break;
+        res[j] = 0;
+        if (MATS == 1 && p.residual != nullptr && n < p.N && j < nb) res[j] = p.residual[(size_t)(b0 + j) * p.N + n];
+    }
+}
+// The epilogue of a 16-column slice (columns b0 .. b0 + nb of the batch): clamp, round, residual add or SwiGLU, store.
+template <int MATS>
+__device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&acc)[MATS][16], int n, int b0, int nb, const uint16_t (&res)[16]) {
+    const float fmax_act = p.bf16 ? 3.3895313892515355e38f : 65504.0f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        if (j >= nb) break;
+        const int b = b0 + j;
         const size_t o = (size_t)b * p.N + n;
-        const float v0 = __half2float(__float2half_rn(fminf(fmaxf(acc[0][j], -65504.0f), 65504.0f)));
+        const float cs = p.col_scale != nullptr ? p.col_scale[b] : 1.0f;
+        const float v0 = ts_round(p, fminf(fmaxf(acc[0][j] * cs, -fmax_act), fmax_act));
         if (MATS == 1) {
             float v = v0;
-            if (p.residual != nullptr) v = res[C0 + j] + v;
-            p.y[o] = __float2half_rn(v);
+            if (p.residual != nullptr) v = ts_float(p, res[j]) + v;
+            p.y[o] = ts_bits(p, v);
         } else {
-            const float v1 = __half2float(__float2half_rn(fminf(fmaxf(acc[MATS - 1][j], -65504.0f), 65504.0f)));
-            if (p.gate_out != nullptr) p.gate_out[o] = __float2half_rn(v0);
-            if (p.up_out != nullptr) p.up_out[o] = __float2half_rn(v1);
-            if (p.act_out != nullptr) p.act_out[o] = __float2half_rn((v0 / (1.0f + expf(-v0))) * v1);
+            const float v1 = ts_round(p, fminf(fmaxf(acc[MATS - 1][j] * cs, -fmax_act), fmax_act));
+            if (p.gate_out != nullptr) p.gate_out[o] = ts_bits(p, v0);
+            if (p.up_out != nullptr) p.up_out[o] = ts_bits(p, v1);
+            if (p.act_out != nullptr) p.act_out[o] = ts_bits(p, (v0 / (1.0f + expf(-v0))) * v1);
         }
     }
 }
 
-// Sum of squares of rmsnorm's input row z = cast(x + residual) for batch row b, by one warp; fixed summation order
-// (lane-strided, then a butterfly), so every CTA and every launch shape gets the same bits.
-__device__ __forceinline__ float row_inv_rms(const TsParams& p, int b, int lane) {
-    float ss = 0.0f;
-    for (int k = lane * 8; k < p.K; k += 256) {
-        const uint4 ux = *reinterpret_cast<const uint4*>(p.x + (size_t)b * p.K + k);
-        const __half2* hx = reinterpret_cast<const __half2*>(&ux);
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { v[2 * i] = __low2float(hx[i]); v[2 * i + 1] = __high2float(hx[i]); }
-        if (p.res_in != nullptr) {
-            const uint4 ur = *reinterpret_cast<const uint4*>(p.res_in + (size_t)b * p.K + k);
-            const __half2* hr = reinterpret_cast<const __half2*>(&ur);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                v[2 * i] = __half2float(__float2half_rn(v[2 * i] + __low2float(hr[i])));
-                v[2 * i + 1] = __half2float(__float2half_rn(v[2 * i + 1] + __high2float(hr[i])));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    return rsqrtf(ss / (float)p.K + p.eps);
-}
-
-template <int BITS, int LOGG, int MATS, bool WHOLE>
-__global__ void __launch_bounds__(ts_threads(WHOLE), WHOLE ? 1 : 2) qgemm_ts_kernel(const __grid_constant__ TsParams p) {
-    constexpr int DW = kDeqWarps;
-    constexpr int kXWarps = ts_xwarps(WHOLE);
+// META: scales arrive by TMA (their rows are a multiple of 16 bytes), else the dequantise warps read them from global memory.
+template <int BITS, int LOGG, int MATS, bool META>
+__global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_constant__ TsParams p) {
     constexpr int KS = kRowBytes * 8 / BITS;           // k per stage: 256 (q4) or 128 (q8)
     constexpr int SC = KS / kChunkK;                   // k-chunks per stage
-    constexpr int APS = SC * MATS;                     // chunks of A per stage
-    constexpr int NG = DW / 4;                         // dequantise groups; chunk a belongs to group a % NG
-    constexpr int kTmaWarp = DW, kMmaWarp = DW + 1, kXWarp0 = DW + 2;
-    constexpr int kThreads = ts_threads(WHOLE);
-    constexpr int GPS = APS < NG ? APS : NG;           // groups that touch one stage
+    constexpr int APS = SC * MATS;                     // chunks of A per stage: 1, 2 or 4
+    constexpr int NG = kGroups;                        // chunk a (counted over the kernel) belongs to group a % NG
+    constexpr int GPS = APS < NG ? APS : NG;           // groups that touch one stage (each with one chunk: APS <= NG)
+    constexpr int MS = (kMetaGroups << LOGG) / KS;     // stages per scale tile
+    constexpr uint32_t kMetaBuf = MATS * 2 * kMetaTile;
+    constexpr int CGR = kChunkK >> LOGG;               // scale groups per chunk: 4, 2 or 1
+    static_assert(APS <= NG, "a group has at most one chunk per stage");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* const sbase = smem_raw + (base - smem_u32(smem_raw));
 
     uint64_t* bars = reinterpret_cast<uint64_t*>(sbase);
-    uint64_t* full_w = bars;                            // [stages] codes + scales of the stage have landed
-    uint64_t* empty_w = full_w + kMaxStages;            // [stages] dequantise warps are done with the codes
-    uint64_t* full_x = empty_w + kMaxStages;            // [x_tiles] the operand tile of a stage is written
-    uint64_t* empty_x = full_x + kMaxXTiles;            // [x_tiles] the MMAs reading the tile are done
-    uint64_t* x_tma = empty_x + kMaxXTiles;             // [x_tiles] the raw activation rows of a stage have landed
-    uint64_t* a_full = x_tma + kMaxXTiles;              // [a_slots] a chunk of A is in tensor memory
-    uint64_t* a_free = a_full + kMaxASlots;             // [a_slots] the MMAs reading the chunk are done
-    uint64_t* d_full = a_free + kMaxASlots;             // the tile's accumulator is complete
+    uint64_t* full_w = bars;                            // [stages] codes of the stage have landed
+    uint64_t* empty_w = full_w + kMaxStages;            // [stages] the dequantise warps are done with them
+    uint64_t* full_x = empty_w + kMaxStages;            // [x_slots] a chunk of activations has landed
+    uint64_t* empty_x = full_x + kMaxXSlots;            // [x_slots] the MMAs reading it are done
+    uint64_t* a_full = empty_x + kMaxXSlots;            // [a_slots] a chunk of A is in tensor memory
+    uint64_t* a_free = a_full + kMaxASlots;             // [a_slots] the MMAs reading it are done
+    uint64_t* full_m = a_free + kMaxASlots;             // [meta_bufs] scales / zero points of kMetaGroups groups have landed
+    uint64_t* empty_m = full_m + kMaxMetaBufs;          // [meta_bufs] every dequantise warp is done with them
+    uint64_t* d_full = empty_m + kMaxMetaBufs;          // the item's accumulator is complete
     uint64_t* d_free = d_full + 1;                      // the epilogue has read the accumulator
     uint64_t* red_bar = d_free + 1;                     // first CTA of a cluster: the other CTAs' partial sums have arrived
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbase + 512);
-    float* inv_rms = reinterpret_cast<float*>(sbase + 576);      // [B <= 64]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbase + 768);
     const uint32_t stage0 = base + 1024;
-    const uint32_t xt0 = base + p.off_xt;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t rank = p.split > 1 ? cluster_rank() : 0u;
-    const int cluster_id = (int)blockIdx.x / p.split;
-    const int n_clusters = (int)gridDim.x / p.split;
+    const int first_item = (int)blockIdx.x / p.split;
+    const int item_step = (int)gridDim.x / p.split;
     const int st_lo = (int)((int64_t)p.n_stage_total * rank / p.split);
     const int st_hi = (int)((int64_t)p.n_stage_total * (rank + 1) / p.split);
     const int n_st = st_hi - st_lo;
-    const int my_tiles = cluster_id < p.tiles ? (p.tiles - cluster_id + n_clusters - 1) / n_clusters : 0;
+    const int my_items = first_item < p.items ? (p.items - first_item + item_step - 1) / item_step : 0;
     const int NS = p.stages;
     const int NA = p.a_slots;
-    const int XT = p.x_tiles;
+    const int XS = p.x_slots;
     const int ncols = p.ncols;
-    const int B = p.B;
+    auto row_of = [&](int it) { return (first_item + it * item_step) / p.nblk * kRows; };        // column blocks of a tile run side by side
+    auto col_of = [&](int it) { return (first_item + it * item_step) % p.nblk * ncols; };
 
-    // ---- set-up: barriers, tensor memory, zeroed operand tiles (rows >= B stay zero for good) ----
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < NS; ++i) {
-            mbar_init(&full_w[i], 1);
-            mbar_init(&empty_w[i], GPS * 4);
+    if (warp == kMmaWarp) {
+        if (lane < NS) { mbar_init(&full_w[lane], 1); mbar_init(&empty_w[lane], GPS * 4); }
+        if (lane < XS) { mbar_init(&full_x[lane], 1); mbar_init(&empty_x[lane], 1); }
+        if (lane < NA) { mbar_init(&a_full[lane], 4); mbar_init(&a_free[lane], 1); }
+        if (META && lane < p.meta_bufs) { mbar_init(&full_m[lane], 1); mbar_init(&empty_m[lane], kDeqWarps); }
+        if (lane == 0) {
+            mbar_init(d_full, 1);
+            mbar_init(d_free, kDeqWarps);
+            mbar_init(red_bar, p.split > 1 ? (uint32_t)(p.split - 1) * kDeqWarps * 32u : 1u);
         }
-        for (int i = 0; i < XT; ++i) {
-            mbar_init(&full_x[i], 1);
-            mbar_init(&empty_x[i], 1);
-            mbar_init(&x_tma[i], 1);
-        }
-        for (int i = 0; i < NA; ++i) {
-            mbar_init(&a_full[i], 4);
-            mbar_init(&a_free[i], 1);
-        }
-        mbar_init(d_full, 1);
-        mbar_init(d_free, 4);
-        mbar_init(red_bar, p.split > 1 ? (uint32_t)(p.split - 1) * 128u : 1u);
         mbar_fence_init();
     }
-    if (warp == kTmaWarp) tmem_alloc(tmem_slot, (uint32_t)p.tmem_cols);
-    for (uint32_t o = threadIdx.x * 16u; o < (uint32_t)XT * p.xt_bytes; o += kThreads * 16u)
-        sts128(xt0 + o, make_uint4(0u, 0u, 0u, 0u));
-    fence_async_smem();
+    if (warp == kTmaWarp) tmem_alloc(tmem_slot, 512u);
     tc_fence_before();
     __syncthreads();
     if (p.split > 1) cluster_sync_all();      // every CTA's barriers exist before a neighbour arrives on one
@@ -381,327 +346,261 @@ __global__ void __launch_bounds__(ts_threads(WHOLE), WHOLE ? 1 : 2) qgemm_ts_ker
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
     pdl_launch_dependents();
 
-    // ================================ TMA producer ================================================
+    // ================================ weight producer =============================================
     if (warp == kTmaWarp) {
+        if (lane == 0) {
+            bool ok = true;
+            int slot = 0, mslot = 0;
+            uint32_t par = 0, mpar = 0;
+            const uint32_t meta_tx = MATS * kMetaTile * (p.has_z ? 2 : 1);
+            for (int it = 0; it < my_items; ++it) {
+                const int n0 = row_of(it);
+                for (int s = st_lo; s < st_hi; ++s) {
+                    if (META && (s == st_lo || s % MS == 0)) {      // scales / zero points of the next MS stages
+                        wait_bar(&empty_m[mslot], mpar ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
+                        uint8_t* mb = sbase + p.off_meta + (size_t)mslot * kMetaBuf;
+                        mbar_arrive_expect_tx(&full_m[mslot], meta_tx);
+                        const int gx = s / MS * (kMetaGroups * 2);
+#pragma unroll
+                        for (int m = 0; m < MATS; ++m) {
+                            tma_load_2d(mb + m * 2 * kMetaTile, &p.smap[m], gx, n0, &full_m[mslot]);
+                            if (p.has_z) tma_load_2d(mb + m * 2 * kMetaTile + kMetaTile, &p.zmap[m], gx, n0, &full_m[mslot]);
+                        }
+                        if (++mslot == p.meta_bufs) { mslot = 0; mpar ^= 1u; }
+                    }
+                    wait_bar(&empty_w[slot], par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
+                    uint8_t* st = sbase + 1024 + (size_t)slot * p.stage_bytes;
+                    mbar_arrive_expect_tx(&full_w[slot], MATS * kWTile);
+#pragma unroll
+                    for (int m = 0; m < MATS; ++m) tma_load_2d(st + m * kWTile, &p.wmap[m], s * kRowBytes, n0, &full_w[slot]);
+                    if (++slot == NS) { slot = 0; par ^= 1u; }
+                }
+            }
+        }
+    }
+    // ================================ row producer ================================================
+    else if (warp == kRowWarp) {
+        pdl_wait();                           // the activations belong to the previous kernel until here
         if (lane == 0) {
             bool ok = true;
             int slot = 0;
             uint32_t par = 0;
-            const uint32_t tx = MATS * (kWTile + kMetaTile * (p.has_z ? 2 : 1));
-            for (int ti = 0; ti < my_tiles; ++ti) {
-                const int n0 = (cluster_id + ti * n_clusters) * kRows;
-                for (int s = st_lo; s < st_hi; ++s) {
-                    wait_bar(&empty_w[slot], par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
-                    uint8_t* st = sbase + 1024 + (size_t)slot * p.stage_bytes;
-                    mbar_arrive_expect_tx(&full_w[slot], tx);
-                    const int gx = (((s * KS) >> LOGG) * 2) & ~15;          // byte column of the stage's scales
-#pragma unroll
-                    for (int m = 0; m < MATS; ++m) {
-                        tma_load_2d(st + m * kWTile, &p.wmap[m], s * kRowBytes, n0, &full_w[slot]);
-                        tma_load_2d(st + p.off_meta + m * 2 * kMetaTile, &p.smap[m], gx, n0, &full_w[slot]);
-                        if (p.has_z)
-                            tma_load_2d(st + p.off_meta + m * 2 * kMetaTile + kMetaTile, &p.zmap[m], gx, n0, &full_w[slot]);
-                    }
-                    if (++slot == NS) { slot = 0; par ^= 1u; }
+            for (int it = 0; it < my_items; ++it) {
+                const int c0 = col_of(it);
+                for (int ch = st_lo * SC; ch < st_hi * SC; ++ch) {
+                    wait_bar(&empty_x[slot], par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
+                    uint8_t* dst = sbase + p.off_x + (size_t)slot * p.x_bytes;
+                    mbar_arrive_expect_tx(&full_x[slot], p.x_bytes);
+                    tma_load_2d(dst, &p.xmap, ch * kChunkK * 2, c0, &full_x[slot]);                       // byte coordinates
+                    tma_load_2d(dst + (p.x_bytes >> 1), &p.xmap, ch * kChunkK * 2 + 128, c0, &full_x[slot]);
+                    if (++slot == XS) { slot = 0; par ^= 1u; }
                 }
             }
         }
     }
     // ================================ MMA issuer ==================================================
     else if (warp == kMmaWarp) {
-        {
-            bool ok = true;
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
-            // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart, descriptor version 1
-            const uint64_t desc_hi = ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61) | (1ull << 16);
-            int xslot = 0, a_slot = 0;
-            uint32_t xpar = 0, a_par = 0;
-            const uint32_t a_base = tmem + (uint32_t)p.a_col0;
-            const uint32_t atom16 = (uint32_t)(ncols * 128) >> 4;      // distance of two 64-k atoms of the tile, in 16-byte units
-            for (int ti = 0; ti < my_tiles; ++ti) {
-                if (ti > 0) wait_bar(d_free, (uint32_t)(ti - 1) & 1u, EV_GEMV_EMPTY_WAIT, ok);
-                tc_fence_after();
-                for (int sl = 0; sl < n_st; ++sl) {
-                    wait_bar(&full_x[xslot], xpar, EV_GEMV_FULL_WAIT, ok);
-                    const uint32_t xb = xt0 + (uint32_t)xslot * p.xt_bytes;
-                    // descriptor of the first K step of the stage's operand tile; the later steps are constant offsets
-                    const uint64_t desc0 = desc_hi | (uint64_t)((xb & 0x3FFFFu) >> 4);
-#pragma unroll
-                    for (int u = 0; u < APS; ++u) {
-                        const int c = u / MATS, m = u % MATS;
-                        wait_bar(&a_full[a_slot], a_par, EV_GEMV_FULL_WAIT, ok);
-                        tc_fence_after();
-                        const uint32_t a_t = a_base + (uint32_t)a_slot * kChunkCols;
-                        const uint32_t d_t = tmem + (uint32_t)(m * ncols);
-                        const uint64_t desc_c = desc0 + (uint64_t)(c * 2) * atom16;
-                        tc_mma_ts(d_t, a_t, desc_c, idesc, (sl == 0 && c == 0) ? 0u : 1u);
-#pragma unroll
-                        for (int i = 1; i < kChunkK / 16; ++i)
-                            tc_mma_ts(d_t, a_t + i * 8, desc_c + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
-                        tc_commit(&a_free[a_slot]);
-                        if (++a_slot == NA) { a_slot = 0; a_par ^= 1u; }
-                    }
-                    tc_commit(&empty_x[xslot]);
-                    if (++xslot == XT) { xslot = 0; xpar ^= 1u; }
-                }
-                tc_commit(d_full);
-            }
-        }
-    }
-    // ================================ activation warps ============================================
-    else if (warp >= kXWarp0) {
-        pdl_wait();
-        const int xw = warp - kXWarp0;
-        constexpr int PPR = KS / 8;                            // 16-byte pieces per batch row and stage
-        const int n_pieces = B * PPR;
-        const int total_st = my_tiles * n_st;
-        const uint32_t res0 = base + p.off_res;
-        // Every activation warp owns the stages q = xw, xw + kXWarps, ... (the fixed cost of finishing a stage - waits,
-        // proxy fence, arrival - is then paid once per kXWarps stages).  One TMA copy per 64 k puts the stage's rows
-        // straight into the operand tile (the 128-byte swizzle of the copy IS the operand layout); the warp then
-        // rewrites the pieces in place where needed (order of the codes for q4, rmsnorm) and hands the tile to the
-        // MMA warp.  With more tiles than activation warps the copies of the warp's next stage are in flight while
-        // it finishes the current one.
-        const int my_total = total_st > xw ? (total_st - xw + kXWarps - 1) / kXWarps : 0;
-        const int ahead = (XT > kXWarps && my_total > 1) ? 1 : 0;
         bool ok = true;
-        auto tile_addr = [&](uint32_t tile, int idx) -> uint32_t {
-            const int b = idx / PPR;
-            const int pc = idx - b * PPR;
-            return tile + (uint32_t)(pc >> 3) * (uint32_t)(ncols * 128) + (uint32_t)(b >> 3) * 1024u + (uint32_t)(b & 7) * 128u +
-                   (uint32_t)(((pc & 7) ^ (b & 7)) << 4);
-        };
-        const uint32_t x_tx = (uint32_t)B * KS * 2 * (p.res_in != nullptr ? 2u : 1u);
-        auto issue = [&](int q) {
-            const int slot = q % XT;
-            // the tile may still be read by the MMAs of the stage that used the slot before
-            wait_bar(&empty_x[slot], (((uint32_t)q / (uint32_t)XT) & 1u) ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
-            if (lane == 0) {
-                uint8_t* tile = sbase + p.off_xt + (size_t)slot * p.xt_bytes;
-                uint8_t* res = sbase + p.off_res + (size_t)slot * p.res_bytes;
-                const int k0 = (st_lo + q % n_st) * KS;
-                mbar_arrive_expect_tx(&x_tma[slot], x_tx);
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+        // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart, descriptor version 1
+        const uint64_t desc_hi = ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61) | (1ull << 16);
+        int xslot = 0, a_slot = 0;
+        uint32_t xpar = 0, a_par = 0;
+        const uint32_t a_base = tmem + (uint32_t)p.a_col0;
+        const uint32_t x0 = base + p.off_x;
+        const uint32_t atom16 = (p.x_bytes >> 1) >> 4;                 // distance of the two 64-k atoms of a chunk, in 16-byte units
+        const int n_ch = n_st * SC;
+        for (int it = 0; it < my_items; ++it) {
+            if (it > 0) wait_bar(d_free, (uint32_t)(it - 1) & 1u, EV_GEMV_EMPTY_WAIT, ok);
+            tc_fence_after();
+            for (int ch = 0; ch < n_ch; ++ch) {
+                wait_bar(&full_x[xslot], xpar, EV_GEMV_FULL_WAIT, ok);
+                const uint64_t desc0 = desc_hi | (uint64_t)(((x0 + (uint32_t)xslot * p.x_bytes) & 0x3FFFFu) >> 4);
 #pragma unroll
-                for (int at = 0; at < KS / 64; ++at) {
-                    tma_load_2d(tile + (size_t)at * ncols * 128, &p.xmap, (k0 + at * 64) * 2, 0, &x_tma[slot]);      // byte coordinates
-                    if (p.res_in != nullptr) tma_load_2d(res + (size_t)at * B * 128, &p.rmap, (k0 + at * 64) * 2, 0, &x_tma[slot]);
+                for (int m = 0; m < MATS; ++m) {
+                    wait_bar(&a_full[a_slot], a_par, EV_GEMV_FULL_WAIT, ok);
+                    tc_fence_after();
+                    const uint32_t a_t = a_base + (uint32_t)a_slot * kChunkCols;
+                    const uint32_t d_t = tmem + (uint32_t)(m * ncols);
+                    tc_mma_ts(d_t, a_t, desc0, idesc, ch == 0 ? 0u : 1u);
+#pragma unroll
+                    for (int i = 1; i < kChunkK / 16; ++i)
+                        tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
+                    tc_commit(&a_free[a_slot]);
+                    if (++a_slot == NA) { a_slot = 0; a_par ^= 1u; }
                 }
+                tc_commit(&empty_x[xslot]);
+                if (++xslot == XS) { xslot = 0; xpar ^= 1u; }
             }
-            __syncwarp();
-        };
-        if (my_total > 0) issue(xw);
-        // rmsnorm prologue: one warp per batch row; with more rows than activation warps the dequantise warps take
-        // their share (they cannot get far before the first operand tile exists anyway)
-        if (p.norm_w != nullptr) {
-            const bool shared = B > kXWarps;
-            const int nw = shared ? kXWarps + DW : kXWarps;
-            for (int b = xw; b < B; b += nw) {
-                const float inv = row_inv_rms(p, b, lane);
-                if (lane == 0) inv_rms[b] = inv;
-            }
-            named_bar_sync(1, nw * 32);
-        }
-        const bool writes_side = cluster_id == 0;              // the cluster of tile 0 covers the whole K range
-        for (int j = 0, q = xw; j < my_total; ++j, q += kXWarps) {
-            if (ahead) {
-                if (j + 1 < my_total) issue(q + kXWarps);
-            } else if (j > 0) {
-                issue(q);                                       // no spare tile: copy, then finish, one stage at a time
-            }
-            const int slot = q % XT;
-            wait_bar(&x_tma[slot], ((uint32_t)q / (uint32_t)XT) & 1u, EV_GEMV_FULL_WAIT, ok);
-            const uint32_t tile = xt0 + (uint32_t)slot * p.xt_bytes;
-            const uint32_t res = res0 + (uint32_t)slot * p.res_bytes;
-            const int k0 = (st_lo + q % n_st) * KS;
-            if (p.norm_w == nullptr) {
-                if (BITS == 4) {
-                    // q4: piece (row i, lane) of the tile; the order in which the dequantise warps emit the 8 codes of a
-                    // 32-bit word is (0,4) (1,5) (2,6) (3,7).  Four pieces in flight per lane.
-                    const uint32_t lane_base = tile + (uint32_t)(lane >> 3) * (uint32_t)(ncols * 128) + (uint32_t)((lane & 7) << 4);
-                    for (int i0 = 0; i0 < B; i0 += 4) {
-                        uint4 u[4];
-                        uint32_t addr[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int i = i0 + e < B ? i0 + e : i0;
-                            addr[e] = (lane_base ^ (uint32_t)((i & 7) << 4)) + (uint32_t)(i >> 3) * 1024u + (uint32_t)(i & 7) * 128u;
-                            u[e] = lds128(addr[e]);
-                        }
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            u[e] = make_uint4(prmt(u[e].x, u[e].z, 0x5410), prmt(u[e].x, u[e].z, 0x7632), prmt(u[e].y, u[e].w, 0x5410),
-                                              prmt(u[e].y, u[e].w, 0x7632));
-                            if (i0 + e < B) sts128(addr[e], u[e]);
-                        }
-                    }
-                }
-            } else {
-                // rows z = cast(x + residual), then cast(z * inv_rms * w): a lane meets the same 8 k of every row it
-                // handles (32 % PPR == 0), so the norm weights are fetched once per stage
-                const int pc = lane % PPR;
-                const int k = k0 + pc * 8;
-                float w8[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) w8[i] = load_as_f32(p.norm_w, p.norm_w_dtype, k + i);
-                const bool side = q < n_st && writes_side;          // first tile of the cluster that owns tile 0
-                for (int idx = lane; idx < n_pieces; idx += 32) {
-                    const int b = idx / PPR;
-                    const uint32_t addr = tile_addr(tile, idx);
-                    uint4 u = lds128(addr);
-                    const __half2* hx = reinterpret_cast<const __half2*>(&u);
-                    float v[8];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) { v[2 * i] = __low2float(hx[i]); v[2 * i + 1] = __high2float(hx[i]); }
-                    if (p.res_in != nullptr) {
-                        const uint4 ur = lds128(res + (uint32_t)(pc >> 3) * (uint32_t)(B * 128) + (uint32_t)b * 128u + (uint32_t)((pc & 7) << 4));
-                        const __half2* hr = reinterpret_cast<const __half2*>(&ur);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            v[2 * i] = __half2float(__float2half_rn(v[2 * i] + __low2float(hr[i])));
-                            v[2 * i + 1] = __half2float(__float2half_rn(v[2 * i + 1] + __high2float(hr[i])));
-                        }
-                    }
-                    if (side && p.z_out != nullptr) {
-                        __half2 zo[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) zo[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-                        *reinterpret_cast<uint4*>(p.z_out + (size_t)b * p.K + k) = *reinterpret_cast<const uint4*>(zo);
-                    }
-                    const float inv = inv_rms[b];
-                    __half2 no[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) no[i] = __floats2half2_rn(v[2 * i] * inv * w8[2 * i], v[2 * i + 1] * inv * w8[2 * i + 1]);
-                    u = *reinterpret_cast<const uint4*>(no);
-                    if (side && p.normed_out != nullptr) *reinterpret_cast<uint4*>(p.normed_out + (size_t)b * p.K + k) = u;
-                    if (BITS == 4)
-                        u = make_uint4(prmt(u.x, u.z, 0x5410), prmt(u.x, u.z, 0x7632), prmt(u.y, u.w, 0x5410), prmt(u.y, u.w, 0x7632));
-                    sts128(addr, u);
-                }
-            }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full_x[slot]);
+            tc_commit(d_full);
         }
     }
-    // ================================ dequantise warps (+ epilogue on warps 0-3) ===================
+    // ================================ dequantise warps + epilogue =================================
     else {
-        const int grp = warp >> 2;                             // chunks a with a % NG == grp
+        const int grp = warp >> 2;
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;                     // weight row inside the tile = lane of tensor memory
         const uint32_t sw = (uint32_t)(r & 7);
+        const uint32_t msw = (uint32_t)((r >> 2) & 1) << 4;    // 32-byte swizzle of the scale tiles
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+        const uint32_t row_u = stage0 + (uint32_t)r * kRowBytes;
         bool ok = true;
-        bool waited_pdl = false;
-        if (p.norm_w != nullptr && B > kXWarps) {
-            pdl_wait();
-            waited_pdl = true;
-            for (int b = kXWarps + warp; b < B; b += kXWarps + DW) {
-                const float inv = row_inv_rms(p, b, lane);
-                if (lane == 0) inv_rms[b] = inv;
-            }
-            named_bar_sync(1, (kXWarps + DW) * 32);
-        }
-        uint32_t a0 = 0;                     // index of the first chunk of A of the current stage (counted over the kernel)
-        int slot = 0, t = grp % NA;          // ring positions of the stage and of this group's next chunk of A
-        uint32_t par = 0, a_par = (uint32_t)(grp / NA) & 1u;
-        for (int ti = 0; ti < my_tiles; ++ti) {
-            const int n0 = (cluster_id + ti * n_clusters) * kRows;
-            for (int s = st_lo; s < st_hi; ++s, a0 += APS) {
-                // this group's chunks of the stage: u with (a0 + u) % NG == grp
-                const int u0 = (int)((grp - (int)(a0 & (NG - 1)) + NG) & (NG - 1));
-                if (u0 < APS) {
-                    wait_bar(&full_w[slot], par, EV_GEMV_FULL_WAIT, ok);
-                    const uint32_t st = stage0 + slot * p.stage_bytes;
-#pragma unroll 1
-                    for (int u = u0; u < APS; u += NG) {
-                        const int c = u / MATS, m = u % MATS;
-                        wait_bar(&a_free[t], a_par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
-                        tc_fence_after();
-                        const uint32_t wrow = st + m * kWTile + (uint32_t)r * kRowBytes;
-                        const uint32_t mrow = st + p.off_meta + m * 2 * kMetaTile + (uint32_t)r * 16;
-                        const int g0 = ((s * KS + c * kChunkK) >> LOGG) & 7;      // first group of the chunk inside the scale tile
-                        // scales / zero points of the chunk's groups (1, 2 or 4 halves)
-                        uint32_t sreg[2] = {0u, 0u}, zreg[2] = {0u, 0u};
-                        if (LOGG == 5) {
-                            sreg[0] = lds32(mrow + g0 * 2); sreg[1] = lds32(mrow + g0 * 2 + 4);
-                            if (p.has_z) { zreg[0] = lds32(mrow + kMetaTile + g0 * 2); zreg[1] = lds32(mrow + kMetaTile + g0 * 2 + 4); }
-                        } else {
-                            const uint32_t sa = lds32(mrow + ((g0 * 2) & ~3));
-                            sreg[0] = (LOGG == 7 && (g0 & 1)) ? sa >> 16 : sa;
-                            if (p.has_z) {
-                                const uint32_t za = lds32(mrow + kMetaTile + ((g0 * 2) & ~3));
-                                zreg[0] = (LOGG == 7 && (g0 & 1)) ? za >> 16 : za;
-                            }
+        int t = grp % NA;                                      // A slot of this group's next chunk
+        uint32_t a_par = (uint32_t)(grp / NA) & 1u;
+        int slot = 0;                                          // weight slot of stage `sl_at`
+        uint32_t par = 0;
+        int mslot = 0;
+        uint32_t mpar = 0;
+        const int n_ch = n_st * APS;                           // chunks of an item
+        for (int it = 0; it < my_items; ++it) {
+            const int n0 = row_of(it);
+            int sl_at = 0;                                     // stage of the item that `slot` stands for
+            int mt_at = 0;                                     // scale tile of the item that `mslot` stands for
+            bool m_waited = false;
+            const int mt0 = st_lo / MS;
+            // scales and zero points of a chunk, read directly (META == false): one chunk ahead of their use
+            uint32_t ns[2] = {0u, 0u}, nz[2] = {0u, 0u};
+            auto fetch_meta = [&](int q) {
+                const int s = st_lo + q / APS, u = q % APS, c = u / MATS, m = u % MATS;
+                const int gi = (s * KS + c * kChunkK) >> LOGG;
+                ns[0] = ns[1] = nz[0] = nz[1] = 0u;
+                if (n0 + r < p.N) {
+                    const size_t at = (size_t)(n0 + r) * p.Gn + gi;
+#pragma unroll
+                    for (int j = 0; j < CGR; ++j)
+                        if (gi + j < p.Gn) {
+                            ns[j >> 1] |= (uint32_t)__ldg(p.s[m] + at + j) << (16 * (j & 1));
+                            if (p.has_z) nz[j >> 1] |= (uint32_t)__ldg(p.z[m] + at + j) << (16 * (j & 1));
                         }
-                        const uint32_t a_t = lane_addr + (uint32_t)(p.a_col0 + t * kChunkCols);
+                }
+            };
+            const int a0 = (int)((uint32_t)it * (uint32_t)n_ch & (uint32_t)(NG - 1));      // chunk number of the item's first, modulo NG
+            const int q0 = (grp - a0 + NG) & (NG - 1);
+            if (!META && q0 < n_ch) fetch_meta(q0);
+#pragma unroll 1
+            for (int q = q0; q < n_ch; q += NG) {
+                const int sl = q / APS, u = q % APS;
+                const int s = st_lo + sl;
+                const int c = u / MATS, m = u % MATS;
+                slot += sl - sl_at;                            // at most NG / APS stages on
+                sl_at = sl;
+                while (slot >= NS) { slot -= NS; par ^= 1u; }
+                uint32_t sreg[2], zreg[2];
+                if (META) {
+                    const int mt = s / MS - mt0;
+                    while (mt_at < mt) {                       // done with the scale tiles before (also one without a chunk of this group)
+                        if (!m_waited) wait_bar(&full_m[mslot], mpar, EV_GEMV_FULL_WAIT, ok);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&empty_m[mslot]);
+                        if (++mslot == p.meta_bufs) { mslot = 0; mpar ^= 1u; }
+                        ++mt_at;
+                        m_waited = false;
+                    }
+                    if (!m_waited) wait_bar(&full_m[mslot], mpar, EV_GEMV_FULL_WAIT, ok);
+                    m_waited = true;
+                    const int g0 = ((s * KS + c * kChunkK) >> LOGG) & (kMetaGroups - 1);      // first group of the chunk inside the scale tile
+                    const uint32_t mrow = base + p.off_meta + (uint32_t)mslot * kMetaBuf + (uint32_t)(m * 2 * kMetaTile) +
+                                          (uint32_t)r * (kMetaGroups * 2) + (((uint32_t)g0 * 2 & ~3u) ^ msw);
+                    sreg[0] = lds32(mrow);
+                    sreg[1] = LOGG == 5 ? lds32(mrow + 4) : 0u;
+                    zreg[0] = zreg[1] = 0u;
+                    if (p.has_z) {
+                        zreg[0] = lds32(mrow + kMetaTile);
+                        if (LOGG == 5) zreg[1] = lds32(mrow + kMetaTile + 4);
+                    }
+                    if (LOGG == 7 && (g0 & 1)) { sreg[0] >>= 16; zreg[0] >>= 16; }
+                } else {
+                    sreg[0] = ns[0]; sreg[1] = ns[1]; zreg[0] = nz[0]; zreg[1] = nz[1];
+                    if (q + NG < n_ch) fetch_meta(q + NG);
+                }
+                wait_bar(&full_w[slot], par, EV_GEMV_FULL_WAIT, ok);
+                const uint32_t wrow = row_u + (uint32_t)slot * p.stage_bytes + (uint32_t)(m * kWTile);
+                const uint32_t a_t = lane_addr + (uint32_t)(p.a_col0 + t * kChunkCols);
+                wait_bar(&a_free[t], a_par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
+                tc_fence_after();
 #pragma unroll
-                        for (int hb = 0; hb < 2; ++hb) {            // halves of the chunk: 64 k -> 32 columns
-                            uint32_t out[32];
+                for (int hb = 0; hb < 2; ++hb) {               // halves of the chunk: 64 k -> 32 columns
+                    uint32_t out[32];
+                    GroupConst gc;
 #pragma unroll
-                            for (int sb = 0; sb < 2; ++sb) {        // 32 k -> 16 columns
-                                const int k32 = hb * 2 + sb;        // 32-k block of the chunk
-                                const int gi = (k32 * 32) >> LOGG;  // group of the chunk (0 for G = 128)
-                                const uint32_t sbits = (gi & 1) ? sreg[gi >> 1] >> 16 : sreg[gi >> 1];
-                                const uint32_t zbits = (gi & 1) ? zreg[gi >> 1] >> 16 : zreg[gi >> 1];
-                                const GroupConst gc = group_const(sbits & 0xFFFFu, zbits & 0xFFFFu);
-                                if (BITS == 4) {
-                                    const uint4 v = lds128(wrow + ((((uint32_t)(c * 4 + k32)) ^ sw) << 4));
-                                    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+                    for (int sb = 0; sb < 2; ++sb) {           // 32 k -> 16 columns
+                        const int k32 = hb * 2 + sb;           // 32-k block of the chunk
+                        const int gi = (k32 * 32) >> LOGG;     // group of the chunk
+                        if (sb == 0 || LOGG == 5)
+                            gc = group_const<BITS>((gi & 1) ? sreg[gi >> 1] >> 16 : sreg[gi >> 1], (gi & 1) ? zreg[gi >> 1] >> 16 : zreg[gi >> 1]);
+                        if (BITS == 4) {
+                            const uint4 v = lds128(wrow + ((((uint32_t)(c * 4 + k32)) ^ sw) << 4));
+                            const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                                    for (int w = 0; w < 4; ++w) {
-                                        const uint32_t lo = w4[w], hi = w4[w] >> 8;
-                                        out[sb * 16 + 4 * w + 0] = hfma2_u32(hadd2_u32(lop3_and_or(lo, 0x000F000Fu, 0x64006400u), gc.c1024), gc.s2, gc.r2);
-                                        out[sb * 16 + 4 * w + 1] = hfma2_u32(hadd2_u32(lop3_and_or(lo, 0x00F000F0u, 0x54005400u), gc.c64), gc.s2, gc.r2);
-                                        out[sb * 16 + 4 * w + 2] = hfma2_u32(hadd2_u32(lop3_and_or(hi, 0x000F000Fu, 0x64006400u), gc.c1024), gc.s2, gc.r2);
-                                        out[sb * 16 + 4 * w + 3] = hfma2_u32(hadd2_u32(lop3_and_or(hi, 0x00F000F0u, 0x54005400u), gc.c64), gc.s2, gc.r2);
-                                    }
-                                } else {
+                            for (int w = 0; w < 4; ++w) {
+                                // byte j of the word holds k = 2j (low nibble) and 2j + 1: [byte, 0x64, byte, 0x54], nibbles masked
+                                const uint32_t p0 = prmt(w4[w], 0x00005464u, 0x5040) & 0xFFF0FF0Fu, p1 = prmt(w4[w], 0x00005464u, 0x5141) & 0xFFF0FF0Fu;
+                                const uint32_t p2 = prmt(w4[w], 0x00005464u, 0x5242) & 0xFFF0FF0Fu, p3 = prmt(w4[w], 0x00005464u, 0x5343) & 0xFFF0FF0Fu;
+                                out[sb * 16 + 4 * w + 0] = hfma2_u32(hadd2_u32(p0, gc.c), gc.s2, gc.r2);
+                                out[sb * 16 + 4 * w + 1] = hfma2_u32(hadd2_u32(p1, gc.c), gc.s2, gc.r2);
+                                out[sb * 16 + 4 * w + 2] = hfma2_u32(hadd2_u32(p2, gc.c), gc.s2, gc.r2);
+                                out[sb * 16 + 4 * w + 3] = hfma2_u32(hadd2_u32(p3, gc.c), gc.s2, gc.r2);
+                            }
+                        } else {
 #pragma unroll
-                                    for (int q16 = 0; q16 < 2; ++q16) {
-                                        const uint4 v = lds128(wrow + ((((uint32_t)(k32 * 2 + q16)) ^ sw) << 4));
-                                        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+                            for (int q16 = 0; q16 < 2; ++q16) {
+                                const uint4 v = lds128(wrow + ((((uint32_t)(k32 * 2 + q16)) ^ sw) << 4));
+                                const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                                        for (int w = 0; w < 4; ++w) {
-                                            out[sb * 16 + q16 * 8 + 2 * w] = hfma2_u32(hadd2_u32(prmt(w4[w], 0x64646464u, 0x4140u), gc.c1024), gc.s2, gc.r2);
-                                            out[sb * 16 + q16 * 8 + 2 * w + 1] = hfma2_u32(hadd2_u32(prmt(w4[w], 0x64646464u, 0x4342u), gc.c1024), gc.s2, gc.r2);
-                                        }
-                                    }
+                                for (int w = 0; w < 4; ++w) {
+                                    out[sb * 16 + q16 * 8 + 2 * w] = hfma2_u32(hadd2_u32(prmt(w4[w], 0x64646464u, 0x4140u), gc.c), gc.s2, gc.r2);
+                                    out[sb * 16 + q16 * 8 + 2 * w + 1] = hfma2_u32(hadd2_u32(prmt(w4[w], 0x64646464u, 0x4342u), gc.c), gc.s2, gc.r2);
                                 }
                             }
-                            tc_st32(a_t + hb * 32, out);
                         }
-                        tc_wait_st();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&a_full[t]);
-                        t += NG;
-                        while (t >= NA) { t -= NA; a_par ^= 1u; }
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty_w[slot]);
+                    tc_st32(a_t + hb * 32, out);
                 }
-                if (++slot == NS) { slot = 0; par ^= 1u; }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty_w[slot]);
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&a_full[t]);
+                t += NG;
+                while (t >= NA) { t -= NA; a_par ^= 1u; }
             }
-            // ---- epilogue of the tile (split == 1; with a split K range it follows the cluster exchange below) ----
-            if (warp < 4 && p.split == 1) {
-                if (!waited_pdl) { pdl_wait(); waited_pdl = true; }
-                const int n = n0 + r;
-                float res[32];
-                ts_load_residual<MATS>(p, n, res);
-                wait_bar(d_full, (uint32_t)ti & 1u, EV_GEMV_FULL_WAIT, ok);
-                tc_fence_after();
-                {
+            // step over the rest of the item's stages and scale tiles
+            slot += n_st - sl_at;
+            while (slot >= NS) { slot -= NS; par ^= 1u; }
+            if (META && n_st > 0) {
+                const int mt_end = (st_hi - 1) / MS - mt0 + 1;
+                while (mt_at < mt_end) {
+                    if (!m_waited) wait_bar(&full_m[mslot], mpar, EV_GEMV_FULL_WAIT, ok);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty_m[mslot]);
+                    if (++mslot == p.meta_bufs) { mslot = 0; mpar ^= 1u; }
+                    ++mt_at;
+                    m_waited = false;
+                }
+            }
+            // ---- epilogue of the item (split == 1; with a split K range it follows the cluster exchange below): the groups of warps
+            //      take 16-column slices in turn ----
+            if (p.split == 1) {
+                if (it == 0) pdl_wait();
+                const int n = n0 + r, c0 = col_of(it);
+                bool first = true;
+                for (int cs = grp * 16; cs < ncols; cs += NG * 16) {
+                    const int nb = min(16, p.B - c0 - cs);
+                    if (nb <= 0) break;
+                    uint16_t res[16];
+                    ts_load_residual<MATS>(p, n, c0 + cs, nb, res);
+                    if (first) {
+                        wait_bar(d_full, (uint32_t)it & 1u, EV_GEMV_FULL_WAIT, ok);
+                        tc_fence_after();
+                        first = false;
+                    }
                     float acc[MATS][16];
 #pragma unroll
-                    for (int m = 0; m < MATS; ++m) tc_ld16(lane_addr + (uint32_t)(m * ncols), acc[m]);
-                    if (n < p.N) ts_store_cols<MATS, 0>(p, acc, n, res);
+                    for (int m = 0; m < MATS; ++m) tc_ld16(lane_addr + (uint32_t)(m * ncols + cs), acc[m]);
+                    if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, nb, res);
                 }
-                if (ncols > 16 && B > 16) {
-                    float acc[MATS][16];
-#pragma unroll
-                    for (int m = 0; m < MATS; ++m) tc_ld16(lane_addr + (uint32_t)(m * ncols + 16), acc[m]);
-                    if (n < p.N) ts_store_cols<MATS, 16>(p, acc, n, res);
-                }
+                if (first) wait_bar(d_full, (uint32_t)it & 1u, EV_GEMV_FULL_WAIT, ok);      // no slice for this group: stay in step
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(d_free);
@@ -709,81 +608,83 @@ __global__ void __launch_bounds__(ts_threads(WHOLE), WHOLE ? 1 : 2) qgemm_ts_ker
         }
     }
 
-    // ---- split K range: the cluster's partial accumulators are summed in rank order by its first CTA (one tile
-    //      per cluster).  Small batches send only their real columns into a dedicated buffer and signal a barrier
-    //      of the first CTA; otherwise the first CTA's weight ring is reused between two cluster-wide barriers. ----
+    // ---- split K range (one item per cluster): the partial accumulators are summed in rank order by the cluster's first CTA.  Small
+    //      batches send only their real columns into a dedicated buffer and signal a barrier of the first CTA; otherwise the first
+    //      CTA's rings are reused between two cluster-wide barriers. ----
     if (p.split > 1) {
         __syncwarp();
-        const int quarter = warp & 3;
-        const int r = quarter * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+        const int grp = warp >> 2;
+        const int r = (warp & 3) * 32 + lane;
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const bool fast = p.off_red != 0;
-        const int rcols = fast ? B : ncols;                  // columns per matrix that travel
+        const int c0 = col_of(0);
+        const int bcols = min(ncols, p.B - c0);               // real columns of the block
+        const int rcols = fast ? min(ncols, p.B) : ncols;     // columns per matrix and part in the buffer
         const uint32_t red_base = fast ? base + p.off_red : stage0;
-        const bool epi = warp < 4 && my_tiles > 0;
+        const bool epi = warp < kDeqWarps && my_items > 0;
         bool ok = true;
         if (epi) {
             wait_bar(d_full, 0u, EV_GEMV_FULL_WAIT, ok);
             tc_fence_after();
         }
-        if (!fast) cluster_sync_all();      // every CTA of the cluster is done with its ring: the first CTA's ring is free
+        if (!fast) cluster_sync_all();      // every CTA of the cluster is done with its rings: the first CTA's are free
         if (epi && rank != 0) {
             for (int m = 0; m < MATS; ++m)
-                for (int c0 = 0; c0 < rcols; c0 += 16) {
+                for (int cs = grp * 16; cs < bcols; cs += kGroups * 16) {
                     float acc[16];
-                    tc_ld16(lane_addr + (uint32_t)(m * ncols + c0), acc);
+                    tc_ld16(lane_addr + (uint32_t)(m * ncols + cs), acc);
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (c0 + j < rcols)
-                            st_cluster_f32(red_base + (uint32_t)(((((int)rank - 1) * MATS + m) * rcols + c0 + j) * kRows + r) * 4u, 0u, acc[j]);
+                        if (cs + j < bcols)
+                            st_cluster_f32(red_base + (uint32_t)(((((int)rank - 1) * MATS + m) * rcols + cs + j) * kRows + r) * 4u, 0u, acc[j]);
                 }
             if (fast) arrive_remote(smem_u32(red_bar), 0u);
         }
         if (!fast) cluster_sync_all();      // the partial sums are in the first CTA's shared memory
         if (epi && rank == 0) {
             pdl_wait();
-            const int n = cluster_id * kRows + r;
-            float res[32];
-            ts_load_residual<MATS>(p, n, res);
-            if (fast) wait_bar_cluster(red_bar, 0u, ok ? kTsWaitLimit : 64u);
+            const int n = row_of(0) + r;
+            bool first = true;
             const float* red = reinterpret_cast<const float*>(sbase + (red_base - base));
-#pragma unroll
-            for (int c0 = 0; c0 < 32; c0 += 16) {
-                if (c0 >= rcols) break;
+            for (int cs = grp * 16; cs < bcols; cs += kGroups * 16) {
+                const int nb = min(16, bcols - cs);
+                uint16_t res[16];
+                ts_load_residual<MATS>(p, n, c0 + cs, nb, res);
+                if (first && fast) wait_bar_cluster(red_bar, 0u, ok ? kTsWaitLimit : 64u);
+                first = false;
                 float acc[MATS][16];
 #pragma unroll
                 for (int m = 0; m < MATS; ++m) {
-                    tc_ld16(lane_addr + (uint32_t)(m * ncols + c0), acc[m]);
+                    tc_ld16(lane_addr + (uint32_t)(m * ncols + cs), acc[m]);
                     for (int q = 1; q < p.split; ++q)
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
-                            if (c0 + j < rcols) acc[m][j] += red[((((q - 1) * MATS + m) * rcols + c0 + j) * kRows + r)];
+                            if (j < nb) acc[m][j] += red[((((q - 1) * MATS + m) * rcols + cs + j) * kRows + r)];
                 }
-                if (n < p.N) {
-                    if (c0 == 0) ts_store_cols<MATS, 0>(p, acc, n, res);
-                    else ts_store_cols<MATS, 16>(p, acc, n, res);
-                }
+                if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, nb, res);
             }
         }
+        // the first CTA must not leave while its neighbours still store into it
+        if (fast && rank == 0 && epi) wait_bar_cluster(red_bar, 0u, ok ? kTsWaitLimit : 64u);
     }
     tc_fence_before();
     __syncthreads();
     if (warp == kTmaWarp) {
         tc_fence_after();
-        tmem_dealloc(tmem, (uint32_t)p.tmem_cols);
+        tmem_dealloc(tmem, 512u);
     }
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------
 struct MapKey {
-    const void* ptr; uint64_t d0, d1; uint32_t b0, b1; int swz;
+    const void* ptr; uint64_t d0, d1; uint32_t b0, b1, swz;
     bool operator==(const MapKey& o) const { return ptr == o.ptr && d0 == o.d0 && d1 == o.d1 && b0 == o.b0 && b1 == o.b1 && swz == o.swz; }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         size_t h = std::hash<const void*>()(k.ptr);
         h = h * 1000003u ^ std::hash<uint64_t>()(k.d0 * 31 + k.d1);
-        h = h * 1000003u ^ std::hash<uint64_t>()(((uint64_t)k.b0 << 32) | (k.b1 * 2 + k.swz));
+        h = h * 1000003u ^ std::hash<uint64_t>()(((uint64_t)k.b0 << 32) | (k.b1 * 4 + k.swz));
         return h;
     }
 };
@@ -793,8 +694,8 @@ PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
 // 2-D byte tensor [d1 rows, d0 bytes] (rows d0 bytes apart), box b0 x b1.  The driver entry point is looked up at run
 // time, so the library has no link-time dependency on libcuda.
-bool tensor_map_2d(const void* ptr, uint64_t d0, uint64_t d1, uint32_t b0, uint32_t b1, bool swizzle128, CUtensorMap* out) {
-    const MapKey key = {ptr, d0, d1, b0, b1, swizzle128 ? 1 : 0};
+bool tensor_map_2d(const void* ptr, uint64_t d0, uint64_t d1, uint32_t b0, uint32_t b1, CUtensorMapSwizzle swizzle, CUtensorMap* out) {
+    const MapKey key = {ptr, d0, d1, b0, b1, (uint32_t)swizzle};
     std::lock_guard<std::mutex> lock(g_map_mu);
     auto it = g_maps.find(key);
     if (it != g_maps.end()) { *out = it->second; return true; }
@@ -811,7 +712,7 @@ bool tensor_map_2d(const void* ptr, uint64_t d0, uint64_t d1, uint32_t b0, uint3
     const cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;
     const CUresult rc = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                                 CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return false;
     if (g_maps.size() > 4096) g_maps.clear();
@@ -822,85 +723,123 @@ bool tensor_map_2d(const void* ptr, uint64_t d0, uint64_t d1, uint32_t b0, uint3
 
 inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <int BITS, int LOGG, int MATS, bool WHOLE>
-int launch_ts(TsParams& p, cudaStream_t stream) {
-    constexpr int KS = kRowBytes * 8 / BITS;
-    const int sms = sm_count();
-    p.n_stage_total = p.K / KS;
-    p.tiles = (p.N + kRows - 1) / kRows;
-    p.off_meta = MATS * kWTile;
-    p.stage_bytes = MATS * (kWTile + 2 * kMetaTile);
-    p.xt_bytes = (uint32_t)p.ncols * KS * 2;
-    p.res_bytes = p.res_in != nullptr ? (uint32_t)p.B * KS * 2 : 0u;
-    // compact shape: a CTA stays below half of an SM's shared memory, registers and tensor memory
-    const uint32_t cap = (uint32_t)max_smem_optin();
-    uint32_t budget = WHOLE ? cap : std::min<uint32_t>(cap, 112u * 1024u);
-    const int forced = tuning_get("ts.smem_kb");
-    if (forced > 0) budget = std::min<uint32_t>(cap, (uint32_t)forced * 1024u);
-    // tensor memory: accumulators below, ring of A chunks above
-    const int dcols = MATS * p.ncols;
-    p.a_col0 = std::max(32, (dcols + 31) / 32 * 32);
-    p.tmem_cols = WHOLE ? 512 : 256;
-    p.a_slots = std::min(kMaxASlots, (p.tmem_cols - p.a_col0) / kChunkCols);
-    if (p.a_slots < 2) return B200Q_ERR_UNSUPPORTED;
-    // K split over a cluster when the tiles do not fill the SMs.  The split (and with it the order in which a row's
-    // partial sums are added) must not depend on how many rows THIS launch holds: a tensor-parallel shard of the rows
-    // has to reproduce the unsharded result bit for bit, so the tile count of the unsharded matrix decides
-    // ("ts.tp_world" = number of equal row shards), and the cap below uses no shape-dependent quantity.
-    const int tiles_full = p.tiles * std::max(1, tuning_get("ts.tp_world"));
-    int split = 1;
-    if (tiles_full < sms) split = std::min(8, sms / tiles_full);
-    split = std::max(1, std::min(split, p.n_stage_total / 2));
-    // the partial sums of the other CTAs of a cluster (real batch columns only) must fit 48 KB of the first CTA's
-    // shared memory; like the split itself the bound depends on the batch alone, not on the shape of this launch
-    constexpr uint32_t kRedCap = 48u * 1024u;
-    const uint32_t part_bytes = (uint32_t)MATS * p.B * kRows * 4;
-    if ((uint32_t)(split - 1) * part_bytes > kRedCap) split = std::max(1, std::min(split, 1 + (int)(kRedCap / part_bytes)));
-    const int fs = tuning_get("ts.split");
-    if (fs > 0) split = std::max(1, std::min({fs, 8, p.n_stage_total}));
-    // they arrive in a dedicated buffer signalled by a barrier (whole-SM shape: up to the 48 KB, compact shape: 8 KB),
-    // else in the first CTA's weight ring between two cluster-wide barriers; both add them in rank order
-    const uint32_t red_bytes = (uint32_t)(split - 1) * part_bytes;
-    const bool fast_red = split > 1 && red_bytes <= (WHOLE ? kRedCap : 8192u) && !tuning_get("ts.slow_reduce");
-    const uint32_t red_alloc = fast_red ? (red_bytes + 1023u) / 1024u * 1024u : 0u;
-    // rings: operand tiles (at least as many as activation warps: a warp must never meet a tile slot two uses ahead of
-    // the MMAs; one more lets it keep the copies of its next stage in flight), then as many weight stages as fit
-    constexpr int XW = ts_xwarps(WHOLE);
-    const uint32_t per_tile = p.xt_bytes + p.res_bytes;
-    const uint32_t base_fixed = 2048u + red_alloc;
-    int xt = XW + 2;
-    while (xt > XW && base_fixed + (uint32_t)xt * per_tile + 3 * p.stage_bytes > budget) --xt;
-    p.x_tiles = std::min(xt, kMaxXTiles);
-    const uint32_t fixed = base_fixed + (uint32_t)p.x_tiles * per_tile;
-    if (fixed + 2 * p.stage_bytes > budget) return B200Q_ERR_UNSUPPORTED;
-    int stages = (int)((budget - fixed) / p.stage_bytes);
-    const int want = tuning_get("ts.stages");
-    if (want > 0) stages = std::min(stages, want);
-    stages = std::min(stages, kMaxStages);
-    if (stages < 2) return B200Q_ERR_UNSUPPORTED;
-    p.stages = stages;
-    if (!fast_red && split > 1 && (uint64_t)(split - 1) * dcols * kRows * 4 > (uint64_t)stages * p.stage_bytes)
-        return B200Q_ERR_UNSUPPORTED;      // only with a forced split
-    p.split = split;
-    p.off_xt = 1024u + (uint32_t)stages * p.stage_bytes;
-    p.off_res = p.off_xt + (uint32_t)p.x_tiles * p.xt_bytes;
-    p.off_red = (fast_red && split > 1) ? p.off_res + (uint32_t)p.x_tiles * p.res_bytes : 0u;
-    const int clusters = split > 1 ? p.tiles : std::min(p.tiles, sms);
-    const uint32_t smem = 1024u + p.off_res + (uint32_t)p.x_tiles * p.res_bytes + red_alloc;
+// Clusters of `size` CTAs of one SM each that can be resident together: GPCs are not a multiple of every size.
+template <typename Kernel>
+int max_clusters(Kernel kernel, int size, uint32_t smem) {
+    static int cached[64][9] = {};      // per device; a race only repeats the query (all instantiations have one CTA per SM)
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = cached[dev & 63][size];
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(size);
+        cfg.blockDim = dim3(kTsThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int got = 0;
+        if (cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) != cudaSuccess || got <= 0) {
+            cudaGetLastError();
+            got = std::max(1, sm_count() / size);
+        }
+        n = got;
+    }
+    return n;
+}
 
-    auto kernel = qgemm_ts_kernel<BITS, LOGG, MATS, WHOLE>;
+template <int BITS, int LOGG, int MATS, bool META>
+int launch_ts(TsParams& p, int K, cudaStream_t stream) {
+    constexpr int KS = kRowBytes * 8 / BITS;
+    constexpr int SC = KS / kChunkK;
+    constexpr int MS = (kMetaGroups << LOGG) / KS;         // stages per scale tile
+    constexpr uint32_t kMetaBuf = META ? MATS * 2 * kMetaTile : 0;
+    const int sms = sm_count();
+    const int tiles = (p.N + kRows - 1) / kRows;
+    p.n_stage_total = (K + KS - 1) / KS;
+    p.stage_bytes = MATS * kWTile;
+    auto kernel = qgemm_ts_kernel<BITS, LOGG, MATS, META>;
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
+    const uint32_t cap = (uint32_t)max_smem_optin();
     if (!configured[dev & 63]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess)
             return B200Q_ERR_LAUNCH;
         configured[dev & 63] = true;
     }
+    // Column blocks and K split by estimated time, in clocks: rounds of items over the SMs, each a chain of chunks whose cost is the
+    // dequantisation's or the tensor pipe's (measured: 22 clocks per MMA up to 32 columns, then half a clock per column).  The choice
+    // must not depend on how many rows THIS launch holds: a tensor-parallel shard of the rows has to reproduce the unsharded result
+    // bit for bit, so the tile count of the unsharded matrix decides ("ts.tp_world" = number of equal row shards).
+    const int tiles_full = tiles * std::max(1, tuning_get("ts.tp_world"));
+    const int forced = tuning_get("ts.split");
+    constexpr uint32_t kRedCap = 48u * 1024u;              // bytes of the dedicated buffer for partial sums
+    double best = 0.0;
+    int cols = 0, split = 1;
+    const int nb0 = (p.B + kMaxCols - 1) / kMaxCols;
+    for (int nb = nb0; nb <= (p.B + 15) / 16 && nb <= 4 * nb0; ++nb) {
+        const int c = ((p.B + nb - 1) / nb + 15) / 16 * 16;
+        const int blocks = (p.B + c - 1) / c;
+        if (blocks != nb) continue;                        // the same blocks as a smaller nb
+        const double chunk = std::max(360.0, 8.0 * std::max(22.2, c * 0.5 + 0.8));
+        for (int sp = 1; sp <= 8; sp *= 2) {
+            if (forced > 0 ? sp != std::min(forced, std::max(1, p.n_stage_total)) : sp > 1 && sp > p.n_stage_total / 2) continue;
+            if (forced <= 0 && sp > 1 && (uint32_t)(sp - 1) * MATS * std::min(c, p.B) * kRows * 4 > kRedCap) continue;
+            const int64_t items = (int64_t)tiles_full * blocks;
+            const int slots = sp == 1 ? sms : max_clusters(kernel, sp, cap - 2048u);
+            if (forced <= 0 && sp > 1 && items > slots) continue;
+            const double rounds = (double)((items + slots - 1) / slots);
+            const double t = rounds * ((double)((p.n_stage_total + sp - 1) / sp * SC * MATS) * chunk + 1500.0 + c * MATS * 10.0) + (sp > 1 ? 1500.0 : 0.0);
+            if (cols == 0 || t < best) { best = t; cols = c; split = sp; }
+        }
+    }
+    if (cols == 0) return B200Q_ERR_UNSUPPORTED;
+    p.ncols = cols;
+    p.nblk = (p.B + cols - 1) / cols;
+    p.items = tiles * p.nblk;
+    p.split = split;
+    // tensor memory: accumulators below, ring of A chunks above
+    const int dcols = MATS * cols;
+    p.a_col0 = std::max(32, (dcols + 31) / 32 * 32);
+    p.a_slots = std::min(kMaxASlots, (512 - p.a_col0) / kChunkCols);
+    // partial sums of a K split: a dedicated buffer signalled by a barrier, else the first CTA's rings between two cluster-wide
+    // barriers; both add them in rank order
+    const uint32_t red_bytes = (uint32_t)(split - 1) * MATS * std::min(cols, p.B) * kRows * 4;
+    const bool fast_red = split > 1 && red_bytes <= kRedCap && !tuning_get("ts.slow_reduce");
+    const uint32_t red_alloc = fast_red ? (red_bytes + 1023u) / 1024u * 1024u : 0u;
+    // rings: scale tiles so deep that the producer never waits for one before it waits for a weight stage, then activation chunks
+    // and weight stages share what is left
+    auto meta_bufs_for = [](int stages) { return META ? std::min(kMaxMetaBufs, (stages + MS - 1) / MS + 1) : 0; };
+    p.x_bytes = (uint32_t)cols * kChunkK * 2;
+    const uint32_t budget = cap - 2048u - red_alloc;       // 1 KB of barriers, up to 1 KB of alignment
+    auto need = [&](int xs, int stages) {
+        return (uint32_t)xs * p.x_bytes + (uint32_t)stages * p.stage_bytes + (uint32_t)meta_bufs_for(stages) * kMetaBuf;
+    };
+    const int want = tuning_get("ts.stages");
+    int xs = std::min(kMaxXSlots, std::max(2, (int)(64u * 1024u / p.x_bytes)));
+    int stages = want > 0 ? std::max(2, std::min(kMaxStages, want)) : kMaxStages;
+    while (stages > 3 && need(xs, stages) > budget) --stages;
+    while (xs > 2 && need(xs, stages) > budget) --xs;
+    while (stages > 2 && need(xs, stages) > budget) --stages;
+    if (need(xs, stages) > budget) return B200Q_ERR_UNSUPPORTED;
+    p.stages = stages;
+    p.x_slots = xs;
+    p.meta_bufs = meta_bufs_for(stages);
+    p.off_x = 1024u + (uint32_t)stages * p.stage_bytes;
+    p.off_meta = p.off_x + (uint32_t)xs * p.x_bytes;
+    const uint32_t rings_end = p.off_meta + (uint32_t)p.meta_bufs * kMetaBuf;
+    p.off_red = fast_red ? rings_end : 0u;
+    if (split > 1 && !fast_red && (uint64_t)(split - 1) * dcols * kRows * 4 > (uint64_t)rings_end - 1024u) return B200Q_ERR_UNSUPPORTED;      // only with a forced split
+
+    if (!tensor_map_2d(p.x, (uint64_t)K * 2, (uint64_t)p.B, 128, (uint32_t)cols, CU_TENSOR_MAP_SWIZZLE_128B, &p.xmap)) return B200Q_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(clusters * split);
-    cfg.blockDim = dim3(ts_threads(WHOLE));
-    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(split > 1 ? p.items * split : std::min(p.items, sms));
+    cfg.blockDim = dim3(kTsThreads);
+    cfg.dynamicSmemBytes = std::max(1024u + rings_end + red_alloc, cap / 2 + 2048u);      // one CTA per SM (it takes all of the tensor memory)
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -922,72 +861,56 @@ int launch_ts(TsParams& p, cudaStream_t stream) {
     return finish_launch();
 }
 
-// The whole-SM shape for matrices large enough that the depth of the rings matters more than overlapping the head
-// of the next kernel (measured: 16 MB of codes and up), and whenever the compact shape does not fit;
-// "ts.big" = 1 / -1 forces / prefers the other.
-template <int BITS, int LOGG, int MATS>
-int launch_ts_shape(TsParams& p, int64_t weight_bytes, cudaStream_t stream) {
-    const int mode = tuning_get("ts.big");
-    // (the size of the UNSHARDED matrix decides, so that a tensor-parallel shard runs the shape, and with it the K
-    // split, of the unsharded launch)
-    const int64_t full_bytes = weight_bytes * std::max(1, tuning_get("ts.tp_world"));
-    const bool big = mode > 0 || (mode == 0 && full_bytes >= (int64_t)16 << 20);
-    if (!big) {
-        const int rc = launch_ts<BITS, LOGG, MATS, false>(p, stream);
-        if (rc != B200Q_ERR_UNSUPPORTED) return rc;
-    }
-    return launch_ts<BITS, LOGG, MATS, true>(p, stream);
+template <int BITS, int LOGG>
+int dispatch_ts_mats(TsParams& p, int K, bool gate_up, bool meta, cudaStream_t stream) {
+    if (gate_up) return meta ? launch_ts<BITS, LOGG, 2, true>(p, K, stream) : launch_ts<BITS, LOGG, 2, false>(p, K, stream);
+    return meta ? launch_ts<BITS, LOGG, 1, true>(p, K, stream) : launch_ts<BITS, LOGG, 1, false>(p, K, stream);
 }
-
 template <int BITS>
-int dispatch_ts(TsParams& p, int G, bool gate_up, int64_t weight_bytes, cudaStream_t stream) {
-    if (gate_up) {
-        if (G == 32) return launch_ts_shape<BITS, 5, 2>(p, weight_bytes, stream);
-        if (G == 64) return launch_ts_shape<BITS, 6, 2>(p, weight_bytes, stream);
-        return launch_ts_shape<BITS, 7, 2>(p, weight_bytes, stream);
-    }
-    if (G == 32) return launch_ts_shape<BITS, 5, 1>(p, weight_bytes, stream);
-    if (G == 64) return launch_ts_shape<BITS, 6, 1>(p, weight_bytes, stream);
-    return launch_ts_shape<BITS, 7, 1>(p, weight_bytes, stream);
+int dispatch_ts(TsParams& p, int K, int G, bool gate_up, bool meta, cudaStream_t stream) {
+    if (G == 32) return dispatch_ts_mats<BITS, 5>(p, K, gate_up, meta, stream);
+    if (G == 64) return dispatch_ts_mats<BITS, 6>(p, K, gate_up, meta, stream);
+    return dispatch_ts_mats<BITS, 7>(p, K, gate_up, meta, stream);
 }
 
 }  // namespace
 
-// Returns B200Q_ERR_UNSUPPORTED when the problem is outside this kernel (the caller then uses the other kernels).
-int qgemm_ts(int bits, const GemvParams& g, bool gate_up, cudaStream_t stream) {
-    if (g.act_dtype != B200Q_F16 || g.scale_dtype != B200Q_F16) return B200Q_ERR_UNSUPPORTED;
-    if (g.G != 32 && g.G != 64 && g.G != 128) return B200Q_ERR_UNSUPPORTED;
-    const int KS = kRowBytes * 8 / bits;
-    if (g.K % KS != 0 || g.K % g.G != 0 || g.Gn % 8 != 0 || g.row_bytes % 16 != 0) return B200Q_ERR_UNSUPPORTED;
-    if (g.B > 32 || g.tp_in.world > 0 || g.tp_out.world > 0) return B200Q_ERR_UNSUPPORTED;    // larger batches: 32 rows per launch
-    const int mats = gate_up ? 2 : 1;
-    for (int m = 0; m < mats; ++m)
-        if (!al16(g.w[m]) || !al16(g.s[m]) || (g.z[m] != nullptr && !al16(g.z[m]))) return B200Q_ERR_UNSUPPORTED;
-    if (gate_up && ((g.z[0] == nullptr) != (g.z[1] == nullptr))) return B200Q_ERR_UNSUPPORTED;
-    if (!al16(g.x) || (g.res_in != nullptr && !al16(g.res_in)) || (g.z_out != nullptr && !al16(g.z_out)) ||
-        (g.normed_out != nullptr && !al16(g.normed_out)))
-        return B200Q_ERR_UNSUPPORTED;
-    if (g.K % 8 != 0) return B200Q_ERR_UNSUPPORTED;
-
-    TsParams p = {};
-    for (int m = 0; m < mats; ++m) {
-        if (!tensor_map_2d(g.w[m], (uint64_t)g.row_bytes, (uint64_t)g.N, kRowBytes, kRows, true, &p.wmap[m])) return B200Q_ERR_UNSUPPORTED;
-        if (!tensor_map_2d(g.s[m], (uint64_t)g.Gn * 2, (uint64_t)g.N, 16, kRows, false, &p.smap[m])) return B200Q_ERR_UNSUPPORTED;
-        if (g.z[m] != nullptr &&
-            !tensor_map_2d(g.z[m], (uint64_t)g.Gn * 2, (uint64_t)g.N, 16, kRows, false, &p.zmap[m]))
-            return B200Q_ERR_UNSUPPORTED;
-    }
-    if (!tensor_map_2d(g.x, (uint64_t)g.K * 2, (uint64_t)g.B, 128, (uint32_t)g.B, true, &p.xmap)) return B200Q_ERR_UNSUPPORTED;
-    if (g.res_in != nullptr && !tensor_map_2d(g.res_in, (uint64_t)g.K * 2, (uint64_t)g.B, 128, (uint32_t)g.B, false, &p.rmap))
-        return B200Q_ERR_UNSUPPORTED;
-    p.x = (const __half*)g.x; p.res_in = (const __half*)g.res_in; p.norm_w = g.norm_w; p.norm_w_dtype = g.norm_w_dtype;
-    p.z_out = (__half*)g.z_out; p.normed_out = (__half*)g.normed_out; p.residual = (const __half*)g.residual;
-    p.y = (__half*)g.y; p.gate_out = (__half*)g.gate_out; p.up_out = (__half*)g.up_out; p.act_out = (__half*)g.act_out;
-    p.eps = g.eps; p.B = g.B; p.N = g.N; p.K = g.K; p.has_z = g.z[0] != nullptr ? 1 : 0;
-    p.ncols = (g.B + 15) / 16 * 16;
-    const int64_t weight_bytes = (int64_t)mats * g.N * g.row_bytes;
-    return bits == 4 ? dispatch_ts<4>(p, g.G, gate_up, weight_bytes, stream) : dispatch_ts<8>(p, g.G, gate_up, weight_bytes, stream);
+// Whether this kernel takes a problem (without looking at the norm prologue, which callers run as a launch of its own).  bf16 rows
+// need `col_scale`: the caller has put them into fp16 with a power of two per row.
+bool qgemm_ts_applies(const GemvParams& g, bool gate_up) {
+    if (g.scale_dtype != B200Q_F16 || (g.act_dtype != B200Q_F16 && g.col_scale == nullptr)) return false;
+    if (g.G != 32 && g.G != 64 && g.G != 128) return false;
+    if (g.K % g.G != 0 || g.K % 8 != 0 || g.row_bytes % 16 != 0 || g.tp_in.world > 0 || g.tp_out.world > 0) return false;
+    for (int m = 0; m < (gate_up ? 2 : 1); ++m)
+        if (!al16(g.w[m])) return false;
+    if (gate_up && ((g.z[0] == nullptr) != (g.z[1] == nullptr))) return false;
+    return al16(g.x);
 }
 
+// Returns B200Q_ERR_UNSUPPORTED when the problem is outside this kernel (the caller then uses the other kernels).
+int qgemm_ts(int bits, const GemvParams& g, bool gate_up, cudaStream_t stream) {
+    if (!qgemm_ts_applies(g, gate_up) || g.norm_w != nullptr) return B200Q_ERR_UNSUPPORTED;
+    const int mats = gate_up ? 2 : 1;
+    bool meta = g.Gn % 8 == 0;
+    for (int m = 0; m < mats; ++m) meta = meta && al16(g.s[m]) && al16(g.z[m]);
+    TsParams p = {};
+    p.B = g.B; p.N = g.N; p.Gn = g.Gn; p.has_z = g.z[0] != nullptr ? 1 : 0;
+    p.bf16 = g.act_dtype == B200Q_BF16;
+    p.col_scale = g.col_scale;
+    for (int m = 0; m < mats; ++m) {
+        p.s[m] = (const uint16_t*)g.s[m];
+        p.z[m] = (const uint16_t*)g.z[m];
+        if (!tensor_map_2d(g.w[m], (uint64_t)g.row_bytes, (uint64_t)g.N, kRowBytes, kRows, CU_TENSOR_MAP_SWIZZLE_128B, &p.wmap[m])) return B200Q_ERR_UNSUPPORTED;
+        if (!meta) continue;
+        if (!tensor_map_2d(g.s[m], (uint64_t)g.Gn * 2, (uint64_t)g.N, kMetaGroups * 2, kRows, CU_TENSOR_MAP_SWIZZLE_32B, &p.smap[m])) return B200Q_ERR_UNSUPPORTED;
+        if (g.z[m] != nullptr &&
+            !tensor_map_2d(g.z[m], (uint64_t)g.Gn * 2, (uint64_t)g.N, kMetaGroups * 2, kRows, CU_TENSOR_MAP_SWIZZLE_32B, &p.zmap[m]))
+            return B200Q_ERR_UNSUPPORTED;
+    }
+    p.residual = (const uint16_t*)g.residual; p.y = (uint16_t*)g.y; p.gate_out = (uint16_t*)g.gate_out; p.up_out = (uint16_t*)g.up_out;
+    p.act_out = (uint16_t*)g.act_out;
+    p.x = g.x;
+    return bits == 4 ? dispatch_ts<4>(p, g.K, g.G, gate_up, meta, stream) : dispatch_ts<8>(p, g.K, g.G, gate_up, meta, stream);
+}
 
 }  // namespace b200q

@@ -29,6 +29,8 @@ SIGNATURES = {
     "b200q_strerror": (_c.c_char_p, [_i]),
     "b200q_device_status": (_i, [_i, _vp]),
     "b200q_set_tuning": (_i, [_c.c_char_p, _i]),
+    "b200q_scratch_next": (_i, [_vp, _sz]),
+    "b200q_scratch_bytes": (_sz, [_i, _i64, _i]),
     "b200q_dequant": (_i, [_i, _vp, _vp, _vp, _vp, _i64, _i64, _i, _i, _i, _vp]),
     "b200q_qmatvec": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i64, _i64, _i, _i, _i, _vp]),
     "b200q_norm_qmatvec": (_i, [_i, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i64, _i64, _i, _i, _i,
@@ -168,6 +170,17 @@ def stream() -> int:
 
 def contiguous(t):
     return t if t is None or t.is_contiguous() else t.contiguous()
+
+
+def scratch_next(rows: int, k: int, x):
+    """Hands the library the scratch that its next matvec / gate-up call on ``rows`` rows of ``k`` can use; the returned tensor
+    has to live until that call is made."""
+    n = load().b200q_scratch_bytes(rows, k, dtype_code(x.dtype))
+    if n == 0:
+        return None
+    buf = torch.empty(n, dtype=torch.uint8, device=x.device)
+    load().b200q_scratch_next(buf.data_ptr(), n)
+    return buf
 
 
 def scale_pair(scales, zeros):

@@ -22,6 +22,7 @@ def norm_quantized_linear(x, norm_weight, w, scales, zeros=None, *, residual_in=
     N = w.shape[0]
     y = torch.empty((R, N), dtype=x.dtype, device=x.device)
     normed = torch.empty_like(x)           # also the staging buffer of the generic (odd-shape) route
+    scratch = _cabi.scratch_next(R, K, x)      # noqa: F841 (held until the call below)
     _cabi.check(
         _cabi.load().b200q_norm_qmatvec(bits, x.data_ptr(), _cabi.ptr(residual_in), norm_weight.data_ptr(),
                                         _cabi.dtype_code(norm_weight.dtype), float(eps), None, normed.data_ptr(),

@@ -171,6 +171,7 @@ def matvec_rows(bits, x2d, codes, scales, zeros, group_size, residual=None):
     B, K = x2d.shape
     N = codes.shape[0]
     y = torch.empty((B, N), dtype=x2d.dtype, device=x2d.device)
+    scratch = _cabi.scratch_next(B, K, x2d)      # noqa: F841 (held until the call below)
     _cabi.check(
         _cabi.load().b200q_qmatvec(bits, x2d.data_ptr(), codes.data_ptr(), scales.data_ptr(), _cabi.ptr(zeros),
                                    _cabi.ptr(residual), y.data_ptr(), B, N, K, group_size,
@@ -294,6 +295,7 @@ def gate_up_rows(bits, x2d, gate_w, up_w, gate_scales, up_scales, gate_zeros, up
             out["z"] = new(R, K)
         # the generic (odd-shape) route needs the normalised rows as a buffer, so always provide it
         out["normed"] = new(R, K)
+    scratch = _cabi.scratch_next(R, K, x2d)      # noqa: F841 (held until the call below)
     _cabi.check(
         _cabi.load().b200q_gate_up_swiglu(
             bits, x2d.data_ptr(), gate_w.data_ptr(), up_w.data_ptr(), gate_scales.data_ptr(), up_scales.data_ptr(),
