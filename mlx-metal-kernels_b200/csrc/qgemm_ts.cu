@@ -13,8 +13,10 @@
 //                                 shared memory 16 bytes at a time (conflict-free through the swizzle), become fp16 weights in
 //                                     w = ((base+q) - (base+rint(z))) * s + (rint(z) - z) * s
 //                                 (exact subtraction, then one fused multiply-add) and go to tensor memory with tcgen05.st
-//   MMA (one warp, one elected    tcgen05.mma.kind::f16, M = 128, N = block columns, K = 16, A from tensor memory; tcgen05.commit
-//        lane issues)             releases the chunk / the operand slot / the accumulator
+//   MMA (two warps, one elected   tcgen05.mma.kind::f16, M = 128, N = block columns, K = 16, A from tensor memory; tcgen05.commit
+//        lane of each issues)     releases the chunk / the operand slot / the accumulator.  Each warp has an accumulator of its own - gate
+//                                 and up, or the even and the odd chunks of one matrix: a ready barrier still costs the warp 150-250
+//                                 clocks beside the busy dequantise warps, which one warp alone cannot hide (MMA_MEASURED)
 //   epilogue (dequantise warps)   tcgen05.ld of D, clamp, round, residual add or SwiGLU, store
 //
 // What bounds it: a chunk (128 x 128 weights) costs the dequantisation 4 x 260 warp instructions, i.e. about 300 clocks on the SM's four
@@ -60,8 +62,9 @@ constexpr int kMaxCols = 128;                  // batch columns per item
 constexpr uint32_t kTsWaitLimit = 1u << 20;
 constexpr int kDeqWarps = 16;
 constexpr int kGroups = kDeqWarps / 4;         // a group = four warps = one per 32-lane quarter of tensor memory
-constexpr int kTmaWarp = kDeqWarps, kMmaWarp = kDeqWarps + 1, kRowWarp = kDeqWarps + 2;
-constexpr int kTsThreads = (kDeqWarps + 3) * 32;
+constexpr int kMmaWarps = 2;                   // one accumulator each
+constexpr int kTmaWarp = kDeqWarps, kRowWarp = kDeqWarps + 1, kMmaWarp0 = kDeqWarps + 2;
+constexpr int kTsThreads = (kDeqWarps + 2 + kMmaWarps) * 32;
 
 struct alignas(64) TsParams {
     CUtensorMap wmap[2];        // codes [N, row_bytes] u8, box 128 B x 128 rows, 128-byte swizzle
@@ -146,17 +149,12 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&v)[32])
         : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
+__device__ __forceinline__ void tc_ld4(uint32_t taddr, float (&v)[4]) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -245,33 +243,33 @@ __device__ __forceinline__ uint16_t ts_bits(const TsParams& p, float v) {
 __device__ __forceinline__ float ts_float(const TsParams& p, uint16_t u) {
     return p.bf16 ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
 }
-// The residual values of output row n for 16 columns, fetched before the accumulators are waited for and before the first
-// store (y may alias the residual rows as far as the compiler knows).
+// The residual values of output row n for 4 columns, fetched ahead of the accumulators and before the first store (y may
+// alias the residual rows as far as the compiler knows).
 template <int MATS>
-__device__ __forceinline__ void ts_load_residual(const TsParams& p, int n, int b0, int nb, uint16_t (&res)[16]) {
+__device__ __forceinline__ void ts_load_residual(const TsParams& p, int n, int b0, int nb, uint16_t (&res)[4]) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < 4; ++j) {
         res[j] = 0;
         if (MATS == 1 && p.residual != nullptr && n < p.N && j < nb) res[j] = p.residual[(size_t)(b0 + j) * p.N + n];
     }
 }
-// The epilogue of a 16-column slice (columns b0 .. b0 + nb of the batch): clamp, round, residual add or SwiGLU, store.
+// The epilogue of 4 columns (b0 .. b0 + nb of the batch): clamp, round, residual add or SwiGLU, store.
 template <int MATS>
-__device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&acc)[MATS][16], int n, int b0, int nb, const uint16_t (&res)[16]) {
+__device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&acc)[2][4], int n, int b0, int nb, const uint16_t (&res)[4]) {
     const float fmax_act = p.bf16 ? 3.3895313892515355e38f : 65504.0f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < 4; ++j) {
         if (j >= nb) break;
         const int b = b0 + j;
         const size_t o = (size_t)b * p.N + n;
         const float cs = p.col_scale != nullptr ? p.col_scale[b] : 1.0f;
-        const float v0 = ts_round(p, fminf(fmaxf(acc[0][j] * cs, -fmax_act), fmax_act));
         if (MATS == 1) {
-            float v = v0;
+            float v = ts_round(p, fminf(fmaxf((acc[0][j] + acc[1][j]) * cs, -fmax_act), fmax_act));
             if (p.residual != nullptr) v = ts_float(p, res[j]) + v;
             p.y[o] = ts_bits(p, v);
         } else {
-            const float v1 = ts_round(p, fminf(fmaxf(acc[MATS - 1][j] * cs, -fmax_act), fmax_act));
+            const float v0 = ts_round(p, fminf(fmaxf(acc[0][j] * cs, -fmax_act), fmax_act));
+            const float v1 = ts_round(p, fminf(fmaxf(acc[1][j] * cs, -fmax_act), fmax_act));
             if (p.gate_out != nullptr) p.gate_out[o] = ts_bits(p, v0);
             if (p.up_out != nullptr) p.up_out[o] = ts_bits(p, v1);
             if (p.act_out != nullptr) p.act_out[o] = ts_bits(p, (v0 / (1.0f + expf(-v0))) * v1);
@@ -326,13 +324,13 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
     auto row_of = [&](int it) { return (first_item + it * item_step) / p.nblk * kRows; };        // column blocks of a tile run side by side
     auto col_of = [&](int it) { return (first_item + it * item_step) % p.nblk * ncols; };
 
-    if (warp == kMmaWarp) {
+    if (warp == kMmaWarp0) {
         if (lane < NS) { mbar_init(&full_w[lane], 1); mbar_init(&empty_w[lane], GPS * 4); }
-        if (lane < XS) { mbar_init(&full_x[lane], 1); mbar_init(&empty_x[lane], 1); }
+        if (lane < XS) { mbar_init(&full_x[lane], 1); mbar_init(&empty_x[lane], MATS); }
         if (lane < NA) { mbar_init(&a_full[lane], 4); mbar_init(&a_free[lane], 1); }
         if (META && lane < p.meta_bufs) { mbar_init(&full_m[lane], 1); mbar_init(&empty_m[lane], kDeqWarps); }
         if (lane == 0) {
-            mbar_init(d_full, 1);
+            mbar_init(d_full, kMmaWarps);
             mbar_init(d_free, kDeqWarps);
             mbar_init(red_bar, p.split > 1 ? (uint32_t)(p.split - 1) * kDeqWarps * 32u : 1u);
         }
@@ -398,39 +396,45 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
             }
         }
     }
-    // ================================ MMA issuer ==================================================
-    else if (warp == kMmaWarp) {
+    // ================================ MMA issuers =================================================
+    else if (warp >= kMmaWarp0) {
+        // warp j: matrix j of every chunk of k (two matrices), or the chunks of k with number = j modulo 2
+        const int j = warp - kMmaWarp0;
         bool ok = true;
         const uint32_t idesc = (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
         // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart, descriptor version 1
         const uint64_t desc_hi = ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61) | (1ull << 16);
-        int xslot = 0, a_slot = 0;
-        uint32_t xpar = 0, a_par = 0;
         const uint32_t a_base = tmem + (uint32_t)p.a_col0;
+        const uint32_t d_t = tmem + (uint32_t)(j * ncols);
         const uint32_t x0 = base + p.off_x;
         const uint32_t atom16 = (p.x_bytes >> 1) >> 4;                 // distance of the two 64-k atoms of a chunk, in 16-byte units
         const int n_ch = n_st * SC;
+        const int step = MATS == 2 ? 1 : 2;
+        int xslot = 0, a_slot = 0, x_at = 0, a_at = 0;                 // ring positions and the chunk numbers they stand for
+        uint32_t xpar = 0, a_par = 0;
         for (int it = 0; it < my_items; ++it) {
             if (it > 0) wait_bar(d_free, (uint32_t)(it - 1) & 1u, EV_GEMV_EMPTY_WAIT, ok);
             tc_fence_after();
-            for (int ch = 0; ch < n_ch; ++ch) {
-                wait_bar(&full_x[xslot], xpar, EV_GEMV_FULL_WAIT, ok);
+            const int first = MATS == 2 ? 0 : j;
+            for (int ch = first; ch < n_ch; ch += step) {
+                const int xn = it * n_ch + ch, an = MATS == 2 ? 2 * xn + j : xn;
+                xslot += xn - x_at;
+                x_at = xn;
+                while (xslot >= XS) { xslot -= XS; xpar ^= 1u; }
+                a_slot += an - a_at;
+                a_at = an;
+                while (a_slot >= NA) { a_slot -= NA; a_par ^= 1u; }
                 const uint64_t desc0 = desc_hi | (uint64_t)(((x0 + (uint32_t)xslot * p.x_bytes) & 0x3FFFFu) >> 4);
+                const uint32_t a_t = a_base + (uint32_t)a_slot * kChunkCols;
+                wait_bar(&full_x[xslot], xpar, EV_GEMV_FULL_WAIT, ok);
+                wait_bar(&a_full[a_slot], a_par, EV_GEMV_FULL_WAIT, ok);
+                tc_fence_after();
+                tc_mma_ts(d_t, a_t, desc0, idesc, ch == first ? 0u : 1u);
 #pragma unroll
-                for (int m = 0; m < MATS; ++m) {
-                    wait_bar(&a_full[a_slot], a_par, EV_GEMV_FULL_WAIT, ok);
-                    tc_fence_after();
-                    const uint32_t a_t = a_base + (uint32_t)a_slot * kChunkCols;
-                    const uint32_t d_t = tmem + (uint32_t)(m * ncols);
-                    tc_mma_ts(d_t, a_t, desc0, idesc, ch == 0 ? 0u : 1u);
-#pragma unroll
-                    for (int i = 1; i < kChunkK / 16; ++i)
-                        tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
-                    tc_commit(&a_free[a_slot]);
-                    if (++a_slot == NA) { a_slot = 0; a_par ^= 1u; }
-                }
+                for (int i = 1; i < kChunkK / 16; ++i)
+                    tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
+                tc_commit(&a_free[a_slot]);
                 tc_commit(&empty_x[xslot]);
-                if (++xslot == XS) { xslot = 0; xpar ^= 1u; }
             }
             tc_commit(d_full);
         }
@@ -452,6 +456,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         int mslot = 0;
         uint32_t mpar = 0;
         const int n_ch = n_st * APS;                           // chunks of an item
+        const bool second = n_st * SC > 1;                     // one matrix: the second accumulator is in use
         for (int it = 0; it < my_items; ++it) {
             const int n0 = row_of(it);
             int sl_at = 0;                                     // stage of the item that `slot` stands for
@@ -579,28 +584,28 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     m_waited = false;
                 }
             }
-            // ---- epilogue of the item (split == 1; with a split K range it follows the cluster exchange below): the groups of warps
-            //      take 16-column slices in turn ----
+            // ---- epilogue of the item (split == 1; with a split K range it follows the cluster exchange below): each group of warps takes
+            //      4 columns of every 16 ----
             if (p.split == 1) {
                 if (it == 0) pdl_wait();
-                const int n = n0 + r, c0 = col_of(it);
-                bool first = true;
-                for (int cs = grp * 16; cs < ncols; cs += NG * 16) {
-                    const int nb = min(16, p.B - c0 - cs);
+                const int n = n0 + r, c0 = col_of(it) + grp * 4;
+                uint16_t res[4];
+                ts_load_residual<MATS>(p, n, c0, p.B - c0, res);
+                wait_bar(d_full, (uint32_t)it & 1u, EV_GEMV_FULL_WAIT, ok);
+                tc_fence_after();
+#pragma unroll 1
+                for (int cs = 0; cs < ncols; cs += 16) {
+                    const int nb = p.B - c0 - cs;              // may be more than 4
                     if (nb <= 0) break;
-                    uint16_t res[16];
-                    ts_load_residual<MATS>(p, n, c0 + cs, nb, res);
-                    if (first) {
-                        wait_bar(d_full, (uint32_t)it & 1u, EV_GEMV_FULL_WAIT, ok);
-                        tc_fence_after();
-                        first = false;
-                    }
-                    float acc[MATS][16];
-#pragma unroll
-                    for (int m = 0; m < MATS; ++m) tc_ld16(lane_addr + (uint32_t)(m * ncols + cs), acc[m]);
+                    uint16_t next[4];
+                    ts_load_residual<MATS>(p, n, c0 + cs + 16, cs + 16 < ncols ? nb - 16 : 0, next);
+                    float acc[2][4] = {};
+                    tc_ld4(lane_addr + (uint32_t)(cs + grp * 4), acc[0]);
+                    if (MATS == 2 || second) tc_ld4(lane_addr + (uint32_t)(ncols + cs + grp * 4), acc[1]);
                     if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, nb, res);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) res[j] = next[j];
                 }
-                if (first) wait_bar(d_full, (uint32_t)it & 1u, EV_GEMV_FULL_WAIT, ok);      // no slice for this group: stay in step
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(d_free);
@@ -628,40 +633,52 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
             tc_fence_after();
         }
         if (!fast) cluster_sync_all();      // every CTA of the cluster is done with its rings: the first CTA's are free
+        const bool second = n_st * SC > 1;                    // one matrix: the second accumulator is in use
         if (epi && rank != 0) {
-            for (int m = 0; m < MATS; ++m)
-                for (int cs = grp * 16; cs < bcols; cs += kGroups * 16) {
-                    float acc[16];
-                    tc_ld16(lane_addr + (uint32_t)(m * ncols + cs), acc);
+#pragma unroll 1
+            for (int cs = grp * 4; cs < bcols; cs += 16) {
+                float acc[2][4] = {};
+                tc_ld4(lane_addr + (uint32_t)cs, acc[0]);
+                if (MATS == 2 || second) tc_ld4(lane_addr + (uint32_t)(ncols + cs), acc[1]);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (cs + j < bcols)
-                            st_cluster_f32(red_base + (uint32_t)(((((int)rank - 1) * MATS + m) * rcols + cs + j) * kRows + r) * 4u, 0u, acc[j]);
+                for (int j = 0; j < 4; ++j) {
+                    if (cs + j >= bcols) break;
+#pragma unroll
+                    for (int m = 0; m < MATS; ++m)
+                        st_cluster_f32(red_base + (uint32_t)(((((int)rank - 1) * MATS + m) * rcols + cs + j) * kRows + r) * 4u, 0u,
+                                       MATS == 1 ? acc[0][j] + acc[1][j] : acc[m][j]);
                 }
+            }
             if (fast) arrive_remote(smem_u32(red_bar), 0u);
         }
         if (!fast) cluster_sync_all();      // the partial sums are in the first CTA's shared memory
         if (epi && rank == 0) {
             pdl_wait();
             const int n = row_of(0) + r;
-            bool first = true;
             const float* red = reinterpret_cast<const float*>(sbase + (red_base - base));
-            for (int cs = grp * 16; cs < bcols; cs += kGroups * 16) {
-                const int nb = min(16, bcols - cs);
-                uint16_t res[16];
-                ts_load_residual<MATS>(p, n, c0 + cs, nb, res);
-                if (first && fast) wait_bar_cluster(red_bar, 0u, ok ? kTsWaitLimit : 64u);
-                first = false;
-                float acc[MATS][16];
+            uint16_t res[4];
+            ts_load_residual<MATS>(p, n, c0 + grp * 4, bcols - grp * 4, res);
+            if (fast) wait_bar_cluster(red_bar, 0u, ok ? kTsWaitLimit : 64u);
+#pragma unroll 1
+            for (int cs = grp * 4; cs < bcols; cs += 16) {
+                uint16_t next[4];
+                ts_load_residual<MATS>(p, n, c0 + cs + 16, bcols - cs - 16, next);
+                float acc[2][4] = {};
+                tc_ld4(lane_addr + (uint32_t)cs, acc[0]);
+                if (MATS == 2 || second) tc_ld4(lane_addr + (uint32_t)(ncols + cs), acc[1]);
+                if (MATS == 1) {
 #pragma unroll
-                for (int m = 0; m < MATS; ++m) {
-                    tc_ld16(lane_addr + (uint32_t)(m * ncols + cs), acc[m]);
-                    for (int q = 1; q < p.split; ++q)
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (j < nb) acc[m][j] += red[((((q - 1) * MATS + m) * rcols + cs + j) * kRows + r)];
+                    for (int j = 0; j < 4; ++j) { acc[0][j] += acc[1][j]; acc[1][j] = 0.0f; }
                 }
-                if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, nb, res);
+                for (int q = 1; q < p.split; ++q)
+#pragma unroll
+                    for (int m = 0; m < MATS; ++m)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (cs + j < bcols) acc[m][j] += red[((((q - 1) * MATS + m) * rcols + cs + j) * kRows + r)];
+                if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, bcols - cs, res);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) res[j] = next[j];
             }
         }
         // the first CTA must not leave while its neighbours still store into it
@@ -803,7 +820,7 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     p.items = tiles * p.nblk;
     p.split = split;
     // tensor memory: accumulators below, ring of A chunks above
-    const int dcols = MATS * cols;
+    const int dcols = 2 * cols;
     p.a_col0 = std::max(32, (dcols + 31) / 32 * 32);
     p.a_slots = std::min(kMaxASlots, (512 - p.a_col0) / kChunkCols);
     // partial sums of a K split: a dedicated buffer signalled by a barrier, else the first CTA's rings between two cluster-wide
@@ -833,7 +850,7 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     p.off_meta = p.off_x + (uint32_t)xs * p.x_bytes;
     const uint32_t rings_end = p.off_meta + (uint32_t)p.meta_bufs * kMetaBuf;
     p.off_red = fast_red ? rings_end : 0u;
-    if (split > 1 && !fast_red && (uint64_t)(split - 1) * dcols * kRows * 4 > (uint64_t)rings_end - 1024u) return B200Q_ERR_UNSUPPORTED;      // only with a forced split
+    if (split > 1 && !fast_red && (uint64_t)(split - 1) * MATS * cols * kRows * 4 > (uint64_t)rings_end - 1024u) return B200Q_ERR_UNSUPPORTED;      // only with a forced split
 
     if (!tensor_map_2d(p.x, (uint64_t)K * 2, (uint64_t)p.B, 128, (uint32_t)cols, CU_TENSOR_MAP_SWIZZLE_128B, &p.xmap)) return B200Q_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
