@@ -15,8 +15,9 @@
 //                                 (exact subtraction, then one fused multiply-add) and go to tensor memory with tcgen05.st
 //   MMA (two warps, one elected   tcgen05.mma.kind::f16, M = 128, N = block columns, K = 16, A from tensor memory; tcgen05.commit
 //        lane of each issues)     releases the chunk / the operand slot / the accumulator.  Each warp has an accumulator of its own - gate
-//                                 and up, or the even and the odd chunks of one matrix: a ready barrier still costs the warp 150-250
-//                                 clocks beside the busy dequantise warps, which one warp alone cannot hide (MMA_MEASURED)
+//                                 and up, or the even and the odd chunks of one matrix - and takes two chunks per round:
+//                                 waits, ring arithmetic and commits cost it 800 clocks a round beside the busy dequantise warps,
+//                                 16 MMAs 360
 //   epilogue (dequantise warps)   tcgen05.ld of D, clamp, round, residual add or SwiGLU, store
 //
 // What bounds it: a chunk (128 x 128 weights) costs the dequantisation 4 x 260 warp instructions, i.e. about 300 clocks on the SM's four
@@ -156,7 +157,6 @@ __device__ __forceinline__ void tc_ld4(uint32_t taddr, float (&v)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -209,13 +209,32 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-__device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int event, bool& ok) {
     const bool got = mbar_wait_bounded(bar, parity, &g_device_status, event, ok ? kTsWaitLimit : 64u);
     ok = ok && got;
     return got;
+}
+
+// One wait of a warp for several barriers: lane i polls its own (address and parity per lane; lanes without one pass `need` false).
+// Beside the busy dequantise warps a ready barrier costs a warp 150-200 clocks, so barriers are polled together, not in turn.
+__device__ __forceinline__ void wait_bars(uint32_t addr, uint32_t parity, bool need, int event, bool& ok) {
+    const uint32_t limit = ok ? kTsWaitLimit : 64u;
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t got = 1;
+        if (need)
+            asm volatile(
+                "{\n"
+                ".reg .pred p;\n"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                "selp.b32 %0, 1, 0, p;\n"
+                "}\n"
+                : "=r"(got)
+                : "r"(addr), "r"(parity)
+                : "memory");
+        if (__all_sync(0xffffffffu, got != 0)) return;
+    }
+    atomicMax(&g_device_status, event);
+    ok = false;
 }
 
 // Per-group constants of the dequantisation, each duplicated into both halves of a register:
@@ -398,7 +417,9 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
     }
     // ================================ MMA issuers =================================================
     else if (warp >= kMmaWarp0) {
-        // warp j: matrix j of every chunk of k (two matrices), or the chunks of k with number = j modulo 2
+        // warp j: matrix j of every chunk of k (two matrices), or the chunks of k with number = j modulo 2 (one matrix).  Two matrices and
+        // few columns: two chunks per round of waits, where the rings are deep enough to hold one round and refill another
+        // (gate and up, 14336 x 4096 q4: 27.6 -> 25.9 us for 8 rows; one matrix and more than 64 columns lose by it: 64 -> 71 us for 256)
         const int j = warp - kMmaWarp0;
         bool ok = true;
         const uint32_t idesc = (1u << 4) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
@@ -409,32 +430,47 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         const uint32_t x0 = base + p.off_x;
         const uint32_t atom16 = (p.x_bytes >> 1) >> 4;                 // distance of the two 64-k atoms of a chunk, in 16-byte units
         const int n_ch = n_st * SC;
-        const int step = MATS == 2 ? 1 : 2;
-        int xslot = 0, a_slot = 0, x_at = 0, a_at = 0;                 // ring positions and the chunk numbers they stand for
+        const int per = MATS == 2 && ncols <= 64 && XS >= 4 && NA >= 5 ? 2 : 1;      // chunks per round
+        const int first = MATS == 2 ? 0 : j;
+        const int skip = MATS == 2 ? 0 : 1;                            // chunks of the other warp between two rounds
+        int xslot = 0, a_slot = 0, x_at = 0;                           // ring positions and the chunk they stand for
         uint32_t xpar = 0, a_par = 0;
+        if (MATS == 2) a_slot = j;                                     // (NA >= 2)
+        auto go = [&](int d) {                                         // d chunks of k on
+            xslot += d;
+            while (xslot >= XS) { xslot -= XS; xpar ^= 1u; }
+            a_slot += MATS * d;
+            while (a_slot >= NA) { a_slot -= NA; a_par ^= 1u; }
+            x_at += d;
+        };
+        auto chunk = [&](int xs, int as, bool start) {
+            const uint64_t desc0 = desc_hi | (uint64_t)(((x0 + (uint32_t)xs * p.x_bytes) & 0x3FFFFu) >> 4);
+            const uint32_t a_t = a_base + (uint32_t)as * kChunkCols;
+            tc_mma_ts(d_t, a_t, desc0, idesc, start ? 0u : 1u);
+#pragma unroll
+            for (int i = 1; i < kChunkK / 16; ++i)
+                tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
+            tc_commit(&a_free[as]);
+            tc_commit(&empty_x[xs]);
+        };
         for (int it = 0; it < my_items; ++it) {
             if (it > 0) wait_bar(d_free, (uint32_t)(it - 1) & 1u, EV_GEMV_EMPTY_WAIT, ok);
             tc_fence_after();
-            const int first = MATS == 2 ? 0 : j;
-            for (int ch = first; ch < n_ch; ch += step) {
-                const int xn = it * n_ch + ch, an = MATS == 2 ? 2 * xn + j : xn;
-                xslot += xn - x_at;
-                x_at = xn;
-                while (xslot >= XS) { xslot -= XS; xpar ^= 1u; }
-                a_slot += an - a_at;
-                a_at = an;
-                while (a_slot >= NA) { a_slot -= NA; a_par ^= 1u; }
-                const uint64_t desc0 = desc_hi | (uint64_t)(((x0 + (uint32_t)xslot * p.x_bytes) & 0x3FFFFu) >> 4);
-                const uint32_t a_t = a_base + (uint32_t)a_slot * kChunkCols;
-                wait_bar(&full_x[xslot], xpar, EV_GEMV_FULL_WAIT, ok);
-                wait_bar(&a_full[a_slot], a_par, EV_GEMV_FULL_WAIT, ok);
+            go(it * n_ch + first - x_at);
+#pragma unroll 1
+            for (int ch = first; ch < n_ch;) {
+                const int xs0 = xslot, as0 = a_slot;
+                const uint32_t xp0 = xpar, ap0 = a_par;
+                const bool two = per == 2 && ch + 1 < n_ch;
+                if (two) go(1);
+                // lanes 0, 1: the first chunk's operands; lanes 2, 3: the second's
+                const uint32_t bar = lane == 0 ? smem_u32(&full_x[xs0]) : lane == 1 ? smem_u32(&a_full[as0]) : lane == 2 ? smem_u32(&full_x[xslot]) : smem_u32(&a_full[a_slot]);
+                wait_bars(bar, lane == 0 ? xp0 : lane == 1 ? ap0 : lane == 2 ? xpar : a_par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
                 tc_fence_after();
-                tc_mma_ts(d_t, a_t, desc0, idesc, ch == first ? 0u : 1u);
-#pragma unroll
-                for (int i = 1; i < kChunkK / 16; ++i)
-                    tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
-                tc_commit(&a_free[a_slot]);
-                tc_commit(&empty_x[xslot]);
+                chunk(xs0, as0, ch == first);
+                if (two) chunk(xslot, a_slot, false);
+                ch += (two ? 2 : 1) + skip;
+                go(1 + skip);
             }
             tc_commit(d_full);
         }
@@ -448,6 +484,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         const uint32_t msw = (uint32_t)((r >> 2) & 1) << 4;    // 32-byte swizzle of the scale tiles
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         const uint32_t row_u = stage0 + (uint32_t)r * kRowBytes;
+        const bool second = n_st * SC > 1;                     // one matrix: the second accumulator is in use
         bool ok = true;
         int t = grp % NA;                                      // A slot of this group's next chunk
         uint32_t a_par = (uint32_t)(grp / NA) & 1u;
@@ -456,7 +493,6 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         int mslot = 0;
         uint32_t mpar = 0;
         const int n_ch = n_st * APS;                           // chunks of an item
-        const bool second = n_st * SC > 1;                     // one matrix: the second accumulator is in use
         for (int it = 0; it < my_items; ++it) {
             const int n0 = row_of(it);
             int sl_at = 0;                                     // stage of the item that `slot` stands for
@@ -501,7 +537,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                         ++mt_at;
                         m_waited = false;
                     }
-                    if (!m_waited) wait_bar(&full_m[mslot], mpar, EV_GEMV_FULL_WAIT, ok);
+                }
+                if (META && !m_waited) wait_bar(&full_m[mslot], mpar, EV_GEMV_FULL_WAIT, ok);
+                wait_bar(&full_w[slot], par, EV_GEMV_FULL_WAIT, ok);
+                if (META) {
                     m_waited = true;
                     const int g0 = ((s * KS + c * kChunkK) >> LOGG) & (kMetaGroups - 1);      // first group of the chunk inside the scale tile
                     const uint32_t mrow = base + p.off_meta + (uint32_t)mslot * kMetaBuf + (uint32_t)(m * 2 * kMetaTile) +
@@ -518,7 +557,6 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     sreg[0] = ns[0]; sreg[1] = ns[1]; zreg[0] = nz[0]; zreg[1] = nz[1];
                     if (q + NG < n_ch) fetch_meta(q + NG);
                 }
-                wait_bar(&full_w[slot], par, EV_GEMV_FULL_WAIT, ok);
                 const uint32_t wrow = row_u + (uint32_t)slot * p.stage_bytes + (uint32_t)(m * kWTile);
                 const uint32_t a_t = lane_addr + (uint32_t)(p.a_col0 + t * kChunkCols);
                 wait_bar(&a_free[t], a_par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
