@@ -10,14 +10,14 @@
 //     same number of pages whatever the length distribution).  A CTA writes one partial
 //     (max, sum, accumulator) per sequence it touches; a second small kernel merges them.
 //   * warp w of a CTA owns kv head w % Hkv (and, when there are fewer than 8 kv heads, every
-//     (8/Hkv)-th page of the range; more than 8 kv heads are cut into chunks of 8, grid.y).  It is self-contained: it looks up
-//     its page ids 32 at a time and copies its pages with cp.async into a private ring in shared memory, several pages
-//     ahead.  No CTA-wide barrier.
+//     (8/Hkv)-th page of the range; more than 8 kv heads are cut into chunks of 8, grid.y).  A ninth warp looks up the page ids and
+//     fetches every page for all the CTA's heads with tensor copies into a ring in shared memory, several pages ahead.
 //   * what a warp does with a page is in paged_attn_page.cuh.
 //
 // Everything else (other head dims, other group sizes) runs the simple kernel: one
 // warp per (sequence, query head), the reference's streaming-softmax loop.
 #include "paged_attn_page.cuh"
+#include "tensor_map.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -54,12 +54,12 @@ struct AttnParams {
     float scale;
     int q_dtype;
     int bits;
-    int stages;                 // pages in flight per warp
+    int stages;                 // pages in flight per range
     int subs;                   // ranges per CTA (8 / hc)
     int hc;                     // kv heads per CTA: Hkv, at most 8
     int row_bytes;              // bytes of one token row of codes, all kv heads
     int scale_row_halves;       // halves of one token row of scales, all kv heads
-    uint32_t off_prefix, off_ring, slot_bytes;
+    uint32_t off_bars, off_desc, off_prefix, slot_bytes;      // the ring comes first
     int grid;
     int sink, window;           // window > 0: only positions < sink or >= length - window are attended
     TpOut tp_out;               // tensor-parallel exchange of the merged rows (world == 0: off)
@@ -128,23 +128,70 @@ __device__ __forceinline__ int find_sequence(const int* prefix, int B, int f) {
     return lo;
 }
 
-// Two shapes of the same kernel.  TWO = true: two CTAs per SM (16 warps hide more latency) with the ring depth that still
-// fits twice into shared memory.  TWO = false: one CTA per SM with a deeper ring, for grids that do not fill the SMs twice
-// anyway, and for plain pages (8 KB per page and head).
-constexpr int ring_depth(int bits, bool two) { return bits == 4 ? (two ? 5 : 10) : bits == 8 ? (two ? 3 : 6) : 3; }
+// pages in flight per warp of the cluster kernel (its widest form has room for one less)
+constexpr int ring_depth(int bits) { return bits == 4 ? 9 : 5; }
+
+// The split-KV kernel: eight consumer warps (process_page) and one producer warp.
+// Bound by HBM (a page of q8 codes and scales is 4.3 KB per kv head: 181 clocks of an SM's share).  What held it back before was the
+// path into shared memory: every warp copied its own head's pages with 16-byte cp.async pieces and 8-byte pieces of scales - 9 (q8) or
+// 17 (plain) such instructions per page and head, 64 L2 requests - and the warps' ldmatrix, shuffles and conversions queued behind
+// them (5 of 12.5 clocks per instruction on short scoreboards, issue 31 %): 303 clocks per page and head, 81 us for 32 x 4097 q8
+// tokens of 8 kv heads (0.55 of the copy rate).  Now one elected lane fetches a page for ALL heads of the block: two
+// 3-D tensor copies (row, token, head) whose swizzle is what ldmatrix wants, and two copies of the scales.
+// The producer also looks up the page descriptors, 32 at a time, and leaves them in shared memory.
+// TWO: two CTAs per SM, 16 consumer warps; otherwise (grids that do not fill the SMs twice, plain pages of 64 KB) one with a deeper ring.
+constexpr int kSplitThreads = kAttnThreads + 32;
+constexpr int kMaxRing = 16;                  // pages in flight per range
+constexpr uint32_t kAttnWaitLimit = 1u << 20;
+constexpr int kDescSlots = 64;                // descriptors per range: the window being issued and the one before (a ring is shorter than 32)
+
+struct alignas(64) SplitParams {
+    CUtensorMap kmap, vmap;     // codes (or values) as bytes [heads (x 2)][tokens][64 or 128], box hc (x 2) x 16 x row
+    CUtensorMap ksmap, vsmap;   // scales as bytes [tokens][row], box 16 x (hc heads); used with more than 8 kv heads only
+    AttnParams a;
+};
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
+}
+// bytes of one range's ring slot: K tiles, V tiles, scales of K, scales of V; a multiple of the swizzle's repeat
+__host__ __device__ constexpr uint32_t split_scale_bytes(int hc, int Gd) { return (uint32_t)(16 * hc * Gd * 2); }
+__host__ __device__ constexpr uint32_t split_slot_bytes(int bits, int hc, int Gd) {
+    const uint32_t tiles = (uint32_t)(2 * hc * 16 * kHeadDim * bits / 8), sc = bits == 16 ? 0u : 2 * split_scale_bytes(hc, Gd);
+    return (tiles + sc + 1023u) & ~1023u;
+}
+
 template <int BITS, int LOGG, bool TWO, bool WIDE>
-__global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged_attn_kernel(const __grid_constant__ AttnParams p) {
-    extern __shared__ __align__(128) uint8_t smem[];
+__global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) paged_attn_kernel(const __grid_constant__ SplitParams sp) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    const AttnParams& p = sp.a;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int D = kHeadDim;
-    constexpr int SLOT = PageShape<BITS>::SLOT;
+    constexpr int TILE = PageShape<BITS>::TILE;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    int* prefix = reinterpret_cast<int*>(smem + p.off_prefix);   // [B + 1]
+    const int NS = p.stages, subs = p.subs, hc = p.hc;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.off_bars);        // [subs][NS]
+    uint64_t* empty = full + subs * NS;
+    uint2* desc = reinterpret_cast<uint2*>(smem + p.off_desc);              // [subs][kDescSlots]: page, sequence << 16 | attended slots
+    int* prefix = reinterpret_cast<int*>(smem + p.off_prefix);              // [B + 1]
+    const uint32_t ring = smem_u32(smem);                                   // [subs][NS] slots
+
+    if (threadIdx.x < subs * NS) {
+        mbar_init(&full[threadIdx.x], 1);
+        mbar_init(&empty[threadIdx.x], hc);
+    }
+    mbar_fence_init();
+    __syncthreads();
 
     pdl_wait();   // lengths / block table / q / the cache itself may be produced by the previous kernel
     pdl_launch_dependents();      // after the wait: the merge kernel may read the lengths before this kernel ends
 
-    // The flattened page list is cut into p.grid equal ranges.  A CTA has 8 warps = 8 (range, kv head) pairs:
+    // The flattened page list is cut into p.grid equal ranges.  A CTA has 8 consumer warps = 8 (range, kv head) pairs:
     // with 8 kv heads one range, with fewer heads several consecutive ranges (subs of them).  Up to 32 sequences, every warp
     // keeps their lengths and page counts in its lanes: one load and a scan, no shared memory and no barrier.
     const bool small = p.B <= 32;
@@ -168,30 +215,16 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
         total = build_prefix(p, prefix);
     }
     const int ppc = (total + p.grid - 1) / p.grid;               // pages per range
-    const int subs = p.subs;
-    const int h = blockIdx.y * p.hc + warp % p.hc;               // kv head of this warp
-    const int sub = warp / p.hc;
-    const int vc = (int)blockIdx.x * subs + sub;                 // range of this warp
-    const int lo = min(total, vc * ppc);
-    const int hi = min(total, lo + ppc);
-    if (lo >= hi || sub >= subs || vc >= p.grid || h >= p.Hkv) return;
-
-    const int group = p.group;
-    constexpr int NS = ring_depth(BITS, TWO);                     // pages in flight per warp
-    const uint32_t my_ring = smem_u32(smem) + p.off_ring + (uint32_t)warp * (NS * SLOT);
-    const int n_my = hi - lo;                                     // pages this warp walks: f = lo + j
-
-    WarpState<BITS, WIDE> acc;
-    state_reset(acc);
-
-    // Page descriptors (page id, sequence, valid tokens) of 32 consecutive pages of this warp, one per
-    // lane.  Two windows: one for the page being consumed, one for the page being issued ahead.
-    struct Desc { int page, b, attended; };   // attended: bit mask of the page's slots
-    auto lookup = [&](int base) -> Desc {
-        const int j = base + lane;
-        const int f = min(lo + j, hi - 1);
-        int b = 0, len, before;
-        if (small) {                           // largest b with pages before it <= f
+    const int h0 = blockIdx.y * hc;                              // first kv head of the CTA
+    auto range = [&](int sub, int& lo, int& hi) {
+        const int vc = (int)blockIdx.x * subs + sub;
+        lo = vc < p.grid ? min(total, vc * ppc) : total;
+        hi = min(total, lo + ppc);
+    };
+    // largest b with pages before it <= f (executed by whole warps)
+    auto sequence_of = [&](int f, int& len, int& before) -> int {
+        int b = 0;
+        if (small) {
 #pragma unroll
             for (int step = 16; step > 0; step >>= 1) {
                 const int v = __shfl_sync(0xffffffffu, pre_l, b + step);
@@ -204,72 +237,116 @@ __global__ void __launch_bounds__(kAttnThreads, TWO ? B200Q_ATTN_CTAS : 1) paged
             len = p.lengths[b];
             before = prefix[b];
         }
-        Desc d = {-1, b, 0};
-        if (j < n_my) {
-            const SeqPages sp = seq_pages(len, cap, p.P, p.sink, p.window);
-            const int idx = f - before;
-            const int pg = idx < sp.sink_pages ? idx : sp.first_recent + (idx - sp.sink_pages);
-            const int page = p.block_table[(int64_t)b * p.max_blocks + pg];
-            d.page = (page < 0 || page >= p.num_pages) ? -1 : page;
-            d.attended = (int)page_mask16(pg, sp.L, p.sink, p.window);
-        }
-        return d;
+        return b;
     };
-    Desc win_c = lookup(0);     // consume window
-    Desc win_i = win_c;         // issue window
-    const PageLanes L = page_lanes<BITS>(lane, h, (uint32_t)p.row_bytes, p.scale_row_halves, p.Gd, p.k_scales, p.v_scales);
-    const size_t page_code_bytes = (size_t)p.P * p.row_bytes;
-    const size_t page_scale_halves = (size_t)p.P * p.scale_row_halves;
-    int slot_i = 0;      // ring slot of the next page to issue
-    // issue the asynchronous copies of page j (descriptor held by lane j % 32 of the issue window)
-    auto issue = [&](int j) {
-        if (j > 0 && (j & 31) == 0) win_i = lookup(j);
-        const int src_lane = j & 31;
-        const int page = __shfl_sync(0xffffffffu, win_i.page, src_lane);
-        issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, L, page, p.k_codes, p.v_codes, page_code_bytes, page_scale_halves);
-        slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1;
-    };
+    const uint32_t limit = kAttnWaitLimit;
 
+    // ================================ producer ================================
+    if (warp == kAttnWarps) {
+        const uint32_t sc_bytes = BITS == 16 ? 0u : split_scale_bytes(hc, p.Gd);
+        const uint32_t tx = (uint32_t)(2 * hc * TILE) + 2 * sc_bytes;
+        bool ok = true;
+        int slot = 0;
+        uint32_t par = 1u;                                       // a fresh barrier's previous phase counts as done
+        for (int j = 0; j < ppc; ++j) {
+            for (int sub = 0; sub < subs; ++sub) {
+                int lo, hi;
+                range(sub, lo, hi);
+                if (lo + j >= hi) continue;
+                uint2* dsub = desc + sub * kDescSlots;
+                if ((j & 31) == 0) {                             // descriptors of this range's next 32 pages, one per lane
+                    const int f = min(lo + j + lane, hi - 1);
+                    int len, before;
+                    const int b = sequence_of(f, len, before);
+                    const SeqPages sq = seq_pages(len, cap, p.P, p.sink, p.window);
+                    const int idx = f - before;
+                    const int pg = idx < sq.sink_pages ? idx : sq.first_recent + (idx - sq.sink_pages);
+                    const int page = p.block_table[(int64_t)b * p.max_blocks + pg];
+                    dsub[(j + lane) & (kDescSlots - 1)] = make_uint2((uint32_t)(page < 0 || page >= p.num_pages ? -1 : page),
+                                                                     ((uint32_t)b << 16) | page_mask16(pg, sq.L, p.sink, p.window));
+                    __syncwarp();
+                }
+                const int bar = sub * NS + slot;
+                ok = mbar_wait_bounded(&empty[bar], par, &g_device_status, EV_ATTN_EMPTY_WAIT, ok ? limit : 64u) && ok;
+                __syncwarp();
+                if (lane == 0) {
+                    const int page = (int)dsub[j & (kDescSlots - 1)].x;
+                    if (page < 0) {
+                        mbar_arrive(&full[bar]);                 // a missing page: nothing to copy, the consumers skip it
+                    } else {
+                        const uint32_t dst = ring + (uint32_t)bar * p.slot_bytes;
+                        mbar_arrive_expect_tx(&full[bar], tx);
+                        tma_load_3d(dst, &sp.kmap, 0, page * 16, BITS == 16 ? 2 * h0 : h0, &full[bar]);
+                        tma_load_3d(dst + hc * TILE, &sp.vmap, 0, page * 16, BITS == 16 ? 2 * h0 : h0, &full[bar]);
+                        if (BITS != 16) {
+                            const uint32_t sdst = dst + 2 * hc * TILE;
+                            if (p.Hkv == hc) {                   // the page's scales are contiguous
+                                const size_t at = (size_t)page * 16 * p.scale_row_halves;
+                                bulk_g2s(smem + (sdst - ring), p.k_scales + at, sc_bytes, &full[bar]);
+                                bulk_g2s(smem + (sdst + sc_bytes - ring), p.v_scales + at, sc_bytes, &full[bar]);
+                            } else {
+                                tma_load_2d(sdst, &sp.ksmap, h0 * p.Gd * 2, page * 16, &full[bar]);
+                                tma_load_2d(sdst + sc_bytes, &sp.vsmap, h0 * p.Gd * 2, page * 16, &full[bar]);
+                            }
+                        }
+                    }
+                }
+            }
+            if (++slot == NS) { slot = 0; par ^= 1u; }
+        }
+        return;
+    }
+
+    // ================================ consumers ================================
+    const int hl = warp % hc, h = h0 + hl;                       // kv head of this warp
+    const int sub = warp / hc;
+    if (sub >= subs) return;
+    const int vc = (int)blockIdx.x * subs + sub;                 // range of this warp
+    int lo, hi;
+    range(sub, lo, hi);
+    if (lo >= hi) return;
+    const int group = p.group;
+    const int n_my = hi - lo;                                    // pages this warp walks: f = lo + j
+
+    WarpState<BITS, WIDE> acc;
+    state_reset(acc);
     auto flush = [&](int b) {
         float* dst = p.partial + ((size_t)(vc + b) * p.Hq + h * group) * (D + 2);
         emit(acc, group, lane, [&](int head, int d, float v) { dst[head * (D + 2) + d] = v; },
              [&](int head, float m, float l) { dst[head * (D + 2) + D] = m; dst[head * (D + 2) + D + 1] = l; });
     };
-
-    // prologue: copies of the first NS - 1 pages
-    for (int j = 0; j < NS - 1; ++j) {
-        if (j < n_my) issue(j);
-        else { cp_async_commit(); slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1; }
-    }
-
-    // the first sequence's queries, while the copies are in flight
     auto queries = [&](int b) {
         load_queries<BITS, LOGG>(acc, reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D, group, p.q_dtype, p.scale, lane);
     };
-    int cur_b = __shfl_sync(0xffffffffu, win_c.b, 0);
-    queries(cur_b);
-
-    int slot_c = 0;     // ring slot of the page being consumed
+    int cur_b;
+    {
+        int len, before;
+        cur_b = sequence_of(lo, len, before);
+    }
+    queries(cur_b);                                              // the first sequence's, while the copies are in flight
+    const PageRead R = box_read<BITS>(lane, hl, hc, p.Gd);
+    const uint2* dsub = desc + sub * kDescSlots;
+    bool ok = true;
+    int slot = 0;
+    uint32_t par = 0;
     for (int j = 0; j < n_my; ++j) {
-        if (j > 0 && (j & 31) == 0) win_c = lookup(j);
-        const int page = __shfl_sync(0xffffffffu, win_c.page, j & 31);
-        const int b = __shfl_sync(0xffffffffu, win_c.b, j & 31);
-        const uint32_t attended = (uint32_t)__shfl_sync(0xffffffffu, win_c.attended, j & 31);
-        // look-ahead: copies of page j + NS - 1 (an empty group keeps the count uniform at the end)
-        if (j + NS - 1 < n_my) issue(j + NS - 1);
-        else cp_async_commit();
-        cp_async_wait<NS - 1>();     // at most NS - 1 groups pending: page j has landed
-        __syncwarp();
-
-        if (b != cur_b) {
+        const int bar = sub * NS + slot;
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[bar], par, &g_device_status, EV_ATTN_FULL_WAIT, ok ? limit : 64u)) && ok;
+        const uint2 d = dsub[j & (kDescSlots - 1)];
+        const int b = (int)(d.y >> 16);
+        if (b != cur_b && ok) {
             flush(cur_b);
             cur_b = b;
             state_reset(acc);
             queries(b);
         }
-        if (page >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, L, attended, lane);
+        if ((int)d.x >= 0 && ok) {
+            const uint32_t sl = ring + (uint32_t)bar * p.slot_bytes;
+            process_page<BITS, LOGG, true>(acc, sl + hl * TILE, sl + (hc + hl) * TILE, sl + 2 * hc * TILE, R, d.y & 0xFFFFu, lane);
+        }
         __syncwarp();   // every lane is done with this slot before it is refilled
-        slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
+        if (lane == 0) mbar_arrive(&empty[bar]);
+        if (++slot == NS) { slot = 0; par ^= 1u; }
     }
     flush(cur_b);
 }
@@ -315,7 +392,7 @@ template <int BITS, int LOGG, bool WIDE>
 __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterAttnParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int D = kHeadDim;
-    constexpr int NS = ring_depth(BITS, false) - (WIDE ? 2 : 1);  // pages in flight per warp (room for the partial results)
+    constexpr int NS = ring_depth(BITS) - (WIDE ? 1 : 0);         // pages in flight per warp (room for the partial results)
     constexpr int SLOT = PageShape<BITS>::SLOT;
     constexpr int PW = D + 2;                                     // floats of one partial: accumulator, max, sum
     const int warp = threadIdx.x >> 5;
@@ -427,6 +504,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     if (n_my > 0) {
         const void* qrows = p.fused ? (const void*)qs : (const void*)(reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D);
         const PageLanes Lp = page_lanes<BITS>(lane, h, (uint32_t)p.row_bytes, p.scale_row_halves, p.Gd, p.k_scales, p.v_scales);
+        const PageRead Rp = ring_read(Lp, lane);
         const size_t page_code_bytes = (size_t)p.P * p.row_bytes;
         const size_t page_scale_halves = (size_t)p.P * p.scale_row_halves;
         const uint32_t my_ring = smem_u32(smem) + p.off_ring + (uint32_t)warp * (NS * SLOT);
@@ -451,7 +529,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
             __syncwarp();
             const int valid = min(p.P, L - (lo + j) * p.P);
             const uint32_t attended = valid >= 16 ? 0xFFFFu : ((1u << max(valid, 0)) - 1u);
-            if (__shfl_sync(0xffffffffu, ids_c, j & 31) >= 0) process_page<BITS, LOGG>(acc, my_ring + slot_c * SLOT, Lp, attended, lane);
+            if (__shfl_sync(0xffffffffu, ids_c, j & 31) >= 0) {
+                const uint32_t sl = my_ring + slot_c * SLOT;
+                process_page<BITS, LOGG, false>(acc, sl, sl + PageShape<BITS>::TILE, sl + 2 * PageShape<BITS>::TILE, Rp, attended, lane);
+            }
             __syncwarp();
             slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
         }
@@ -739,7 +820,7 @@ int cluster_size_for(int B, int Hkv) {
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     const bool g32 = p.G == 32, wide = p.group > 4;
     const int slot = p.bits == 4 ? PageShape<4>::SLOT : PageShape<8>::SLOT;
-    const int ns = ring_depth(p.bits, false) - (wide ? 2 : 1);
+    const int ns = ring_depth(p.bits) - (wide ? 1 : 0);
     uint32_t off = 0;
     p.off_q = off;      off += align_up_u32((uint32_t)p.group * 128 * 2, 128);
     p.off_wpart = off;  off += align_up_u32((uint32_t)kAttnWarps * p.group * 130 * 4, 128);
@@ -785,12 +866,35 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     return finish_launch();
 }
 
+// Byte tensor [heads][tokens][row] of a page pool whose token rows are `pitch` bytes apart; box = heads of a CTA x 16 tokens x row.
+bool page_map(const void* ptr, uint32_t row, int64_t tokens, int heads, int pitch, int box_heads, CUtensorMap* out) {
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
+    const cuuint64_t dims[3] = {row, (cuuint64_t)tokens, (cuuint64_t)heads};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch, row};
+    const cuuint32_t box[3] = {row, 16, (cuuint32_t)box_heads};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtensorMap* out) {
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)tokens};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, 16};
+    const cuuint32_t estr[2] = {1, 1};
+    return encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int launch_split_attention(AttnParams& p, cudaStream_t stream) {
     const int bits = p.bits;
     p.hc = std::min(p.Hkv, kAttnWarps);
     p.subs = subs_for(p.hc);
     const int chunks = p.Hkv / p.hc;
-    p.slot_bytes = bits == 4 ? PageShape<4>::SLOT : bits == 8 ? PageShape<8>::SLOT : PageShape<16>::SLOT;
+    p.slot_bytes = split_slot_bytes(bits, p.hc, p.Gd);
     int ctas_per_sm = tuning_get("attn.ctas_per_sm");
     if (ctas_per_sm <= 0) ctas_per_sm = bits == 16 ? 1 : B200Q_ATTN_CTAS;
     // At least three pages per range (by the block table's capacity; the lengths live on the device): short
@@ -806,19 +910,29 @@ int launch_split_attention(AttnParams& p, cudaStream_t stream) {
     p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(std::min({kMaxRanges, kMaxGrid * full_subs, want}), (pages_cap + min_pages - 1) / min_pages));
     const int launch_grid = (p.grid + p.subs - 1) / p.subs;   // CTAs: each covers `subs` ranges
     const bool two = bits != 16 && launch_grid * chunks > sm_count();
-    const int stages = ring_depth(bits, two);
-
-    uint32_t off = 0;
-    p.off_prefix = off; off += align_up_u32((p.B + 1) * sizeof(int), 16);
-    off = align_up_u32(off, 128);
-    p.off_ring = off;
+    // shared memory: [1 KB alignment] ring, barriers, descriptors, prefix sums
     const uint32_t cap = (uint32_t)max_smem_optin();
-    const uint32_t total_smem = off + stages * kAttnWarps * p.slot_bytes;
-    if (total_smem > cap) return B200Q_ERR_UNSUPPORTED;
-    p.stages = stages;
+    const uint32_t fixed = 1024 + align_up_u32(2 * p.subs * kMaxRing * 8, 128) + p.subs * kDescSlots * 8 + align_up_u32((p.B + 1) * sizeof(int), 128);
+    const uint32_t budget = two ? (cap + 1024) / 2 - 1024 : cap;       // an SM keeps 1 KB per resident CTA
+    p.stages = (int)std::min<uint32_t>(kMaxRing, (budget - std::min(budget, fixed)) / (p.subs * p.slot_bytes));
+    if (p.stages < 2) return B200Q_ERR_UNSUPPORTED;
+    p.off_bars = p.subs * p.stages * p.slot_bytes;
+    p.off_desc = p.off_bars + align_up_u32(2 * p.subs * p.stages * 8, 128);
+    p.off_prefix = p.off_desc + p.subs * kDescSlots * 8;
+    const uint32_t total_smem = 1024 + p.off_prefix + align_up_u32((p.B + 1) * sizeof(int), 128);
+    SplitParams sp = {};
+    sp.a = p;
+    const uint32_t row = bits == 4 ? 64 : 128, tiles = bits == 16 ? 2 : 1;       // a plain row is two tiles of 128 bytes
+    if (!page_map(p.k_codes, row, p.num_pages * 16, p.Hkv * tiles, p.row_bytes, p.hc * tiles, &sp.kmap) ||
+        !page_map(p.v_codes, row, p.num_pages * 16, p.Hkv * tiles, p.row_bytes, p.hc * tiles, &sp.vmap))
+        return B200Q_ERR_LAUNCH;
+    if (bits != 16 && chunks > 1 &&
+        (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hc * p.Gd * 2, &sp.ksmap) ||
+         !scale_map(p.v_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hc * p.Gd * 2, &sp.vsmap)))
+        return B200Q_ERR_LAUNCH;
 
     const bool g32 = p.G == 32, wide_group = p.group > 4, bf = p.q_dtype == B200Q_BF16;
-    using KernelFn = void (*)(AttnParams);
+    using KernelFn = void (*)(SplitParams);
 #define B200Q_ATTN_PAIR(BITS, LOGG, TWO) {paged_attn_kernel<BITS, LOGG, TWO, false>, paged_attn_kernel<BITS, LOGG, TWO, true>}
     static const KernelFn quantised[2][2][2][2] = {      // [q4][group 32][two][wide]
         {{B200Q_ATTN_PAIR(8, 6, false), B200Q_ATTN_PAIR(8, 6, true)}, {B200Q_ATTN_PAIR(8, 5, false), B200Q_ATTN_PAIR(8, 5, true)}},
@@ -841,12 +955,12 @@ int launch_split_attention(AttnParams& p, cudaStream_t stream) {
     {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(launch_grid, chunks);
-        cfg.blockDim = dim3(kAttnThreads);
+        cfg.blockDim = dim3(kSplitThreads);
         cfg.dynamicSmemBytes = total_smem;
         cfg.stream = stream;
         cfg.attrs = attr;
         cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
-        if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return B200Q_ERR_LAUNCH;
+        if (cudaLaunchKernelEx(&cfg, kernel, sp) != cudaSuccess) return B200Q_ERR_LAUNCH;
     }
     {
         cudaLaunchConfig_t cfg = {};
@@ -902,14 +1016,15 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
                          ((uintptr_t)q % 16 == 0) && ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) &&
                          ((uintptr_t)k_scales % 8 == 0) && ((uintptr_t)v_scales % 8 == 0);
     if (!fast_ok && tp_out_slot >= 0) return B200Q_ERR_UNSUPPORTED;   // the exchange exists only in the split-KV kernels
-    if (!fast_ok) {
+    auto simple = [&]() -> int {
         SimpleParams sp = {q, k_codes, v_codes, k_scales, v_scales, block_table, lengths, out,
                            B, Hq, Hkv, D, page_size, max_blocks, group_size, Gd, bits, q_dtype, scale_dtype,
                            num_pages, scale, sink_tokens, window_size, nullptr, 0, 0, 0};
         const int warps = 4;
         paged_attn_simple_kernel<<<(B * Hq + warps - 1) / warps, warps * 32, 0, stream>>>(sp);
         return finish_launch();
-    }
+    };
+    if (!fast_ok) return simple();
     // small batches: one cluster per (sequence, kv head), merged on chip - no workspace, no second launch
     const int cluster = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_size_for(B, Hkv) : 0;
     if (cluster > 0) {
@@ -925,6 +1040,8 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
         const int rc = launch_cluster_attention(c, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
     }
+    // the split kernel copies scales in 16-byte pieces
+    if (((uintptr_t)k_scales | (uintptr_t)v_scales) % 16 != 0) return tp_out_slot >= 0 ? (int)B200Q_ERR_UNSUPPORTED : simple();
     if (workspace == nullptr || workspace_bytes < paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D)) return B200Q_ERR_WORKSPACE;
 
     AttnParams p = {};
@@ -938,7 +1055,8 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     p.window = window_size;
     p.row_bytes = Hkv * dp;
     p.scale_row_halves = Hkv * Gd;
-    return launch_split_attention(p, stream);
+    const int rc = launch_split_attention(p, stream);
+    return rc == B200Q_ERR_UNSUPPORTED && tp_out_slot < 0 ? simple() : rc;      // scales of very many kv heads do not fit a ring
 }
 
 // Plain fp16 / bf16 pages on the split-KV kernels; B200Q_ERR_UNSUPPORTED outside their shapes.

@@ -49,6 +49,11 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
 __device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], uint32_t a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a));
+    return r;
+}
 __device__ __forceinline__ void lds64(uint32_t (&r)[2], uint32_t a) {
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
 }
@@ -206,6 +211,31 @@ __device__ __forceinline__ PageLanes page_lanes(int lane, int h, uint32_t row_by
     L.rd = (uint32_t)up * 256 + (uint32_t)((lane >> 3) & 1) * 128 + (uint32_t)(((lane & 7) ^ (BITS == 4 ? 2 * up : up)) << 4);
     return L;
 }
+// Where process_page finds a page: the warp's own ring slot (page_lanes above, BOX = false), or one head of a page that a tensor copy put
+// down for all heads of the block (BOX = true: [head][16 tokens][row], rows of 64 or 128 bytes swizzled by the copy, plain rows
+// as two halves of 128 bytes; scales [16 tokens][heads] of K, then of V).
+struct PageRead {
+    uint32_t rd;                      // ldmatrix row address inside a tile, first pair of chunks
+    uint32_t sc, sc8, scv;            // scales of token g; distances to token g + 8 and to V's
+};
+__device__ __forceinline__ PageRead ring_read(const PageLanes& L, int lane) { return {L.rd, (uint32_t)(lane >> 2) * 8, 64, 128}; }
+template <int BITS>
+__device__ __forceinline__ PageRead box_read(int lane, int head, int heads, int Gd) {
+    const int up = lane >> 4, row = (lane & 7) + ((lane >> 3) & 1) * 8;
+    PageRead R;
+    R.rd = BITS == 4 ? (uint32_t)row * 64 + (uint32_t)((up ^ ((row >> 1) & 3)) << 4) : (uint32_t)row * 128 + (uint32_t)((up ^ (row & 7)) << 4);
+    R.sc = (uint32_t)(((lane >> 2) * heads + head) * Gd * 2);
+    R.sc8 = (uint32_t)(8 * heads * Gd * 2);
+    R.scv = 2 * R.sc8;
+    return R;
+}
+// ldmatrix address of chunks 2c, 2c + 1
+template <int BITS, bool BOX>
+__device__ __forceinline__ uint32_t chunk_pair(uint32_t rd, int c) {
+    if (!BOX) return (rd ^ (uint32_t)(((BITS == 4 ? 4 * c : 2 * c) & 7) << 4)) + 2 * c * 256;
+    return (rd ^ (uint32_t)(((2 * c) & 7) << 4)) + (BITS == 16 ? (uint32_t)(c >> 2) * 2048 : 0u);
+}
+
 // Asynchronous copies of one page into a ring slot: one commit group, empty for a missing page.  Whole pages are copied; slots
 // past the length are masked where they are used.
 template <int BITS, int LOGG>
@@ -229,14 +259,13 @@ __device__ __forceinline__ void issue_page(uint32_t slot, const PageLanes& L, in
     cp_async_commit();
 }
 
-// One page: `attended` = bit mask of the token slots that take part (at least one).
-template <int BITS, int LOGG, bool WIDE>
-__device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t slot, const PageLanes& L, uint32_t attended, int lane) {
-    using P = PageShape<BITS>;
+// One page: its K and V tile and its scales in shared memory; `attended` = bit mask of the token slots that take part (at least one).
+template <int BITS, int LOGG, bool BOX, bool WIDE>
+__device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t k_tile, uint32_t v_tile, uint32_t scales, const PageRead& R, uint32_t attended, int lane) {
     constexpr int ST = WarpState<BITS, WIDE>::ST;
     constexpr bool BF = BITS == 16 && LOGG == 1;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t kr = slot + L.rd, vr = kr + P::TILE;
+    const uint32_t kr = k_tile + R.rd, vr = v_tile + R.rd;
     const bool in0 = (attended >> g) & 1u, in1 = (attended >> (g + 8)) & 1u;
 
     // ---------------- scores of tokens g, g + 8 ----------------
@@ -247,7 +276,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             uint32_t r[4];
-            ldsm4(r, (kr ^ (uint32_t)(((2 * i) & 7) << 4)) + 2 * i * 256);
+            ldsm4(r, chunk_pair<BITS, BOX>(kr, i));
             mma_f16<BF>(c, r[0], r[1], r[2], r[3], a.qb[0][i][0], a.qb[0][i][1]);
         }
         s[0][0] = c[0] * a.qs[0];
@@ -255,8 +284,13 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
         if constexpr (WIDE) { s[ST - 1][0] = c[1] * a.qs[0]; s[ST - 1][1] = c[3] * a.qs[0]; }
     } else {
         uint32_t ks0[2], ks1[2], vs0[2], vs1[2];
-        const uint32_t sc = slot + 2 * P::TILE + g * 8;
-        lds64(ks0, sc); lds64(ks1, sc + 64); lds64(vs0, sc + 128); lds64(vs1, sc + 192);
+        const uint32_t sc = scales + R.sc;
+        if (BOX && LOGG == 6) {                            // two scales per token and head
+            ks0[0] = lds32(sc); ks1[0] = lds32(sc + R.sc8); vs0[0] = lds32(sc + R.scv); vs1[0] = lds32(sc + R.scv + R.sc8);
+            ks0[1] = ks1[1] = vs0[1] = vs1[1] = 0u;
+        } else {
+            lds64(ks0, sc); lds64(ks1, sc + R.sc8); lds64(vs0, sc + R.scv); lds64(vs1, sc + R.scv + R.sc8);
+        }
         float acc[ST][2];
 #pragma unroll
         for (int x = 0; x < ST; ++x) acc[x][0] = acc[x][1] = 0.0f;
@@ -266,12 +300,12 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
         for (int i = 0; i < 4; ++i) {
             uint32_t w[4];
             if constexpr (BITS == 4) {
-                if (i % 2 == 0) ldsm4(r, (kr ^ (uint32_t)((2 * i) << 4)) + i * 256);
+                if (i % 2 == 0) ldsm4(r, chunk_pair<BITS, BOX>(kr, i / 2));
                 const uint32_t w0 = r[(i & 1) * 2], w1 = r[(i & 1) * 2 + 1];
                 w[0] = w0 & 0x0F0F0F0Fu; w[1] = w1 & 0x0F0F0F0Fu;
                 w[2] = (w0 >> 4) & 0x0F0F0F0Fu; w[3] = (w1 >> 4) & 0x0F0F0F0Fu;
             } else {
-                ldsm4(w, (kr ^ (uint32_t)((2 * i) << 4)) + 2 * i * 256);
+                ldsm4(w, chunk_pair<BITS, BOX>(kr, i));
             }
 #pragma unroll
             for (int x = 0; x < ST; ++x) {
@@ -390,7 +424,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             uint32_t r[4];
-            ldsm4_trans(r, (vr ^ (uint32_t)(((2 * i) & 7) << 4)) + 2 * i * 256);
+            ldsm4_trans(r, chunk_pair<BITS, BOX>(vr, i));
             if (attended != 0xFFFFu) { r[0] &= mask0; r[2] &= mask0; r[1] &= mask1; r[3] &= mask1; }
             mma_f16<BF>(a.o[i], r[0], r[2], r[1], r[3], b[0][0], b[0][1]);
             if constexpr (WIDE) mma_f16<BF>(a.o[i], r[0], r[2], r[1], r[3], b[1][0], b[1][1]);
@@ -416,7 +450,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
             }
             if constexpr (BITS == 4) {
                 uint32_t r[4];
-                ldsm4_trans(r, (vr ^ (uint32_t)((4 * cp) << 4)) + 2 * cp * 256);
+                ldsm4_trans(r, chunk_pair<BITS, BOX>(vr, cp));
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {           // 32 dims: this lane's 4 codes of two token pairs
                     const uint32_t x = r[2 * cc], y = r[2 * cc + 1], x8 = x >> 8, y8 = y >> 8;
@@ -433,7 +467,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {           // 32 dims = chunks 4cp + 2cc and the next
                     uint32_t r[4];
-                    ldsm4_trans(r, (vr ^ (uint32_t)((4 * cp + 2 * cc) << 4)) + (4 * cp + 2 * cc) * 256);
+                    ldsm4_trans(r, chunk_pair<BITS, BOX>(vr, 2 * cp + cc));
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         const uint32_t x = r[2 * q], y = r[2 * q + 1];

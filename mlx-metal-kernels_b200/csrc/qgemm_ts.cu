@@ -34,8 +34,7 @@
 // carries on without the data so that it always terminates and frees its tensor memory.
 #include "gemv_params.cuh"
 
-#include <cuda.h>
-#include <cudaTypedefs.h>
+#include "tensor_map.cuh"
 
 #include <algorithm>
 #include <functional>
@@ -745,28 +744,21 @@ struct MapKeyHash {
 };
 std::mutex g_map_mu;
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
-// 2-D byte tensor [d1 rows, d0 bytes] (rows d0 bytes apart), box b0 x b1.  The driver entry point is looked up at run
-// time, so the library has no link-time dependency on libcuda.
+// 2-D byte tensor [d1 rows, d0 bytes] (rows d0 bytes apart), box b0 x b1.
 bool tensor_map_2d(const void* ptr, uint64_t d0, uint64_t d1, uint32_t b0, uint32_t b1, CUtensorMapSwizzle swizzle, CUtensorMap* out) {
     const MapKey key = {ptr, d0, d1, b0, b1, (uint32_t)swizzle};
     std::lock_guard<std::mutex> lock(g_map_mu);
     auto it = g_maps.find(key);
     if (it != g_maps.end()) { *out = it->second; return true; }
-    if (g_encode == nullptr) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || fn == nullptr)
-            return false;
-        g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    }
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
     const cuuint64_t dims[2] = {d0, d1};
     const cuuint64_t strides[1] = {d0};
     const cuuint32_t box[2] = {b0, b1};
     const cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;
-    const CUresult rc = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+    const CUresult rc = encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return false;
@@ -966,6 +958,16 @@ int qgemm_ts(int bits, const GemvParams& g, bool gate_up, cudaStream_t stream) {
     p.act_out = (uint16_t*)g.act_out;
     p.x = g.x;
     return bits == 4 ? dispatch_ts<4>(p, g.K, g.G, gate_up, meta, stream) : dispatch_ts<8>(p, g.K, g.G, gate_up, meta, stream);
+}
+
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess) fn = nullptr;
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }();
+    return encode;
 }
 
 }  // namespace b200q
