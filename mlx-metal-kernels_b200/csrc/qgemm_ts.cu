@@ -852,7 +852,13 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     // tensor memory: accumulators below, ring of A chunks above
     const int dcols = 2 * cols;
     p.a_col0 = std::max(32, (dcols + 31) / 32 * 32);
-    p.a_slots = std::min(kMaxASlots, (512 - p.a_col0) / kChunkCols);
+    // A barrier is waited for by its parity, so whoever waits on a slot has to have seen the slot's phase before.  Ring depths see to
+    // that: an even number of A slots (and, one matrix, of activation slots) gives every slot to the same MMA warp each time round, and
+    // a stage slot serves the same groups of warps each time (chunk n goes to group n modulo kGroups).  Four A slots or more cover
+    // the groups' waits for a free one: the chunk a group wrote before lies at most one round of the ring back.
+    p.a_slots = std::min(kMaxASlots, (512 - p.a_col0) / kChunkCols) & ~1;
+    constexpr int kXStep = MATS == 2 ? 1 : 2;
+    constexpr int kStageStep = std::max(1, kGroups / (SC * MATS));
     // partial sums of a K split: a dedicated buffer signalled by a barrier, else the first CTA's rings between two cluster-wide
     // barriers; both add them in rank order
     const uint32_t red_bytes = (uint32_t)(split - 1) * MATS * std::min(cols, p.B) * kRows * 4;
@@ -867,11 +873,12 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
         return (uint32_t)xs * p.x_bytes + (uint32_t)stages * p.stage_bytes + (uint32_t)meta_bufs_for(stages) * kMetaBuf;
     };
     const int want = tuning_get("ts.stages");
-    int xs = std::min(kMaxXSlots, std::max(2, (int)(64u * 1024u / p.x_bytes)));
-    int stages = want > 0 ? std::max(2, std::min(kMaxStages, want)) : kMaxStages;
-    while (stages > 3 && need(xs, stages) > budget) --stages;
-    while (xs > 2 && need(xs, stages) > budget) --xs;
-    while (stages > 2 && need(xs, stages) > budget) --stages;
+    int xs = std::min(kMaxXSlots, std::max(2, (int)(64u * 1024u / p.x_bytes))) / kXStep * kXStep;
+    constexpr int kMinStages = std::max(2, kStageStep);
+    int stages = (want > 0 ? std::max(kMinStages, std::min(kMaxStages, want)) : kMaxStages) / kStageStep * kStageStep;
+    while (stages > kMinStages + kStageStep && need(xs, stages) > budget) stages -= kStageStep;
+    while (xs > 2 && need(xs, stages) > budget) xs -= kXStep;
+    while (stages > kMinStages && need(xs, stages) > budget) stages -= kStageStep;
     if (need(xs, stages) > budget) return B200Q_ERR_UNSUPPORTED;
     p.stages = stages;
     p.x_slots = xs;
