@@ -1,0 +1,45 @@
+"""The tcgen05 matvec where it can go wrong: a K range that ends inside a stage, group counts whose scale rows no tensor copy can
+fetch, one chunk only, column blocks on both sides of every width, bf16 rows, and ring slots that change hands between warps
+(results have to repeat bit for bit however the warps interleave)."""
+import pytest
+import torch
+
+from helpers import cabi, quant_ops, rel_l2, synth, to_dev
+from oracle import quant_ops as oq
+
+pytestmark = pytest.mark.gpu
+
+
+def _ref(bits):
+    return oq.reference_q4_matvec_decode if bits == 4 else oq.reference_q8_matvec_decode
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("B,N,K,G", [(5, 128, 128, 64), (6, 300, 1152, 128), (16, 129, 2592, 32), (17, 257, 1056, 32), (33, 64, 4096, 64), (65, 500, 640, 64),
+                                     (128, 200, 1024, 64), (129, 333, 512, 64), (256, 130, 1536, 32)])
+@pytest.mark.parametrize("dtype,tol", [(torch.float16, 1e-3), (torch.bfloat16, 6e-3)])
+def test_shapes(cuda, bits, B, N, K, G, dtype, tol):
+    w, s, z = synth.quantized_weight(N, K, bits, G, seed=N + K)
+    x = synth.activations((B, K), 7, "cpu", dtype)
+    for zeros in (z, None):
+        want = _ref(bits)(x, w, s, zeros, group_size=G)
+        got = quant_ops.matvec_rows(bits, *to_dev(cuda, x, w, s, zeros), G)
+        assert rel_l2(got, want) <= tol
+    assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("B,N,K,G", [(8, 4096, 4096, 64), (40, 3000, 4096, 32), (130, 14336, 2048, 64), (200, 9000, 1024, 128)])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_results_repeat(cuda, bits, B, N, K, G):
+    g, u = (tuple(t.to(cuda) for t in synth.quantized_weight(N, K, bits, G, seed=i)) for i in (1, 2))
+    x = synth.activations((B, K), 3, cuda)
+    plain = quant_ops.matvec_rows(bits, x, *g, G)
+    pair = quant_ops.q4_gate_up_matvec_tiled if bits == 4 else quant_ops.q8_gate_up_matvec_tiled
+    both = pair(x, g[0], u[0], g[1], u[1], g[2], u[2], group_size=G)
+    other = torch.empty(64 << 20, dtype=torch.uint8, device=cuda)
+    for i in range(20):
+        if i % 4 == 0:
+            other.zero_()                                  # the next launch starts from a cold cache
+        assert torch.equal(quant_ops.matvec_rows(bits, x, *g, G), plain)
+        assert all(torch.equal(a, b) for a, b in zip(pair(x, g[0], u[0], g[1], u[1], g[2], u[2], group_size=G), both))
+    assert cabi.device_status() == 0
