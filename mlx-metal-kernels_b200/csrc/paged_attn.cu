@@ -128,9 +128,6 @@ __device__ __forceinline__ int find_sequence(const int* prefix, int B, int f) {
     return lo;
 }
 
-// pages in flight per warp of the cluster kernel (its widest form has room for one less)
-constexpr int ring_depth(int bits) { return bits == 4 ? 9 : 5; }
-
 // The split-KV kernel: eight consumer warps (process_page) and one producer warp.
 // Bound by HBM (a page of q8 codes and scales is 4.3 KB per kv head: 181 clocks of an SM's share).  What held it back before was the
 // path into shared memory: every warp copied its own head's pages with 16-byte cp.async pieces and 8-byte pieces of scales - 9 (q8) or
@@ -154,6 +151,7 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
@@ -342,7 +340,7 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
         }
         if ((int)d.x >= 0 && ok) {
             const uint32_t sl = ring + (uint32_t)bar * p.slot_bytes;
-            process_page<BITS, LOGG, true>(acc, sl + hl * TILE, sl + (hc + hl) * TILE, sl + 2 * hc * TILE, R, d.y & 0xFFFFu, lane);
+            process_page<BITS, LOGG>(acc, sl + hl * TILE, sl + (hc + hl) * TILE, sl + 2 * hc * TILE, R, d.y & 0xFFFFu, lane);
         }
         __syncwarp();   // every lane is done with this slot before it is refilled
         if (lane == 0) mbar_arrive(&empty[bar]);
@@ -378,9 +376,18 @@ struct ClusterAttnParams {
     int64_t num_pages;
     float scale;
     int row_bytes, scale_row_halves;
-    uint32_t off_q, off_wpart, off_cpart, off_ring;
+    int hs;                     // kv heads whose scales one copy brings: Hkv, at most 8
+    int stages;                 // pages in flight per warp
+    uint32_t slot_bytes;        // K tile, V tile, scales of K, scales of V
+    uint32_t off_bars, off_q, off_cpart;      // the warps' rings come first
     TpOut tp_out;
 };
+struct alignas(64) ClusterParams {
+    CUtensorMap kmap, vmap;     // as in SplitParams, box of one head
+    CUtensorMap ksmap, vsmap;   // used with more than 8 kv heads only
+    ClusterAttnParams a;
+};
+constexpr int kMaxClusterRing = 8;
 
 __device__ __forceinline__ uint32_t cluster_rank_x() {
     uint32_t r;
@@ -388,12 +395,19 @@ __device__ __forceinline__ uint32_t cluster_rank_x() {
     return r;
 }
 
+// Bound by latency: one launch of a few microseconds whose chain is lengths -> page ids -> pages -> merge of the warps -> merge of the
+// CTAs.  A warp's pages come by tensor copies that one lane issues as soon as the page ids are there, before the queries are
+// rotated (16-byte cp.async pieces kept the CTA's memory path busy for 9100 of the kernel's 20000 clocks at one sequence of 4096 q8
+// tokens); the scales come whole, all heads of the page, which costs less than sixteen pieces of 8 bytes.  Only the page that the new
+// token goes to waits for its append.
 template <int BITS, int LOGG, bool WIDE>
-__global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterAttnParams p) {
-    extern __shared__ __align__(128) uint8_t smem[];
+__global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterParams cp) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    const ClusterAttnParams& p = cp.a;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int D = kHeadDim;
-    constexpr int NS = ring_depth(BITS) - (WIDE ? 1 : 0);         // pages in flight per warp (room for the partial results)
-    constexpr int SLOT = PageShape<BITS>::SLOT;
+    constexpr int TILE = PageShape<BITS>::TILE;
+    const int NS = p.stages;
     constexpr int PW = D + 2;                                     // floats of one partial: accumulator, max, sum
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -403,9 +417,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     const int group = p.group;
     const int S = p.S;
     __half* qs = reinterpret_cast<__half*>(smem + p.off_q);              // [group][D] rotated query rows
-    float* wpart = reinterpret_cast<float*>(smem + p.off_wpart);         // [8 warps][group][PW]
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.off_bars) + warp * NS;      // this warp's ring
+    uint8_t* my_ring = smem + (size_t)warp * NS * p.slot_bytes;
+    const int wstride = NS * (int)p.slot_bytes / 4;                      // a warp's partial [group][PW] takes the place of its pages
+    const float* wpart = reinterpret_cast<const float*>(smem);
     float* cpart = reinterpret_cast<float*>(smem + p.off_cpart);         // [S][group][PW] (used in the first CTA)
 
+    if (lane < NS) mbar_init(&full[lane], 1);
+    mbar_fence_init();
+    __syncwarp();
     pdl_launch_dependents();
     pdl_wait();
 
@@ -422,6 +442,36 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
         const int page = j < n_my ? p.block_table[(size_t)b * p.max_blocks + lo + j] : -1;
         return page >= p.num_pages ? -1 : page;
     };
+    int ids_c = page_ids(0), ids_i = ids_c;                              // page ids of 32 consecutive pages, one per lane: consumed / issued window
+    const uint32_t sc_bytes = split_scale_bytes(p.hs, p.Gd);
+    auto issue = [&](int j) {                                            // copies of page j into its slot
+        if (j > 0 && (j & 31) == 0) ids_i = page_ids(j);
+        const int page = __shfl_sync(0xffffffffu, ids_i, j & 31);
+        if (lane == 0) {
+            uint64_t* bar = &full[j % NS];
+            if (page < 0) {
+                mbar_arrive(bar);                                        // a missing page: nothing to copy, skipped where it is used
+            } else {
+                uint8_t* dst = my_ring + (size_t)(j % NS) * p.slot_bytes;
+                mbar_arrive_expect_tx(bar, 2 * TILE + 2 * sc_bytes);
+                tma_load_3d(smem_u32(dst), &cp.kmap, 0, page * 16, h, bar);
+                tma_load_3d(smem_u32(dst + TILE), &cp.vmap, 0, page * 16, h, bar);
+                if (p.Hkv == p.hs) {
+                    const size_t at = (size_t)page * 16 * p.scale_row_halves;
+                    bulk_g2s(dst + 2 * TILE, p.k_scales + at, sc_bytes, bar);
+                    bulk_g2s(dst + 2 * TILE + sc_bytes, p.v_scales + at, sc_bytes, bar);
+                } else {
+                    const int x = (h & ~7) * p.Gd * 2;
+                    tma_load_2d(smem_u32(dst + 2 * TILE), &cp.ksmap, x, page * 16, bar);
+                    tma_load_2d(smem_u32(dst + 2 * TILE + sc_bytes), &cp.vsmap, x, page * 16, bar);
+                }
+            }
+        }
+    };
+    // the page of the new token is copied after its append
+    const int j_app = p.fused && p.positions[b] >= 0 ? p.positions[b] / p.P - lo : -1;
+    for (int j = 0; j < min(NS, n_my); ++j)
+        if (j != j_app) issue(j);
 
     if (p.fused) {
         const int heads = p.Hq + 2 * p.Hkv;
@@ -493,9 +543,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
                         (uint16_t)(codes[0] | (codes[1] << 4) | (codes[2] << 8) | (codes[3] << 12));
                 if ((lane % lanes_per_group) == 0) sdst[tok * p.Gd + d0 / p.G] = __float2half_rn(sc);
             }
-            __threadfence();          // the appended bytes are in global memory before this CTA's copies read the page
+            // the appended bytes are in global memory, also for the copy engine, before this CTA's copies read the page
+            __threadfence();
+            fence_async_proxy();
         }
         __syncthreads();
+        fence_async_proxy();
+        if (j_app >= 0 && j_app < min(NS, n_my)) issue(j_app);
     }
 
     // ---- this warp's pages ----
@@ -503,54 +557,42 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     state_reset(acc);
     if (n_my > 0) {
         const void* qrows = p.fused ? (const void*)qs : (const void*)(reinterpret_cast<const uint16_t*>(p.q) + ((size_t)b * p.Hq + h * group) * D);
-        const PageLanes Lp = page_lanes<BITS>(lane, h, (uint32_t)p.row_bytes, p.scale_row_halves, p.Gd, p.k_scales, p.v_scales);
-        const PageRead Rp = ring_read(Lp, lane);
-        const size_t page_code_bytes = (size_t)p.P * p.row_bytes;
-        const size_t page_scale_halves = (size_t)p.P * p.scale_row_halves;
-        const uint32_t my_ring = smem_u32(smem) + p.off_ring + (uint32_t)warp * (NS * SLOT);
-        int ids_c = page_ids(0), ids_i = ids_c;                  // page ids of 32 consecutive pages, one per lane: consumed / issued window
-        int slot_i = 0, slot_c = 0;
-        auto issue = [&](int j) {
-            if (j < n_my) {
-                if (j > 0 && (j & 31) == 0) ids_i = page_ids(j);
-                issue_page<BITS, LOGG>(my_ring + slot_i * SLOT, Lp, __shfl_sync(0xffffffffu, ids_i, j & 31), p.k_codes, p.v_codes,
-                                       page_code_bytes, page_scale_halves);
-            } else {
-                cp_async_commit();
-            }
-            slot_i = (slot_i + 1 == NS) ? 0 : slot_i + 1;
-        };
-        for (int j = 0; j < NS - 1; ++j) issue(j);
+        const PageRead R = box_read<BITS>(lane, h % p.hs, p.hs, p.Gd);
         load_queries<BITS, LOGG>(acc, qrows, group, p.fused ? B200Q_F16 : p.q_dtype, p.scale, lane);
+        bool ok = true;
+        int slot = 0;
+        uint32_t par = 0;
         for (int j = 0; j < n_my; ++j) {
             if (j > 0 && (j & 31) == 0) ids_c = page_ids(j);
-            issue(j + NS - 1);
-            cp_async_wait<NS - 1>();
-            __syncwarp();
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[slot], par, &g_device_status, EV_ATTN_FULL_WAIT, ok ? kAttnWaitLimit : 64u)) && ok;
             const int valid = min(p.P, L - (lo + j) * p.P);
             const uint32_t attended = valid >= 16 ? 0xFFFFu : ((1u << max(valid, 0)) - 1u);
-            if (__shfl_sync(0xffffffffu, ids_c, j & 31) >= 0) {
-                const uint32_t sl = my_ring + slot_c * SLOT;
-                process_page<BITS, LOGG, false>(acc, sl, sl + PageShape<BITS>::TILE, sl + 2 * PageShape<BITS>::TILE, Rp, attended, lane);
+            if (__shfl_sync(0xffffffffu, ids_c, j & 31) >= 0 && ok) {
+                const uint32_t k_tile = smem_u32(my_ring) + (uint32_t)slot * p.slot_bytes;
+                process_page<BITS, LOGG>(acc, k_tile, k_tile + TILE, k_tile + 2 * TILE, R, attended, lane);
             }
-            __syncwarp();
-            slot_c = (slot_c + 1 == NS) ? 0 : slot_c + 1;
+            __syncwarp();                                                // every lane is done with this slot before it is refilled
+            if (j + NS < n_my) issue(j + NS);
+            if (++slot == NS) { slot = 0; par ^= 1u; }
         }
     }
     {
-        float* dst = wpart + (size_t)warp * group * PW;
+        float* dst = reinterpret_cast<float*>(my_ring);
         emit(acc, group, lane, [&](int head, int d, float v) { dst[head * PW + d] = v; },
              [&](int head, float m, float l) { dst[head * PW + D] = m; dst[head * PW + D + 1] = l; });
     }
     __syncthreads();
     // ---- merge the 8 warps (fixed order) into this CTA's partial; thread -> (head, d) ----
-    auto merge = [&](const float* src, int n, int head, int d, float& m_tot, float& l_tot) -> float {
+    auto merge = [&](const float* src, int n, int stride, int head, int d, float& m_tot, float& l_tot) -> float {
+        src += head * PW;
         m_tot = -INFINITY;
-        for (int i = 0; i < n; ++i) m_tot = fmaxf(m_tot, src[((size_t)i * group + head) * PW + D]);
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) m_tot = fmaxf(m_tot, src[i * stride + D]);
         float accv = 0.0f;
         l_tot = 0.0f;
+#pragma unroll 8
         for (int i = 0; i < n; ++i) {
-            const float* ps = src + ((size_t)i * group + head) * PW;
+            const float* ps = src + i * stride;
             const float m = ps[D];
             const float w = m == -INFINITY ? 0.0f : exp2f(m - m_tot);      // the maxima are in log2 units
             accv = fmaf(w, ps[d], accv);
@@ -562,7 +604,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     for (int idx = threadIdx.x; idx < group * D; idx += kAttnThreads) {
         const int head = idx / D, d = idx - head * D;
         float m_tot, l_tot;
-        const float v = merge(wpart, kAttnWarps, head, d, m_tot, l_tot);
+        const float v = merge(wpart, kAttnWarps, wstride, head, d, m_tot, l_tot);
         // slot `rank` of the first CTA's table (its own slot for the first CTA itself)
         const uint32_t base = cpart_u + (uint32_t)((rank * group + head) * PW) * 4u;
         auto put = [&](uint32_t off, float val) {
@@ -579,7 +621,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
         for (int idx = threadIdx.x; idx < group * D; idx += kAttnThreads) {
             const int head = idx / D, d = idx - head * D;
             float m_tot, l_tot;
-            const float v = merge(cpart, S, head, d, m_tot, l_tot);
+            const float v = merge(cpart, S, group * PW, head, d, m_tot, l_tot);
             const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
             const unsigned short bits16 = p.fused || p.q_dtype == B200Q_F16 ? __half_as_ushort(__float2half_rn(v * inv))
                                                                             : __bfloat16_as_ushort(__float2bfloat16_rn(v * inv));
@@ -817,18 +859,52 @@ int cluster_size_for(int B, int Hkv) {
     return size;
 }
 
+// Byte tensor [heads][tokens][row] of a page pool whose token rows are `pitch` bytes apart; box = heads of a CTA x 16 tokens x row.
+bool page_map(const void* ptr, uint32_t row, int64_t tokens, int heads, int pitch, int box_heads, CUtensorMap* out) {
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
+    const cuuint64_t dims[3] = {row, (cuuint64_t)tokens, (cuuint64_t)heads};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch, row};
+    const cuuint32_t box[3] = {row, 16, (cuuint32_t)box_heads};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtensorMap* out) {
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)tokens};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, 16};
+    const cuuint32_t estr[2] = {1, 1};
+    return encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     const bool g32 = p.G == 32, wide = p.group > 4;
-    const int slot = p.bits == 4 ? PageShape<4>::SLOT : PageShape<8>::SLOT;
-    const int ns = ring_depth(p.bits) - (wide ? 1 : 0);
-    uint32_t off = 0;
-    p.off_q = off;      off += align_up_u32((uint32_t)p.group * 128 * 2, 128);
-    p.off_wpart = off;  off += align_up_u32((uint32_t)kAttnWarps * p.group * 130 * 4, 128);
-    p.off_cpart = off;  off += align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
-    p.off_ring = off;   off += (uint32_t)kAttnWarps * ns * slot;
-    const uint32_t cap = (uint32_t)max_smem_optin();
-    if (off > cap) return B200Q_ERR_UNSUPPORTED;
-    using KernelFn = void (*)(ClusterAttnParams);
+    p.hs = std::min(p.Hkv, kAttnWarps);
+    p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024);
+    // shared memory: [1 KB alignment] rings, barriers, query rows, the CTAs' partials
+    const uint32_t q_bytes = align_up_u32((uint32_t)p.group * 128 * 2, 128), c_bytes = align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
+    const uint32_t cap = (uint32_t)max_smem_optin(), fixed = 1024 + 128 * 8 + q_bytes + c_bytes;
+    p.stages = (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (kAttnWarps * p.slot_bytes));
+    if (p.stages < 2 || ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0) return B200Q_ERR_UNSUPPORTED;
+    p.off_bars = kAttnWarps * p.stages * p.slot_bytes;
+    p.off_q = p.off_bars + 128 * 8;
+    p.off_cpart = p.off_q + q_bytes;
+    const uint32_t off = 1024 + p.off_cpart + c_bytes;
+    ClusterParams cp = {};
+    cp.a = p;
+    const uint32_t row = p.bits == 4 ? 64 : 128;
+    if (!page_map(p.k_codes, row, p.num_pages * 16, p.Hkv, p.row_bytes, 1, &cp.kmap) ||
+        !page_map(p.v_codes, row, p.num_pages * 16, p.Hkv, p.row_bytes, 1, &cp.vmap))
+        return B200Q_ERR_LAUNCH;
+    if (p.Hkv > p.hs && (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.ksmap) ||
+                         !scale_map(p.v_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.vsmap)))
+        return B200Q_ERR_LAUNCH;
+    using KernelFn = void (*)(ClusterParams);
     static const KernelFn kernels[2][2][2] = {{{paged_attn_cluster_kernel<8, 6, false>, paged_attn_cluster_kernel<8, 6, true>},
                                                {paged_attn_cluster_kernel<8, 5, false>, paged_attn_cluster_kernel<8, 5, true>}},
                                               {{paged_attn_cluster_kernel<4, 6, false>, paged_attn_cluster_kernel<4, 6, true>},
@@ -862,31 +938,8 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return B200Q_ERR_LAUNCH;
+    if (cudaLaunchKernelEx(&cfg, kernel, cp) != cudaSuccess) return B200Q_ERR_LAUNCH;
     return finish_launch();
-}
-
-// Byte tensor [heads][tokens][row] of a page pool whose token rows are `pitch` bytes apart; box = heads of a CTA x 16 tokens x row.
-bool page_map(const void* ptr, uint32_t row, int64_t tokens, int heads, int pitch, int box_heads, CUtensorMap* out) {
-    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-    if (encode == nullptr) return false;
-    const cuuint64_t dims[3] = {row, (cuuint64_t)tokens, (cuuint64_t)heads};
-    const cuuint64_t strides[2] = {(cuuint64_t)pitch, row};
-    const cuuint32_t box[3] = {row, 16, (cuuint32_t)box_heads};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtensorMap* out) {
-    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-    if (encode == nullptr) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)tokens};
-    const cuuint64_t strides[1] = {(cuuint64_t)pitch};
-    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, 16};
-    const cuuint32_t estr[2] = {1, 1};
-    return encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 int launch_split_attention(AttnParams& p, cudaStream_t stream) {

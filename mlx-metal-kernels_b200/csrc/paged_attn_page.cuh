@@ -4,8 +4,7 @@
 // A page of q4 codes is 2.3 KB per kv head and an SM receives one every 100 clocks at the HBM rate, so the instructions per page
 // decide.  (The form before this one dequantised K and V to fp16 with three operations per pair and took 591 warp
 // instructions per page and kv head; it ran at 58 % issue and 0.27 of the DRAM rate.)
-//   * copies: every lane moves 16-byte pieces with cp.async, rows whole, into a ring slot laid out chunk-major
-//     ([16-byte chunk of a row][16 tokens], positions XORed so that neither the copies nor ldmatrix meet bank conflicts).
+//   * copies: tensor copies put a page down token-major and swizzled, so that ldmatrix meets no bank conflicts.
 //   * S = K Q^T: ldmatrix hands every lane the word of its token row; raw codes go into mma.sync.m16n8k32 u8 x s8 (a q4 word costs
 //     two masks and a shift, a q8 word nothing).  The queries are 16-bit fixed point relative to the head's largest
 //     element, as two signed bytes = two columns of the B operand; the offset of the codes is the accumulator's start value.
@@ -30,19 +29,8 @@ constexpr float kQLevels = 32638.0f;          // the largest 16-bit value whose 
 template <int BITS> struct PageShape {
     static constexpr int ROW = kHeadDim * BITS / 8;        // bytes of one token row of one kv head
     static constexpr int TILE = 16 * ROW;                  // K (or V) bytes of a page
-    static constexpr int SLOT = 2 * TILE + (BITS == 16 ? 0 : 256);   // ring slot: K, V, scales of K, scales of V
-    static constexpr int NCH = ROW / 16;                   // 16-byte chunks of a row
 };
 
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-template <int BYTES>
-__device__ __forceinline__ void cp_async_small(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
@@ -185,40 +173,12 @@ __device__ __forceinline__ void load_queries(WarpState<BITS, WIDE>& a, const voi
     }
 }
 
-// Per-lane source and ring offsets of a page copy for kv head h.
-struct PageLanes {
-    uint32_t src, dst;                // first 16-byte piece of this lane
-    uint32_t step;                    // source distance of its next piece (another token row)
-    uint32_t sc_src, sc_dst;          // scales: lanes 0-15 copy K's, lanes 16-31 V's (halves / bytes)
-    const __half* sc_base;
-    uint32_t rd;                      // ldmatrix row address inside a tile, first pair of chunks
-};
-template <int BITS>
-__device__ __forceinline__ PageLanes page_lanes(int lane, int h, uint32_t row_bytes, int scale_row_halves, int Gd, const __half* k_scales,
-                                                const __half* v_scales) {
-    using P = PageShape<BITS>;
-    constexpr int LPR = P::NCH;                            // lanes that share a token row: 4, 8, 16
-    const int row = lane / LPR, ch = lane % LPR;
-    PageLanes L;
-    L.src = (uint32_t)row * row_bytes + (uint32_t)h * P::ROW + 16u * ch;
-    L.step = (uint32_t)(32 / LPR) * row_bytes;
-    L.dst = (uint32_t)ch * 256 + (uint32_t)(((row & 7) ^ ((BITS == 4 ? 2 * ch : ch) & 7)) << 4);
-    L.sc_src = (uint32_t)(lane & 15) * scale_row_halves + h * Gd;
-    L.sc_dst = 2 * P::TILE + (lane < 16 ? 0 : 128) + (lane & 15) * 8;
-    L.sc_base = lane < 16 ? k_scales : v_scales;
-    // matrices of an x4 load: chunk c tokens 0-7, chunk c tokens 8-15, chunk c + 1 tokens 0-7, chunk c + 1 tokens 8-15
-    const int up = lane >> 4;
-    L.rd = (uint32_t)up * 256 + (uint32_t)((lane >> 3) & 1) * 128 + (uint32_t)(((lane & 7) ^ (BITS == 4 ? 2 * up : up)) << 4);
-    return L;
-}
-// Where process_page finds a page: the warp's own ring slot (page_lanes above, BOX = false), or one head of a page that a tensor copy put
-// down for all heads of the block (BOX = true: [head][16 tokens][row], rows of 64 or 128 bytes swizzled by the copy, plain rows
-// as two halves of 128 bytes; scales [16 tokens][heads] of K, then of V).
+// Where process_page finds a page: tiles [16 tokens][row] that a tensor copy put down (rows of 64 or 128 bytes swizzled by the copy,
+// plain rows as two halves of 128 bytes) and scales [16 tokens][heads] of K, then of V.
 struct PageRead {
     uint32_t rd;                      // ldmatrix row address inside a tile, first pair of chunks
     uint32_t sc, sc8, scv;            // scales of token g; distances to token g + 8 and to V's
 };
-__device__ __forceinline__ PageRead ring_read(const PageLanes& L, int lane) { return {L.rd, (uint32_t)(lane >> 2) * 8, 64, 128}; }
 template <int BITS>
 __device__ __forceinline__ PageRead box_read(int lane, int head, int heads, int Gd) {
     const int up = lane >> 4, row = (lane & 7) + ((lane >> 3) & 1) * 8;
@@ -230,37 +190,13 @@ __device__ __forceinline__ PageRead box_read(int lane, int head, int heads, int 
     return R;
 }
 // ldmatrix address of chunks 2c, 2c + 1
-template <int BITS, bool BOX>
+template <int BITS>
 __device__ __forceinline__ uint32_t chunk_pair(uint32_t rd, int c) {
-    if (!BOX) return (rd ^ (uint32_t)(((BITS == 4 ? 4 * c : 2 * c) & 7) << 4)) + 2 * c * 256;
     return (rd ^ (uint32_t)(((2 * c) & 7) << 4)) + (BITS == 16 ? (uint32_t)(c >> 2) * 2048 : 0u);
 }
 
-// Asynchronous copies of one page into a ring slot: one commit group, empty for a missing page.  Whole pages are copied; slots
-// past the length are masked where they are used.
-template <int BITS, int LOGG>
-__device__ __forceinline__ void issue_page(uint32_t slot, const PageLanes& L, int page, const uint8_t* k, const uint8_t* v, size_t page_bytes,
-                                           size_t page_scale_halves) {
-    using P = PageShape<BITS>;
-    if (page >= 0) {
-        const uint8_t* kb = k + (size_t)page * page_bytes + L.src;
-        const uint8_t* vb = v + (size_t)page * page_bytes + L.src;
-        constexpr int N = P::TILE / 512;                   // pieces per lane
-        constexpr int RPS = 32 / P::NCH;                   // token rows per step: 8, 4, 2
-#pragma unroll
-        for (int s = 0; s < N; ++s) {
-            // row = lane row + s * RPS: bits of the row below 8 toggle the position, the others move by half a chunk
-            const uint32_t d = (L.dst ^ (uint32_t)(((s * RPS) & 7) << 4)) + (uint32_t)((s * RPS) >> 3) * 128;
-            cp_async_16(slot + d, kb + (size_t)s * L.step);
-            cp_async_16(slot + P::TILE + d, vb + (size_t)s * L.step);
-        }
-        if constexpr (BITS != 16) cp_async_small<LOGG == 5 ? 8 : 4>(slot + L.sc_dst, L.sc_base + (size_t)page * page_scale_halves + L.sc_src);
-    }
-    cp_async_commit();
-}
-
 // One page: its K and V tile and its scales in shared memory; `attended` = bit mask of the token slots that take part (at least one).
-template <int BITS, int LOGG, bool BOX, bool WIDE>
+template <int BITS, int LOGG, bool WIDE>
 __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t k_tile, uint32_t v_tile, uint32_t scales, const PageRead& R, uint32_t attended, int lane) {
     constexpr int ST = WarpState<BITS, WIDE>::ST;
     constexpr bool BF = BITS == 16 && LOGG == 1;
@@ -276,7 +212,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             uint32_t r[4];
-            ldsm4(r, chunk_pair<BITS, BOX>(kr, i));
+            ldsm4(r, chunk_pair<BITS>(kr, i));
             mma_f16<BF>(c, r[0], r[1], r[2], r[3], a.qb[0][i][0], a.qb[0][i][1]);
         }
         s[0][0] = c[0] * a.qs[0];
@@ -285,7 +221,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
     } else {
         uint32_t ks0[2], ks1[2], vs0[2], vs1[2];
         const uint32_t sc = scales + R.sc;
-        if (BOX && LOGG == 6) {                            // two scales per token and head
+        if (LOGG == 6) {                            // two scales per token and head
             ks0[0] = lds32(sc); ks1[0] = lds32(sc + R.sc8); vs0[0] = lds32(sc + R.scv); vs1[0] = lds32(sc + R.scv + R.sc8);
             ks0[1] = ks1[1] = vs0[1] = vs1[1] = 0u;
         } else {
@@ -300,12 +236,12 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
         for (int i = 0; i < 4; ++i) {
             uint32_t w[4];
             if constexpr (BITS == 4) {
-                if (i % 2 == 0) ldsm4(r, chunk_pair<BITS, BOX>(kr, i / 2));
+                if (i % 2 == 0) ldsm4(r, chunk_pair<BITS>(kr, i / 2));
                 const uint32_t w0 = r[(i & 1) * 2], w1 = r[(i & 1) * 2 + 1];
                 w[0] = w0 & 0x0F0F0F0Fu; w[1] = w1 & 0x0F0F0F0Fu;
                 w[2] = (w0 >> 4) & 0x0F0F0F0Fu; w[3] = (w1 >> 4) & 0x0F0F0F0Fu;
             } else {
-                ldsm4(w, chunk_pair<BITS, BOX>(kr, i));
+                ldsm4(w, chunk_pair<BITS>(kr, i));
             }
 #pragma unroll
             for (int x = 0; x < ST; ++x) {
@@ -424,7 +360,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             uint32_t r[4];
-            ldsm4_trans(r, chunk_pair<BITS, BOX>(vr, i));
+            ldsm4_trans(r, chunk_pair<BITS>(vr, i));
             if (attended != 0xFFFFu) { r[0] &= mask0; r[2] &= mask0; r[1] &= mask1; r[3] &= mask1; }
             mma_f16<BF>(a.o[i], r[0], r[2], r[1], r[3], b[0][0], b[0][1]);
             if constexpr (WIDE) mma_f16<BF>(a.o[i], r[0], r[2], r[1], r[3], b[1][0], b[1][1]);
@@ -450,7 +386,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
             }
             if constexpr (BITS == 4) {
                 uint32_t r[4];
-                ldsm4_trans(r, chunk_pair<BITS, BOX>(vr, cp));
+                ldsm4_trans(r, chunk_pair<BITS>(vr, cp));
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {           // 32 dims: this lane's 4 codes of two token pairs
                     const uint32_t x = r[2 * cc], y = r[2 * cc + 1], x8 = x >> 8, y8 = y >> 8;
@@ -467,7 +403,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {           // 32 dims = chunks 4cp + 2cc and the next
                     uint32_t r[4];
-                    ldsm4_trans(r, chunk_pair<BITS, BOX>(vr, 2 * cp + cc));
+                    ldsm4_trans(r, chunk_pair<BITS>(vr, 2 * cp + cc));
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         const uint32_t x = r[2 * q], y = r[2 * q + 1];
