@@ -842,21 +842,25 @@ inline int subs_for(int hc) { return kAttnWarps % hc == 0 ? kAttnWarps / hc : 1;
 inline bool heads_ok(int Hkv) { return Hkv <= kAttnWarps || Hkv % kAttnWarps == 0; }
 
 // ---- cluster kernel: host side ----
-int cluster_size_for(int B, int Hkv) {
+struct ClusterChoice { int size; bool preferred; };      // size 0: not possible
+ClusterChoice cluster_choice(int B, int Hkv) {
     const int mode = tuning_get("attn.cluster");      // 1: whenever possible, -1: never, 0: small batches
-    if (mode < 0) return 0;
-    const int pairs = B * Hkv;
-    const int sms = sm_count();
+    if (mode < 0 || (mode > 0 && B * Hkv > 65535)) return {0, false};
     // the choice follows the kv heads of the UNSHARDED cache ("ts.tp_world" equal head shards), so that a
     // tensor-parallel rank runs the same kernel, and the same summation order, as the unsharded call
-    if (mode == 0 && pairs * std::max(1, tuning_get("ts.tp_world")) * 8 > 2 * sms) return 0;
-    if (mode > 0 && pairs > 65535) return 0;
+    const int64_t ctas = (int64_t)B * Hkv * std::max(1, tuning_get("ts.tp_world")) * 8;
+    // Preferred while the clusters fill at most three quarters of the SMs; beyond that the split-KV kernel, which uses all of them and
+    // fetches a page once for all heads, is the faster one (layer of the decode stack, 8 kv heads, context 4096: one
+    // sequence 54.6 against 58.0 us, two 73.5 against 70.0, three 88.0 against 84.0, four 103 against 91).  Up to two waves of
+    // clusters stay possible for callers without a workspace.
+    if (mode == 0 && ctas > 2 * sm_count()) return {0, false};
+    const bool preferred = mode > 0 || ctas * 4 <= 3 * sm_count();
     // 8 CTAs per cluster; the opt-in size 16 measured slower (placing one cluster per GPC costs more than the shorter
     // page walk saves: 17.8 us against 12.9 us per stage at batch 1, context 4096)
     int size = 8;
     const int forced = tuning_get("attn.cluster_size");
     if (forced == 8 || forced == 16 || forced == 4) size = forced;
-    return size;
+    return {size, preferred};
 }
 
 // Byte tensor [heads][tokens][row] of a page pool whose token rows are `pitch` bytes apart; box = heads of a CTA x 16 tokens x row.
@@ -1034,7 +1038,7 @@ int launch_split_attention(AttnParams& p, cudaStream_t stream) {
 
 int attention_stage_launches_impl(int B, int Hkv, int with_append) {
     if (B <= 0 || Hkv <= 0) return 0;
-    if (B <= 65535 && cluster_size_for(B, Hkv) > 0) return 1;
+    if (B <= 65535 && cluster_choice(B, Hkv).preferred) return 1;
     return 2 + (with_append ? 1 : 0);
 }
 
@@ -1079,7 +1083,9 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     };
     if (!fast_ok) return simple();
     // small batches: one cluster per (sequence, kv head), merged on chip - no workspace, no second launch
-    const int cluster = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_size_for(B, Hkv) : 0;
+    const bool have_workspace = workspace != nullptr && workspace_bytes >= paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D);
+    const ClusterChoice choice = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv) : ClusterChoice{0, false};
+    const int cluster = choice.preferred || !have_workspace ? choice.size : 0;
     if (cluster > 0) {
         ClusterAttnParams c = {};
         if (tp_out_slot >= 0) c.tp_out = tp_slot(tp_out_slot)->out;
@@ -1095,7 +1101,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     }
     // the split kernel copies scales in 16-byte pieces
     if (((uintptr_t)k_scales | (uintptr_t)v_scales) % 16 != 0) return tp_out_slot >= 0 ? (int)B200Q_ERR_UNSUPPORTED : simple();
-    if (workspace == nullptr || workspace_bytes < paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D)) return B200Q_ERR_WORKSPACE;
+    if (!have_workspace) return B200Q_ERR_WORKSPACE;
 
     AttnParams p = {};
     if (tp_out_slot >= 0) p.tp_out = tp_slot(tp_out_slot)->out;
@@ -1159,7 +1165,9 @@ int rope_append_attention_impl(const void* qkv, const float* cos_table, const fl
                          group <= 8 && heads_ok(Hkv) && page_size == 16 && B <= 65535 && ((uintptr_t)qkv % 16 == 0) &&
                          ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) && ((uintptr_t)k_scales % 8 == 0) &&
                          ((uintptr_t)v_scales % 8 == 0);
-    const int cluster = fast_ok ? cluster_size_for(B, Hkv) : 0;
+    const ClusterChoice choice = fast_ok ? cluster_choice(B, Hkv) : ClusterChoice{0, false};
+    const bool two_stages = q_scratch != nullptr && workspace != nullptr && workspace_bytes >= paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D);
+    const int cluster = choice.preferred || !two_stages ? choice.size : 0;
     if (cluster > 0) {
         int tp_in_slot = -1, tp_out_slot = -1;
         tp_take(&tp_in_slot, &tp_out_slot);
