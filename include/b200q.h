@@ -213,6 +213,15 @@ int b200q_paged_fp16_gqa_decode(const void* q, const void* k_pages, const void* 
                                 int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
                                 void* stream);
 
+/* The same for head_dim 128 and pages of 16 tokens, with a word on the lengths for a host that has to check them: the kernel
+ * writes 1 to *verdict (device-writable host memory, zero before the call) once it has read them and all lie in
+ * [0, max_blocks * page_size], else 2 - at its start, so that the host need not wait for the result or for a copy.
+ * B200Q_ERR_UNSUPPORTED or B200Q_ERR_WORKSPACE, with nothing launched, for other problems. */
+int b200q_paged_fp16_gqa_decode_checked(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table,
+                                        const int32_t* lengths, void* out, void* workspace, size_t workspace_bytes, int B, int Hq,
+                                        int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
+                                        int32_t* verdict, void* stream);
+
 /* The same attention for callers that cannot allocate device memory at all.  (No counterpart in the
  * reference: its runtime allocates every kernel output itself.)  Some hosts of this library may not
  * call cudaMalloc: a plugin running inside another runtime's memory budget, a worker that must not

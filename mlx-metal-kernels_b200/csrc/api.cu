@@ -106,6 +106,10 @@ int paged_fp16_gqa_decode_impl(const void* q, const void* k_pages, const void* v
                                const int32_t* lengths, void* out, void* workspace, size_t workspace_bytes, int B, int Hq,
                                int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
                                cudaStream_t stream);
+int paged_fp16_gqa_decode_checked_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table,
+                                       const int32_t* lengths, void* out, void* workspace, size_t workspace_bytes, int B, int Hq,
+                                       int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
+                                       int32_t* verdict, cudaStream_t stream);
 size_t paged_gqa_workspace_bytes_impl(int B, int Hq, int Hkv, int D);
 int attention_stage_launches_impl(int B, int Hkv, int with_append);
 size_t paged_gqa_static_scratch_bytes_impl();
@@ -603,6 +607,15 @@ int b200q_paged_fp16_gqa_decode(const void* q, const void* k_pages, const void* 
     tp_discard();
     return paged_fp16_gqa_decode_impl(q, k_pages, v_pages, block_table, lengths, out, workspace, workspace_bytes, B, Hq,
                                       Hkv, D, page_size, num_pages, max_blocks, scale, dtype, (cudaStream_t)stream);
+}
+
+int b200q_paged_fp16_gqa_decode_checked(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table,
+                                        const int32_t* lengths, void* out, void* workspace, size_t workspace_bytes, int B, int Hq,
+                                        int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
+                                        int32_t* verdict, void* stream) {
+    tp_discard();
+    return paged_fp16_gqa_decode_checked_impl(q, k_pages, v_pages, block_table, lengths, out, workspace, workspace_bytes, B, Hq,
+                                              Hkv, D, page_size, num_pages, max_blocks, scale, dtype, verdict, (cudaStream_t)stream);
 }
 
 int b200q_quantize_kv(int bits, const void* values, uint8_t* codes, void* scales, int64_t rows, int D, int group_size,

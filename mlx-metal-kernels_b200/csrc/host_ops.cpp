@@ -45,6 +45,8 @@ int (*p_attn_window)(int, const void*, const uint8_t*, const uint8_t*, const voi
 size_t (*p_plain_ws)(int, int, int, int) = nullptr;
 int (*p_plain_attn)(const void*, const void*, const void*, const int32_t*, const int32_t*, void*, void*, size_t, int, int, int, int, int,
                     int64_t, int, float, int, void*) = nullptr;
+int (*p_plain_checked)(const void*, const void*, const void*, const int32_t*, const int32_t*, void*, void*, size_t, int, int, int, int, int,
+                       int64_t, int, float, int, int32_t*, void*) = nullptr;
 int (*p_quant_pair)(int, const void*, const void*, uint8_t*, uint8_t*, void*, void*, int64_t, int, int, int, void*) = nullptr;
 int (*p_dequant_pair)(int, const uint8_t*, const uint8_t*, const void*, const void*, void*, void*, int64_t, int, int, void*) = nullptr;
 
@@ -246,8 +248,10 @@ PyObject* paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 }
 
 // plain_attention(q, K, V, block_table, lengths, scale or None) -> out or None: fp16 / bf16 pages.  The lengths are
-// range-checked on the host, as the operator promises; they are copied out ahead of the kernels on the same stream, the
-// kernels are enqueued (they clamp what they read), and only then the host waits for that copy - the GPU goes on meanwhile.
+// range-checked on the host, as the operator promises.  The split-KV kernel reports on them at its start, into pinned memory that
+// the host polls while the GPU goes on (a copy on the stream took 10 of 42 us per call at 16 sequences: it kept the kernel from
+// starting under the one before).  Elsewhere they are copied out ahead of the kernels, which clamp what they read,
+// and the host waits for that copy once the kernels are enqueued.
 PyObject* plain_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (p_plain_attn == nullptr || n_args != 6 || safe_mode()) return none();
     const Tensor *q = as_tensor(a[0]), *k = as_tensor(a[1]), *v = as_tensor(a[2]), *bt = as_tensor(a[3]), *len = as_tensor(a[4]);
@@ -272,15 +276,35 @@ PyObject* plain_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     cudaStream_t st = (cudaStream_t)stream_of(dev);
     cudaStreamCaptureStatus capture;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return none();
+    Tensor out = empty(q->sizes(), q->scalar_type(), dev);
+    const size_t ws_bytes = p_plain_ws((int)B, (int)Hq, (int)Hkv, (int)mb);
+    Tensor ws = empty({(int64_t)std::max<size_t>(ws_bytes, 16)}, at::kByte, dev);
+    if (D == 128 && P == 16) {
+        Tensor word = at::detail::empty_cpu({1}, at::kInt, std::nullopt, std::nullopt, /*pin_memory=*/true, std::nullopt);
+        volatile int32_t* verdict = static_cast<volatile int32_t*>(word.mutable_data_ptr());
+        *verdict = 0;
+        const int rc = p_plain_checked(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), static_cast<const int32_t*>(bt->const_data_ptr()),
+                                       static_cast<const int32_t*>(len->const_data_ptr()), out.mutable_data_ptr(), ws.mutable_data_ptr(), ws_bytes,
+                                       (int)B, (int)Hq, (int)Hkv, (int)D, (int)P, pages, (int)mb, (float)scale, dtype_code(q->scalar_type()),
+                                       const_cast<int32_t*>(verdict), st);
+        if (rc == 0) {
+            Py_BEGIN_ALLOW_THREADS
+            // the stream is asked now and then, so that a kernel that never ran (an earlier error) ends the wait
+            for (uint32_t i = 1; *verdict == 0; ++i) {
+                if (i % 4096 == 0 && cudaStreamQuery(st) != cudaErrorNotReady) break;
+                __builtin_ia32_pause();
+            }
+            Py_END_ALLOW_THREADS
+            if (*verdict == 0) cudaStreamSynchronize(st);          // everything has ended: no write to the word is left
+            return *verdict == 1 ? THPVariable_Wrap(std::move(out)) : none();      // 2: the Python body raises
+        }
+    }
     static thread_local cudaEvent_t copied[kMaxDevices] = {};      // one per thread and device that ever calls this
     if (copied[dev] == nullptr && cudaEventCreateWithFlags(&copied[dev], cudaEventDisableTiming) != cudaSuccess) return none();
     Tensor host = at::detail::empty_cpu({B}, at::kInt, std::nullopt, std::nullopt, /*pin_memory=*/true, std::nullopt);
     if (cudaMemcpyAsync(host.mutable_data_ptr(), len->const_data_ptr(), (size_t)B * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaEventRecord(copied[dev], st) != cudaSuccess)
         return none();
-    Tensor out = empty(q->sizes(), q->scalar_type(), dev);
-    const size_t ws_bytes = p_plain_ws((int)B, (int)Hq, (int)Hkv, (int)mb);
-    Tensor ws = empty({(int64_t)std::max<size_t>(ws_bytes, 16)}, at::kByte, dev);
     const int rc = p_plain_attn(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), static_cast<const int32_t*>(bt->const_data_ptr()),
                                 static_cast<const int32_t*>(len->const_data_ptr()), out.mutable_data_ptr(), ws.mutable_data_ptr(), ws_bytes,
                                 (int)B, (int)Hq, (int)Hkv, (int)D, (int)P, pages, (int)mb, (float)scale, dtype_code(q->scalar_type()), st);
@@ -359,6 +383,7 @@ PyObject* bind(PyObject*, PyObject* table) {
         {"b200q_paged_gqa_workspace_bytes", (void**)&p_attn_ws}, {"b200q_attention_stage_launches", (void**)&p_attn_launches},
         {"b200q_paged_gqa_decode", (void**)&p_attn}, {"b200q_paged_gqa_decode_window", (void**)&p_attn_window},
         {"b200q_paged_fp16_gqa_workspace_bytes", (void**)&p_plain_ws}, {"b200q_paged_fp16_gqa_decode", (void**)&p_plain_attn},
+        {"b200q_paged_fp16_gqa_decode_checked", (void**)&p_plain_checked},
         {"b200q_quantize_kv_pair", (void**)&p_quant_pair}, {"b200q_dequantize_kv_pair", (void**)&p_dequant_pair},
     };
     for (const auto& w : want) {

@@ -63,6 +63,7 @@ struct AttnParams {
     int grid;
     int sink, window;           // window > 0: only positions < sink or >= length - window are attended
     TpOut tp_out;               // tensor-parallel exchange of the merged rows (world == 0: off)
+    int32_t* verdict;           // host-visible word: 1 or 2 once the lengths are read, all in range or not (null: off)
 };
 
 __device__ __forceinline__ int clamp_len(int len, int cap) { return max(0, min(len, cap)); }
@@ -211,6 +212,15 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
         total = __shfl_sync(0xffffffffu, incl, 31);
     } else {
         total = build_prefix(p, prefix);
+    }
+    if (p.verdict != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && warp == kAttnWarps) {
+        bool good = true;
+        for (int b = lane; b < p.B; b += 32) {
+            const int len = small ? len_l : p.lengths[b];
+            good = good && len >= 0 && len <= cap;
+        }
+        good = __all_sync(0xffffffffu, good);
+        if (lane == 0) *reinterpret_cast<volatile int32_t*>(p.verdict) = good ? 1 : 2;
     }
     const int ppc = (total + p.grid - 1) / p.grid;               // pages per range
     const int h0 = blockIdx.y * hc;                              // first kv head of the CTA
@@ -1118,10 +1128,10 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     return rc == B200Q_ERR_UNSUPPORTED && tp_out_slot < 0 ? simple() : rc;      // scales of very many kv heads do not fit a ring
 }
 
-// Plain fp16 / bf16 pages on the split-KV kernels; B200Q_ERR_UNSUPPORTED outside their shapes.
+// Plain fp16 / bf16 pages on the split-KV kernels; B200Q_ERR_UNSUPPORTED outside their shapes.  `verdict`: see AttnParams.
 int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table, const int32_t* lengths,
                                void* out, void* workspace, size_t workspace_bytes, int B, int Hq, int Hkv, int D, int page_size,
-                               int64_t num_pages, int max_blocks, float scale, int dtype, cudaStream_t stream) {
+                               int64_t num_pages, int max_blocks, float scale, int dtype, int32_t* verdict, cudaStream_t stream) {
     if (tuning_get("attn.force_simple") || D != kHeadDim || page_size != 16 || Hq / Hkv > 8 || !heads_ok(Hkv) || B > kMaxBatchFast ||
         ((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) % 16 != 0)
         return B200Q_ERR_UNSUPPORTED;
@@ -1132,6 +1142,7 @@ int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v
     p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.P = page_size; p.max_blocks = max_blocks;
     p.group = Hq / Hkv; p.num_pages = num_pages; p.scale = scale; p.q_dtype = dtype; p.bits = 16;
     p.row_bytes = Hkv * kHeadDim * 2;
+    p.verdict = verdict;
     return launch_split_attention(p, stream);
 }
 

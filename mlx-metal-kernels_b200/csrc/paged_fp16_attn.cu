@@ -214,13 +214,26 @@ int splits_for(int B, int Hkv, int max_blocks) {
 size_t paged_gqa_workspace_bytes_impl(int B, int Hq, int Hkv, int D);
 int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table, const int32_t* lengths,
                                void* out, void* workspace, size_t workspace_bytes, int B, int Hq, int Hkv, int D, int page_size,
-                               int64_t num_pages, int max_blocks, float scale, int dtype, cudaStream_t stream);
+                               int64_t num_pages, int max_blocks, float scale, int dtype, int32_t* verdict, cudaStream_t stream);
 
 size_t paged_fp16_workspace_bytes_impl(int B, int Hq, int Hkv, int max_blocks) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || max_blocks <= 0) return 0;
     if (max_blocks == 1) return 0;      // one page per sequence: the general kernel in one CTA per kv head
     const int s = splits_for(B, Hkv, max_blocks);
     return std::max((size_t)s * B * Hq * kPartStride * sizeof(float), paged_gqa_workspace_bytes_impl(B, Hq, Hkv, 128));
+}
+
+// The split-KV kernels only: B200Q_ERR_UNSUPPORTED or B200Q_ERR_WORKSPACE, with nothing launched, where they do not apply.
+int paged_fp16_gqa_decode_checked_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table,
+                                       const int32_t* lengths, void* out, void* workspace, size_t workspace_bytes, int B, int Hq,
+                                       int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
+                                       int32_t* verdict, cudaStream_t stream) {
+    if (q == nullptr || k_pages == nullptr || v_pages == nullptr || block_table == nullptr || lengths == nullptr || out == nullptr ||
+        verdict == nullptr || B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || D <= 0 || page_size <= 0 || num_pages <= 0 || max_blocks <= 0)
+        return B200Q_ERR_BAD_ARG;
+    if (dtype != B200Q_F16 && dtype != B200Q_BF16) return B200Q_ERR_UNSUPPORTED;
+    return paged_plain_attention_impl(q, k_pages, v_pages, block_table, lengths, out, workspace, workspace_bytes, B, Hq, Hkv, D, page_size,
+                                      num_pages, max_blocks, scale, dtype, verdict, stream);
 }
 
 int paged_fp16_gqa_decode_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table,
@@ -235,7 +248,7 @@ int paged_fp16_gqa_decode_impl(const void* q, const void* k_pages, const void* v
     if (D > 128 || (dtype != B200Q_F16 && dtype != B200Q_BF16) || Hkv > 65535 || B > 65535) return B200Q_ERR_UNSUPPORTED;
     // a workspace too small for the split-KV kernels (a caller that knows this kernel's own need) stays here
     const int rc0 = paged_plain_attention_impl(q, k_pages, v_pages, block_table, lengths, out, workspace, workspace_bytes, B, Hq, Hkv, D,
-                                               page_size, num_pages, max_blocks, scale, dtype, stream);
+                                               page_size, num_pages, max_blocks, scale, dtype, nullptr, stream);
     if (rc0 != B200Q_ERR_UNSUPPORTED && rc0 != B200Q_ERR_WORKSPACE) return rc0;
     Fp16AttnParams p = {};
     p.q = q; p.k_pages = k_pages; p.v_pages = v_pages; p.block_table = block_table; p.lengths = lengths; p.out = out;
