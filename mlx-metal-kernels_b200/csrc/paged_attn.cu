@@ -148,6 +148,7 @@ struct alignas(64) SplitParams {
     CUtensorMap ksmap, vsmap;   // scales as bytes [tokens][row], box 16 x (hc heads); used with more than 8 kv heads only
     AttnParams a;
 };
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
@@ -180,6 +181,10 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
     int* prefix = reinterpret_cast<int*>(smem + p.off_prefix);              // [B + 1]
     const uint32_t ring = smem_u32(smem);                                   // [subs][NS] slots
 
+    if (threadIdx.x == kAttnThreads) {
+        prefetch_map(&sp.kmap);
+        prefetch_map(&sp.vmap);
+    }
     if (threadIdx.x < subs * NS) {
         mbar_init(&full[threadIdx.x], 1);
         mbar_init(&empty[threadIdx.x], hc);
@@ -433,6 +438,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     const float* wpart = reinterpret_cast<const float*>(smem);
     float* cpart = reinterpret_cast<float*>(smem + p.off_cpart);         // [S][group][PW] (used in the first CTA)
 
+    if (threadIdx.x == 0) {
+        prefetch_map(&cp.kmap);
+        prefetch_map(&cp.vmap);
+    }
     if (lane < NS) mbar_init(&full[lane], 1);
     mbar_fence_init();
     __syncwarp();
@@ -673,6 +682,7 @@ template <int kMergeWarps>
 __global__ void __launch_bounds__(kMergeWarps * 32) paged_attn_merge_kernel(const __grid_constant__ AttnParams p) {
     __shared__ float red[kMergeWarps][128];
     __shared__ float red_s[2][kMergeWarps];
+    pdl_launch_dependents();      // what follows waits for this kernel's end; until then it may set itself up or fetch its weights
     const int D = p.D;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
