@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
 
     // Lengths and block table may still change until the wait below, so what is read here is a hint (past L1, which must not keep it):
     // it brings the table's lines and the first pages of the CTA's ranges into L2 while the kernel before ends (16 ragged sequences
-    // of bf16 pages: 35.6 -> 33.7 us; the decode stack's q8 attention 1 us).  Not for q4, whose ranges are short in bytes: 30.2 -> 30.6.
+    // of bf16 pages: 35.6 -> 33.7 us; the decode stack's q8 attention 1 us).  Not for q4: no gain (16 x 4096 tokens: 27.6 against 28.0 us).
     if (BITS != 4 && small && warp == kAttnWarps) {
         scan(lane < p.B ? __ldcg(p.lengths + lane) : 0);
         for (int sub = 0; sub < subs; ++sub) {
