@@ -513,7 +513,7 @@ def run_own(args):
                    "cuda_graph": True},
         "step_hbm": {"algorithmic_bytes_per_gpu": step_bytes, "achieved_gbs_per_gpu": round(step_bytes / sec_per_step / 1e9, 1),
                      "frac_of_peak": round(step_bytes / sec_per_step / 1e9 / peak, 4)},
-        "roofline": {"bound": "hbm", "kernel": "qgemv_kernel (all q4 matvec launches of one step, timed alone)",
+        "roofline": {"bound": "hbm", "kernel": "qgemv_i8_kernel (all q4 matvec launches of one step, timed alone)",
                      "achieved": round(gemv_gbs, 1), "peak": peak, "unit": "GB/s", "frac": round(gemv_gbs / peak, 4),
                      "traffic": round(gemv_traffic / n_gemv), "traffic_source": "per-shape ncu captures (profiles/qgemv_kernel_c5_stack_shapes_b1.md): dram bytes read+written / algorithmic bytes 1.002-1.008 for the QKV, O, gate/up and down shapes, applied to this launch mix",
                      "peak_kind": peak_kind, "launches": n_gemv,
