@@ -70,7 +70,7 @@ def _build_host(verbose: bool, force: bool) -> None:
 
 def build(verbose: bool = False, force: bool = False) -> Path:
     sources = sorted(CSRC.glob("*.cu"))
-    headers = sorted(CSRC.glob("*.cuh")) + [HEADER]
+    headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [HEADER]
     OBJ.mkdir(exist_ok=True)
     LIB.parent.mkdir(exist_ok=True)
     nvcc = _nvcc()

@@ -35,6 +35,7 @@
 // carries on without the data so that it always terminates and frees its tensor memory.
 #include "gemv_params.cuh"
 
+#include "ring.h"
 #include "tensor_map.cuh"
 
 #include <algorithm>
@@ -431,18 +432,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         const uint32_t atom16 = (p.x_bytes >> 1) >> 4;                 // distance of the two 64-k atoms of a chunk, in 16-byte units
         const int n_ch = n_st * SC;
         const int per = MATS == 2 && ncols <= 64 && XS >= 4 && NA >= 5 ? 2 : 1;      // chunks per round
-        const int first = MATS == 2 ? 0 : j;
-        const int skip = MATS == 2 ? 0 : 1;                            // chunks of the other warp between two rounds
-        int xslot = 0, a_slot = 0, x_at = 0;                           // ring positions and the chunk they stand for
-        uint32_t xpar = 0, a_par = 0;
-        if (MATS == 2) a_slot = j;                                     // (NA >= 2)
-        auto go = [&](int d) {                                         // d chunks of k on
-            xslot += d;
-            while (xslot >= XS) { xslot -= XS; xpar ^= 1u; }
-            a_slot += MATS * d;
-            while (a_slot >= NA) { a_slot -= NA; a_par ^= 1u; }
-            x_at += d;
-        };
+        const int first = ChunkWalk<MATS>::first(j);
+        ChunkWalk<MATS> at(j);                                         // (NA >= 2)
         auto chunk = [&](int xs, int as, bool start) {
             const uint64_t desc0 = desc_hi | (uint64_t)(((x0 + (uint32_t)xs * p.x_bytes) & 0x3FFFFu) >> 4);
             const uint32_t a_t = a_base + (uint32_t)as * kChunkCols;
@@ -456,21 +447,19 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         for (int it = 0; it < my_items; ++it) {
             if (it > 0) wait_bar(d_free, (uint32_t)(it - 1) & 1u, EV_GEMV_EMPTY_WAIT, ok);
             tc_fence_after();
-            go(it * n_ch + first - x_at);
 #pragma unroll 1
             for (int ch = first; ch < n_ch;) {
-                const int xs0 = xslot, as0 = a_slot;
-                const uint32_t xp0 = xpar, ap0 = a_par;
+                at.to(it * n_ch + ch, XS, NA);
+                const RingPos x = at.x, a = at.a;
                 const bool two = per == 2 && ch + 1 < n_ch;
-                if (two) go(1);
+                if (two) at.to(it * n_ch + ch + 1, XS, NA);
                 // lanes 0, 1: the first chunk's operands; lanes 2, 3: the second's
-                const uint32_t bar = lane == 0 ? smem_u32(&full_x[xs0]) : lane == 1 ? smem_u32(&a_full[as0]) : lane == 2 ? smem_u32(&full_x[xslot]) : smem_u32(&a_full[a_slot]);
-                wait_bars(bar, lane == 0 ? xp0 : lane == 1 ? ap0 : lane == 2 ? xpar : a_par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
+                const uint32_t bar = lane == 0 ? smem_u32(&full_x[x.slot]) : lane == 1 ? smem_u32(&a_full[a.slot]) : lane == 2 ? smem_u32(&full_x[at.x.slot]) : smem_u32(&a_full[at.a.slot]);
+                wait_bars(bar, lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
                 tc_fence_after();
-                chunk(xs0, as0, ch == first);
-                if (two) chunk(xslot, a_slot, false);
-                ch += (two ? 2 : 1) + skip;
-                go(1 + skip);
+                chunk(x.slot, a.slot, ch == first);
+                if (two) chunk(at.x.slot, at.a.slot, false);
+                ch += (two ? 2 : 1) + ChunkWalk<MATS>::kSkip;
             }
             tc_commit(d_full);
         }
@@ -853,10 +842,12 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     // tensor memory: accumulators below, ring of A chunks above
     const int dcols = 2 * cols;
     p.a_col0 = std::max(32, (dcols + 31) / 32 * 32);
-    // A barrier is waited for by its parity, so whoever waits on a slot has to have seen the slot's phase before.  Ring depths see to
-    // that: an even number of A slots (and, one matrix, of activation slots) gives every slot to the same MMA warp each time round, and
-    // a stage slot serves the same groups of warps each time (chunk n goes to group n modulo kGroups).  Four A slots or more cover
-    // the groups' waits for a free one: the chunk a group wrote before lies at most one round of the ring back.
+    // A barrier is waited for by its parity, so whoever waits on a slot has to know that the slot's phase before has ended.  Ring depths
+    // see to that: an even number of A slots (and, one matrix, of activation slots) gives every slot to the same MMA warp each time
+    // round within an item, and a stage slot serves the same groups of warps each time (chunk n goes to group n modulo kGroups).
+    // From one item to the next the MMA warps of one matrix change places when an item has an odd number of chunks; their wait for d_free
+    // in between covers it, since the accumulators are read only after every chunk of the item has been consumed.  Four A slots or
+    // more cover the groups' waits for a free one: the chunk a group wrote before lies at most one round of the ring back.
     p.a_slots = std::min(kMaxASlots, (512 - p.a_col0) / kChunkCols) & ~1;
     constexpr int kXStep = MATS == 2 ? 1 : 2;
     constexpr int kStageStep = std::max(1, kGroups / (SC * MATS));

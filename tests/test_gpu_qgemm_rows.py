@@ -43,3 +43,18 @@ def test_results_repeat(cuda, bits, B, N, K, G):
         assert torch.equal(quant_ops.matvec_rows(bits, x, *g, G), plain)
         assert all(torch.equal(a, b) for a, b in zip(pair(x, g[0], u[0], g[1], u[1], g[2], u[2], group_size=G), both))
     assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("B,N,K", [(5, 20480, 640), (6, 20000, 896), (40, 19300, 2944), (1024, 4096, 5504)])
+def test_odd_chunk_counts_over_several_items(cuda, B, N, K):
+    """q8 matrices with an odd number of 128-k chunks and more work items than SMs: the two MMA warps change places from one
+    item to the next."""
+    w, s, z = synth.quantized_weight(N, K, 8, 64, seed=K)
+    x = synth.activations((B, K), 8)
+    want = _ref(8)(x, w, s, z, group_size=64)
+    args = to_dev(cuda, x, w, s, z)
+    got = quant_ops.matvec_rows(8, *args, 64)
+    assert rel_l2(got, want) <= 1e-3
+    for _ in range(5):
+        assert torch.equal(quant_ops.matvec_rows(8, *args, 64), got)
+    assert cabi.device_status() == 0
