@@ -59,6 +59,7 @@ struct AttnParams {
     int hc;                     // kv heads per CTA: Hkv, at most 8
     int row_bytes;              // bytes of one token row of codes, all kv heads
     int scale_row_halves;       // halves of one token row of scales, all kv heads
+    int scales8;                // the scales are aligned to 8 bytes only: no bulk copies of them
     uint32_t off_bars, off_desc, off_prefix, slot_bytes;      // the ring comes first
     int grid;
     int sink, window;           // window > 0: only positions < sink or >= length - window are attended
@@ -169,6 +170,21 @@ __host__ __device__ constexpr uint32_t split_slot_bytes(int bits, int hc, int Gd
     return (tiles + sc + 1023u) & ~1023u;
 }
 
+// Scales that are aligned to 8 bytes only (a view that starts inside a tensor): copied by a whole warp in 8-byte pieces, `rows` rows of
+// `row8` pieces that lie `pitch` bytes apart, into the same place and order as the bulk copies.  Every lane then arrives on the
+// slot's barrier (whose count includes the 32 lanes) when its pieces are there.  16 x 4096 tokens of q4, 8 kv heads: 40 us against
+// 38 us aligned, one cold call by events; the kernel for every shape, one warp per head, took 7675 us.
+__device__ __forceinline__ void copy_scales8(uint32_t dst, const void* src, int rows, int row8, int64_t pitch, int lane) {
+    for (int i = lane; i < rows * row8; i += 32) {
+        const int r = i / row8;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + (uint32_t)i * 8),
+                     "l"(static_cast<const uint8_t*>(src) + r * pitch + (i - r * row8) * 8) : "memory");
+    }
+}
+__device__ __forceinline__ void arrive_on_copies(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 template <int BITS, int LOGG, bool TWO, bool WIDE>
 __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) paged_attn_kernel(const __grid_constant__ SplitParams sp) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -190,7 +206,7 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
         prefetch_map(&sp.vmap);
     }
     if (threadIdx.x < subs * NS) {
-        mbar_init(&full[threadIdx.x], 1);
+        mbar_init(&full[threadIdx.x], BITS != 16 && p.scales8 ? 33 : 1);
         mbar_init(&empty[threadIdx.x], hc);
     }
     mbar_fence_init();
@@ -286,7 +302,8 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
     // ================================ producer ================================
     if (warp == kAttnWarps) {
         const uint32_t sc_bytes = BITS == 16 ? 0u : split_scale_bytes(hc, p.Gd);
-        const uint32_t tx = (uint32_t)(2 * hc * TILE) + 2 * sc_bytes;
+        const bool scales8 = BITS != 16 && p.scales8;
+        const uint32_t tx = (uint32_t)(2 * hc * TILE) + (scales8 ? 0u : 2 * sc_bytes);
         bool ok = true;
         int slot = 0;
         uint32_t par = 1u;                                       // a fresh barrier's previous phase counts as done
@@ -310,8 +327,19 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
                 const int bar = sub * NS + slot;
                 ok = mbar_wait_bounded(&empty[bar], par, &g_device_status, EV_ATTN_EMPTY_WAIT, ok ? limit : 64u) && ok;
                 __syncwarp();
+                const int page = (int)dsub[j & (kDescSlots - 1)].x;
+                if (scales8) {
+                    if (page >= 0) {
+                        const uint32_t sdst = ring + (uint32_t)bar * p.slot_bytes + 2 * hc * TILE;
+                        const bool whole = p.Hkv == hc;          // the page's scales are contiguous
+                        const int rows = whole ? 1 : 16, row8 = (int)(sc_bytes / 8) / rows;
+                        const size_t at = (size_t)page * 16 * p.scale_row_halves + (whole ? 0 : h0 * p.Gd);
+                        copy_scales8(sdst, p.k_scales + at, rows, row8, (int64_t)p.scale_row_halves * 2, lane);
+                        copy_scales8(sdst + sc_bytes, p.v_scales + at, rows, row8, (int64_t)p.scale_row_halves * 2, lane);
+                    }
+                    arrive_on_copies(&full[bar]);
+                }
                 if (lane == 0) {
-                    const int page = (int)dsub[j & (kDescSlots - 1)].x;
                     if (page < 0) {
                         mbar_arrive(&full[bar]);                 // a missing page: nothing to copy, the consumers skip it
                     } else {
@@ -319,7 +347,7 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
                         mbar_arrive_expect_tx(&full[bar], tx);
                         tma_load_3d(dst, &sp.kmap, 0, page * 16, BITS == 16 ? 2 * h0 : h0, &full[bar]);
                         tma_load_3d(dst + hc * TILE, &sp.vmap, 0, page * 16, BITS == 16 ? 2 * h0 : h0, &full[bar]);
-                        if (BITS != 16) {
+                        if (BITS != 16 && !scales8) {
                             const uint32_t sdst = dst + 2 * hc * TILE;
                             if (p.Hkv == hc) {                   // the page's scales are contiguous
                                 const size_t at = (size_t)page * 16 * p.scale_row_halves;
@@ -335,6 +363,7 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
             }
             if (++slot == NS) { slot = 0; par ^= 1u; }
         }
+        if (scales8) asm volatile("cp.async.wait_all;" ::: "memory");
         return;
     }
 
@@ -443,7 +472,8 @@ __device__ __forceinline__ uint32_t cluster_rank_x() {
 // rotated (16-byte cp.async pieces kept the CTA's memory path busy for 9100 of the kernel's 20000 clocks at one sequence of 4096 q8
 // tokens); the scales come whole, all heads of the page, which costs less than sixteen pieces of 8 bytes.  Only the page that the new
 // token goes to waits for its append.
-template <int BITS, int LOGG, bool WIDE>
+// SC8: scales aligned to 8 bytes only (a template parameter: asked at run time it cost the aligned form 0.3 of 9.9 us).
+template <int BITS, int LOGG, bool WIDE, bool SC8>
 __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterParams cp) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const ClusterAttnParams& p = cp.a;
@@ -470,7 +500,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
         prefetch_map(&cp.kmap);
         prefetch_map(&cp.vmap);
     }
-    if (lane < NS) mbar_init(&full[lane], 1);
+    if (lane < NS) mbar_init(&full[lane], SC8 ? 33 : 1);
     mbar_fence_init();
     __syncwarp();
     pdl_launch_dependents();
@@ -494,16 +524,28 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     auto issue = [&](int j) {                                            // copies of page j into its slot
         if (j > 0 && (j & 31) == 0) ids_i = page_ids(j);
         const int page = __shfl_sync(0xffffffffu, ids_i, j & 31);
+        if constexpr (SC8) {
+            if (page >= 0) {
+                const uint32_t sdst = smem_u32(my_ring + (size_t)(j % NS) * p.slot_bytes + 2 * TILE);
+                const bool whole = p.Hkv == p.hs;
+                const int rows = whole ? 1 : 16, row8 = (int)(sc_bytes / 8) / rows;
+                const size_t at = (size_t)page * 16 * p.scale_row_halves + (whole ? 0 : (h & ~7) * p.Gd);
+                copy_scales8(sdst, p.k_scales + at, rows, row8, (int64_t)p.scale_row_halves * 2, lane);
+                copy_scales8(sdst + sc_bytes, p.v_scales + at, rows, row8, (int64_t)p.scale_row_halves * 2, lane);
+            }
+            arrive_on_copies(&full[j % NS]);
+        }
         if (lane == 0) {
             uint64_t* bar = &full[j % NS];
             if (page < 0) {
                 mbar_arrive(bar);                                        // a missing page: nothing to copy, skipped where it is used
             } else {
                 uint8_t* dst = my_ring + (size_t)(j % NS) * p.slot_bytes;
-                mbar_arrive_expect_tx(bar, 2 * TILE + 2 * sc_bytes);
+                mbar_arrive_expect_tx(bar, 2 * TILE + (SC8 ? 0u : 2 * sc_bytes));
                 tma_load_3d(smem_u32(dst), &cp.kmap, 0, page * 16, h, bar);
                 tma_load_3d(smem_u32(dst + TILE), &cp.vmap, 0, page * 16, h, bar);
-                if (p.Hkv == p.hs) {
+                if (SC8) {
+                } else if (p.Hkv == p.hs) {
                     const size_t at = (size_t)page * 16 * p.scale_row_halves;
                     bulk_g2s(dst + 2 * TILE, p.k_scales + at, sc_bytes, bar);
                     bulk_g2s(dst + 2 * TILE + sc_bytes, p.v_scales + at, sc_bytes, bar);
@@ -935,14 +977,14 @@ bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtens
 }
 
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
-    const bool g32 = p.G == 32, wide = p.group > 4;
+    const bool g32 = p.G == 32, wide = p.group > 4, sc8 = ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     p.hs = std::min(p.Hkv, kAttnWarps);
     p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024);
     // shared memory: [1 KB alignment] rings, barriers, query rows, the CTAs' partials
     const uint32_t q_bytes = align_up_u32((uint32_t)p.group * 128 * 2, 128), c_bytes = align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
     const uint32_t cap = (uint32_t)max_smem_optin(), fixed = 1024 + 128 * 8 + q_bytes + c_bytes;
     p.stages = (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (kAttnWarps * p.slot_bytes));
-    if (p.stages < 2 || ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0) return B200Q_ERR_UNSUPPORTED;
+    if (p.stages < 2) return B200Q_ERR_UNSUPPORTED;
     p.off_bars = kAttnWarps * p.stages * p.slot_bytes;
     p.off_q = p.off_bars + 128 * 8;
     p.off_cpart = p.off_q + q_bytes;
@@ -953,23 +995,26 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     if (!page_map(p.k_codes, row, p.num_pages * 16, p.Hkv, p.row_bytes, 1, &cp.kmap) ||
         !page_map(p.v_codes, row, p.num_pages * 16, p.Hkv, p.row_bytes, 1, &cp.vmap))
         return B200Q_ERR_LAUNCH;
-    if (p.Hkv > p.hs && (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.ksmap) ||
+    if (p.Hkv > p.hs && !sc8 && (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.ksmap) ||
                          !scale_map(p.v_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.vsmap)))
         return B200Q_ERR_LAUNCH;
     using KernelFn = void (*)(ClusterParams);
-    static const KernelFn kernels[2][2][2] = {{{paged_attn_cluster_kernel<8, 6, false>, paged_attn_cluster_kernel<8, 6, true>},
-                                               {paged_attn_cluster_kernel<8, 5, false>, paged_attn_cluster_kernel<8, 5, true>}},
-                                              {{paged_attn_cluster_kernel<4, 6, false>, paged_attn_cluster_kernel<4, 6, true>},
-                                               {paged_attn_cluster_kernel<4, 5, false>, paged_attn_cluster_kernel<4, 5, true>}}};
-    KernelFn kernel = kernels[p.bits == 4][g32][wide];
-    static bool configured[2][2][2][64] = {};
+#define B200Q_CLUSTER_PAIR(BITS, LOGG, WIDE) {paged_attn_cluster_kernel<BITS, LOGG, WIDE, false>, paged_attn_cluster_kernel<BITS, LOGG, WIDE, true>}
+    static const KernelFn kernels[2][2][2][2] = {{{B200Q_CLUSTER_PAIR(8, 6, false), B200Q_CLUSTER_PAIR(8, 6, true)},      // [q4][group 32][wide][sc8]
+                                                  {B200Q_CLUSTER_PAIR(8, 5, false), B200Q_CLUSTER_PAIR(8, 5, true)}},
+                                                 {{B200Q_CLUSTER_PAIR(4, 6, false), B200Q_CLUSTER_PAIR(4, 6, true)},
+                                                  {B200Q_CLUSTER_PAIR(4, 5, false), B200Q_CLUSTER_PAIR(4, 5, true)}}};
+#undef B200Q_CLUSTER_PAIR
+    KernelFn kernel = kernels[p.bits == 4][g32][wide][sc8];
+    static bool configured[16][64] = {};
+    const int slot = (p.bits == 4) * 8 + g32 * 4 + wide * 2 + sc8;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!configured[p.bits == 4][g32][wide][dev & 63]) {
+    if (!configured[slot][dev & 63]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess ||
             cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
             return B200Q_ERR_LAUNCH;
-        configured[p.bits == 4][g32][wide][dev & 63] = true;
+        configured[slot][dev & 63] = true;
     }
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -1000,6 +1045,7 @@ int launch_split_attention(AttnParams& p, cudaStream_t stream) {
     p.subs = subs_for(p.hc);
     const int chunks = p.Hkv / p.hc;
     p.slot_bytes = split_slot_bytes(bits, p.hc, p.Gd);
+    p.scales8 = bits != 16 && ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     int ctas_per_sm = tuning_get("attn.ctas_per_sm");
     if (ctas_per_sm <= 0) ctas_per_sm = bits == 16 ? 1 : B200Q_ATTN_CTAS;
     // At least three pages per range (by the block table's capacity; the lengths live on the device): short
@@ -1031,7 +1077,7 @@ int launch_split_attention(AttnParams& p, cudaStream_t stream) {
     if (!page_map(p.k_codes, row, p.num_pages * 16, p.Hkv * tiles, p.row_bytes, p.hc * tiles, &sp.kmap) ||
         !page_map(p.v_codes, row, p.num_pages * 16, p.Hkv * tiles, p.row_bytes, p.hc * tiles, &sp.vmap))
         return B200Q_ERR_LAUNCH;
-    if (bits != 16 && chunks > 1 &&
+    if (bits != 16 && chunks > 1 && !p.scales8 &&
         (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hc * p.Gd * 2, &sp.ksmap) ||
          !scale_map(p.v_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hc * p.Gd * 2, &sp.vsmap)))
         return B200Q_ERR_LAUNCH;
@@ -1147,8 +1193,6 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
         const int rc = launch_cluster_attention(c, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
     }
-    // the split kernel copies scales in 16-byte pieces
-    if (((uintptr_t)k_scales | (uintptr_t)v_scales) % 16 != 0) return tp_out_slot >= 0 ? (int)B200Q_ERR_UNSUPPORTED : simple();
     if (!have_workspace) return B200Q_ERR_WORKSPACE;
 
     AttnParams p = {};

@@ -92,3 +92,33 @@ def test_plain_pages(cuda, dtype, Hq, Hkv, lengths):
     bad[0] = 10 ** 6
     with pytest.raises(ValueError, match="positions must be in"):
         gqa_ops.paged_gqa_decode_attention(*args[:4], bad)
+
+
+@pytest.mark.parametrize("bits,G", [(4, 32), (8, 64)])
+@pytest.mark.parametrize("Hq,Hkv,lengths", [(8, 1, [1, 300, 17]), (6, 3, [129, 5]), (32, 8, [700, 0, 40]), (32, 16, [40, 0, 250])])
+@pytest.mark.parametrize("shifted", ["k_scales", "v_scales", "both"])
+def test_scales_aligned_to_eight_bytes(cuda, bits, G, Hq, Hkv, lengths, shifted):
+    """Views of scales that start 8 bytes into a 16-byte piece give the same bits as aligned ones, in both kernels, with a page missing."""
+    pages = sum((n + 15) // 16 for n in lengths) + 3
+    table, ln = _table(lengths, pages, 1).to(cuda), torch.tensor(lengths, dtype=torch.int32, device=cuda)
+    if table.shape[1] > 1:
+        table[0, 1] = -1
+    k, v = (synth.activations((pages, 16, Hkv, 128), s, cuda) for s in (31, 32))
+    q = synth.activations((len(lengths), 1, Hq, 128), 33, cuda)
+    cache = pq_ops.quantize_kv_pages(k, v, table, ln, pq_ops.PagedQuantizedKVConfig(bits=bits, group_size=G))
+    aligned = {name: getattr(cache, name) for name in ("k_scales", "v_scales")}
+    for cluster in (-1, 1):
+        cabi.set_tuning("attn.cluster", cluster)
+        try:
+            for name in aligned:
+                setattr(cache, name, aligned[name])
+            want = pq_ops.paged_quantized_kv_gqa_decode_attention(q, cache, backend="cuda")
+            for name in aligned:
+                if shifted in (name, "both"):
+                    setattr(cache, name, torch.cat([aligned[name].new_zeros(4), aligned[name].flatten()])[4:].view(aligned[name].shape))
+                    assert getattr(cache, name).data_ptr() % 16 == 8
+            got = pq_ops.paged_quantized_kv_gqa_decode_attention(q, cache, backend="cuda")
+        finally:
+            cabi.set_tuning("attn.cluster", 0)
+        assert torch.equal(got, want)
+    assert cabi.device_status() == 0
