@@ -155,7 +155,12 @@ int b200q_block_table_lookup(const int32_t* block_table, const int32_t* position
  *   k/v codes   [num_pages, page_size, Hkv, D] (bits=8) or [.., ceil(D/2)] (bits=4)
  *   k/v scales  [num_pages, page_size, Hkv, ceil(D/group)] in scale_dtype
  *   block_table [B, max_blocks] int32, lengths [B] int32
- *   workspace   b200q_paged_gqa_workspace_bytes(B, Hq, Hkv, D) bytes of scratch (split-KV partials)
+ *   workspace   b200q_paged_gqa_workspace_bytes(B, Hq, Hkv, D) bytes of scratch (split-KV partials).  Less is served
+ *               with fewer partial results down to (304 + B) * Hq * (D + 2) * 4 bytes and refused with
+ *               B200Q_ERR_WORKSPACE below that.  bf16 q or more than 8 kv heads: never refused - without room
+ *               for one partial result per SM and sequence they run the one-warp-per-head kernel.
+ *   The fast kernels (head_dim 128, pages of 16 tokens, groups of 32 or 64, fp16 scales) want q and codes aligned to 16
+ *   bytes and scales to 8; scales aligned to 16 are the fastest.
  */
 size_t b200q_paged_gqa_workspace_bytes(int B, int Hq, int Hkv, int D);
 int b200q_paged_gqa_decode(int bits, const void* q, const uint8_t* k_codes, const uint8_t* v_codes,
@@ -231,18 +236,18 @@ int b200q_paged_fp16_gqa_decode_checked(const void* q, const void* k_pages, cons
  * entry point keeps them in a fixed array of b200q_paged_gqa_static_scratch_bytes() (8 MiB) that is
  * part of the library image: every GPU that loads the library holds those 8 MiB until the process
  * exits.  It allocates nothing and calls no allocating routine.
- *   - Limit: returns B200Q_ERR_STATIC_SCRATCH when
- *     b200q_paged_gqa_workspace_bytes(B, Hq, Hkv, D) exceeds the array (for 32 query heads of
- *     head_dim 128 over 8 kv heads that is a batch of 200 sequences); use the workspace variant then.
+ *   - Limit: returns B200Q_ERR_STATIC_SCRATCH when fp16 q over up to 8 kv heads needs more than the array:
+ *     (304 + B) * Hq * (D + 2) * 4 bytes (for 32 query heads of head_dim 128 that is a batch of 200
+ *     sequences); use the workspace variant then.
  *   - The first call on each device looks up the array's device address (with that device current)
  *     and remembers it.  Make that first call outside any stream capture.
  *   - Every call on a device shares the one array.  Nothing in it has to start at zero: each call
  *     writes every partial result it later reads, so leftovers of the previous call are never seen.
  *     Two calls whose kernels overlap on the GPU (different streams, or graphs replayed
  *     concurrently) would overwrite each other's partials: keep calls on one device stream-ordered.
- *   - Dense attention only (there is no windowed form of this entry point).  Shapes that run the
- *     one-warp-per-head kernel (head_dim != 128, bf16 q, page sizes other than 16 ...) use no scratch and are
- *     never refused for size.
+ *   - Dense attention only (there is no windowed form of this entry point).  bf16 q, more than 8 kv heads and
+ *     shapes that run the one-warp-per-head kernel (head_dim != 128, page sizes other than 16 ...) are never
+ *     refused for size.
  * Arguments and results are those of b200q_paged_gqa_decode without workspace / workspace_bytes. */
 size_t b200q_paged_gqa_static_scratch_bytes(void);
 int b200q_paged_gqa_decode_static(int bits, const void* q, const uint8_t* k_codes, const uint8_t* v_codes,

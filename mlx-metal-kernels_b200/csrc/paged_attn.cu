@@ -1039,7 +1039,8 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     return finish_launch();
 }
 
-int launch_split_attention(AttnParams& p, cudaStream_t stream) {
+// max_ranges: what the workspace has room for.
+int launch_split_attention(AttnParams& p, int max_ranges, cudaStream_t stream) {
     const int bits = p.bits;
     p.hc = std::min(p.Hkv, kAttnWarps);
     p.subs = subs_for(p.hc);
@@ -1058,7 +1059,7 @@ int launch_split_attention(AttnParams& p, cudaStream_t stream) {
     // shards), so that a head's partial results do not depend on the sharding.
     const int full_subs = subs_for(std::min(p.Hkv * std::max(1, tuning_get("ts.tp_world")), kAttnWarps));
     const int want = std::max(1, sm_count() * ctas_per_sm / chunks) * full_subs;
-    p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(std::min({kMaxRanges, kMaxGrid * full_subs, want}), (pages_cap + min_pages - 1) / min_pages));
+    p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(std::min({max_ranges, kMaxRanges, kMaxGrid * full_subs, want}), (pages_cap + min_pages - 1) / min_pages));
     const int launch_grid = (p.grid + p.subs - 1) / p.subs;   // CTAs: each covers `subs` ranges
     const bool two = bits != 16 && launch_grid * chunks > sm_count();
     // shared memory: [1 KB alignment] ring, barriers, descriptors, prefix sums
@@ -1142,6 +1143,19 @@ size_t paged_gqa_workspace_bytes_impl(int B, int Hq, int Hkv, int D) {
     return (size_t)(ranges + B) * Hq * (D + 2) * sizeof(float);
 }
 
+// Calls that the kernel without scratch served before the split-KV kernels took them on: a workspace that is missing or too small
+// sends them back to it and is no error.
+static bool scratch_optional(int Hkv, int q_dtype) { return q_dtype != B200Q_F16 || Hkv > kAttnWarps; }
+// Page ranges that a workspace has room for (range r and sequence b meet in slot r + b); 0: too few, or no workspace.  kMaxGrid ranges
+// fill every SM twice; more only serve the warps that fewer than 8 kv heads leave over, so a workspace without room for them is cut to,
+// not refused.  Where scratch is optional, one range per SM is enough to be faster than one warp per head.
+static int split_ranges(const void* workspace, size_t bytes, int B, int Hq, int Hkv, int D, int q_dtype) {
+    if (workspace == nullptr) return 0;
+    const int64_t ranges = (int64_t)(bytes / ((size_t)Hq * (D + 2) * sizeof(float))) - B;
+    const int chunks = std::max(1, Hkv / kAttnWarps), at_least = scratch_optional(Hkv, q_dtype) ? (sm_count() + chunks - 1) / chunks : kMaxGrid;
+    return ranges >= at_least ? (int)std::min<int64_t>(ranges, kMaxRanges) : 0;
+}
+
 int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const uint8_t* v_codes, const void* k_scales,
                           const void* v_scales, const int32_t* block_table, const int32_t* lengths, void* out,
                           void* workspace, size_t workspace_bytes, int B, int Hq, int Hkv, int D, int page_size,
@@ -1177,9 +1191,9 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     };
     if (!fast_ok) return simple();
     // small batches: one cluster per (sequence, kv head), merged on chip - no workspace, no second launch
-    const bool have_workspace = workspace != nullptr && workspace_bytes >= paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D);
+    const int ranges = split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, q_dtype);
     const ClusterChoice choice = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv) : ClusterChoice{0, false};
-    const int cluster = choice.preferred || !have_workspace ? choice.size : 0;
+    const int cluster = choice.preferred || ranges == 0 ? choice.size : 0;
     if (cluster > 0) {
         ClusterAttnParams c = {};
         if (tp_out_slot >= 0) c.tp_out = tp_slot(tp_out_slot)->out;
@@ -1193,7 +1207,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
         const int rc = launch_cluster_attention(c, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
     }
-    if (!have_workspace) return B200Q_ERR_WORKSPACE;
+    if (ranges == 0) return scratch_optional(Hkv, q_dtype) && tp_out_slot < 0 ? simple() : (int)B200Q_ERR_WORKSPACE;
 
     AttnParams p = {};
     if (tp_out_slot >= 0) p.tp_out = tp_slot(tp_out_slot)->out;
@@ -1206,7 +1220,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     p.window = window_size;
     p.row_bytes = Hkv * dp;
     p.scale_row_halves = Hkv * Gd;
-    const int rc = launch_split_attention(p, stream);
+    const int rc = launch_split_attention(p, ranges, stream);
     return rc == B200Q_ERR_UNSUPPORTED && tp_out_slot < 0 ? simple() : rc;      // scales of very many kv heads do not fit a ring
 }
 
@@ -1225,7 +1239,7 @@ int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v
     p.group = Hq / Hkv; p.num_pages = num_pages; p.scale = scale; p.q_dtype = dtype; p.bits = 16;
     p.row_bytes = Hkv * kHeadDim * 2;
     p.verdict = verdict;
-    return launch_split_attention(p, stream);
+    return launch_split_attention(p, kMaxRanges, stream);
 }
 
 // Decode-layer attention in one call: split + rotate + append (as rope_kv_append_impl) followed by the attention over
@@ -1259,7 +1273,7 @@ int rope_append_attention_impl(const void* qkv, const float* cos_table, const fl
                          ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) && ((uintptr_t)k_scales % 8 == 0) &&
                          ((uintptr_t)v_scales % 8 == 0);
     const ClusterChoice choice = fast_ok ? cluster_choice(B, Hkv) : ClusterChoice{0, false};
-    const bool two_stages = q_scratch != nullptr && workspace != nullptr && workspace_bytes >= paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D);
+    const bool two_stages = q_scratch != nullptr && split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, B200Q_F16) > 0;
     const int cluster = choice.preferred || !two_stages ? choice.size : 0;
     if (cluster > 0) {
         int tp_in_slot = -1, tp_out_slot = -1;
