@@ -127,10 +127,9 @@ PyObject* matvec(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     Matrix m;
     if (B <= 0 || B > INT32_MAX || K <= 0 || !matrix(m, a[2], a[3], a[4], (int)bits, K, group, dev)) return none();
     Tensor y = empty({B, m.n}, x->scalar_type(), dev), scratch;
-    if (const size_t n = p_scratch_bytes((int)B, K, dtype_code(x->scalar_type()))) {
-        scratch = empty({(int64_t)n}, at::kByte, dev);
-        p_scratch_next(scratch.mutable_data_ptr(), n);
-    }
+    const size_t scratch_bytes = p_scratch_bytes((int)B, K, dtype_code(x->scalar_type()));
+    if (scratch_bytes) scratch = empty({(int64_t)scratch_bytes}, at::kByte, dev);
+    p_scratch_next(scratch_bytes ? scratch.mutable_data_ptr() : nullptr, scratch_bytes);      // the call below takes it, always
     const int rc = p_qmatvec((int)bits, x->const_data_ptr(), codes(m.w), ptr(m.s), ptr(m.z), nullptr, y.mutable_data_ptr(), (int)B, m.n,
                              K, (int)group, dtype_code(x->scalar_type()), dtype_code(m.s->scalar_type()), stream_of(dev));
     return rc == 0 ? THPVariable_Wrap(std::move(y)) : none();

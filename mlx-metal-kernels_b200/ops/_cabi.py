@@ -174,15 +174,18 @@ def contiguous(t):
     return t if t is None or t.is_contiguous() else t.contiguous()
 
 
-def scratch_next(rows: int, k: int, x):
-    """Hands the library the scratch that its next matvec / gate-up call on ``rows`` rows of ``k`` can use; the returned tensor
-    has to live until that call is made."""
-    n = load().b200q_scratch_bytes(rows, k, dtype_code(x.dtype))
-    if n == 0:
-        return None
-    buf = torch.empty(n, dtype=torch.uint8, device=x.device)
-    load().b200q_scratch_next(buf.data_ptr(), n)
-    return buf
+def call_with_scratch(symbol: str, rows: int, k: int, x, *args) -> None:
+    """Makes the matvec / gate-up call ``symbol(*args)`` on ``rows`` rows of ``k`` with the scratch it can use.  The library keeps
+    the scratch's address for the next call of the thread: it is handed over when the arguments are ready, and taken back
+    whatever becomes of the call, so that no later call finds the address of freed memory."""
+    lib = load()
+    n = lib.b200q_scratch_bytes(rows, k, dtype_code(x.dtype))
+    buf = torch.empty(n, dtype=torch.uint8, device=x.device) if n else None
+    lib.b200q_scratch_next(ptr(buf), n)
+    try:
+        check(getattr(lib, symbol)(*args), symbol)
+    finally:
+        lib.b200q_scratch_next(None, 0)
 
 
 def scale_pair(scales, zeros):

@@ -22,15 +22,10 @@ def norm_quantized_linear(x, norm_weight, w, scales, zeros=None, *, residual_in=
     N = w.shape[0]
     y = torch.empty((R, N), dtype=x.dtype, device=x.device)
     normed = torch.empty_like(x)           # also the staging buffer of the generic (odd-shape) route
-    scratch = _cabi.scratch_next(R, K, x)      # noqa: F841 (held until the call below)
-    _cabi.check(
-        _cabi.load().b200q_norm_qmatvec(bits, x.data_ptr(), _cabi.ptr(residual_in), norm_weight.data_ptr(),
-                                        _cabi.dtype_code(norm_weight.dtype), float(eps), None, normed.data_ptr(),
-                                        w.data_ptr(), scales.data_ptr(), _cabi.ptr(zeros), None, y.data_ptr(), R, N, K,
-                                        group_size, _cabi.dtype_code(x.dtype), _cabi.dtype_code(scales.dtype),
-                                        _cabi.stream()),
-        "b200q_norm_qmatvec",
-    )
+    _cabi.call_with_scratch("b200q_norm_qmatvec", R, K, x, bits, x.data_ptr(), _cabi.ptr(residual_in), norm_weight.data_ptr(),
+                            _cabi.dtype_code(norm_weight.dtype), float(eps), None, normed.data_ptr(), w.data_ptr(),
+                            scales.data_ptr(), _cabi.ptr(zeros), None, y.data_ptr(), R, N, K, group_size,
+                            _cabi.dtype_code(x.dtype), _cabi.dtype_code(scales.dtype), _cabi.stream())
     return (y, normed) if return_normed else y
 
 

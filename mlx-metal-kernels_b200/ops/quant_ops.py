@@ -171,13 +171,9 @@ def matvec_rows(bits, x2d, codes, scales, zeros, group_size, residual=None):
     B, K = x2d.shape
     N = codes.shape[0]
     y = torch.empty((B, N), dtype=x2d.dtype, device=x2d.device)
-    scratch = _cabi.scratch_next(B, K, x2d)      # noqa: F841 (held until the call below)
-    _cabi.check(
-        _cabi.load().b200q_qmatvec(bits, x2d.data_ptr(), codes.data_ptr(), scales.data_ptr(), _cabi.ptr(zeros),
-                                   _cabi.ptr(residual), y.data_ptr(), B, N, K, group_size,
-                                   _cabi.dtype_code(x2d.dtype), _cabi.dtype_code(scales.dtype), _cabi.stream()),
-        "b200q_qmatvec",
-    )
+    _cabi.call_with_scratch("b200q_qmatvec", B, K, x2d, bits, x2d.data_ptr(), codes.data_ptr(), scales.data_ptr(), _cabi.ptr(zeros),
+                            _cabi.ptr(residual), y.data_ptr(), B, N, K, group_size, _cabi.dtype_code(x2d.dtype),
+                            _cabi.dtype_code(scales.dtype), _cabi.stream())
     return y
 
 
@@ -295,17 +291,12 @@ def gate_up_rows(bits, x2d, gate_w, up_w, gate_scales, up_scales, gate_zeros, up
             out["z"] = new(R, K)
         # the generic (odd-shape) route needs the normalised rows as a buffer, so always provide it
         out["normed"] = new(R, K)
-    scratch = _cabi.scratch_next(R, K, x2d)      # noqa: F841 (held until the call below)
-    _cabi.check(
-        _cabi.load().b200q_gate_up_swiglu(
-            bits, x2d.data_ptr(), gate_w.data_ptr(), up_w.data_ptr(), gate_scales.data_ptr(), up_scales.data_ptr(),
-            _cabi.ptr(gate_zeros), _cabi.ptr(up_zeros), _cabi.ptr(out.get("gate")), _cabi.ptr(out.get("up")),
-            _cabi.ptr(out.get("act")), _cabi.ptr(residual_in), _cabi.ptr(norm_weight),
-            _cabi.dtype_code(norm_weight.dtype) if norm_weight is not None else _cabi.F16, float(eps),
-            _cabi.ptr(out.get("z")), _cabi.ptr(out.get("normed")), R, N, K, group_size, _cabi.dtype_code(adt),
-            _cabi.dtype_code(dt), _cabi.stream()),
-        "b200q_gate_up_swiglu",
-    )
+    _cabi.call_with_scratch(
+        "b200q_gate_up_swiglu", R, K, x2d, bits, x2d.data_ptr(), gate_w.data_ptr(), up_w.data_ptr(), gate_scales.data_ptr(),
+        up_scales.data_ptr(), _cabi.ptr(gate_zeros), _cabi.ptr(up_zeros), _cabi.ptr(out.get("gate")), _cabi.ptr(out.get("up")),
+        _cabi.ptr(out.get("act")), _cabi.ptr(residual_in), _cabi.ptr(norm_weight),
+        _cabi.dtype_code(norm_weight.dtype) if norm_weight is not None else _cabi.F16, float(eps), _cabi.ptr(out.get("z")),
+        _cabi.ptr(out.get("normed")), R, N, K, group_size, _cabi.dtype_code(adt), _cabi.dtype_code(dt), _cabi.stream())
     if not want_normed:
         out.pop("normed", None)
     return out
