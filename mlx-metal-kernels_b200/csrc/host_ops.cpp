@@ -51,6 +51,7 @@ int (*p_quant_pair)(int, const void*, const void*, uint8_t*, uint8_t*, void*, vo
 int (*p_dequant_pair)(int, const uint8_t*, const uint8_t*, const void*, const void*, void*, void*, int64_t, int, int, void*) = nullptr;
 
 constexpr int kMaxDevices = 64;
+constexpr int kErrUnsupported = -2, kErrWorkspace = -4;      // B200Q_ERR_*
 constexpr int kMinNormRows = 5;      // from this many rows on the library runs the rmsnorm as a launch of its own
 
 PyObject* none() { Py_RETURN_NONE; }
@@ -246,6 +247,24 @@ PyObject* paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     return rc == 0 ? THPVariable_Wrap(std::move(out)) : none();
 }
 
+// Queries and waits on a stream are refused to every thread while one captures a graph in the default mode, unless the thread asks
+// for the relaxed one.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// Memory that a kernel on the stream may still write to goes back to its allocator when the stream has ended; if even the wait
+// fails it is kept for good.
+void release_after_stream(Tensor word, cudaStream_t st) {
+    cudaError_t err;
+    Py_BEGIN_ALLOW_THREADS
+    const RelaxedCapture relaxed;
+    err = cudaStreamSynchronize(st);
+    Py_END_ALLOW_THREADS
+    if (err != cudaSuccess) new Tensor(std::move(word));
+}
+
 // plain_attention(q, K, V, block_table, lengths, scale or None) -> out or None: fp16 / bf16 pages.  The lengths are
 // range-checked on the host, as the operator promises.  The split-KV kernel reports on them at its start, into pinned memory that
 // the host polls while the GPU goes on (a copy on the stream took 10 of 42 us per call at 16 sequences: it kept the kernel from
@@ -289,28 +308,37 @@ PyObject* plain_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         if (rc == 0) {
             Py_BEGIN_ALLOW_THREADS
             // the stream is asked now and then, so that a kernel that never ran (an earlier error) ends the wait
+            const RelaxedCapture relaxed;
             for (uint32_t i = 1; *verdict == 0; ++i) {
                 if (i % 4096 == 0 && cudaStreamQuery(st) != cudaErrorNotReady) break;
                 __builtin_ia32_pause();
             }
             Py_END_ALLOW_THREADS
-            if (*verdict == 0) cudaStreamSynchronize(st);          // everything has ended: no write to the word is left
+            if (*verdict == 0) release_after_stream(word, st);
             return *verdict == 1 ? THPVariable_Wrap(std::move(out)) : none();      // 2: the Python body raises
+        }
+        if (rc != kErrUnsupported && rc != kErrWorkspace) {      // nothing is launched with these two; else the main kernel may be
+            release_after_stream(word, st);
+            return none();
         }
     }
     static thread_local cudaEvent_t copied[kMaxDevices] = {};      // one per thread and device that ever calls this
     if (copied[dev] == nullptr && cudaEventCreateWithFlags(&copied[dev], cudaEventDisableTiming) != cudaSuccess) return none();
     Tensor host = at::detail::empty_cpu({B}, at::kInt, std::nullopt, std::nullopt, /*pin_memory=*/true, std::nullopt);
     if (cudaMemcpyAsync(host.mutable_data_ptr(), len->const_data_ptr(), (size_t)B * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaEventRecord(copied[dev], st) != cudaSuccess)
+        cudaEventRecord(copied[dev], st) != cudaSuccess) {
+        release_after_stream(host, st);
         return none();
+    }
     const int rc = p_plain_attn(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), static_cast<const int32_t*>(bt->const_data_ptr()),
                                 static_cast<const int32_t*>(len->const_data_ptr()), out.mutable_data_ptr(), ws.mutable_data_ptr(), ws_bytes,
                                 (int)B, (int)Hq, (int)Hkv, (int)D, (int)P, pages, (int)mb, (float)scale, dtype_code(q->scalar_type()), st);
     cudaError_t err;
     Py_BEGIN_ALLOW_THREADS
+    const RelaxedCapture relaxed;
     err = cudaEventSynchronize(copied[dev]);
     Py_END_ALLOW_THREADS
+    if (err != cudaSuccess) release_after_stream(host, st);
     if (rc != 0 || err != cudaSuccess) return none();
     const int32_t* n = static_cast<const int32_t*>(host.const_data_ptr());
     for (int64_t b = 0; b < B; ++b)

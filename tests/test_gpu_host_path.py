@@ -1,5 +1,7 @@
 """The operators' native call path against their Python bodies: the same launches, bit for bit, on the ordinary arguments;
 None (the Python body takes the call) on everything else."""
+import ctypes
+
 import pytest
 import torch
 
@@ -76,3 +78,28 @@ def test_quantised_pages_equal_python_body(cuda, bits, pages, D, G, dtype):
         s = scales.reshape(rows, -1).abs()
         ref = quant_ops.dequant_codes(bits, codes.reshape(rows, -1), s, torch.full_like(s, off), rows, D, G, torch.float16)
         assert torch.equal(out.reshape(rows, D), ref)
+
+
+@pytest.mark.parametrize("code,falls_through", [(-2, True), (-4, True), (-3, False), (-1, False)])
+def test_plain_attention_falls_through_only_where_nothing_was_launched(cuda, code, falls_through):
+    """The entry point that reports on the lengths fails with ``code``: after a failed launch its kernel may be under way, so the
+    general one must not be launched on the same workspace.  The entry points are stand-ins: no kernel runs."""
+    lib, host, calls = cabi.load(), cabi.host(), []
+
+    def stand_in(name, result):
+        restype, argtypes = cabi.SIGNATURES[name]
+        return ctypes.CFUNCTYPE(restype, *argtypes)(lambda *args: calls.append(name) or result)
+
+    fakes = {"b200q_paged_fp16_gqa_decode_checked": stand_in("b200q_paged_fp16_gqa_decode_checked", code),
+             "b200q_paged_fp16_gqa_decode": stand_in("b200q_paged_fp16_gqa_decode", -2)}
+    table = {name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in cabi.SIGNATURES}
+    pages = synth.activations((4, 16, 8, 128), 1, cuda)
+    q = synth.activations((1, 1, 8, 128), 2, cuda)
+    bt, ln = torch.arange(4, dtype=torch.int32, device=cuda).reshape(1, 4), torch.tensor([50], dtype=torch.int32, device=cuda)
+    host.bind({**table, **{name: ctypes.cast(fn, ctypes.c_void_p).value for name, fn in fakes.items()}})
+    try:
+        assert host.plain_attention(q, pages, pages, bt, ln, None) is None
+    finally:
+        host.bind(table)
+    assert calls == list(fakes)[:2 if falls_through else 1]
+    assert host.plain_attention(q, pages, pages, bt, ln, None) is not None
