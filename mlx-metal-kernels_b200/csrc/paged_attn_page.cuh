@@ -5,10 +5,13 @@
 // decide.  (The form before this one dequantised K and V to fp16 with three operations per pair and took 591 warp
 // instructions per page and kv head; it ran at 58 % issue and 0.27 of the DRAM rate.)
 //   * copies: tensor copies put a page down token-major and swizzled, so that ldmatrix meets no bank conflicts.
-//   * S = K Q^T: ldmatrix hands every lane the word of its token row; raw codes go into mma.sync.m16n8k32 u8 x s8 (a q4 word costs
-//     two masks and a shift, a q8 word nothing).  The queries are 16-bit fixed point relative to the head's largest
-//     element, as two signed bytes = two columns of the B operand; the offset of the codes is the accumulator's start value.
-//     The scale is applied once per token and group in fp32, so K is not rounded at all.
+//   * S = K Q^T: ldmatrix hands every lane the word of its token row; code - offset as exact fp16 integers takes two operations per
+//     pair, the queries enter as they are, and the scale is applied once per token and group in fp32.  So neither side is rounded.
+//     (The form before multiplied raw codes in u8 x s8 with queries in two signed bytes.  It saved these operations but rounded every
+//     query at 2^-16 of its head's largest: with one channel 100 times the rest and K zero there the result's relative error was
+//     9.2e-4 instead of 2.8e-4.  One column per head instead of two and no accumulator start values make up for the operations:
+//     16 x 8192 tokens, 8 kv heads, groups of 8: q4 77.8 -> 51.3 us, q8 77.4 -> 59.9; groups of 4: q4 42.3 -> 44.0, 32 x 4096
+//     q8 54.7 -> 54.4.)
 //   * softmax: a lane holds one head (two when there are more than four query heads per kv head) of tokens g and g + 8.  The
 //     reference maximum only moves when a score exceeds it by 2^8, decided by one vote per page; no shuffles otherwise.
 //   * O^T += V^T P: ldmatrix.trans delivers the codes of two tokens side by side, exact fp16 code - offset takes two operations per
@@ -23,7 +26,6 @@ namespace attn {
 
 constexpr int kHeadDim = 128;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kQLevels = 32638.0f;          // the largest 16-bit value whose high digit still fits a signed byte, less one for the product's rounding
 
 // BITS: 4, 8 (codes) or 16 (plain).  LOGG: log2 of the scale group, 5 or 6; for plain pages 0 = fp16, 1 = bf16.
 template <int BITS> struct PageShape {
@@ -50,16 +52,6 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ void mma_u8s8_start(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0, int c1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
-                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1));
-}
-__device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 template <bool BF>
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     if constexpr (BF) {
@@ -76,12 +68,21 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// code - offset as exact halves: the nibbles (0, 4) (1, 5) (2, 6) (3, 7) of a q4 word; two bytes of a q8 word
+__device__ __forceinline__ void q4_values(uint32_t w, uint32_t (&v)[4]) {
+    const uint32_t w8 = w >> 8;
+    v[0] = hsub2_u32(lop3_and_or(w, 0x000F000Fu, 0x64006400u), 0x64086408u);
+    v[1] = hsub2_u32(lop3_and_or(w, 0x00F000F0u, 0x54005400u), 0x54805480u);
+    v[2] = hsub2_u32(lop3_and_or(w8, 0x000F000Fu, 0x64006400u), 0x64086408u);
+    v[3] = hsub2_u32(lop3_and_or(w8, 0x00F000F0u, 0x54005400u), 0x54805480u);
+}
+__device__ __forceinline__ uint32_t q8_values(uint32_t w, uint32_t sel) { return hsub2_u32(prmt(w, 0x64646464u, sel), 0x64806480u); }
+
 // WIDE: five to eight query heads per kv head.  ST: heads ("streams") a lane holds: head t, and head 4 + t when WIDE.
 template <int BITS, bool WIDE> struct WarpState {
     static constexpr int ST = WIDE ? 2 : 1;
-    uint32_t qb[BITS == 16 ? 1 : ST][BITS == 16 ? 8 : 4][2];      // queries as B operand, per mma
-    int c0[BITS == 16 ? 1 : ST][BITS == 16 ? 1 : 4][2];           // -offset * (sum of the group's query digits): accumulator start
-    float qs[ST];               // factor of the integer scores: digit step * softmax scale * log2(e)
+    uint32_t qb[8][2];          // queries as B operand, per mma
+    float qs[ST];               // factor of the scores: softmax scale * log2(e) (bf16 queries of codes: and their power of two)
     float m[ST], l[ST];         // reference maximum (log2 units), this lane's share of the sum
     float vk;                   // power of two on the V scales inside the probabilities
     float o[8][4];              // O^T tiles; see out_value()
@@ -103,72 +104,55 @@ __device__ __forceinline__ void load_queries(WarpState<BITS, WIDE>& a, const voi
     constexpr int ST = WarpState<BITS, WIDE>::ST;
     const int g = lane >> 2, t = lane & 3;
     const uint16_t* q = reinterpret_cast<const uint16_t*>(rows);
+    // column 2h is head h, column 2h + 1 head 4 + h (when WIDE): this lane feeds column g
+    const int head = (g >> 1) + ((g & 1) ? 4 : 0);
+    const bool live = ((g & 1) == 0 || WIDE) && head < group;
+    const uint16_t* row = q + (size_t)head * kHeadDim;
+#pragma unroll
+    for (int s = 0; s < ST; ++s) a.qs[s] = sm_scale * kLog2e;
     if constexpr (BITS == 16) {
-        // column 2h is head h, column 2h + 1 head 4 + h (when WIDE): this lane feeds column g
-        const int head = (g >> 1) + ((g & 1) ? 4 : 0);
-        const bool live = ((g & 1) == 0 || WIDE) && head < group;
 #pragma unroll
         for (int s = 0; s < 8; ++s)
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                a.qb[0][s][h] = live ? *reinterpret_cast<const uint32_t*>(q + (size_t)head * kHeadDim + 16 * s + 8 * h + 2 * t) : 0u;
-#pragma unroll
-        for (int s = 0; s < ST; ++s) a.qs[s] = sm_scale * kLog2e;
+            for (int h = 0; h < 2; ++h) a.qb[s][h] = live ? *reinterpret_cast<const uint32_t*>(row + 16 * s + 8 * h + 2 * t) : 0u;
     } else {
 #pragma unroll
-        for (int s = 0; s < ST; ++s) {
-            // column 2h is the high digit of head h (+ 4), column 2h + 1 its low digit: this lane feeds column g
-            const int head = (g >> 1) + 4 * s;
-            float v[4][8], mx = 0.0f;
+        for (int i = 0; i < 4; ++i) {                      // 32 dims, two mma
+            if constexpr (BITS == 4) {
+                // d = 8t .. 8t + 7 of the 32, in the order in which the masks take the nibbles of a word: (0, 4) (1, 5) (2, 6) (3, 7)
+                const uint4 u = live ? *reinterpret_cast<const uint4*>(row + 32 * i + 8 * t) : make_uint4(0u, 0u, 0u, 0u);
+                a.qb[2 * i][0] = prmt(u.x, u.z, 0x5410);
+                a.qb[2 * i][1] = prmt(u.x, u.z, 0x7632);
+                a.qb[2 * i + 1][0] = prmt(u.y, u.w, 0x5410);
+                a.qb[2 * i + 1][1] = prmt(u.y, u.w, 0x7632);
+            } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t w[4] = {0u, 0u, 0u, 0u};
-                if (head < group) {
-                    const uint16_t* row = q + (size_t)head * kHeadDim + 32 * i;
-                    if (BITS == 4) {      // d = 8t .. 8t + 7 of the 32
-                        const uint4 u = *reinterpret_cast<const uint4*>(row + 8 * t);
-                        w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
-                    } else {              // d = 4t .. 4t + 3 and 16 + 4t ..
-                        const uint2 u0 = *reinterpret_cast<const uint2*>(row + 4 * t), u1 = *reinterpret_cast<const uint2*>(row + 16 + 4 * t);
-                        w[0] = u0.x; w[1] = u0.y; w[2] = u1.x; w[3] = u1.y;
-                    }
+                for (int c = 0; c < 2; ++c) {              // d = 4t .. 4t + 3 of 16
+                    const uint2 u = live ? *reinterpret_cast<const uint2*>(row + 32 * i + 16 * c + 4 * t) : make_uint2(0u, 0u);
+                    a.qb[2 * i + c][0] = u.x;
+                    a.qb[2 * i + c][1] = u.y;
                 }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    v[i][2 * j] = dtype == B200Q_F16 ? half_lo(w[j]) : __uint_as_float(w[j] << 16);
-                    v[i][2 * j + 1] = dtype == B200Q_F16 ? half_hi(w[j]) : __uint_as_float(w[j] & 0xFFFF0000u);
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) mx = v[i][j] == v[i][j] ? fmaxf(mx, fabsf(v[i][j])) : INFINITY;
             }
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            const float up = mx > 0.0f ? kQLevels / mx : 0.0f;
-            int sum[4];
+        }
+        if (dtype != B200Q_F16) {
+            // bf16 queries in fp16: a power of two brings the head's largest element to [2^13, 2^14); bf16 has 8 significant bits, so all
+            // within 2^-30 of the largest are exact
+            uint32_t mx = 0u;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t dig[8];
+            for (int s = 0; s < 8; ++s)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int x = __float2int_rn(v[i][j] * up);
-                    const int hi = (x + 128) >> 8;
-                    dig[j] = (uint32_t)((g & 1) ? x - (hi << 8) : hi) & 0xFFu;
-                }
-                // q4: even elements, then odd ones (low and high nibbles of the code word); q8: the two runs of four
-                constexpr int E = BITS == 4 ? 2 : 1, O = BITS == 4 ? 1 : 4;
-                a.qb[s][i][0] = dig[0] | (dig[E] << 8) | (dig[2 * E] << 16) | (dig[3 * E] << 24);
-                a.qb[s][i][1] = dig[O] | (dig[O + E] << 8) | (dig[O + 2 * E] << 16) | (dig[O + 3 * E] << 24);
-                sum[i] = __dp4a((int)a.qb[s][i][0], 0x01010101, __dp4a((int)a.qb[s][i][1], 0x01010101, 0));
-                sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 1);
-                sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 2);
-            }
-            if (LOGG == 6) { sum[0] += sum[1]; sum[2] += sum[3]; }
-            // as accumulator owner this lane holds columns 2t, 2t + 1: head t (+ 4)
+                for (int h = 0; h < 2; ++h) mx = max(mx, max(a.qb[s][h] & 0x7FFFu, (a.qb[s][h] >> 16) & 0x7FFFu));
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const uint32_t e = max(mx >> 7, 14u);
+            const float up = __uint_as_float((267u - e) << 23), down = __uint_as_float((e - 13u) << 23);      // 2^(140 - e) and its inverse
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int s = 0; s < 8; ++s)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) a.c0[s][i][e] = (BITS == 4 ? -8 : -128) * __shfl_sync(0xffffffffu, sum[i], (2 * t + e) * 4);
-            a.qs[s] = __shfl_sync(0xffffffffu, mx, 2 * t * 4) / kQLevels * (sm_scale * kLog2e);
+                for (int h = 0; h < 2; ++h) a.qb[s][h] = pack_h2(__uint_as_float(a.qb[s][h] << 16) * up, __uint_as_float(a.qb[s][h] & 0xFFFF0000u) * up);
+            // as accumulator owner this lane holds columns 2t, 2t + 1
+#pragma unroll
+            for (int s = 0; s < ST; ++s) a.qs[s] *= __shfl_sync(0xffffffffu, down, 8 * t + 4 * s);
         }
     }
 }
@@ -213,7 +197,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
         for (int i = 0; i < 8; ++i) {
             uint32_t r[4];
             ldsm4(r, chunk_pair<BITS>(kr, i));
-            mma_f16<BF>(c, r[0], r[1], r[2], r[3], a.qb[0][i][0], a.qb[0][i][1]);
+            mma_f16<BF>(c, r[0], r[1], r[2], r[3], a.qb[i][0], a.qb[i][1]);
         }
         s[0][0] = c[0] * a.qs[0];
         s[0][1] = c[2] * a.qs[0];
@@ -230,28 +214,34 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
         float acc[ST][2];
 #pragma unroll
         for (int x = 0; x < ST; ++x) acc[x][0] = acc[x][1] = 0.0f;
-        int c[ST][4];
+        float c[4];
         uint32_t r[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            uint32_t w[4];
+            if (LOGG == 5 || i % 2 == 0) c[0] = c[1] = c[2] = c[3] = 0.0f;
             if constexpr (BITS == 4) {
                 if (i % 2 == 0) ldsm4(r, chunk_pair<BITS>(kr, i / 2));
-                const uint32_t w0 = r[(i & 1) * 2], w1 = r[(i & 1) * 2 + 1];
-                w[0] = w0 & 0x0F0F0F0Fu; w[1] = w1 & 0x0F0F0F0Fu;
-                w[2] = (w0 >> 4) & 0x0F0F0F0Fu; w[3] = (w1 >> 4) & 0x0F0F0F0Fu;
+                uint32_t x[4], y[4];
+                q4_values(r[(i & 1) * 2], x);
+                q4_values(r[(i & 1) * 2 + 1], y);
+                mma_m16n8k16(c, x[0], y[0], x[1], y[1], a.qb[2 * i][0], a.qb[2 * i][1]);
+                mma_m16n8k16(c, x[2], y[2], x[3], y[3], a.qb[2 * i + 1][0], a.qb[2 * i + 1][1]);
             } else {
-                ldsm4(w, chunk_pair<BITS>(kr, i));
-            }
+                ldsm4(r, chunk_pair<BITS>(kr, i));
 #pragma unroll
-            for (int x = 0; x < ST; ++x) {
-                if (LOGG == 5 || i % 2 == 0) mma_u8s8_start(c[x], w, a.qb[x][i][0], a.qb[x][i][1], a.c0[x][i][0], a.c0[x][i][1]);
-                else mma_u8s8(c[x], w, a.qb[x][i][0], a.qb[x][i][1]);
-                if (LOGG == 5 || i % 2 == 1) {
-                    const int gi = LOGG == 5 ? i : i / 2;
-                    const uint32_t k0 = ks0[gi / 2] & 0x7FFF7FFFu, k1 = ks1[gi / 2] & 0x7FFF7FFFu;
-                    acc[x][0] = fmaf((gi & 1) ? half_hi(k0) : half_lo(k0), (float)((c[x][0] << 8) + c[x][1]), acc[x][0]);
-                    acc[x][1] = fmaf((gi & 1) ? half_hi(k1) : half_lo(k1), (float)((c[x][2] << 8) + c[x][3]), acc[x][1]);
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t x = r[2 * h], y = r[2 * h + 1];
+                    mma_m16n8k16(c, q8_values(x, 0x4140u), q8_values(y, 0x4140u), q8_values(x, 0x4342u), q8_values(y, 0x4342u), a.qb[2 * i + h][0], a.qb[2 * i + h][1]);
+                }
+            }
+            if (LOGG == 5 || i % 2 == 1) {
+                const int gi = LOGG == 5 ? i : i / 2;
+                const uint32_t k0 = ks0[gi / 2] & 0x7FFF7FFFu, k1 = ks1[gi / 2] & 0x7FFF7FFFu;
+                const float f0 = (gi & 1) ? half_hi(k0) : half_lo(k0), f1 = (gi & 1) ? half_hi(k1) : half_lo(k1);
+#pragma unroll
+                for (int x = 0; x < ST; ++x) {
+                    acc[x][0] = fmaf(f0, c[x], acc[x][0]);
+                    acc[x][1] = fmaf(f1, c[2 + x], acc[x][1]);
                 }
             }
         }
@@ -389,15 +379,11 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
                 ldsm4_trans(r, chunk_pair<BITS>(vr, cp));
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {           // 32 dims: this lane's 4 codes of two token pairs
-                    const uint32_t x = r[2 * cc], y = r[2 * cc + 1], x8 = x >> 8, y8 = y >> 8;
-                    mma_m16n8k16(a.o[4 * cp + 2 * cc], hsub2_u32(lop3_and_or(x, 0x000F000Fu, 0x64006400u), 0x64086408u),
-                                 hsub2_u32(lop3_and_or(x, 0x00F000F0u, 0x54005400u), 0x54805480u),
-                                 hsub2_u32(lop3_and_or(y, 0x000F000Fu, 0x64006400u), 0x64086408u),
-                                 hsub2_u32(lop3_and_or(y, 0x00F000F0u, 0x54005400u), 0x54805480u), b[cc][0], b[cc][1]);
-                    mma_m16n8k16(a.o[4 * cp + 2 * cc + 1], hsub2_u32(lop3_and_or(x8, 0x000F000Fu, 0x64006400u), 0x64086408u),
-                                 hsub2_u32(lop3_and_or(x8, 0x00F000F0u, 0x54005400u), 0x54805480u),
-                                 hsub2_u32(lop3_and_or(y8, 0x000F000Fu, 0x64006400u), 0x64086408u),
-                                 hsub2_u32(lop3_and_or(y8, 0x00F000F0u, 0x54005400u), 0x54805480u), b[cc][0], b[cc][1]);
+                    uint32_t x[4], y[4];
+                    q4_values(r[2 * cc], x);
+                    q4_values(r[2 * cc + 1], y);
+                    mma_m16n8k16(a.o[4 * cp + 2 * cc], x[0], x[1], y[0], y[1], b[cc][0], b[cc][1]);
+                    mma_m16n8k16(a.o[4 * cp + 2 * cc + 1], x[2], x[3], y[2], y[3], b[cc][0], b[cc][1]);
                 }
             } else {
 #pragma unroll
@@ -407,9 +393,7 @@ __device__ __forceinline__ void process_page(WarpState<BITS, WIDE>& a, uint32_t 
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         const uint32_t x = r[2 * q], y = r[2 * q + 1];
-                        mma_m16n8k16(a.o[4 * cp + 2 * cc + q], hsub2_u32(prmt(x, 0x64646464u, 0x4240u), 0x64806480u),
-                                     hsub2_u32(prmt(x, 0x64646464u, 0x4341u), 0x64806480u), hsub2_u32(prmt(y, 0x64646464u, 0x4240u), 0x64806480u),
-                                     hsub2_u32(prmt(y, 0x64646464u, 0x4341u), 0x64806480u), b[cc][0], b[cc][1]);
+                        mma_m16n8k16(a.o[4 * cp + 2 * cc + q], q8_values(x, 0x4240u), q8_values(x, 0x4341u), q8_values(y, 0x4240u), q8_values(y, 0x4341u), b[cc][0], b[cc][1]);
                     }
                 }
             }

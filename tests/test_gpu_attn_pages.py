@@ -4,7 +4,7 @@ that hold anything at all."""
 import pytest
 import torch
 
-from helpers import cabi, pq_ops, synth
+from helpers import cabi, pq_ops, rel_l2, synth
 import importlib
 
 gqa_ops = importlib.import_module("mlx_metal_kernels_b200.ops.gqa_ops")
@@ -121,4 +121,52 @@ def test_scales_aligned_to_eight_bytes(cuda, bits, G, Hq, Hkv, lengths, shifted)
         finally:
             cabi.set_tuning("attn.cluster", 0)
         assert torch.equal(got, want)
+    assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("bits,G", [(4, 32), (4, 64), (8, 32), (8, 64)])
+@pytest.mark.parametrize("Hq,Hkv", [(8, 2), (16, 2), (5, 1)])
+@pytest.mark.parametrize("kind", ["one_head", "all_heads", "two_channels", "alone_in_group"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_query_heads_with_outliers(cuda, bits, G, Hq, Hkv, kind, dtype):
+    """Queries with a channel far above the rest, where K is (nearly) zero: the scores depend on elements that lie 60 to 2000 times below
+    the largest.  Queries and K enter unrounded; what is left is p * scale and the result rounded once each, 2^-12 (fp16 result) or
+    2^-9 (bf16) of a value at most and about 0.6 of that in the norm, so 5e-4 and 2.4e-3 bound the relative error (queries rounded
+    at 2^-16 of the largest give 9e-4 and 1.9e-3 for a factor of 100, and grow with the factor)."""
+    L, pages = 700, 100
+    table, ln = _table([L, 33], pages, 5), torch.tensor([L, 33], dtype=torch.int32)
+    k, v = (synth.activations((pages, 16, Hkv, 128), s) for s in (41, 42))
+    q = synth.activations((2, 1, Hq, 128), 43, "cpu", torch.float32)
+    if kind == "one_head":
+        k[..., 37] = 0
+        q[:, :, 1 % Hq, 37] = 100.0
+    elif kind == "all_heads":
+        k[..., 37] = 0
+        q[..., 37] = -2000.0
+    elif kind == "two_channels":
+        k[..., 5] *= 1e-3
+        k[..., 99] *= 1e-3
+        q[..., 5], q[..., 99] = 300.0, -300.0
+    else:                                                 # nothing but the outlier in the first 32 elements
+        k[..., :32] *= 0.05
+        q[..., :32] = 0.0
+        q[..., 3] = 60.0
+    q = q.to(dtype)
+    cache = pq_ops.quantize_kv_pages(k.to(cuda), v.to(cuda), table.to(cuda), ln.to(cuda), pq_ops.PagedQuantizedKVConfig(bits=bits, group_size=G))
+    off = 8.0 if bits == 4 else 128.0
+
+    def exact(codes, scales):
+        codes, scales = codes.cpu(), scales.cpu().double().abs()
+        if bits == 4:
+            codes = torch.stack([codes & 15, codes >> 4], -1).reshape(*codes.shape[:-1], 128)
+        return (codes.double() - off) * scales.repeat_interleave(G, -1)
+
+    want = _expected(q, exact(cache.k_pages_q, cache.k_scales), exact(cache.v_pages_q, cache.v_scales), table, [L, 33])
+    for cluster in (-1, 1):
+        cabi.set_tuning("attn.cluster", cluster)
+        try:
+            got = pq_ops.paged_quantized_kv_gqa_decode_attention(q.to(cuda), cache, backend="cuda")
+        finally:
+            cabi.set_tuning("attn.cluster", 0)
+        assert rel_l2(got, want) <= (5e-4 if dtype == torch.float16 else 2.4e-3)
     assert cabi.device_status() == 0
