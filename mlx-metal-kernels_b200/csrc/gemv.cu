@@ -126,16 +126,23 @@ bool fast_path_ok(const GemvParams& p) {
     return true;
 }
 
-// Which kernel takes a launch: "gemv.ts" = 1 sends everything the tcgen05 kernel supports to it, -1 nothing,
-// 0 (default) the batches of gemv.ts_min_batch rows and more (default 5: measured crossover at the Llama-3-8B
-// shapes; the integer kernel's work grows with every batch row, this one's does not).
+// Which kernel takes a launch: "gemv.ts" = 1 sends everything the tcgen05 kernel supports to it, -1 nothing, 0 (default) the batches
+// of gemv.ts_min_batch rows and more.  Default 5: the integer kernel has no instance above four rows, and against the fp16 mma.sync
+// kernel tcgen05 wins from there on (fp16 rows, 14336 x 4096 q4: 15.6 against 19.1 us at five rows; 4096 x 14336: 16.4 against 26.4).
+// One region of bf16 rows goes the other way: their weights take two terms there, which doubles the chain of chunks, and with a
+// row tile for more than half of the SMs no K split can shorten it; up to eight rows are one launch of the mma.sync kernel
+// (11008 x 4096 q4, eight rows: 20.4 against 25.4 us, gate and up 28.9 against 42.4; 2048 or 8192 long rows: 18.0 against 15.1,
+// 56.7 against 46.0).
 bool prefer_ts(const GemvParams& p) {
     const int mode = tuning_get("gemv.ts");
     if (mode < 0) return false;
     if (mode > 0) return true;
-    int min_b = tuning_get("gemv.ts_min_batch");
-    if (min_b <= 0) min_b = 5;
-    return p.B >= min_b;
+    const int min_b = tuning_get("gemv.ts_min_batch");
+    if (min_b > 0) return p.B >= min_b;
+    if (p.B < 5) return false;
+    const int64_t rows_full = (int64_t)p.N * std::max(1, tuning_get("ts.tp_world"));      // of the unsharded matrix: a shard takes the same kernel
+    const bool scale_rows = p.scale_dtype == B200Q_F16 && p.Gn % 8 == 0 && aligned16(p.s[0]) && aligned16(p.z[0]) && aligned16(p.s[1]) && aligned16(p.z[1]);
+    return !(p.act_dtype == B200Q_BF16 && p.B <= 8 && scale_rows && rows_full > 64 * sm_count() && p.K > 2048 && p.K < 8192);
 }
 
 // bf16 rows in fp16 for the tcgen05 kernel: one power of two per row brings the largest element to [2^13, 2^14); bf16 has 8
@@ -188,14 +195,8 @@ int rows_to_fp16(const void* x, void* out, float* scale, int rows, int K, cudaSt
 
 int dispatch_fast(int bits, GemvParams& p, bool gate_up, cudaStream_t stream) {
     if (p.B <= 4 && tuning_get("gemv.i8") >= 0) {
-        int rc = bits == 4 ? gemv_i8_q4(p, gate_up, stream) : gemv_i8_q8(p, gate_up, stream);
-        if (rc != B200Q_ERR_UNSUPPORTED) return rc;
-        // three or four long rows do not fit into its shared memory: there the tcgen05 kernel comes next (4096 x 14336, four
-        // rows: 17 us against 23 us of the fp16 mma.sync kernel)
-        if (p.B >= 3 && tuning_get("gemv.ts") == 0) {
-            rc = qgemm_ts(bits, p, gate_up, stream);
-            if (rc != B200Q_ERR_UNSUPPORTED) return rc;
-        }
+        const int rc = bits == 4 ? gemv_i8_q4(p, gate_up, stream) : gemv_i8_q8(p, gate_up, stream);
+        if (rc != B200Q_ERR_UNSUPPORTED) return rc;      // three or four long rows do not fit into its shared memory
     }
     if (p.B > 16) return B200Q_ERR_UNSUPPORTED;
     return bits == 4 ? gemv_fast_q4(p, gate_up, stream) : gemv_fast_q8(p, gate_up, stream);

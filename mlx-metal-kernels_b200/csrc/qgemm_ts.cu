@@ -50,8 +50,8 @@ B200Q_DEFINE_STATUS_WORD(qgemm_ts_read_status)
 namespace {
 
 constexpr int kRows = 128;                     // weight rows per tile = lanes of tensor memory
-constexpr int kChunkK = 128;                   // k per chunk of A in tensor memory (64 columns of 2 halves)
-constexpr int kChunkCols = kChunkK / 2;
+constexpr int kChunkCols = 64;                 // tensor-memory columns of a chunk of A (2 halves each): 128 k, or 64 k in two terms
+constexpr int chunk_k(bool split) { return split ? 64 : 128; }
 constexpr int kRowBytes = 128;                 // bytes of one weight row per stage = the swizzle span
 constexpr int kWTile = kRows * kRowBytes;      // 16 KB of codes per stage and matrix
 constexpr int kMetaGroups = 16;                // groups per scale tile: 32 bytes of a row (one sector), several stages' worth
@@ -148,6 +148,13 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&v)[32])
         "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
         "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
         "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -298,17 +305,19 @@ __device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&a
 }
 
 // META: scales arrive by TMA (their rows are a multiple of 16 bytes), else the dequantise warps read them from global memory.
-template <int BITS, int LOGG, int MATS, bool META>
+// SPLIT: weights in two fp16 terms, w = hi + lo with hi = (q - rint(z)) * s rounded and lo = what the rounding left out + (rint(z) - z) * s (see
+// qgemm_ts for whom).  A chunk then holds 64 k: hi in its first 32 columns, lo in the others, both multiplied with the same
+// activations.  14336 x 4096 q4, 32 bf16 rows: 27.1 us against 18.2 with one term and 93.8 of the mma.sync kernel.
+template <int BITS, int LOGG, int MATS, bool META, bool SPLIT>
 __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_constant__ TsParams p) {
     constexpr int KS = kRowBytes * 8 / BITS;           // k per stage: 256 (q4) or 128 (q8)
-    constexpr int SC = KS / kChunkK;                   // k-chunks per stage
-    constexpr int APS = SC * MATS;                     // chunks of A per stage: 1, 2 or 4
+    constexpr int CK = chunk_k(SPLIT);                 // k per chunk
+    constexpr int SC = KS / CK;                        // k-chunks per stage
+    constexpr int APS = SC * MATS;                     // chunks of A per stage: 1, 2, 4 or 8
     constexpr int NG = kGroups;                        // chunk a (counted over the kernel) belongs to group a % NG
-    constexpr int GPS = APS < NG ? APS : NG;           // groups that touch one stage (each with one chunk: APS <= NG)
     constexpr int MS = (kMetaGroups << LOGG) / KS;     // stages per scale tile
     constexpr uint32_t kMetaBuf = MATS * 2 * kMetaTile;
-    constexpr int CGR = kChunkK >> LOGG;               // scale groups per chunk: 4, 2 or 1
-    static_assert(APS <= NG, "a group has at most one chunk per stage");
+    constexpr int CGR = CK >> LOGG > 1 ? CK >> LOGG : 1;      // scale groups of a chunk: 4, 2 or 1
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* const sbase = smem_raw + (base - smem_u32(smem_raw));
@@ -345,7 +354,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
     auto col_of = [&](int it) { return (first_item + it * item_step) % p.nblk * ncols; };
 
     if (warp == kMmaWarp0) {
-        if (lane < NS) { mbar_init(&full_w[lane], 1); mbar_init(&empty_w[lane], GPS * 4); }
+        if (lane < NS) { mbar_init(&full_w[lane], 1); mbar_init(&empty_w[lane], APS * 4); }
         if (lane < XS) { mbar_init(&full_x[lane], 1); mbar_init(&empty_x[lane], MATS); }
         if (lane < NA) { mbar_init(&a_full[lane], 4); mbar_init(&a_free[lane], 1); }
         if (META && lane < p.meta_bufs) { mbar_init(&full_m[lane], 1); mbar_init(&empty_m[lane], kDeqWarps); }
@@ -409,8 +418,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     wait_bar(&empty_x[slot], par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
                     uint8_t* dst = sbase + p.off_x + (size_t)slot * p.x_bytes;
                     mbar_arrive_expect_tx(&full_x[slot], p.x_bytes);
-                    tma_load_2d(dst, &p.xmap, ch * kChunkK * 2, c0, &full_x[slot]);                       // byte coordinates
-                    tma_load_2d(dst + (p.x_bytes >> 1), &p.xmap, ch * kChunkK * 2 + 128, c0, &full_x[slot]);
+                    tma_load_2d(dst, &p.xmap, ch * CK * 2, c0, &full_x[slot]);                            // byte coordinates
+                    if (!SPLIT) tma_load_2d(dst + (p.x_bytes >> 1), &p.xmap, ch * CK * 2 + 128, c0, &full_x[slot]);
                     if (++slot == XS) { slot = 0; par ^= 1u; }
                 }
             }
@@ -439,8 +448,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
             const uint32_t a_t = a_base + (uint32_t)as * kChunkCols;
             tc_mma_ts(d_t, a_t, desc0, idesc, start ? 0u : 1u);
 #pragma unroll
-            for (int i = 1; i < kChunkK / 16; ++i)
-                tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((i >> 2) * atom16 + (i & 3) * 2), idesc, 1u);
+            for (int i = 1; i < 8; ++i)
+                tc_mma_ts(d_t, a_t + i * 8, desc0 + (uint64_t)((SPLIT ? 0 : (i >> 2) * atom16) + (i & 3) * 2), idesc, 1u);
             tc_commit(&a_free[as]);
             tc_commit(&empty_x[xs]);
         };
@@ -492,7 +501,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
             uint32_t ns[2] = {0u, 0u}, nz[2] = {0u, 0u};
             auto fetch_meta = [&](int q) {
                 const int s = st_lo + q / APS, u = q % APS, c = u / MATS, m = u % MATS;
-                const int gi = (s * KS + c * kChunkK) >> LOGG;
+                const int gi = (s * KS + c * CK) >> LOGG;
                 ns[0] = ns[1] = nz[0] = nz[1] = 0u;
                 if (n0 + r < p.N) {
                     const size_t at = (size_t)(n0 + r) * p.Gn + gi;
@@ -531,17 +540,17 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                 wait_bar(&full_w[slot], par, EV_GEMV_FULL_WAIT, ok);
                 if (META) {
                     m_waited = true;
-                    const int g0 = ((s * KS + c * kChunkK) >> LOGG) & (kMetaGroups - 1);      // first group of the chunk inside the scale tile
+                    const int g0 = ((s * KS + c * CK) >> LOGG) & (kMetaGroups - 1);      // first group of the chunk inside the scale tile
                     const uint32_t mrow = base + p.off_meta + (uint32_t)mslot * kMetaBuf + (uint32_t)(m * 2 * kMetaTile) +
                                           (uint32_t)r * (kMetaGroups * 2) + (((uint32_t)g0 * 2 & ~3u) ^ msw);
                     sreg[0] = lds32(mrow);
-                    sreg[1] = LOGG == 5 ? lds32(mrow + 4) : 0u;
+                    sreg[1] = CGR == 4 ? lds32(mrow + 4) : 0u;
                     zreg[0] = zreg[1] = 0u;
                     if (p.has_z) {
                         zreg[0] = lds32(mrow + kMetaTile);
-                        if (LOGG == 5) zreg[1] = lds32(mrow + kMetaTile + 4);
+                        if (CGR == 4) zreg[1] = lds32(mrow + kMetaTile + 4);
                     }
-                    if (LOGG == 7 && (g0 & 1)) { sreg[0] >>= 16; zreg[0] >>= 16; }
+                    if (CGR == 1 && (g0 & 1)) { sreg[0] >>= 16; zreg[0] >>= 16; }
                 } else {
                     sreg[0] = ns[0]; sreg[1] = ns[1]; zreg[0] = nz[0]; zreg[1] = nz[1];
                     if (q + NG < n_ch) fetch_meta(q + NG);
@@ -550,43 +559,64 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                 const uint32_t a_t = lane_addr + (uint32_t)(p.a_col0 + t * kChunkCols);
                 wait_bar(&a_free[t], a_par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
                 tc_fence_after();
+                // exact integers q - rint(z) of 32 k, in k order, two per register
+                auto integers = [&](int k32, const GroupConst& gc, uint32_t* d) {
+                    if (BITS == 4) {
+                        const uint4 v = lds128(wrow + ((((uint32_t)(c * (CK / 32) + k32)) ^ sw) << 4));
+                        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int hb = 0; hb < 2; ++hb) {               // halves of the chunk: 64 k -> 32 columns
-                    uint32_t out[32];
-                    GroupConst gc;
+                        for (int w = 0; w < 4; ++w) {
+                            // byte j of the word holds k = 2j (low nibble) and 2j + 1: [byte, 0x64, byte, 0x54], nibbles masked
+                            d[4 * w + 0] = hadd2_u32(prmt(w4[w], 0x00005464u, 0x5040) & 0xFFF0FF0Fu, gc.c);
+                            d[4 * w + 1] = hadd2_u32(prmt(w4[w], 0x00005464u, 0x5141) & 0xFFF0FF0Fu, gc.c);
+                            d[4 * w + 2] = hadd2_u32(prmt(w4[w], 0x00005464u, 0x5242) & 0xFFF0FF0Fu, gc.c);
+                            d[4 * w + 3] = hadd2_u32(prmt(w4[w], 0x00005464u, 0x5343) & 0xFFF0FF0Fu, gc.c);
+                        }
+                    } else {
 #pragma unroll
-                    for (int sb = 0; sb < 2; ++sb) {           // 32 k -> 16 columns
-                        const int k32 = hb * 2 + sb;           // 32-k block of the chunk
-                        const int gi = (k32 * 32) >> LOGG;     // group of the chunk
-                        if (sb == 0 || LOGG == 5)
-                            gc = group_const<BITS>((gi & 1) ? sreg[gi >> 1] >> 16 : sreg[gi >> 1], (gi & 1) ? zreg[gi >> 1] >> 16 : zreg[gi >> 1]);
-                        if (BITS == 4) {
-                            const uint4 v = lds128(wrow + ((((uint32_t)(c * 4 + k32)) ^ sw) << 4));
+                        for (int q16 = 0; q16 < 2; ++q16) {
+                            const uint4 v = lds128(wrow + ((((uint32_t)(c * (CK / 16) + k32 * 2 + q16)) ^ sw) << 4));
                             const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                             for (int w = 0; w < 4; ++w) {
-                                // byte j of the word holds k = 2j (low nibble) and 2j + 1: [byte, 0x64, byte, 0x54], nibbles masked
-                                const uint32_t p0 = prmt(w4[w], 0x00005464u, 0x5040) & 0xFFF0FF0Fu, p1 = prmt(w4[w], 0x00005464u, 0x5141) & 0xFFF0FF0Fu;
-                                const uint32_t p2 = prmt(w4[w], 0x00005464u, 0x5242) & 0xFFF0FF0Fu, p3 = prmt(w4[w], 0x00005464u, 0x5343) & 0xFFF0FF0Fu;
-                                out[sb * 16 + 4 * w + 0] = hfma2_u32(hadd2_u32(p0, gc.c), gc.s2, gc.r2);
-                                out[sb * 16 + 4 * w + 1] = hfma2_u32(hadd2_u32(p1, gc.c), gc.s2, gc.r2);
-                                out[sb * 16 + 4 * w + 2] = hfma2_u32(hadd2_u32(p2, gc.c), gc.s2, gc.r2);
-                                out[sb * 16 + 4 * w + 3] = hfma2_u32(hadd2_u32(p3, gc.c), gc.s2, gc.r2);
-                            }
-                        } else {
-#pragma unroll
-                            for (int q16 = 0; q16 < 2; ++q16) {
-                                const uint4 v = lds128(wrow + ((((uint32_t)(k32 * 2 + q16)) ^ sw) << 4));
-                                const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                                for (int w = 0; w < 4; ++w) {
-                                    out[sb * 16 + q16 * 8 + 2 * w] = hfma2_u32(hadd2_u32(prmt(w4[w], 0x64646464u, 0x4140u), gc.c), gc.s2, gc.r2);
-                                    out[sb * 16 + q16 * 8 + 2 * w + 1] = hfma2_u32(hadd2_u32(prmt(w4[w], 0x64646464u, 0x4342u), gc.c), gc.s2, gc.r2);
-                                }
+                                d[q16 * 8 + 2 * w] = hadd2_u32(prmt(w4[w], 0x64646464u, 0x4140u), gc.c);
+                                d[q16 * 8 + 2 * w + 1] = hadd2_u32(prmt(w4[w], 0x64646464u, 0x4342u), gc.c);
                             }
                         }
                     }
-                    tc_st32(a_t + hb * 32, out);
+                };
+                auto constants = [&](int k32) {                // of the 32-k block's group
+                    const int gi = (k32 * 32) >> LOGG;
+                    return group_const<BITS>((gi & 1) ? sreg[gi >> 1] >> 16 : sreg[gi >> 1], (gi & 1) ? zreg[gi >> 1] >> 16 : zreg[gi >> 1]);
+                };
+                if constexpr (!SPLIT) {
+#pragma unroll
+                    for (int hb = 0; hb < 2; ++hb) {           // halves of the chunk: 64 k -> 32 columns
+                        uint32_t out[32];
+                        GroupConst gc;
+#pragma unroll
+                        for (int sb = 0; sb < 2; ++sb) {       // 32 k -> 16 columns
+                            if (sb == 0 || LOGG == 5) gc = constants(hb * 2 + sb);
+                            integers(hb * 2 + sb, gc, out + sb * 16);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) out[sb * 16 + i] = hfma2_u32(out[sb * 16 + i], gc.s2, gc.r2);
+                        }
+                        tc_st32(a_t + hb * 32, out);
+                    }
+                } else {
+                    GroupConst gc;
+#pragma unroll
+                    for (int k32 = 0; k32 < 2; ++k32) {        // 32 k -> 16 columns of each term
+                        if (k32 == 0 || LOGG == 5) gc = constants(k32);
+                        uint32_t d[16], hi[16];
+                        integers(k32, gc, d);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) hi[i] = hmul2_u32(d[i], gc.s2);
+                        tc_st16(a_t + k32 * 16, hi);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) d[i] = hadd2_u32(hfma2_u32(d[i], gc.s2, hi[i] ^ 0x80008000u), gc.r2);
+                        tc_st16(a_t + 32 + k32 * 16, d);
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty_w[slot]);
@@ -788,17 +818,17 @@ int max_clusters(Kernel kernel, int size, uint32_t smem) {
     return n;
 }
 
-template <int BITS, int LOGG, int MATS, bool META>
+template <int BITS, int LOGG, int MATS, bool META, bool SPLIT>
 int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     constexpr int KS = kRowBytes * 8 / BITS;
-    constexpr int SC = KS / kChunkK;
+    constexpr int CK = chunk_k(SPLIT), SC = KS / CK;
     constexpr int MS = (kMetaGroups << LOGG) / KS;         // stages per scale tile
     constexpr uint32_t kMetaBuf = META ? MATS * 2 * kMetaTile : 0;
     const int sms = sm_count();
     const int tiles = (p.N + kRows - 1) / kRows;
     p.n_stage_total = (K + KS - 1) / KS;
     p.stage_bytes = MATS * kWTile;
-    auto kernel = qgemm_ts_kernel<BITS, LOGG, MATS, META>;
+    auto kernel = qgemm_ts_kernel<BITS, LOGG, MATS, META, SPLIT>;
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -822,7 +852,7 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
         const int c = ((p.B + nb - 1) / nb + 15) / 16 * 16;
         const int blocks = (p.B + c - 1) / c;
         if (blocks != nb) continue;                        // the same blocks as a smaller nb
-        const double chunk = std::max(360.0, 8.0 * std::max(22.2, c * 0.5 + 0.8));
+        const double chunk = std::max(SPLIT ? 300.0 : 360.0, 8.0 * std::max(22.2, c * 0.5 + 0.8));
         for (int sp = 1; sp <= 8; sp *= 2) {
             if (forced > 0 ? sp != std::min(forced, std::max(1, p.n_stage_total)) : sp > 1 && sp > p.n_stage_total / 2) continue;
             if (forced <= 0 && sp > 1 && (uint32_t)(sp - 1) * MATS * std::min(c, p.B) * kRows * 4 > kRedCap) continue;
@@ -859,7 +889,7 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     // rings: scale tiles so deep that the producer never waits for one before it waits for a weight stage, then activation chunks
     // and weight stages share what is left
     auto meta_bufs_for = [](int stages) { return META ? std::min(kMaxMetaBufs, (stages + MS - 1) / MS + 1) : 0; };
-    p.x_bytes = (uint32_t)cols * kChunkK * 2;
+    p.x_bytes = (uint32_t)cols * CK * 2;
     const uint32_t budget = cap - 2048u - red_alloc;       // 1 KB of barriers, up to 1 KB of alignment
     auto need = [&](int xs, int stages) {
         return (uint32_t)xs * p.x_bytes + (uint32_t)stages * p.stage_bytes + (uint32_t)meta_bufs_for(stages) * kMetaBuf;
@@ -907,16 +937,20 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     return finish_launch();
 }
 
+template <int BITS, int LOGG, int MATS>
+int dispatch_ts_form(TsParams& p, int K, bool meta, bool split, cudaStream_t stream) {
+    if (!meta) return launch_ts<BITS, LOGG, MATS, false, true>(p, K, stream);
+    return split ? launch_ts<BITS, LOGG, MATS, true, true>(p, K, stream) : launch_ts<BITS, LOGG, MATS, true, false>(p, K, stream);
+}
 template <int BITS, int LOGG>
-int dispatch_ts_mats(TsParams& p, int K, bool gate_up, bool meta, cudaStream_t stream) {
-    if (gate_up) return meta ? launch_ts<BITS, LOGG, 2, true>(p, K, stream) : launch_ts<BITS, LOGG, 2, false>(p, K, stream);
-    return meta ? launch_ts<BITS, LOGG, 1, true>(p, K, stream) : launch_ts<BITS, LOGG, 1, false>(p, K, stream);
+int dispatch_ts_mats(TsParams& p, int K, bool gate_up, bool meta, bool split, cudaStream_t stream) {
+    return gate_up ? dispatch_ts_form<BITS, LOGG, 2>(p, K, meta, split, stream) : dispatch_ts_form<BITS, LOGG, 1>(p, K, meta, split, stream);
 }
 template <int BITS>
-int dispatch_ts(TsParams& p, int K, int G, bool gate_up, bool meta, cudaStream_t stream) {
-    if (G == 32) return dispatch_ts_mats<BITS, 5>(p, K, gate_up, meta, stream);
-    if (G == 64) return dispatch_ts_mats<BITS, 6>(p, K, gate_up, meta, stream);
-    return dispatch_ts_mats<BITS, 7>(p, K, gate_up, meta, stream);
+int dispatch_ts(TsParams& p, int K, int G, bool gate_up, bool meta, bool split, cudaStream_t stream) {
+    if (G == 32) return dispatch_ts_mats<BITS, 5>(p, K, gate_up, meta, split, stream);
+    if (G == 64) return dispatch_ts_mats<BITS, 6>(p, K, gate_up, meta, split, stream);
+    return dispatch_ts_mats<BITS, 7>(p, K, gate_up, meta, split, stream);
 }
 
 }  // namespace
@@ -956,7 +990,11 @@ int qgemm_ts(int bits, const GemvParams& g, bool gate_up, cudaStream_t stream) {
     p.residual = (const uint16_t*)g.residual; p.y = (uint16_t*)g.y; p.gate_out = (uint16_t*)g.gate_out; p.up_out = (uint16_t*)g.up_out;
     p.act_out = (uint16_t*)g.act_out;
     p.x = g.x;
-    return bits == 4 ? dispatch_ts<4>(p, g.K, g.G, gate_up, meta, stream) : dispatch_ts<8>(p, g.K, g.G, gate_up, meta, stream);
+    // Weights in two terms where the kernel that these calls had before, fp16 mma.sync with up to 16 rows a launch, takes codes and scales
+    // unrounded: bf16 rows, and scale rows that no tensor copy can fetch.  Relative error against fp64, 12 x 4561 x 1280 q4 groups
+    // of 128: 2.93e-4 with one term, 2.07e-4 with two (the result's own rounding).
+    const bool split = p.bf16 || !meta;
+    return bits == 4 ? dispatch_ts<4>(p, g.K, g.G, gate_up, meta, split, stream) : dispatch_ts<8>(p, g.K, g.G, gate_up, meta, split, stream);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {

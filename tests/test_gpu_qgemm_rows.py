@@ -58,3 +58,45 @@ def test_odd_chunk_counts_over_several_items(cuda, B, N, K):
     for _ in range(5):
         assert torch.equal(quant_ops.matvec_rows(8, *args, 64), got)
     assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("B,N,K,G,dtype", [(9, 130, 1024, 64, torch.bfloat16), (40, 257, 4096, 128, torch.bfloat16), (130, 200, 1024, 32, torch.bfloat16),
+                                           (6, 10000, 4096, 64, torch.bfloat16), (9, 130, 1152, 128, torch.float16), (17, 300, 2592, 32, torch.float16),
+                                           (150, 140, 1088, 64, torch.float16)])
+def test_weights_are_not_rounded(cuda, bits, B, N, K, G, dtype):
+    """bf16 rows, and scale rows that no tensor copy can fetch: every result is the difference of two weights whose scales are
+    neighbouring halves, 2^-10 of a weight or less, so that a weight rounded to fp16 (2^-12 of it) would show as a quarter of the result."""
+    g = torch.Generator().manual_seed(B)
+    codes = torch.randint(1, 16 if bits == 4 else 256, (N, 1), generator=g, dtype=torch.int32).expand(N, K).to(torch.uint8)
+    w = quant_ops.pack_q4(codes) if bits == 4 else codes.contiguous()
+    groups = K // G
+    base = (torch.rand((N, 1), generator=g) * 0.5 + 1.0).half()
+    step = torch.arange(groups) % 2                                 # scale s, s + ulp, s, ...
+    scales = (base.view(torch.int16) + step.to(torch.int16)).view(torch.float16).contiguous()
+    x = torch.zeros((B, K), dtype=dtype)
+    for b in range(B):                                              # one element of an odd group against one of the group before it
+        first = 2 * (b % (groups // 2))
+        x[b, (first + 1) * G + b % G], x[b, first * G + (7 * b) % G] = 1.0, -1.0
+    want = codes[:, 0].double() * (scales[:, 1].double() - scales[:, 0].double())
+    for gate_up in (False, True):
+        args = to_dev(cuda, x, w, scales)
+        if gate_up:
+            out = quant_ops.gate_up_rows(bits, args[0], args[1], args[1], args[2], args[2], None, None, G)
+            got = torch.stack([out["gate"], out["up"]]).cpu()
+        else:
+            got = quant_ops.matvec_rows(bits, *args, None, G).cpu()[None]
+        err = (got.double() - want).abs() / want
+        assert err.max() <= (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8)      # twice the rounding of the result
+    assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("bits,B,N,K,G", [(4, 12, 4561, 1280, 128), (8, 24, 1000, 1088, 64), (4, 6, 700, 2592, 32)])
+def test_error_is_the_rounding_of_the_result(cuda, bits, B, N, K, G):
+    """Against fp64, fractional zero points among them: one rounding to fp16 is 2^-12 of a value at most (2.9e-4 in the norm with
+    weights rounded to fp16)."""
+    w, s, z = synth.quantized_weight(N, K, bits, G, seed=N)
+    x = synth.activations((B, K), 3)
+    q = (torch.stack([w & 15, w >> 4], -1).reshape(N, K) if bits == 4 else w).double()
+    want = x.double() @ ((q - z.double().repeat_interleave(G, 1)) * s.double().repeat_interleave(G, 1)).T
+    assert rel_l2(quant_ops.matvec_rows(bits, *to_dev(cuda, x, w, s, z), G), want) <= 2.0 ** -12
