@@ -77,9 +77,13 @@ int b200q_set_tuning(const char* key, int value);
 /* Scratch for the NEXT b200q_qmatvec / b200q_norm_qmatvec / b200q_gate_up_swiglu call of this thread (device memory, 16-byte
  * aligned, stream-ordered like the other buffers; NULL = none).  b200q_scratch_bytes(rows, K, act_dtype) is what such a call on
  * rows [rows, K] can use: bf16 rows from batch 5 on (0 otherwise).  With it they run on the tcgen05 kernel - as fp16 with a
- * power of two per row - instead of 16 rows per launch. */
+ * power of two per row - instead of 16 rows per launch.
+ * b200q_norm_scratch_bytes is what a call with a norm prologue but without a normed_out buffer can use, in fp16 and bf16, from
+ * batch 5 on: the normalised rows then lie in the scratch.  With neither buffer nor scratch such a call runs 16 rows per
+ * launch, and every CTA repeats the norm (32 rows, 4096 -> 2 x 14336 q4: 188 us against 38 us). */
 int b200q_scratch_next(void* ptr, size_t bytes);
 size_t b200q_scratch_bytes(int rows, int64_t K, int act_dtype);
+size_t b200q_norm_scratch_bytes(int rows, int64_t K, int act_dtype);
 
 /* Group-wise dequantisation, bit-exact: out = cast(fp32(code - zero) * scale) with two
  * separately rounded fp32 operations.  Replaces kernels/dequant_q4.metal, dequant_q8.metal as
@@ -102,7 +106,8 @@ int b200q_qmatvec(int bits, const void* x, const uint8_t* codes, const void* sca
 /* The same matvec with the RMSNorm (and residual add) that precedes it fused in: the rows fed to the
  * projection are rmsnorm(x + residual_in) (residual_in may be NULL).  Replaces rms_norm followed by the
  * QKV matvec of llama_layer_decode_step (ops/llama_layer_ops.py:255-259,
- * ops/quantized_decode_block_ops.py:113-131).  z_out / normed_out are written when not NULL. */
+ * ops/quantized_decode_block_ops.py:113-131).  z_out / normed_out are written when not NULL.  From five rows on give
+ * normed_out, or scratch of b200q_norm_scratch_bytes: the norm then runs once, ahead of the matvec. */
 int b200q_norm_qmatvec(int bits, const void* x, const void* residual_in, const void* norm_weight, int norm_w_dtype,
                        float eps, void* z_out, void* normed_out, const uint8_t* codes, const void* scales,
                        const void* zeros, const void* residual, void* y, int B, int64_t N, int64_t K,
@@ -118,7 +123,8 @@ int b200q_norm_qmatvec(int bits, const void* x, const void* residual_in, const v
  * rmsnorm(x + residual_in) as in quantized_mlp_block (ops/mlp_block_ops.py:339-340;
  * kernels/residual_add.metal, kernels/rms_norm.metal); z_out = cast(x + residual_in) and
  * normed_out = cast(z * rsqrt(mean(z^2) + eps) * norm_weight) are written when not NULL.
- * residual_in may be NULL (z = x); norm_weight [K] is read in norm_w_dtype. */
+ * residual_in may be NULL (z = x); norm_weight [K] is read in norm_w_dtype.  From five rows on give normed_out or
+ * scratch, as for b200q_norm_qmatvec. */
 int b200q_gate_up_swiglu(int bits, const void* x, const uint8_t* gate_codes, const uint8_t* up_codes,
                          const void* gate_scales, const void* up_scales, const void* gate_zeros,
                          const void* up_zeros, void* gate_out, void* up_out, void* act_out,

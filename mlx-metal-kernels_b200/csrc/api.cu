@@ -69,6 +69,7 @@ int peer_read_status(int reset, cudaStream_t stream);
 int stack_read_status(int reset, cudaStream_t stream);
 void scratch_next(void* ptr, size_t bytes);
 size_t scratch_bytes_impl(int rows, int64_t K, int act_dtype);
+size_t norm_scratch_bytes_impl(int rows, int64_t K, int act_dtype);
 int quantize_kv_pair_impl(int bits, const void* k, const void* v, uint8_t* k_codes, uint8_t* v_codes, void* k_scales, void* v_scales,
                           int64_t rows, int D, int group_size, int in_dtype, cudaStream_t stream);
 int dequantize_kv_pair_impl(int bits, const uint8_t* k_codes, const uint8_t* v_codes, const void* k_scales, const void* v_scales, void* k,
@@ -442,6 +443,7 @@ int b200q_scratch_next(void* ptr, size_t bytes) {
     return B200Q_OK;
 }
 size_t b200q_scratch_bytes(int rows, int64_t K, int act_dtype) { return scratch_bytes_impl(rows, K, act_dtype); }
+size_t b200q_norm_scratch_bytes(int rows, int64_t K, int act_dtype) { return norm_scratch_bytes_impl(rows, K, act_dtype); }
 
 int b200q_set_tuning(const char* key, int value) {
     if (key == nullptr) return B200Q_ERR_BAD_ARG;

@@ -208,6 +208,10 @@ struct ScratchGuard {                            // a call that ends early must 
     ~ScratchGuard() { t_scratch = nullptr; t_scratch_bytes = 0; }
 };
 
+constexpr int kMinApart = 5;                     // rows from which on the norm, or the conversion of bf16 rows, is a launch of its own
+size_t scratch_rows(int rows, int64_t K) { return ((size_t)rows * K * 2 + 255) / 256 * 256; }
+size_t scratch_scales(int rows) { return ((size_t)rows * 4 + 255) / 256 * 256; }
+
 // rows b0 .. b0 + bn of a problem
 GemvParams slice(const GemvParams& a, int b0, int bn) {
     GemvParams p = a;
@@ -227,23 +231,28 @@ int run_rows(int bits, GemvParams all, bool gate_up, cudaStream_t stream) {
     const size_t scratch_bytes = t_scratch_bytes;
     const bool tp_used = all.tp_in.world > 0 || all.tp_out.world > 0;
     const bool tensor_cores = !tuning_get("gemv.force_generic");
-    // From five rows on the norm is a launch of its own where the caller gives the buffer: inside the matvec kernels every CTA would
-    // repeat it (fp16 mma.sync kernel, 4096 -> 2 x 14336 at batch 8: 40 us fused against 30 + 3).
+    const bool bf = all.act_dtype == B200Q_BF16;
+    // the scratch: bf16 rows as fp16 and their powers of two, then normalised rows
+    const size_t rows_bytes = scratch_rows(all.B, all.K), fp16_bytes = bf ? rows_bytes + scratch_scales(all.B) : 0;
+    const bool usable = scratch != nullptr && aligned16(scratch), room = !bf || (usable && scratch_bytes >= fp16_bytes);
+    void* normed = all.normed_out;
+    if (normed == nullptr && usable && scratch_bytes >= fp16_bytes + rows_bytes) normed = static_cast<uint8_t*>(scratch) + fp16_bytes;
+    // From five rows on the norm is a launch of its own where there is a buffer for its rows, the caller's or scratch: inside the matvec
+    // kernels every CTA would repeat it, and only mma.sync kernels of up to 16 rows have it at all (4096 -> 2 x 14336 q4, cold calls by
+    // events: 8 rows 53 us fused, 36 apart; 32 rows 188 and 38).
     auto norm_first = [&]() -> int {
-        if (all.norm_w == nullptr || all.normed_out == nullptr) return B200Q_OK;
-        const int rc = rmsnorm_residual_launch(all.x, all.res_in, all.norm_w, all.normed_out, all.z_out, all.B, all.K, all.eps, all.act_dtype,
+        if (all.norm_w == nullptr || normed == nullptr) return B200Q_OK;
+        const int rc = rmsnorm_residual_launch(all.x, all.res_in, all.norm_w, normed, all.z_out, all.B, all.K, all.eps, all.act_dtype,
                                                all.norm_w_dtype, stream);
-        all.x = all.normed_out;
+        all.x = normed;
         all.norm_w = nullptr; all.res_in = nullptr; all.z_out = nullptr; all.normed_out = nullptr;
         return rc;
     };
-    if (!tp_used && tensor_cores && prefer_ts(all)) {
-        const bool bf = all.act_dtype == B200Q_BF16;
-        const size_t rows_bytes = ((size_t)all.B * all.K * 2 + 255) / 256 * 256;
-        const bool room = !bf || (scratch != nullptr && (reinterpret_cast<uintptr_t>(scratch) & 15u) == 0 && scratch_bytes >= rows_bytes + (size_t)all.B * 4);
+    const bool ts = !tp_used && tensor_cores && prefer_ts(all);
+    if (ts) {
         GemvParams probe = all;
         if (bf) probe.col_scale = reinterpret_cast<const float*>(scratch);
-        if (probe.norm_w != nullptr) probe.x = probe.normed_out;
+        if (probe.norm_w != nullptr) probe.x = normed;
         if (room && probe.x != nullptr && qgemm_ts_applies(probe, gate_up)) {
             int rc = norm_first();
             if (rc != B200Q_OK) return rc;
@@ -258,10 +267,10 @@ int run_rows(int bits, GemvParams all, bool gate_up, cudaStream_t stream) {
             rc = qgemm_ts(bits, p, gate_up, stream);
             if (rc != B200Q_ERR_UNSUPPORTED) return rc;
         }
-        if (fast_path_ok(slice(all, 0, std::min(all.B, 16)))) {
-            const int rc = norm_first();
-            if (rc != B200Q_OK) return rc;
-        }
+    }
+    if ((ts || (!tp_used && all.B >= kMinApart && tuning_get("gemv.ts") >= 0)) && fast_path_ok(slice(all, 0, std::min(all.B, 16)))) {
+        const int rc = norm_first();
+        if (rc != B200Q_OK) return rc;
     }
     int chunk = 16;      // batch rows per launch; halved when a kernel's shared-memory plan does not fit
     for (int b0 = 0; b0 < all.B;) {
@@ -310,8 +319,12 @@ void scratch_next(void* ptr, size_t bytes) {
     t_scratch_bytes = ptr != nullptr ? bytes : 0;
 }
 size_t scratch_bytes_impl(int rows, int64_t K, int act_dtype) {
-    if (K <= 0 || act_dtype != B200Q_BF16 || rows < 5) return 0;
-    return ((size_t)rows * K * 2 + 255) / 256 * 256 + ((size_t)rows * 4 + 255) / 256 * 256;
+    if (K <= 0 || act_dtype != B200Q_BF16 || rows < kMinApart) return 0;
+    return scratch_rows(rows, K) + scratch_scales(rows);
+}
+size_t norm_scratch_bytes_impl(int rows, int64_t K, int act_dtype) {
+    if (K <= 0 || !is_act_dtype(act_dtype) || rows < kMinApart) return 0;
+    return scratch_bytes_impl(rows, K, act_dtype) + scratch_rows(rows, K);
 }
 
 int qmatvec_impl(int bits, const void* x, const uint8_t* codes, const void* scales, const void* zeros,

@@ -31,6 +31,7 @@ SIGNATURES = {
     "b200q_set_tuning": (_i, [_c.c_char_p, _i]),
     "b200q_scratch_next": (_i, [_vp, _sz]),
     "b200q_scratch_bytes": (_sz, [_i, _i64, _i]),
+    "b200q_norm_scratch_bytes": (_sz, [_i, _i64, _i]),
     "b200q_dequant": (_i, [_i, _vp, _vp, _vp, _vp, _i64, _i64, _i, _i, _i, _vp]),
     "b200q_qmatvec": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i64, _i64, _i, _i, _i, _vp]),
     "b200q_norm_qmatvec": (_i, [_i, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i64, _i64, _i, _i, _i,

@@ -100,3 +100,42 @@ def test_error_is_the_rounding_of_the_result(cuda, bits, B, N, K, G):
     q = (torch.stack([w & 15, w >> 4], -1).reshape(N, K) if bits == 4 else w).double()
     want = x.double() @ ((q - z.double().repeat_interleave(G, 1)) * s.double().repeat_interleave(G, 1)).T
     assert rel_l2(quant_ops.matvec_rows(bits, *to_dev(cuda, x, w, s, z), G), want) <= 2.0 ** -12
+
+
+@pytest.mark.parametrize("rows", [5, 8, 33])
+@pytest.mark.parametrize("dtype,tol", [(torch.float16, 1e-3), (torch.bfloat16, 6e-3)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_norm_prologue_without_a_buffer(cuda, rows, dtype, tol, wide):
+    """A norm in front of the matvec with no buffer for its rows: with scratch the same launches and bits as with the buffer; with scratch
+    too small for it, or none, the fused kernels and the same result up to rounding."""
+    lib = cabi.load()
+    N, K, G = (9600, 2560, 64) if wide else (384, 1024, 64)
+    w, s, z = (t.to(cuda) for t in synth.quantized_weight(N, K, 4, G, seed=9))
+    x, res = (synth.activations((rows, K), i, cuda, dtype) for i in (1, 2))
+    nw = (torch.rand(K, generator=torch.Generator().manual_seed(3)) + 0.5).half().to(cuda)
+    code = cabi.dtype_code(dtype)
+    need = lib.b200q_norm_scratch_bytes(rows, K, code)
+    assert need >= rows * K * 2 and lib.b200q_norm_scratch_bytes(4, K, code) == 0
+
+    def call(gate_up, normed, scratch):
+        out, zs = torch.empty((rows, N), dtype=dtype, device=cuda), torch.empty_like(x)
+        lib.b200q_scratch_next(cabi.ptr(scratch), 0 if scratch is None else scratch.numel())
+        if gate_up:
+            rc = lib.b200q_gate_up_swiglu(4, x.data_ptr(), w.data_ptr(), w.data_ptr(), s.data_ptr(), s.data_ptr(), z.data_ptr(), z.data_ptr(), None, None,
+                                          out.data_ptr(), res.data_ptr(), nw.data_ptr(), cabi.F16, 1e-5, zs.data_ptr(), cabi.ptr(normed), rows, N, K, G,
+                                          code, cabi.F16, cabi.stream())
+        else:
+            rc = lib.b200q_norm_qmatvec(4, x.data_ptr(), res.data_ptr(), nw.data_ptr(), cabi.F16, 1e-5, zs.data_ptr(), cabi.ptr(normed), w.data_ptr(),
+                                        s.data_ptr(), z.data_ptr(), None, out.data_ptr(), rows, N, K, G, code, cabi.F16, cabi.stream())
+        assert rc == 0
+        return out, zs
+
+    new = lambda n: torch.empty(n, dtype=torch.uint8, device=cuda)
+    for gate_up in (False, True):
+        want = call(gate_up, torch.empty_like(x), new(need))
+        got = call(gate_up, None, new(need))
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        for scratch in (None, new(lib.b200q_scratch_bytes(rows, K, code) or 256)):
+            got = call(gate_up, None, scratch)
+            assert rel_l2(got[0], want[0]) <= 2 * tol and torch.equal(got[1], want[1])
+    assert cabi.device_status() == 0
