@@ -1,6 +1,6 @@
-"""GPU parity of the tcgen05 matvec kernel (weights dequantised into tensor memory) against the CPU oracle:
-rel-L2 <= 1e-3 for fp16 activations with fp32 accumulation, on both of its shapes (compact: two kernels per SM;
-whole SM), with and without a K split over a thread-block cluster, plain / gate-up / fused-norm entry points."""
+"""GPU parity of the tcgen05 matvec kernel (weights dequantised into tensor memory) against the CPU oracle: rel-L2 <= 1e-3 for fp16
+activations with fp32 accumulation, with and without a K split over a thread-block cluster, plain and gate-up, inside the MLP
+block, and row shards bit for bit."""
 import pytest
 import torch
 
@@ -17,7 +17,7 @@ def tcgen05(cuda):
     """Routes every supported launch to the tcgen05 kernel; restores the default routing afterwards."""
     cabi.set_tuning("gemv.ts", 1)
     yield cuda
-    for key in ("gemv.ts", "ts.big", "ts.split", "ts.slow_reduce", "ts.stages", "gemv.fuse_norm"):
+    for key in ("gemv.ts", "ts.split", "ts.slow_reduce", "ts.stages"):
         cabi.set_tuning(key, 0)
     assert cabi.device_status() == 0
 
@@ -39,11 +39,12 @@ SHAPES = [
 ]
 
 
-@pytest.mark.parametrize("big", [-1, 1])
+@pytest.mark.parametrize("stages", [0, 4])
 @pytest.mark.parametrize("case", SHAPES)
-def test_matvec_shapes(tcgen05, case, big):
+def test_matvec_shapes(tcgen05, case, stages):
+    """With the deepest ring of weight stages that fits, and with the shortest one."""
     bits, B, N, K, G = case
-    cabi.set_tuning("ts.big", big)
+    cabi.set_tuning("ts.stages", stages)
     w, s, z = synth.quantized_weight(N, K, bits, G, seed=N + K + bits)
     x = synth.activations((B, K), 7)
     want = _ref(bits)(x, w, s, z, group_size=G)
@@ -92,9 +93,11 @@ def test_non_integer_and_negative_zero_points_and_scales(tcgen05):
 
 
 @pytest.mark.parametrize("bits,B,N,K", [(4, 1, 512, 1024), (4, 8, 14336, 4096), (4, 32, 1792, 4096), (8, 3, 1024, 1024)])
-@pytest.mark.parametrize("big", [-1, 1])
-def test_gate_up_swiglu(tcgen05, bits, B, N, K, big):
-    cabi.set_tuning("ts.big", big)
+@pytest.mark.parametrize("split,slow", [(0, 0), (2, 0), (4, 1)])
+def test_gate_up_swiglu(tcgen05, bits, B, N, K, split, slow):
+    """K split as the launcher chooses, and forced, with the partial sums in their own buffer and through the rings."""
+    cabi.set_tuning("ts.split", split)
+    cabi.set_tuning("ts.slow_reduce", slow)
     gw, gs, gz = synth.quantized_weight(N, K, bits, 64, seed=41)
     uw, us, uz = synth.quantized_weight(N, K, bits, 64, seed=42)
     x = synth.activations((B, K), 43)
@@ -109,13 +112,9 @@ def test_gate_up_swiglu(tcgen05, bits, B, N, K, big):
 
 
 @pytest.mark.parametrize("B,with_res", [(1, False), (6, True), (32, True)])
-@pytest.mark.parametrize("big", [-1, 1])
-@pytest.mark.parametrize("fuse_norm", [1, 0])
-def test_fused_norm_prologue_and_residual_epilogue(tcgen05, B, with_res, big, fuse_norm):
-    """quantized_mlp_block through the tcgen05 kernel: [add + rmsnorm + gate/up + SwiGLU] and [down + residual], the
-    norm in the kernel's prologue (fuse_norm) or as the row kernel's launch in front of it (the default)."""
-    cabi.set_tuning("ts.big", big)
-    cabi.set_tuning("gemv.fuse_norm", fuse_norm)
+def test_mlp_block_with_norm_and_residual(tcgen05, B, with_res):
+    """quantized_mlp_block through the tcgen05 kernel: the row kernel's [add + rmsnorm], [gate/up + SwiGLU] and
+    [down + residual]."""
     hidden, inter = 1024, 2048
     gw, gs, gz = synth.quantized_weight(inter, hidden, 4, 64, seed=51)
     uw, us, uz = synth.quantized_weight(inter, hidden, 4, 64, seed=52)
@@ -140,7 +139,7 @@ def test_fused_norm_prologue_and_residual_epilogue(tcgen05, B, with_res, big, fu
                                               (8, 6, 2048, 2048, 2)])
 def test_row_shards_reproduce_the_unsharded_rows_bit_for_bit(tcgen05, bits, B, N, K, world):
     """Tensor parallelism shards the weight rows.  With "ts.tp_world" set, a shard's launch splits K exactly as the
-    unsharded launch does, so its rows are the unsharded rows bit for bit - on either shape of the kernel."""
+    unsharded launch does, so its rows are the unsharded rows bit for bit."""
     w, s, z = synth.quantized_weight(N, K, bits, 64, seed=71)
     x = synth.activations((B, K), 72)
     d = lambda t: t.to(tcgen05).contiguous()
@@ -148,22 +147,19 @@ def test_row_shards_reproduce_the_unsharded_rows_bit_for_bit(tcgen05, bits, B, N
     assert rel_l2(full, _ref(bits)(x, w, s, z, group_size=64)) <= TOL
     per = N // world
     try:
-        for big in (-1, 1):
-            cabi.set_tuning("ts.tp_world", world)
-            cabi.set_tuning("ts.big", big)
-            for r in (0, world - 1):
-                rows = slice(r * per, (r + 1) * per)
-                part = _fn(bits)(d(x), d(w[rows]), d(s[rows]), d(z[rows]), group_size=64)
-                assert torch.equal(part, full[:, rows]), (big, r)
+        cabi.set_tuning("ts.tp_world", world)
+        for r in (0, world - 1):
+            rows = slice(r * per, (r + 1) * per)
+            part = _fn(bits)(d(x), d(w[rows]), d(s[rows]), d(z[rows]), group_size=64)
+            assert torch.equal(part, full[:, rows]), r
     finally:
         cabi.set_tuning("ts.tp_world", 0)
 
 
 def test_default_routing_takes_batches_of_five_and_more(cuda):
-    """With no tuning set, batch 4 runs the mma.sync kernel and batch 5 the tcgen05 kernel; both agree with the
-    oracle, and with each other to within the parity bound."""
-    for key in ("gemv.ts", "ts.big"):
-        cabi.set_tuning(key, 0)
+    """With no tuning set, batch 4 runs the integer kernel and batch 5 the tcgen05 kernel (which "gemv.ts" = 1 therefore
+    does not change, while -1, the mma.sync kernel, may); all agree with the oracle to within the parity bound."""
+    cabi.set_tuning("gemv.ts", 0)
     w, s, z = synth.quantized_weight(1024, 2048, 4, 64, seed=61)
     x = synth.activations((5, 2048), 62)
     want = oq.reference_q4_matvec_decode(x, w, s, z, group_size=64)
@@ -171,6 +167,8 @@ def test_default_routing_takes_batches_of_five_and_more(cuda):
     y5 = quant_ops.q4_matvec_decode(d(x), d(w), d(s), d(z), group_size=64)
     y4 = quant_ops.q4_matvec_decode(d(x[:4]), d(w), d(s), d(z), group_size=64)
     assert rel_l2(y5, want) <= TOL and rel_l2(y4, want[:4]) <= TOL
+    cabi.set_tuning("gemv.ts", 1)
+    assert torch.equal(quant_ops.q4_matvec_decode(d(x), d(w), d(s), d(z), group_size=64), y5)
     cabi.set_tuning("gemv.ts", -1)
     y5_old = quant_ops.q4_matvec_decode(d(x), d(w), d(s), d(z), group_size=64)
     cabi.set_tuning("gemv.ts", 0)
