@@ -207,6 +207,11 @@ __device__ __forceinline__ uint32_t hadd2_u32(uint32_t a, uint32_t b) {
     asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+__device__ __forceinline__ uint32_t hfms2_u32(uint32_t a, uint32_t b, uint32_t c) {      // a * b - c; the negation is part of the instruction
+    uint32_t r;
+    asm("{\n.reg .b32 n;\nneg.f16x2 n, %3;\nfma.rn.f16x2 %0, %1, %2, n;\n}" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
@@ -307,7 +312,7 @@ __device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&a
 // META: scales arrive by TMA (their rows are a multiple of 16 bytes), else the dequantise warps read them from global memory.
 // SPLIT: weights in two fp16 terms, w = hi + lo with hi = (q - rint(z)) * s rounded and lo = what the rounding left out + (rint(z) - z) * s (see
 // qgemm_ts for whom).  A chunk then holds 64 k: hi in its first 32 columns, lo in the others, both multiplied with the same
-// activations.  14336 x 4096 q4, 32 bf16 rows: 27.1 us against 18.2 with one term and 93.8 of the mma.sync kernel.
+// activations.  14336 x 4096 q4, 32 bf16 rows: 26.4 us against 18.2 with one term and 93.8 of the mma.sync kernel.
 template <int BITS, int LOGG, int MATS, bool META, bool SPLIT>
 __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_constant__ TsParams p) {
     constexpr int KS = kRowBytes * 8 / BITS;           // k per stage: 256 (q4) or 128 (q8)
@@ -614,7 +619,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                         for (int i = 0; i < 16; ++i) hi[i] = hmul2_u32(d[i], gc.s2);
                         tc_st16(a_t + k32 * 16, hi);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) d[i] = hadd2_u32(hfma2_u32(d[i], gc.s2, hi[i] ^ 0x80008000u), gc.r2);
+                        for (int i = 0; i < 16; ++i) d[i] = hadd2_u32(hfms2_u32(d[i], gc.s2, hi[i]), gc.r2);
                         tc_st16(a_t + 32 + k32 * 16, d);
                     }
                 }
@@ -839,7 +844,9 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
         configured[dev & 63] = true;
     }
     // Column blocks and K split by estimated time, in clocks: rounds of items over the SMs, each a chain of chunks whose cost is the
-    // dequantisation's or the tensor pipe's (measured: 22 clocks per MMA up to 32 columns, then half a clock per column).  The choice
+    // dequantisation's or the tensor pipe's (measured: 22 clocks per MMA up to 32 columns, then half a clock per column; 64 k in two
+    // terms take 540 to 600 clocks beside the other groups, so wide blocks cost them nothing: gate and up of 14336 x 4096 q4 for
+    // 128 bf16 rows 72.6 us with 300 here, 64.8 with 540).  The choice
     // must not depend on how many rows THIS launch holds: a tensor-parallel shard of the rows has to reproduce the unsharded result
     // bit for bit, so the tile count of the unsharded matrix decides ("ts.tp_world" = number of equal row shards).
     const int tiles_full = tiles * std::max(1, tuning_get("ts.tp_world"));
@@ -852,7 +859,7 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
         const int c = ((p.B + nb - 1) / nb + 15) / 16 * 16;
         const int blocks = (p.B + c - 1) / c;
         if (blocks != nb) continue;                        // the same blocks as a smaller nb
-        const double chunk = std::max(SPLIT ? 300.0 : 360.0, 8.0 * std::max(22.2, c * 0.5 + 0.8));
+        const double chunk = std::max(SPLIT ? 540.0 : 360.0, 8.0 * std::max(22.2, c * 0.5 + 0.8));
         for (int sp = 1; sp <= 8; sp *= 2) {
             if (forced > 0 ? sp != std::min(forced, std::max(1, p.n_stage_total)) : sp > 1 && sp > p.n_stage_total / 2) continue;
             if (forced <= 0 && sp > 1 && (uint32_t)(sp - 1) * MATS * std::min(c, p.B) * kRows * 4 > kRedCap) continue;
