@@ -39,9 +39,9 @@ WORKLOAD = "c5_llama3_8b_shaped_q4_stack_32_layers_q8_paged_kv_ctx4096"
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of one batch-1 matvec launch, per shape of the
-# stack, from the ncu captures summarised in profiles/qgemv_kernel_c5_stack_shapes_b1.md (one kernel, two launches
-# each, `bench.py --profile-case <shape>_q4_b1`); the kernels read every weight byte once.
-DRAM_TRAFFIC_RATIO = {"qkv": 1.0040, "o": 1.0064, "gate": 1.0075, "down": 1.0018}
+# stack, from the ncu captures summarised in profiles/qgemv_i8_kernel_c5_stack_shapes_b1.md (one kernel, two launches
+# each, `bench.py --profile-case <shape>_q4_b1`); the kernel reads every weight byte once.
+DRAM_TRAFFIC_RATIO = {"qkv": 1.0023, "o": 1.0039, "gate": 1.0053, "down": 1.0013}
 
 
 def measured_peaks():
@@ -515,7 +515,7 @@ def run_own(args):
                      "frac_of_peak": round(step_bytes / sec_per_step / 1e9 / peak, 4)},
         "roofline": {"bound": "hbm", "kernel": "qgemv_i8_kernel (all q4 matvec launches of one step, timed alone)",
                      "achieved": round(gemv_gbs, 1), "peak": peak, "unit": "GB/s", "frac": round(gemv_gbs / peak, 4),
-                     "traffic": round(gemv_traffic / n_gemv), "traffic_source": "per-shape ncu captures (profiles/qgemv_kernel_c5_stack_shapes_b1.md): dram bytes read+written / algorithmic bytes 1.002-1.008 for the QKV, O, gate/up and down shapes, applied to this launch mix",
+                     "traffic": round(gemv_traffic / n_gemv), "traffic_source": "per-shape ncu captures (profiles/qgemv_i8_kernel_c5_stack_shapes_b1.md): dram bytes read+written / algorithmic bytes 1.001-1.005 for the QKV, O, gate/up and down shapes, applied to this launch mix",
                      "peak_kind": peak_kind, "launches": n_gemv,
                      "algorithmic_bytes_per_launch": round(gemv_bytes / n_gemv), "us_per_launch": round(gemv_sec / n_gemv * 1e6, 3)},
         "e2e": {"value": round(B / e2e_sec, 2), "unit": "tokens/s", "ms_per_step": round(e2e_sec * 1e3, 4),

@@ -93,7 +93,8 @@ int b200q_dequant(int bits, const uint8_t* codes, const void* scales, const void
                   int64_t M, int64_t K, int group_size, int scale_dtype, int out_dtype, void* stream);
 
 /* y[b, n] = sum_k x[b, k] * (code[n, k] - zero[n, k/G]) * scale[n, k/G], fp32 accumulation,
- * saturated to the finite range of act_dtype.  One implementation serves the reference's
+ * saturated to the finite range of act_dtype (rows with an infinity or NaN have no defined result: the kernels of up to
+ * 16 rows form inf - inf for them and store the negative limit).  One implementation serves the reference's
  * `metal`, `metal_parallel` and `metal_tiled` launches of q4/q8_matvec_decode
  * (ops/quant_ops.py:407-506, 529-631; kernels/q{4,8}_matvec_decode{,_parallel,_tiled}.metal).
  * If `residual` is not NULL the result is cast(residual + cast(y)), the residual_add that
@@ -280,7 +281,7 @@ int b200q_rope_kv_append(const void* qkv, const float* cos_table, const float* s
 /* b200q_rope_kv_append followed by b200q_paged_gqa_decode over the cache that now holds the new token, as one entry
  * point: the attention stage of llama_layer_decode_step (ops/llama_layer_ops.py:262-330: reference_gqa_qkv_split_rope,
  * cache update, GQA decode attention) on a paged quantized cache.  fp16 rows and fp16 cache scales.  For small batches
- * (batch x kv heads up to a quarter of the SM count) the whole stage is ONE kernel: a thread-block cluster per
+ * (8 x batch x kv heads up to three quarters of the SM count) the whole stage is ONE kernel: a thread-block cluster per
  * (sequence, kv head) rotates q, appends the head's k / v to the page of positions[b], walks the sequence's pages and
  * merges its partial results through distributed shared memory - no workspace traffic and no merge launch.  Larger
  * batches run the two stages back to back; q_scratch [B, Hq, D] then receives the rotated queries (it may be NULL only

@@ -9,8 +9,8 @@
 //   * mma.sync.m16n8k32 u8 x s8: a q4 word gives its even codes with one mask and its odd ones with a shift and a mask, a
 //     q8 word is the operand as it lies.  512 codes per instruction, exact in int32.
 //   * the activations become integers.  Per quantisation group they are scaled by a power of two to 22-bit fixed point
-//     (an element below 2^-11 of its group's largest is rounded at 2^-23 of that, the size of an fp32 sum's own rounding; all
-//     others are exact) and cut into three signed bytes.  The three digits of a row are three columns of the 8-wide B
+//     (an element below 2^-11 of its group's largest is rounded, by at most 2^-22 of that, the size of an fp32 sum's own rounding;
+//     all others are exact) and cut into three signed bytes.  The three digits of a row are three columns of the 8-wide B
 //     operand, which a matvec leaves empty anyway; digit sums meet in int32 and fp32.
 //   * per group, in fp32: y += scale * ((c2 2^16 + c1 2^8 + c0) 2^-e - zero * X), X = sum of the group's activations.  With
 //     one batch row two neighbouring groups sit side by side in the 8 columns and share this step.

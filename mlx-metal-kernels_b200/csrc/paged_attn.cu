@@ -945,8 +945,9 @@ ClusterChoice cluster_choice(int B, int Hkv) {
     // clusters stay possible for callers without a workspace.
     if (mode == 0 && ctas > 2 * sm_count()) return {0, false};
     const bool preferred = mode > 0 || ctas * 4 <= 3 * sm_count();
-    // 8 CTAs per cluster; the opt-in size 16 measured slower (placing one cluster per GPC costs more than the shorter
-    // page walk saves: 17.8 us against 12.9 us per stage at batch 1, context 4096)
+    // 8 CTAs per cluster: the opt-in size 16 is slower at every length (placing one cluster per GPC costs more than the shorter page walk
+    // saves) and 4 from some length on (one sequence of q8, 8 kv heads, cold calls by events, sizes 4 / 8 / 16: 1024 tokens 14.3 /
+    // 12.3 / 18.4 us, 4096 18.4 / 16.4 / 20.5, 8192 26.6 / 20.5 / 24.6)
     int size = 8;
     const int forced = tuning_get("attn.cluster_size");
     if (forced == 8 || forced == 16 || forced == 4) size = forced;

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) quantize_kv_kernel(const T* __restrict__ 
 // run of groups, so a thread takes 8 consecutive values wherever they lie: one 16-byte load, the group's maximum over the
 // G/8 neighbouring lanes, one 8-byte (q8) or 4-byte (q4) store.  The kernel is bound by HBM (2 bytes in, 1 or 1/2 out per
 // value); four pieces per thread are in flight.  K and V go in one launch (blockIdx.y).  Against one thread per group of
-// strided 2-byte loads and byte stores, quantising 2 x 33.5 M fp16 values to q8 groups of 32 and reading them back: 646 -> 66 us
+// strided 2-byte loads and byte stores, quantising 2 x 33.5 M fp16 values to q8 groups of 32 and reading them back: 646 -> 71 us
 // (the copies and the general dequantiser on the way back included).
 constexpr int kVecPerThread = 4;
 struct KvPair {
