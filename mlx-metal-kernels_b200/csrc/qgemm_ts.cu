@@ -222,29 +222,42 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
+// A probe that suspends the warp for up to a microsecond.  Probes that come back at once are repeated, and those of the waiting warps
+// took a third of the issue slots of a busy SM from the dequantising ones (537 instructions per chunk and scheduler, 340 of them the
+// dequantisation's): 6144 x 4096 q4 for 32 rows 11.2 -> 10.4 us, gate and up of 11008 x 4096 for 256 rows 65.5 -> 60.8.
+__device__ __forceinline__ bool probe_bar(uint32_t addr, uint32_t parity) {
+    uint32_t got;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.b32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(got)
+        : "r"(addr), "r"(parity), "r"(1000u)
+        : "memory");
+    return got != 0;
+}
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int event, bool& ok) {
-    const bool got = mbar_wait_bounded(bar, parity, &g_device_status, event, ok ? kTsWaitLimit : 64u);
-    ok = ok && got;
-    return got;
+    const uint32_t addr = smem_u32(bar);
+    if (probe_bar(addr, parity)) return true;      // mostly it is there
+    const uint32_t limit = ok ? kTsWaitLimit : 64u;
+#pragma unroll 1
+    for (uint32_t i = 0; i < limit; ++i)
+        if (probe_bar(addr, parity)) return true;
+    atomicMax(&g_device_status, event);
+    ok = false;
+    return false;
 }
 
 // One wait of a warp for several barriers: lane i polls its own (address and parity per lane; lanes without one pass `need` false).
-// Beside the busy dequantise warps a ready barrier costs a warp 150-200 clocks, so barriers are polled together, not in turn.
+// For the operands of two chunks at once (gate and up, few columns): polled together 25.4 us, in turn 25.7 (14336 x 4096 q4, 32 rows).  The two
+// barriers of a single chunk are waited for in turn: together 66.2 us, in turn 62.4 (gate and up of 11008 x 4096, 256 rows).
 __device__ __forceinline__ void wait_bars(uint32_t addr, uint32_t parity, bool need, int event, bool& ok) {
     const uint32_t limit = ok ? kTsWaitLimit : 64u;
     for (uint32_t i = 0; i < limit; ++i) {
-        uint32_t got = 1;
-        if (need)
-            asm volatile(
-                "{\n"
-                ".reg .pred p;\n"
-                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                "selp.b32 %0, 1, 0, p;\n"
-                "}\n"
-                : "=r"(got)
-                : "r"(addr), "r"(parity)
-                : "memory");
-        if (__all_sync(0xffffffffu, got != 0)) return;
+        const bool got = !need || probe_bar(addr, parity);
+        if (__all_sync(0xffffffffu, got)) return;
     }
     atomicMax(&g_device_status, event);
     ok = false;
@@ -259,21 +272,24 @@ __device__ __forceinline__ GroupConst group_const(uint32_t s_bits, uint32_t z_bi
     GroupConst c;
     c.s2 = prmt(s_bits, s_bits, 0x1010);
     const uint32_t z2 = prmt(z_bits, z_bits, 0x1010);
-    const __half2 zi = h2rint(*reinterpret_cast<const __half2*>(&z2));
-    const uint32_t zi2 = *reinterpret_cast<const uint32_t*>(&zi);
+    // z rounded to an integer by adding and taking away 1536 with its sign (an even integer from 512 on: all that matters is that codes less zi
+    // are exact, r holds the rest).  h2rint takes 16 clocks of a scheduler, this 4: gate and up of 14336 x 4096 q4 26.2 -> 25.1 us
+    const uint32_t magic = (z2 & 0x80008000u) | 0x66006600u;
+    const uint32_t zi2 = hsub2_u32(hadd2_u32(z2, magic), magic);
     c.r2 = hmul2_u32(hsub2_u32(zi2, z2), c.s2);
     c.c = hsub2_u32(BITS == 4 ? 0xD400E400u : 0xE400E400u, zi2);        // exact: integers below 2048
     return c;
 }
 
-__device__ __forceinline__ float ts_round(const TsParams& p, float v) {
-    return p.bf16 ? __bfloat162float(__float2bfloat16_rn(v)) : __half2float(__float2half_rn(v));
+// bf: the outputs are bf16 (a constant for weights in one term, which only fp16 calls have)
+__device__ __forceinline__ float ts_round(bool bf, float v) {
+    return bf ? __bfloat162float(__float2bfloat16_rn(v)) : __half2float(__float2half_rn(v));
 }
-__device__ __forceinline__ uint16_t ts_bits(const TsParams& p, float v) {
-    return p.bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+__device__ __forceinline__ uint16_t ts_bits(bool bf, float v) {
+    return bf ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
 }
-__device__ __forceinline__ float ts_float(const TsParams& p, uint16_t u) {
-    return p.bf16 ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
+__device__ __forceinline__ float ts_float(bool bf, uint16_t u) {
+    return bf ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
 }
 // The residual values of output row n for 4 columns, fetched ahead of the accumulators and before the first store (y may
 // alias the residual rows as far as the compiler knows).
@@ -286,25 +302,26 @@ __device__ __forceinline__ void ts_load_residual(const TsParams& p, int n, int b
     }
 }
 // The epilogue of 4 columns (b0 .. b0 + nb of the batch): clamp, round, residual add or SwiGLU, store.
-template <int MATS>
+template <int MATS, bool SPLIT>
 __device__ __forceinline__ void ts_store_cols(const TsParams& p, const float (&acc)[2][4], int n, int b0, int nb, const uint16_t (&res)[4]) {
-    const float fmax_act = p.bf16 ? 3.3895313892515355e38f : 65504.0f;
+    const bool bf = SPLIT && p.bf16;
+    const float fmax_act = bf ? 3.3895313892515355e38f : 65504.0f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (j >= nb) break;
         const int b = b0 + j;
         const size_t o = (size_t)b * p.N + n;
-        const float cs = p.col_scale != nullptr ? p.col_scale[b] : 1.0f;
+        const float cs = SPLIT && p.col_scale != nullptr ? p.col_scale[b] : 1.0f;
         if (MATS == 1) {
-            float v = ts_round(p, fminf(fmaxf((acc[0][j] + acc[1][j]) * cs, -fmax_act), fmax_act));
-            if (p.residual != nullptr) v = ts_float(p, res[j]) + v;
-            p.y[o] = ts_bits(p, v);
+            float v = ts_round(bf, fminf(fmaxf((acc[0][j] + acc[1][j]) * cs, -fmax_act), fmax_act));
+            if (p.residual != nullptr) v = ts_float(bf, res[j]) + v;
+            p.y[o] = ts_bits(bf, v);
         } else {
-            const float v0 = ts_round(p, fminf(fmaxf(acc[0][j] * cs, -fmax_act), fmax_act));
-            const float v1 = ts_round(p, fminf(fmaxf(acc[1][j] * cs, -fmax_act), fmax_act));
-            if (p.gate_out != nullptr) p.gate_out[o] = ts_bits(p, v0);
-            if (p.up_out != nullptr) p.up_out[o] = ts_bits(p, v1);
-            if (p.act_out != nullptr) p.act_out[o] = ts_bits(p, (v0 / (1.0f + expf(-v0))) * v1);
+            const float v0 = ts_round(bf, fminf(fmaxf(acc[0][j] * cs, -fmax_act), fmax_act));
+            const float v1 = ts_round(bf, fminf(fmaxf(acc[1][j] * cs, -fmax_act), fmax_act));
+            if (p.gate_out != nullptr) p.gate_out[o] = ts_bits(bf, v0);
+            if (p.up_out != nullptr) p.up_out[o] = ts_bits(bf, v1);
+            if (p.act_out != nullptr) p.act_out[o] = ts_bits(bf, (v0 / (1.0f + expf(-v0))) * v1);
         }
     }
 }
@@ -467,9 +484,14 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                 const RingPos x = at.x, a = at.a;
                 const bool two = per == 2 && ch + 1 < n_ch;
                 if (two) at.to(it * n_ch + ch + 1, XS, NA);
-                // lanes 0, 1: the first chunk's operands; lanes 2, 3: the second's
-                const uint32_t bar = lane == 0 ? smem_u32(&full_x[x.slot]) : lane == 1 ? smem_u32(&a_full[a.slot]) : lane == 2 ? smem_u32(&full_x[at.x.slot]) : smem_u32(&a_full[at.a.slot]);
-                wait_bars(bar, lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
+                if (two) {
+                    // lanes 0, 1: the first chunk's operands; lanes 2, 3: the second's
+                    const uint32_t bar = lane == 0 ? smem_u32(&full_x[x.slot]) : lane == 1 ? smem_u32(&a_full[a.slot]) : lane == 2 ? smem_u32(&full_x[at.x.slot]) : smem_u32(&a_full[at.a.slot]);
+                    wait_bars(bar, lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par, lane < 4, EV_GEMV_FULL_WAIT, ok);
+                } else {
+                    wait_bar(&full_x[x.slot], x.par, EV_GEMV_FULL_WAIT, ok);
+                    wait_bar(&a_full[a.slot], a.par, EV_GEMV_FULL_WAIT, ok);
+                }
                 tc_fence_after();
                 chunk(x.slot, a.slot, ch == first);
                 if (two) chunk(at.x.slot, at.a.slot, false);
@@ -521,14 +543,25 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
             const int a0 = (int)((uint32_t)it * (uint32_t)n_ch & (uint32_t)(NG - 1));      // chunk number of the item's first, modulo NG
             const int q0 = (grp - a0 + NG) & (NG - 1);
             if (!META && q0 < n_ch) fetch_meta(q0);
+            // Up to four chunks a stage, a group always takes the same ones: their place in a stage is worked out once
+            constexpr bool kSame = NG % APS == 0;
+            constexpr int kPieces = CK * BITS / 128;           // 16-byte pieces of a chunk in one weight row
+            uint32_t piece[kPieces];
+            auto place = [&](int u) {
+#pragma unroll
+                for (int i = 0; i < kPieces; ++i) piece[i] = row_u + (uint32_t)((u % MATS) * kWTile) + ((((uint32_t)(u / MATS * kPieces + i)) ^ sw) << 4);
+            };
+            if (kSame) place(q0 % APS);
+            const int u_same = q0 % APS;
 #pragma unroll 1
             for (int q = q0; q < n_ch; q += NG) {
-                const int sl = q / APS, u = q % APS;
+                const int sl = q / APS, u = kSame ? u_same : q % APS;
                 const int s = st_lo + sl;
                 const int c = u / MATS, m = u % MATS;
                 slot += sl - sl_at;                            // at most NG / APS stages on
                 sl_at = sl;
-                while (slot >= NS) { slot -= NS; par ^= 1u; }
+                if (slot >= NS) { slot -= NS; par ^= 1u; }     // a ring holds more stages than a group steps over
+                if (!kSame) place(u);
                 uint32_t sreg[2], zreg[2];
                 if (META) {
                     const int mt = s / MS - mt0;
@@ -560,14 +593,14 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     sreg[0] = ns[0]; sreg[1] = ns[1]; zreg[0] = nz[0]; zreg[1] = nz[1];
                     if (q + NG < n_ch) fetch_meta(q + NG);
                 }
-                const uint32_t wrow = row_u + (uint32_t)slot * p.stage_bytes + (uint32_t)(m * kWTile);
+                const uint32_t wslot = (uint32_t)slot * p.stage_bytes;
                 const uint32_t a_t = lane_addr + (uint32_t)(p.a_col0 + t * kChunkCols);
                 wait_bar(&a_free[t], a_par ^ 1u, EV_GEMV_EMPTY_WAIT, ok);
                 tc_fence_after();
                 // exact integers q - rint(z) of 32 k, in k order, two per register
                 auto integers = [&](int k32, const GroupConst& gc, uint32_t* d) {
                     if (BITS == 4) {
-                        const uint4 v = lds128(wrow + ((((uint32_t)(c * (CK / 32) + k32)) ^ sw) << 4));
+                        const uint4 v = lds128(wslot + piece[k32]);
                         const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int w = 0; w < 4; ++w) {
@@ -580,7 +613,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     } else {
 #pragma unroll
                         for (int q16 = 0; q16 < 2; ++q16) {
-                            const uint4 v = lds128(wrow + ((((uint32_t)(c * (CK / 16) + k32 * 2 + q16)) ^ sw) << 4));
+                            const uint4 v = lds128(wslot + piece[k32 * 2 + q16]);
                             const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                             for (int w = 0; w < 4; ++w) {
@@ -630,7 +663,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&a_full[t]);
                 t += NG;
-                while (t >= NA) { t -= NA; a_par ^= 1u; }
+                if (t >= NA) { t -= NA; a_par ^= 1u; }
             }
             // step over the rest of the item's stages and scale tiles
             slot += n_st - sl_at;
@@ -664,7 +697,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     float acc[2][4] = {};
                     tc_ld4(lane_addr + (uint32_t)(cs + grp * 4), acc[0]);
                     if (MATS == 2 || second) tc_ld4(lane_addr + (uint32_t)(ncols + cs + grp * 4), acc[1]);
-                    if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, nb, res);
+                    if (n < p.N) ts_store_cols<MATS, SPLIT>(p, acc, n, c0 + cs, nb, res);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) res[j] = next[j];
                 }
@@ -738,7 +771,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
                             if (cs + j < bcols) acc[m][j] += red[((((q - 1) * MATS + m) * rcols + cs + j) * kRows + r)];
-                if (n < p.N) ts_store_cols<MATS>(p, acc, n, c0 + cs, bcols - cs, res);
+                if (n < p.N) ts_store_cols<MATS, SPLIT>(p, acc, n, c0 + cs, bcols - cs, res);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) res[j] = next[j];
             }

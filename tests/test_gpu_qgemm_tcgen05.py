@@ -79,6 +79,23 @@ def test_symmetric_codes_without_zero_points(tcgen05, bits):
     assert rel_l2(got, want) <= TOL
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("around", [0.0, 511.5, -511.5, 900.0, -900.0, 1023.5])
+def test_zero_points_up_to_the_limit(tcgen05, bits, around):
+    """Zero points whose integer part is taken off the codes exactly: fractions, both signs, and the range from 512 on, where fp16 itself has
+    only halves and the part taken off is an even integer.  A weight is rounded to fp16 once, by at most 2^-11 of itself."""
+    g = torch.Generator().manual_seed(int(around) + bits)
+    codes, scales, _ = synth.quantized_weight(160, 512, bits, 64, seed=5)
+    zeros = (around + torch.randn((160, 8), generator=g) * 0.4).clamp(-1024, 1024).to(torch.float16)
+    scales = (scales.float() / (1.0 + abs(around) / 8)).to(torch.float16)
+    x = synth.activations((6, 512), 6)
+    w = (torch.stack((codes & 15, codes >> 4), -1).reshape(160, 512) if bits == 4 else codes).double()
+    dense = (w.reshape(160, 8, 64) - zeros.double()[..., None]) * scales.double()[..., None]
+    want = x.double() @ dense.reshape(160, 512).T
+    got = _fn(bits)(*(t.to(tcgen05) for t in (x, codes, scales, zeros)), group_size=64)
+    assert rel_l2(got, want) <= 6e-4
+
+
 def test_non_integer_and_negative_zero_points_and_scales(tcgen05):
     """The reference's own tests draw scales and zero points from N(0,1): any sign, any fraction."""
     g = torch.Generator().manual_seed(5)
