@@ -5,7 +5,12 @@
 // What bounds it: HBM.  At 6.5 TB/s an SM receives 23 bytes, i.e. 46 q4 codes, per clock, so the code path has to stay
 // well below 4 issue slots per 46 codes.  The kernel it replaces for these batches (gemv_fast.cuh) turns every code pair into
 // fp16 (5 logic instructions and 2 mma.sync per 512 codes and row half) and needed 2.2 slots per clock at 0.49 of the
-// copy rate (2 x 14336 x 4096 q4, one row: 20.7 us; here 14.8 us, 0.69; 6144 x 4096: 6.8 -> 5.5 us).
+// copy rate (2 x 14336 x 4096 q4, one row: 20.7 us; here 12.5 us, 0.82).
+// Beside HBM it was loads from shared memory: 13 of them per 1 KB of codes and warp held up the rest (stall "MIO throttle" first, by the
+// counters; without the five of the affine step the same launch ran at the copy rate).  Hence digits in the order of the
+// mma, two mma per 16-byte load, scales eight groups per load, constants two steps per load, 6.5 loads in all, and no conversions in the
+// affine step.  Cold weights, passes back to back, before -> after: q4 2 x 14336 x 4096 one row 14.3 -> 12.5 us, four rows 24.6 -> 20.0;
+// 4096 x 14336 11.2 -> 10.1; 4096 x 4096 5.1 -> 4.8; q8 8192 x 3008 groups of 32 8.9 -> 8.4.
 //   * mma.sync.m16n8k32 u8 x s8: a q4 word gives its even codes with one mask and its odd ones with a shift and a mask, a
 //     q8 word is the operand as it lies.  512 codes per instruction, exact in int32.
 //   * the activations become integers.  Per quantisation group they are scaled by a power of two to 22-bit fixed point
@@ -13,7 +18,8 @@
 //     all others are exact) and cut into three signed bytes.  The three digits of a row are three columns of the 8-wide B
 //     operand, which a matvec leaves empty anyway; digit sums meet in int32 and fp32.
 //   * per group, in fp32: y += scale * ((c2 2^16 + c1 2^8 + c0) 2^-e - zero * X), X = sum of the group's activations.  With
-//     one batch row two neighbouring groups sit side by side in the 8 columns and share this step.
+//     one batch row two neighbouring groups sit side by side in the 8 columns and share this step (and the operand: the codes of
+//     both meet the digits of both, each lane takes the sums of its own).
 // The weights are not rounded at all.
 //
 // Work: rows are dealt evenly to the CTAs (one per SM), cut into tiles of at most 16 rows; a unit is a tile x 256 bytes of every
@@ -43,6 +49,12 @@ constexpr int kI8Threads = kI8Warps * 32;
 constexpr int kI8UnitBytes = 256;             // bytes of a unit in one row: four 64-byte pieces
 constexpr uint32_t kI8OnePerSm = 116 * 1024;  // shared memory that keeps a second CTA off the SM
 constexpr int kI8MaxRes = 1024;               // residual values kept in shared memory
+// A group's digit sum S, at most 255 * 128 * 128 < 2^22 in magnitude, is added to these bits: as a float they are then kI8Magic + S, exactly,
+// and no conversion is needed.
+constexpr uint32_t kI8MagicBits = 0x4B400000u;
+constexpr float kI8Magic = 12582912.0f;       // 1.5 * 2^23
+// Digit sums are taken times 2^-kI8Shift until the end of a unit, so that kI8Magic times a digit's weight stays finite for every finite row.
+constexpr int kI8Shift = 20;
 
 struct I8Params {
     const void* x;          // [B, K]
@@ -64,11 +76,10 @@ struct I8Params {
     int rows_lo, rem;       // CTA c owns rows_lo (+1 if c < rem) rows
     int units;              // units per (tile, matrix)
     int batch;              // tiles whose sums fit into shared memory at once
-    int meta_vec;           // a row's groups fill whole units: the scales of a unit are aligned pieces
     TpOut tp_out;
     TpIn tp_in;
     uint32_t off_zero, off_xd, off_cst, off_res, off_part, off_meta, off_ring;
-    uint32_t xstride, meta_slot;
+    uint32_t xstride, cstride, meta_slot;
 };
 
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
@@ -152,10 +163,10 @@ __device__ __forceinline__ uint32_t s_ld32(uint32_t a) {
 __device__ __forceinline__ void s_ld64(uint32_t a, uint32_t& x, uint32_t& y) {
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(a));
 }
-__device__ __forceinline__ float s_ldh(uint32_t a) {
+__device__ __forceinline__ uint32_t s_ldu16(uint32_t a) {
     uint16_t v;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-    return __half2float(__ushort_as_half(v));
+    return v;
 }
 template <int NW>
 __device__ __forceinline__ void s_ldw(uint32_t a, uint32_t (&w)[NW]) {
@@ -168,13 +179,13 @@ __device__ __forceinline__ void s_ldw(uint32_t a, uint32_t (&w)[NW]) {
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(a));
     }
 }
-// D(16x8, s32) (+)= A(16x32, u8, row) * B(32x8, s8, col)
+// D(16x8, s32) (+)= A(16x32, u8, row) * B(32x8, s8, col).  FIRST: the sums start from the bits of kI8Magic.
 template <bool FIRST>
 __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     if constexpr (FIRST) {
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(kI8MagicBits));
     } else {
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
@@ -182,36 +193,30 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, 
     }
 }
 
-// One group of 16 rows against every column tile: rows g and g + 8 at `a_addr` (+ 512), digits at bx + bofs.
-template <int BITS, int LOGG, int NT, bool FIRST>
-__device__ __forceinline__ void i8_group_mma(int (&acc)[NT][4], uint32_t a_addr, const uint32_t (&bx)[NT], uint32_t bofs) {
-    constexpr int GB = (1 << LOGG) * BITS / 8;
-    constexpr int NW = (GB / 4 > 16 ? 16 : GB / 4) / 4;
-    constexpr int MI = BITS == 4 ? NW : NW / 2;
+// This lane's A operands of one group of 16 rows, rows g and g + 8 at `a_addr` (+ 512): mma i of the group.
+template <int BITS, int LOGG> struct I8Words {
+    static constexpr int GB = (1 << LOGG) * BITS / 8;
+    static constexpr int H = GB == 128 ? 2 : 1;              // 64-byte pieces
+    static constexpr int NW = (GB / 4 > 16 ? 16 : GB / 4) / 4;
+    static constexpr int MI = BITS == 4 ? NW : NW / 2;       // mma per piece
+    uint32_t a[H][NW], b[H][NW];
+    __device__ __forceinline__ void load(uint32_t a_addr) {
 #pragma unroll
-    for (int h = 0; h < (GB == 128 ? 2 : 1); ++h) {
-        uint32_t wa[NW], wb[NW];
-        s_ldw<NW>(a_addr + h * 1024, wa);
-        s_ldw<NW>(a_addr + h * 1024 + 512, wb);
-#pragma unroll
-        for (int i = 0; i < MI; ++i) {
-            uint32_t a0, a1, a2, a3;
-            if constexpr (BITS == 4) {
-                a0 = wa[i] & 0x0F0F0F0Fu; a1 = wb[i] & 0x0F0F0F0Fu;
-                a2 = (wa[i] >> 4) & 0x0F0F0F0Fu; a3 = (wb[i] >> 4) & 0x0F0F0F0Fu;
-            } else {
-                a0 = wa[2 * i]; a1 = wb[2 * i]; a2 = wa[2 * i + 1]; a3 = wb[2 * i + 1];
-            }
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                uint32_t b0, b1;
-                s_ld64(bx[nt] + bofs + (h * MI + i) * 96, b0, b1);
-                if (FIRST && h == 0 && i == 0) mma_u8s8<true>(acc[nt], a0, a1, a2, a3, b0, b1);
-                else mma_u8s8<false>(acc[nt], a0, a1, a2, a3, b0, b1);
-            }
+        for (int h = 0; h < H; ++h) {
+            s_ldw<NW>(a_addr + h * 1024, a[h]);
+            s_ldw<NW>(a_addr + h * 1024 + 512, b[h]);
         }
     }
-}
+    __device__ __forceinline__ void operands(int i, uint32_t (&r)[4]) const {
+        const int h = i / MI, j = i % MI;
+        if constexpr (BITS == 4) {
+            r[0] = a[h][j] & 0x0F0F0F0Fu; r[1] = b[h][j] & 0x0F0F0F0Fu;
+            r[2] = (a[h][j] >> 4) & 0x0F0F0F0Fu; r[3] = (b[h][j] >> 4) & 0x0F0F0F0Fu;
+        } else {
+            r[0] = a[h][2 * j]; r[1] = b[h][2 * j]; r[2] = a[h][2 * j + 1]; r[3] = b[h][2 * j + 1];
+        }
+    }
+};
 
 struct I8Pos { int tile, m, i; };             // a unit: tile, matrix, position in the row
 __device__ __forceinline__ void i8_advance(I8Pos& u, int by, int U, int mats) {
@@ -233,16 +238,16 @@ template <int BITS, int LOGG> struct I8Shape {
     static constexpr int CG = CP * 64 / GB;                  // groups per chunk: 4, 2 or 1
     static constexpr int MB = GU * 2;                        // bytes of a unit's scales in one row: 32 .. 4
     static constexpr int WIN = MB > 16 ? 3 : 2;              // 16-byte pieces of an aligned window around them
-    static constexpr int XG = 96 * NM;                       // digit bytes of one group: [mma][digit][lane t] 8 bytes
-    static constexpr int XU = GU * XG;                       // ... of a unit: 1536 (q4) or 768 (q8)
+    static constexpr int XU = GU * 96 * NM;                  // digit bytes of a unit: 1536 (q4) or 768 (q8)
 };
 
-template <int BITS, int LOGG, int NB, bool PACKETS>
+// VEC: the groups of a row fill whole units, so the scales of a unit are aligned pieces.  (One kernel with a run-time switch: gate and up of
+// 14336 x 4096 13.7 us instead of 13.3.)
+template <int BITS, int LOGG, int NB, bool PACKETS, bool VEC>
 __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
     using S = I8Shape<BITS, LOGG>;
     constexpr int G = S::G, GB = S::GB, NM = S::NM, GU = S::GU, CP = S::CP, CH = S::CH, CG = S::CG, MB = S::MB, WIN = S::WIN;
-    constexpr uint32_t XG = S::XG;
     constexpr int NT = NB <= 2 ? 1 : NB / 2;          // 8-column tiles: one batch row takes 4 columns (3 digits)
 
     const int warp = threadIdx.x >> 5;
@@ -261,7 +266,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
     const int tile_rows = (r_cnt + n_tiles - 1) / n_tiles;
     const int U = p.units, mats = p.mats, B = p.B, Gn = p.Gn;
 
-    if (threadIdx.x < S::XU / 16) *reinterpret_cast<uint4*>(smem + p.off_zero + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < (S::XU + 128) / 16) *reinterpret_cast<uint4*>(smem + p.off_zero + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
     pdl_launch_dependents();
 
     // ---------------- the warp's stream: the chunks of its units, in order ----------------
@@ -291,15 +296,15 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                 const int64_t first = (int64_t)(row0 + m_row) * Gn;
                 const int64_t at = (first + nu.i * GU) * 2;
                 leftM = MB;
-                if (!p.meta_vec) leftM = (int)min((int64_t)(WIN * 16), (first + Gn) * 2 - (at & ~(int64_t)15));
-                srcM = reinterpret_cast<const uint8_t*>(mb) + (p.meta_vec ? at : at & ~(int64_t)15);
+                if (!VEC) leftM = (int)min((int64_t)(WIN * 16), (first + Gn) * 2 - (at & ~(int64_t)15));
+                srcM = reinterpret_cast<const uint8_t*>(mb) + (VEC ? at : at & ~(int64_t)15);
                 if (mb == nullptr) leftM = -1;
             }
         }
     };
     auto issue = [&](int c, uint32_t meta) {           // chunk c of that unit; its scales ride on the first
         if (c == 0 && leftM > 0) {
-            if (p.meta_vec) {
+            if (VEC) {
                 const uint32_t dst = meta + (uint32_t)(t * 8 + g) * MB;
                 if constexpr (MB == 32) { cp16(dst, srcM); cp16(dst + 16, srcM + 16); }
                 else if constexpr (MB == 16) cp16(dst, srcM);
@@ -311,7 +316,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                 for (int q = 0; q < WIN; ++q) cp16_part(dst + q * 16, srcM + (leftM > q * 16 ? q * 16 : 0), (uint32_t)max(0, min(16, leftM - q * 16)));
             }
         } else if (c == 0 && leftM < 0) {
-            const uint32_t stride = p.meta_vec ? MB : WIN * 16;
+            const uint32_t stride = VEC ? MB : WIN * 16;
             for (uint32_t q = 0; q < stride; q += 4) asm volatile("st.shared.u32 [%0], %1;" ::"r"(meta + (uint32_t)(t * 8 + g) * stride + q), "r"(0) : "memory");
         }
 #pragma unroll
@@ -346,8 +351,9 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
     // and gained nothing on rows of 14336.
     const int pieces = U * GU * (G / 8);
     const int total = B * pieces;
+    auto row_of = [&](int it) { return NB == 1 ? 0 : it / pieces; };
     auto load_item = [&](int it, uint32_t (&w)[4]) -> bool {
-        const int b = it / pieces, k = (it - b * pieces) * 8;
+        const int b = row_of(it), k = (it - b * pieces) * 8;
         w[0] = w[1] = w[2] = w[3] = 0u;
         if (k < p.K) i8_load_z<PACKETS>(p, (int64_t)b * p.K + k, xsrc, w);
         return k < p.K;
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
     }
 #pragma unroll 1
     for (int it = threadIdx.x; it < total; it += kI8Threads) {      // whole warps (shuffles below)
-        const int b = it / pieces, pc = it - b * pieces;
+        const int b = row_of(it), pc = it - b * pieces;
         const int k = pc * 8;
         const int64_t idx = (int64_t)b * p.K + k;
         uint32_t w[4];
@@ -401,12 +407,15 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
         const float up = __uint_as_float((uint32_t)(e + 127) << 23);
         uint32_t u[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) u[i] = (uint32_t)(__float2int_rn(v[i] * up) + 0x808080);      // three digits, each + 128
+        for (int i = 0; i < 8; ++i) u[i] = __float_as_uint(fmaf(v[i], up, kI8Magic)) + (0x808080u - kI8MagicBits);      // three digits, each + 128
         const int in = pc & (G / 8 - 1), grp = pc / (G / 8);
         int tt, ii;                                    // lane and mma that meet these 8 values
         if (GB == 128) { tt = (in & 7) >> 1; ii = ((in >> 3) << 1) | (in & 1); }      // two 16-byte pieces per lane
         else { tt = in / NM; ii = in & (NM - 1); }
-        uint8_t* dst = smem + p.off_xd + (size_t)b * p.xstride + (uint32_t)grp * XG + ii * 96 + tt * 8;
+        // digits lie in the order of the mma they enter, two mma to a 16-byte piece: [mma pair][digit][lane tt]; one batch row: even groups
+        // of the unit, then odd ones
+        const int unit = grp / GU, gl = grp & (GU - 1), m = (NB == 1 ? gl >> 1 : gl) * NM + ii;
+        uint8_t* dst = smem + p.off_xd + (size_t)b * p.xstride + (uint32_t)unit * S::XU + (NB == 1 ? (gl & 1) * (S::XU / 2) : 0) + (m >> 1) * 192 + tt * 16 + (m & 1) * 8;
         uint32_t d[3][2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -419,11 +428,14 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
             d[0][h] = prmt(prmt(a, b2, 0x0062), prmt(c, d2, 0x0062), 0x5410) ^ 0x80808080u;
         }
 #pragma unroll
-        for (int s = 0; s < 3; ++s) *reinterpret_cast<uint2*>(dst + s * 32) = make_uint2(d[s][0], d[s][1]);
+        for (int s = 0; s < 3; ++s) *reinterpret_cast<uint2*>(dst + s * 64) = make_uint2(d[s][0], d[s][1]);
         if (in == 0) {
-            const float down = mx < INFINITY ? __uint_as_float((uint32_t)(127 + 8 - e) << 23) : NAN;     // 2^(8 - e)
-            // even lanes own the two high digits (c2 2^8 + c1), odd lanes the low one and the zero-point term
-            reinterpret_cast<float4*>(smem + p.off_cst)[b * U * GU + grp] = make_float4(down, 0.0f, down * 1.52587890625e-05f, X);
+            // 2^(16 - e - shift), the weight of the high digit (e is at most 120, so all three weights are exact).  Even lanes own the two high
+            // digits, odd lanes the low one and the zero-point term: [lane t & 1, one batch row: and parity of the group][step]
+            const float high = mx < INFINITY ? __uint_as_float((uint32_t)(127 + 16 - kI8Shift - e) << 23) : NAN;
+            float2* cst = reinterpret_cast<float2*>(smem + p.off_cst + (size_t)b * p.cstride) + unit * (2 * GU) + (NB == 1 ? (gl & 1) * GU + (gl >> 1) : gl);
+            cst[0] = make_float2(high, 0.0f);
+            cst[NB == 1 ? GU / 2 : GU] = make_float2(high * 0x1p-16f, X * __uint_as_float((uint32_t)(127 - kI8Shift) << 23));
         }
     }
     __syncthreads();
@@ -431,16 +443,21 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
     // ---------------- per-lane constants of the consumer ----------------
     const int col_b = g >> 2;                          // batch row of this lane's B column inside a tile; one batch row: parity of the group
     const bool digit = (g & 3) < 3;
-    const uint32_t zaddr = smem0 + p.off_zero + t * 8;
-    const uint32_t xlane = smem0 + p.off_xd + (uint32_t)(g & 3) * 32 + t * 8;
-    const uint32_t cbase = smem0 + p.off_cst + (uint32_t)(t & 1) * 8 + (NB == 1 ? (t >> 1) * 16 : 0);
+    const uint32_t zaddr = smem0 + p.off_zero + 64 + t * 16;             // + 64: other banks than the third digit, which is read together with it
+    const uint32_t xlane = smem0 + p.off_xd + (uint32_t)(g & 3) * 64 + t * 16;
+    constexpr int FL = NB == 1 ? GU / 2 : GU;          // affine steps of a unit: a group, or with one batch row two neighbouring ones
+    constexpr int CV = FL < 2 || NB == 4 ? 1 : 2;      // steps whose constants are read at once (four rows: no registers to spare)
+    const uint32_t cbase = smem0 + p.off_cst + (uint32_t)(NB == 1 ? (t >> 1) * 2 + (t & 1) : t & 1) * (FL * 8);
+    const float k_mid = (t & 1) ? 0.0f : 0x1p-8f;                        // weight of the second column by that of the first
+    const float k_off = (t & 1) ? -kI8Magic : -kI8Magic * 1.00390625f;   // what the magic number adds to both, negative
+    const uint32_t sel_par = t >> 1 ? 0x4432u : 0x4410u;                 // one batch row: the half of a pair of scales that is this lane's
     constexpr int LPP = GB >= 64 ? 16 : GB / 4;        // lane pitch in a row
     const uint32_t a_lane = (((uint32_t)(t * LPP) & ~15u) ^ sw) + ((uint32_t)(t * LPP) & 15u);
     uint32_t a_grp[CG];                                // this lane's bytes of the chunk's groups (first chunk)
 #pragma unroll
     for (int q = 0; q < CG; ++q) a_grp[q] = ring + (uint32_t)g * 64 + (a_lane ^ (uint32_t)(q * GB));
-    const uint32_t m_stride = p.meta_vec ? MB : WIN * 16;
-    const uint32_t m_lane = (uint32_t)g * m_stride + (NB == 1 ? (t >> 1) * 2 : 0);
+    const uint32_t m_stride = VEC ? MB : WIN * 16;
+    const uint32_t m_lane = (uint32_t)g * m_stride;
 
     I8Pos cu = nu;
     uint32_t cmeta = 0;                                // scale buffer of the unit being consumed
@@ -450,42 +467,72 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
 #pragma unroll 1
         while (cu.tile < t1) {
             uint32_t m_s0 = meta0 + cmeta + m_lane, m_s1 = m_s0 + 8 * m_stride;
-            if (!p.meta_vec) {
+            if (!VEC) {
                 const uint32_t e = (uint32_t)(r_lo + cu.tile * tile_rows + g) * (uint32_t)Gn + cu.i * GU;      // low bits are enough
                 m_s0 += (e * 2) & 15u;
                 m_s1 += ((e + 8u * Gn) * 2) & 15u;
             }
             const uint32_t m_z0 = m_s0 + 16 * m_stride, m_z1 = m_s1 + 16 * m_stride;
             float y[NT][2];
-            // B operand addresses: a lane without a digit (or with the other group's column) reads zeros
-            uint32_t xb[NT], xo[NT], cc[NT];
+            // B operand addresses: a lane without a digit reads zeros
+            uint32_t xb[NT], cc[NT];
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 y[nt][0] = y[nt][1] = 0.0f;
                 const int b = NB == 1 ? 0 : 2 * nt + col_b;
-                const uint32_t a = xlane + (uint32_t)b * p.xstride + (uint32_t)cu.i * S::XU;
-                xb[nt] = digit && (NB == 1 ? col_b == 0 : b < B) ? a : zaddr;
-                xo[nt] = digit && col_b == 1 ? a : zaddr;
+                const uint32_t a = xlane + (uint32_t)b * p.xstride + (uint32_t)cu.i * S::XU + (NB == 1 ? (uint32_t)col_b * (S::XU / 2) : 0u);
+                xb[nt] = digit && b < B ? a : zaddr;
                 const int cb = NB == 1 ? 0 : min(2 * nt + (t >> 1), B - 1);
-                cc[nt] = cbase + (uint32_t)(cb * U + cu.i) * (GU * 16);
+                cc[nt] = cbase + (uint32_t)cb * p.cstride + (uint32_t)cu.i * (GU * 16);
             }
 
             i8_advance(nu, kI8Warps, U, mats);
             locate();
-            int acc[NT][4];
-            // affine step of group `gl` of the unit (one batch row: of groups gl and gl + 1 at once)
-            auto flush = [&](int gl) {
-                const float s0 = s_ldh(m_s0 + gl * 2), s1 = s_ldh(m_s1 + gl * 2), z0 = s_ldh(m_z0 + gl * 2), z1 = s_ldh(m_z1 + gl * 2);
+            // scales (and zero points) of rows g and g + 8, eight groups at a time, two to a register
+            constexpr int SG = GU < 8 ? GU : 8;
+            uint32_t sw0[SG / 2], sw1[SG / 2], zw0[SG / 2], zw1[SG / 2];
+            auto scales = [&](int gl) {
+                if (!VEC) return;
+                s_ldw<SG / 2>(m_s0 + gl * 2, sw0);
+                s_ldw<SG / 2>(m_s1 + gl * 2, sw1);
+                s_ldw<SG / 2>(m_z0 + gl * 2, zw0);
+                s_ldw<SG / 2>(m_z1 + gl * 2, zw1);
+            };
+            auto scale_of = [&](const uint32_t (&w)[SG / 2], uint32_t row, int f) -> float {      // of affine step f
+                if (!VEC) {                     // rows of scales that start anywhere: one at a time
+                    const uint32_t h = s_ldu16(row + (NB == 1 ? f * 4 + (t >> 1) * 2 : f * 2));
+                    return __low2float(*reinterpret_cast<const __half2*>(&h));
+                }
+                if constexpr (NB == 1) {
+                    const uint32_t h = prmt(w[f % (SG / 2)], 0u, sel_par);
+                    return __low2float(*reinterpret_cast<const __half2*>(&h));
+                } else {
+                    const __half2 h = *reinterpret_cast<const __half2*>(&w[f % SG / 2]);
+                    return f & 1 ? __high2float(h) : __low2float(h);
+                }
+            };
+            constexpr int AC = NB == 1 ? 2 : NT;               // one batch row: sums of the even and of the odd group
+            int acc[AC][4];
+            uint32_t cw[NT][2 * CV];
+            // affine step f:  y += s * (digits - zero * X)
+            auto flush = [&](int f) {
+                const float s0 = scale_of(sw0, m_s0, f), s1 = scale_of(sw1, m_s1, f), z0 = scale_of(zw0, m_z0, f), z1 = scale_of(zw1, m_z1, f);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    uint32_t wq, xq;
-                    s_ld64(cc[nt] + gl * 16, wq, xq);
-                    const float wf = __uint_as_float(wq), xf = __uint_as_float(xq);
-                    const float f0 = (float)((acc[nt][0] << 8) + acc[nt][1]) * wf, f1 = (float)((acc[nt][2] << 8) + acc[nt][3]) * wf;
+                    if (f % CV == 0) s_ldw<2 * CV>(cc[nt] + f * 8, cw[nt]);
+                    const float w0 = __uint_as_float(cw[nt][f % CV * 2]), xf = __uint_as_float(cw[nt][f % CV * 2 + 1]), w1 = w0 * k_mid, off = w0 * k_off;
+                    float c[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) c[e] = __int_as_float(NB == 1 ? (t >> 1 ? acc[AC - 1][e] : acc[0][e]) : acc[nt % AC][e]);
+                    const float f0 = fmaf(c[1], w1, fmaf(c[0], w0, off)), f1 = fmaf(c[3], w1, fmaf(c[2], w0, off));
                     y[nt][0] = fmaf(s0, fmaf(-z0, xf, f0), y[nt][0]);
                     y[nt][1] = fmaf(s1, fmaf(-z1, xf, f1), y[nt][1]);
                 }
             };
+            // Digits of two mma per load.  One batch row: the lanes of columns 0-3 hold the even group's, those of columns 4-7 the odd group's,
+            // and both groups' codes meet the same operand; each lane then takes the sums that are its own.
+            constexpr int BP = NM < 2 ? 1 : NM / 2;            // 16-byte pieces of a group's digits
+            uint32_t bq[NT][BP][4];
 #pragma unroll
             for (int c = 0; c < CH; ++c) {
                 asm volatile("cp.async.wait_group %0;" ::"n"(CH - 1) : "memory");
@@ -493,15 +540,29 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                 // groups past the end of the row have zero digits: whatever their codes are, they add nothing
 #pragma unroll
                 for (int q = 0; q < CG; ++q) {
-                    const int gl = c * CG + q;
-                    if constexpr (NB == 1) {
-                        if (gl % 2 == 0) i8_group_mma<BITS, LOGG, NT, true>(acc, a_grp[q] + c * CP * 1024, xb, gl * XG);
-                        else i8_group_mma<BITS, LOGG, NT, false>(acc, a_grp[q] + c * CP * 1024, xo, gl * XG);
-                        if (gl % 2 == 1) flush(gl - 1);
-                    } else {
-                        i8_group_mma<BITS, LOGG, NT, true>(acc, a_grp[q] + c * CP * 1024, xb, gl * XG);
-                        flush(gl);
+                    const int gl = c * CG + q, f = NB == 1 ? gl >> 1 : gl;
+                    if (gl % SG == 0) scales(gl);
+                    if ((NB != 1 || gl % 2 == 0) && (f * NM) % 2 == 0) {
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                            for (int i = 0; i < BP; ++i) s_ldw<4>(xb[nt] + (f * NM / 2 + i) * 192, bq[nt][i]);
                     }
+                    I8Words<BITS, LOGG> words;
+                    words.load(a_grp[q] + c * CP * 1024);
+#pragma unroll
+                    for (int i = 0; i < NM; ++i) {
+                        uint32_t r[4];
+                        words.operands(i, r);
+                        const int piece = i / 2, h = (f * NM + i) % 2 * 2;
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) {
+                            int (&d)[4] = acc[NB == 1 ? gl % 2 : nt % AC];
+                            if (i == 0) mma_u8s8<true>(d, r[0], r[1], r[2], r[3], bq[nt][piece][h], bq[nt][piece][h + 1]);
+                            else mma_u8s8<false>(d, r[0], r[1], r[2], r[3], bq[nt][piece][h], bq[nt][piece][h + 1]);
+                        }
+                    }
+                    if (NB != 1 || gl % 2 == 1) flush(f);
                 }
                 __syncwarp();
                 issue(c, meta0 + (cmeta ^ p.meta_slot));
@@ -512,7 +573,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    float v = y[nt][h];
+                    float v = y[nt][h] * (float)(1 << kI8Shift);
                     v += __shfl_xor_sync(0xffffffffu, v, 1);
                     if (NB == 1) v += __shfl_xor_sync(0xffffffffu, v, 2);
                     if ((NB == 1 ? t == 0 : (t & 1) == 0)) dst[(g + 8 * h) * NB + (NB == 1 ? 0 : 2 * nt + (t >> 1))] = v;
@@ -525,13 +586,13 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
         const float fmax_act = p.act_dtype == B200Q_F16 ? 65504.0f : 3.3895313892515355e38f;
         const int rb0 = t0 * tile_rows, n_rows = min(r_cnt, t1 * tile_rows) - rb0;
         for (int it = threadIdx.x; it < n_rows * B; it += kI8Threads) {
-            const int b = it / n_rows, rr = it - b * n_rows;
+            const int b = NB == 1 ? 0 : it / n_rows, rr = it - b * n_rows;
             const int tl = rr / tile_rows, r = rr - tl * tile_rows;
             const float* src = part + (size_t)tl * mats * U * (16 * NB) + r * NB + b;
             float val[2] = {0.0f, 0.0f};
             for (int m = 0; m < mats; ++m) {
                 float sum = 0.0f;
-#pragma unroll 4
+#pragma unroll 8
                 for (int i = 0; i < U; ++i) sum += src[(m * U + i) * (16 * NB)];
                 val[m] = i8_round_act(fminf(fmaxf(sum, -fmax_act), fmax_act), p.act_dtype);
             }
@@ -591,8 +652,8 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
     p.eps = q.eps; p.B = q.B; p.N = q.N; p.K = q.K; p.Gn = q.Gn; p.act_dtype = q.act_dtype; p.norm_w_dtype = q.norm_w_dtype;
     p.row_bytes = q.row_bytes; p.tp_out = q.tp_out; p.tp_in = q.tp_in;
     p.units = (p.row_bytes + kI8UnitBytes - 1) / kI8UnitBytes;
-    p.meta_vec = p.Gn % S::GU == 0;
-    p.meta_slot = 32u * (p.meta_vec ? S::MB : S::WIN * 16);
+    const bool vec = p.Gn % S::GU == 0;
+    p.meta_slot = 32u * (vec ? S::MB : S::WIN * 16);
     // a CTA per SM, fewer only when a CTA would own less than four rows
     const int grid = std::max(1, std::min(sm_count(), (p.N + 3) / 4));
     p.rows_lo = p.N / grid;
@@ -600,29 +661,40 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
     const int r_max = p.rows_lo + (p.rem ? 1 : 0);
     const int tile_bytes = p.mats * p.units * 16 * NB * 4;
     p.batch = std::min((r_max + 15) / 16, std::max(1, 24 * 1024 / tile_bytes));
-    p.xstride = (uint32_t)p.units * S::GU * S::XG + 32;      // + 32: the two batch rows of a B operand fall into different banks
-    uint32_t off = i8_align((uint32_t)q.B * p.units * S::GU * (S::G / 8) / 32 * 4, 128);
-    p.off_zero = off;  off += S::XU;
-    p.off_xd = off;    off += i8_align((uint32_t)q.B * p.xstride, 128);
-    p.off_cst = off;   off += (uint32_t)q.B * p.units * S::GU * 16;
-    p.off_res = off;   off += p.residual != nullptr ? i8_align((uint32_t)std::min(r_max * q.B, kI8MaxRes) * 2, 128) : 0;
-    off = i8_align(off, 128);
-    p.off_part = off;  off += i8_align((uint32_t)(p.batch * tile_bytes), 128);
-    p.off_meta = off;  off += kI8Warps * 2 * p.meta_slot;
-    off = i8_align(off, 1024);
-    p.off_ring = off;  off = std::max<uint32_t>(off + kI8Warps * 4096, kI8OnePerSm);
+    p.xstride = (uint32_t)p.units * S::XU;
+    p.cstride = (uint32_t)p.units * S::GU * 16 + (q.B > 1 ? 32 : 0);      // + 32: two batch rows are read together, from different banks
+    auto plan = [&]() -> uint32_t {
+        uint32_t off = i8_align((uint32_t)q.B * p.units * S::GU * (S::G / 8) / 32 * 4, 128);
+        p.off_zero = off;  off += S::XU + 128;
+        p.off_xd = off;    off += i8_align((uint32_t)q.B * p.xstride, 128);
+        p.off_cst = off;   off += (uint32_t)q.B * p.cstride;
+        p.off_res = off;   off += p.residual != nullptr ? i8_align((uint32_t)std::min(r_max * q.B, kI8MaxRes) * 2, 128) : 0;
+        off = i8_align(off, 128);
+        p.off_part = off;  off += i8_align((uint32_t)(p.batch * tile_bytes), 128);
+        p.off_meta = off;  off += kI8Warps * 2 * p.meta_slot;
+        off = i8_align(off, 1024);
+        p.off_ring = off;
+        return std::max<uint32_t>(off + kI8Warps * 4096, kI8OnePerSm);
+    };
+    uint32_t off = plan();
+    while (off > (uint32_t)max_smem_optin() && p.batch > 1) {      // long rows: fewer tiles whose sums lie in shared memory together
+        --p.batch;
+        off = plan();
+    }
     if (off > (uint32_t)max_smem_optin()) return B200Q_ERR_UNSUPPORTED;
 
     const bool packets = p.tp_in.world > 0 && p.tp_in.packets;
-    auto kernel = qgemv_i8_kernel<BITS, LOGG, NB, false>;
-    if (packets) kernel = qgemv_i8_kernel<BITS, LOGG, NB, true>;
-    static bool configured[2][64] = {};   // per instantiation and device; a race only repeats the call
+    using KernelFn = void (*)(I8Params);
+    static const KernelFn kernels[2][2] = {{qgemv_i8_kernel<BITS, LOGG, NB, false, false>, qgemv_i8_kernel<BITS, LOGG, NB, false, true>},
+                                           {qgemv_i8_kernel<BITS, LOGG, NB, true, false>, qgemv_i8_kernel<BITS, LOGG, NB, true, true>}};
+    KernelFn kernel = kernels[packets][vec];
+    static bool configured[4][64] = {};   // per instantiation and device; a race only repeats the call
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!configured[packets][dev & 63]) {
+    if (!configured[packets * 2 + vec][dev & 63]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()) != cudaSuccess)
             return B200Q_ERR_LAUNCH;
-        configured[packets][dev & 63] = true;
+        configured[packets * 2 + vec][dev & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);

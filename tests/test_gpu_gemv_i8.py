@@ -39,6 +39,33 @@ def test_outliers_and_empty_groups(cuda):
     assert rel_l2(got[:1], want[:1]) <= 1e-3 and rel_l2(got[1:], want[1:]) <= 6e-3      # the second row's results are subnormal halves
 
 
+@pytest.mark.parametrize("bits,G", [(8, 128), (8, 32), (4, 128), (4, 64)])
+@pytest.mark.parametrize("rows", [1, 2, 4])
+def test_largest_digit_sums(cuda, bits, G, rows):
+    """Codes and activations at their limits of one sign: the digit sums of a group come within 0.4 % of the range that the integers added
+    to a float's bits have.  fp32 sums of equal terms: error below 2^-11 of the result from its rounding to fp16."""
+    N, K = 50, 4 * G + 32 * (G == 32)
+    codes = torch.full((N, K * bits // 8), 255, dtype=torch.uint8)
+    scales = torch.full((N, K // G), 2.0 ** -12, dtype=torch.float16)
+    zeros = torch.full((N, K // G), 3.0, dtype=torch.float16)
+    for value in (-1.0, 0.99951171875):
+        x = torch.full((rows, K), value, dtype=torch.float16)
+        want = torch.full((rows, N), K * value * (2 ** bits - 1 - 3) * 2.0 ** -12, dtype=torch.float64)
+        got = quant_ops.matvec_rows(bits, *to_dev(cuda, x, codes, scales, zeros), G)
+        assert rel_l2(got, want) <= 2.0 ** -11
+
+
+@pytest.mark.parametrize("power", [120, 100, -60, -100])
+def test_bf16_rows_near_both_ends_of_the_range(cuda, power):
+    """bf16 rows times a power of two give the same results times that power, bit for bit, as long as these are in range."""
+    w, s, z = synth.quantized_weight(70, 256, 4, 64, seed=8)
+    x = synth.activations((2, 256), 9, "cpu", torch.bfloat16)
+    s = (s.float() * 2.0 ** -6).to(torch.float16)
+    near = quant_ops.matvec_rows(4, *to_dev(cuda, x, w, s, z), 64)
+    far = quant_ops.matvec_rows(4, *to_dev(cuda, (x.float() * 2.0 ** power).to(torch.bfloat16), w, s, z), 64)
+    assert torch.equal(far.float() * 2.0 ** -power, near.float())
+
+
 @pytest.mark.parametrize("rows", [1, 2, 4])
 @pytest.mark.parametrize("lo,hi", [(0, 96), (96, 333), (5, 6)])
 def test_row_shards_reproduce_the_unsharded_rows(cuda, rows, lo, hi):
