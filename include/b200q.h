@@ -66,8 +66,8 @@ int b200q_device_status(int reset, void* stream);
  *                        the tcgen05 kernel then splits K, and the attention picks its kernel, as the unsharded call
  *                        would, which keeps a shard's rows bit-identical to the unsharded result
  *   "attn.ctas_per_sm", "attn.min_pages"                grid sizing of the split-KV attention kernel
- *   "attn.cluster"       1 = the one-kernel cluster form of the attention whenever it applies, -1 = never, 0 = small batches
- *   "attn.cluster_size"  CTAs per cluster of that form: 4, 8 (default) or 16
+ *   "attn.cluster"       1 = the one-kernel cluster form of the attention whenever it applies, -1 = never, 0 = small batches and short ones
+ *   "attn.cluster_size"  CTAs per cluster of that form: 1, 2, 4, 8 or 16 (default: by heads and length)
  *   "attn.force_simple"  1 = always the one-warp-per-head attention kernel
  *   "peer.spin_limit", "tp.spin_limit"   flag probes after which b200q_peer_allgather / the wait of an exchange fused
  *                        into a kernel gives up and records event 5 (default 2^22; tests shorten it)
@@ -298,6 +298,9 @@ int b200q_rope_append_paged_gqa_decode(const void* qkv, const float* cos_table, 
  * cluster kernel applies (with or without the append), else 2 (split-KV + merge) plus 1 for the append.  For callers
  * that report launch counts; no counterpart in the reference. */
 int b200q_attention_stage_launches(int B, int Hkv, int with_append);
+/* The same for a block table of max_blocks pages per sequence, given a workspace: with short tables the cluster kernel takes more
+ * sequences.  (The function above answers for tables of any length, and tells who needs no workspace.) */
+int b200q_attention_launches(int B, int Hkv, int max_blocks, int with_append);
 
 /* Symmetric group-wise quantisation of KV rows with the rule of the reference cache
  * (_quantize_group_symmetric_8 / _4, ops/paged_quantized_kv_ops.py:146-153, 168-175, as applied by quantize_kv_pages,

@@ -112,7 +112,7 @@ int paged_fp16_gqa_decode_checked_impl(const void* q, const void* k_pages, const
                                        int Hkv, int D, int page_size, int64_t num_pages, int max_blocks, float scale, int dtype,
                                        int32_t* verdict, cudaStream_t stream);
 size_t paged_gqa_workspace_bytes_impl(int B, int Hq, int Hkv, int D);
-int attention_stage_launches_impl(int B, int Hkv, int with_append);
+int attention_stage_launches_impl(int B, int Hkv, int max_blocks, int with_append);
 size_t paged_gqa_static_scratch_bytes_impl();
 int paged_gqa_decode_static_impl(int bits, const void* q, const uint8_t* k_codes, const uint8_t* v_codes,
                                  const void* k_scales, const void* v_scales, const int32_t* block_table,
@@ -559,7 +559,10 @@ int b200q_block_table_lookup(const int32_t* block_table, const int32_t* position
     return finish_launch();
 }
 
-int b200q_attention_stage_launches(int B, int Hkv, int with_append) { return attention_stage_launches_impl(B, Hkv, with_append); }
+int b200q_attention_stage_launches(int B, int Hkv, int with_append) { return attention_stage_launches_impl(B, Hkv, INT32_MAX / 16, with_append); }
+int b200q_attention_launches(int B, int Hkv, int max_blocks, int with_append) {
+    return max_blocks <= 0 ? 0 : attention_stage_launches_impl(B, Hkv, max_blocks, with_append);
+}
 
 size_t b200q_paged_gqa_workspace_bytes(int B, int Hq, int Hkv, int D) { return paged_gqa_workspace_bytes_impl(B, Hq, Hkv, D); }
 

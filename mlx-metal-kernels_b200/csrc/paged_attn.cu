@@ -460,6 +460,7 @@ struct alignas(64) ClusterParams {
     ClusterAttnParams a;
 };
 constexpr int kMaxClusterRing = 8;
+constexpr int kClusterWarps = 16, kClusterThreads = kClusterWarps * 32;
 
 __device__ __forceinline__ uint32_t cluster_rank_x() {
     uint32_t r;
@@ -474,7 +475,7 @@ __device__ __forceinline__ uint32_t cluster_rank_x() {
 // token goes to waits for its append.
 // SC8: scales aligned to 8 bytes only (a template parameter: asked at run time it cost the aligned form 0.3 of 9.9 us).
 template <int BITS, int LOGG, bool WIDE, bool SC8>
-__global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterParams cp) {
+__global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterParams cp) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const ClusterAttnParams& p = cp.a;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -489,6 +490,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     const int b = blockIdx.z;
     const int group = p.group;
     const int S = p.S;
+    const int n_warps = (int)(blockDim.x >> 5);
     __half* qs = reinterpret_cast<__half*>(smem + p.off_q);              // [group][D] rotated query rows
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.off_bars) + warp * NS;      // this warp's ring
     uint8_t* my_ring = smem + (size_t)warp * NS * p.slot_bytes;
@@ -510,7 +512,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     const int n_pages = (L + p.P - 1) / p.P;
     const int ppc = (n_pages + S - 1) / S;                               // pages per CTA
     const int c_lo = min(n_pages, (int)rank * ppc), c_hi = min(n_pages, c_lo + ppc);
-    const int ppw = (c_hi - c_lo + kAttnWarps - 1) / kAttnWarps;         // pages per warp
+    const int ppw = (c_hi - c_lo + n_warps - 1) / n_warps;         // pages per warp
     const int lo = min(c_hi, c_lo + warp * ppw), hi = min(c_hi, lo + ppw);
 
     const int n_my = hi - lo;
@@ -690,10 +692,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
         return accv;
     };
     const uint32_t cpart_u = smem_u32(cpart);
-    for (int idx = threadIdx.x; idx < group * D; idx += kAttnThreads) {
+    for (int idx = threadIdx.x; idx < group * D; idx += blockDim.x) {
         const int head = idx / D, d = idx - head * D;
         float m_tot, l_tot;
-        const float v = merge(wpart, kAttnWarps, wstride, head, d, m_tot, l_tot);
+        const float v = merge(wpart, n_warps, wstride, head, d, m_tot, l_tot);
         // slot `rank` of the first CTA's table (its own slot for the first CTA itself)
         const uint32_t base = cpart_u + (uint32_t)((rank * group + head) * PW) * 4u;
         auto put = [&](uint32_t off, float val) {
@@ -707,7 +709,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attn_cluster_kernel(con
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (rank == 0) {
-        for (int idx = threadIdx.x; idx < group * D; idx += kAttnThreads) {
+        for (int idx = threadIdx.x; idx < group * D; idx += blockDim.x) {
             const int head = idx / D, d = idx - head * D;
             float m_tot, l_tot;
             const float v = merge(cpart, S, group * PW, head, d, m_tot, l_tot);
@@ -933,25 +935,41 @@ inline bool heads_ok(int Hkv) { return Hkv <= kAttnWarps || Hkv % kAttnWarps == 
 
 // ---- cluster kernel: host side ----
 struct ClusterChoice { int size; bool preferred; };      // size 0: not possible
-ClusterChoice cluster_choice(int B, int Hkv) {
-    const int mode = tuning_get("attn.cluster");      // 1: whenever possible, -1: never, 0: small batches
+// fused: the launch also stands for the append (three launches against one).  split: the split-KV kernels could take the call; without them
+// (no workspace) the rule is the one for tables of any length, so a call is not refused or served by its length.
+ClusterChoice cluster_choice(int B, int Hkv, int max_blocks, bool fused, bool split) {
+    const int mode = tuning_get("attn.cluster");      // 1: whenever possible, -1: never, 0: by the rule below
     if (mode < 0 || (mode > 0 && B * Hkv > 65535)) return {0, false};
     // the choice follows the kv heads of the UNSHARDED cache ("ts.tp_world" equal head shards), so that a
     // tensor-parallel rank runs the same kernel, and the same summation order, as the unsharded call
-    const int64_t ctas = (int64_t)B * Hkv * std::max(1, tuning_get("ts.tp_world")) * 8;
-    // Preferred while the clusters fill at most three quarters of the SMs; beyond that the split-KV kernel, which uses all of them and
-    // fetches a page once for all heads, is the faster one (layer of the decode stack, 8 kv heads, context 4096: one
-    // sequence 54.6 against 58.0 us, two 73.5 against 70.0, three 88.0 against 84.0, four 103 against 91).  Up to two waves of
-    // clusters stay possible for callers without a workspace.
-    if (mode == 0 && ctas > 2 * sm_count()) return {0, false};
-    const bool preferred = mode > 0 || ctas * 4 <= 3 * sm_count();
-    // 8 CTAs per cluster: the opt-in size 16 is slower at every length (placing one cluster per GPC costs more than the shorter page walk
-    // saves) and 4 from some length on (one sequence of q8, 8 kv heads, cold calls by events, sizes 4 / 8 / 16: 1024 tokens 14.3 /
-    // 12.3 / 18.4 us, 4096 18.4 / 16.4 / 20.5, 8192 26.6 / 20.5 / 24.6)
-    int size = 8;
+    const int64_t heads = (int64_t)B * Hkv * std::max(1, tuning_get("ts.tp_world"));
     const int forced = tuning_get("attn.cluster_size");
-    if (forced == 8 || forced == 16 || forced == 4) size = forced;
-    return {size, preferred};
+    if (forced == 1 || forced == 2 || forced == 4 || forced == 8 || forced == 16) return {mode == 0 && heads * forced > 2 * sm_count() ? 0 : forced, mode > 0 || heads * forced * 4 <= 3 * sm_count()};
+    // Eight CTAs per cluster while the clusters fill at most three quarters of the SMs, whatever the length (the opt-in size 16 is slower at
+    // every length: one sequence of q8, 8 kv heads, sizes 4 / 8 / 16: 1024 tokens 14.3 / 12.3 / 18.4 us, 8192 26.6 / 20.5 / 24.6).
+    if (mode > 0 || heads * 8 * 4 <= 3 * sm_count()) return {8, true};
+    // More heads: as many CTAs per cluster as leave all clusters resident at once, if a warp's walk is short.  A page costs a warp about
+    // one microsecond (it walks alone), the launch 5 us; the split-KV kernel balances ragged batches over all SMs, but with its partial
+    // results and the merge launch takes 9 to 17 us for the shortest ones.  The block table's capacity bounds the walk (the lengths
+    // live on the device).  Split-KV / cluster, us, q4, 8 kv heads, equal lengths and ragged ones down to an eighth: 2 sequences of 2048
+    // tokens 11.1 / 8.2 and 9.1 / 8.1 (of 4096 in q8 13.0 / 12.1 and 11.1 / 11.5: not taken); 7 of 1024 15.7 / 8.2 and 14.4 / 8.0, of 3072
+    // 20.2 / 15.6 and 16.5 / 14.6; 16 of 128 10.5 / 5.8, of 1024 15.1 / 12.6 and 13.4 / 11.1.  Fewer than 8 kv heads cost the split-KV
+    // kernel more: 2 heads, 16 sequences of 4096 tokens 18.7 / 13.1 and 14.5 / 11.4 (of 8192, 7 sequences, 19.3 / 17.8 and 15.4 / 16.8).  With
+    // the append in the same launch the cluster wins 1 to 3 us more (a layer of 2 sequences of 4000 tokens 65.2 / 63.8, 8 of 3000
+    // 91.4 / 86.8, 16 of 1000 89.5 / 87.9).
+    const int kv_full = Hkv * std::max(1, tuning_get("ts.tp_world"));
+    for (int size = 4; split && size >= 1; size /= 2) {
+        if (heads * size * 8 > 7 * (int64_t)sm_count()) continue;
+        const int walk = (max_blocks + size * kClusterWarps - 1) / (size * kClusterWarps);
+        int longest = 4;
+        if (size == 4 && heads < 24) longest = kv_full >= kAttnWarps ? 2 : 3;
+        if (size == 4 && kv_full < 4) longest = 5;
+        if (size == 2) longest = (int)heads / 10;
+        if (walk <= longest + (fused ? 2 : 0)) return {size, true};
+        break;
+    }
+    // up to two waves of clusters stay possible for callers without a workspace
+    return {heads * 8 <= 2 * sm_count() ? 8 : 0, false};
 }
 
 // Byte tensor [heads][tokens][row] of a page pool whose token rows are `pitch` bytes apart; box = heads of a CTA x 16 tokens x row.
@@ -978,15 +996,20 @@ bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtens
 }
 
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
+    // Sixteen warps where eight would have more than a page each: a page costs a warp about a microsecond, the merge of eight more partial
+    // results 0.2 (one sequence, one page a warp: q8 5.4 us with eight, 5.7 with sixteen; two sequences of 2048 tokens 9.2 and 8.5).
+    int warps = p.max_blocks > p.S * 8 ? kClusterWarps : 8;
     const bool g32 = p.G == 32, wide = p.group > 4, sc8 = ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     p.hs = std::min(p.Hkv, kAttnWarps);
     p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024);
     // shared memory: [1 KB alignment] rings, barriers, query rows, the CTAs' partials
     const uint32_t q_bytes = align_up_u32((uint32_t)p.group * 128 * 2, 128), c_bytes = align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
     const uint32_t cap = (uint32_t)max_smem_optin(), fixed = 1024 + 128 * 8 + q_bytes + c_bytes;
-    p.stages = (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (kAttnWarps * p.slot_bytes));
+    auto depth = [&]() { return (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (warps * p.slot_bytes)); };
+    if (depth() < 2) warps = 8;
+    p.stages = depth();
     if (p.stages < 2) return B200Q_ERR_UNSUPPORTED;
-    p.off_bars = kAttnWarps * p.stages * p.slot_bytes;
+    p.off_bars = warps * p.stages * p.slot_bytes;
     p.off_q = p.off_bars + 128 * 8;
     p.off_cpart = p.off_q + q_bytes;
     const uint32_t off = 1024 + p.off_cpart + c_bytes;
@@ -1031,7 +1054,7 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     ++na;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.S, p.Hkv, p.B);
-    cfg.blockDim = dim3(kAttnThreads);
+    cfg.blockDim = dim3(warps * 32);
     cfg.dynamicSmemBytes = off;
     cfg.stream = stream;
     cfg.attrs = attr;
@@ -1132,9 +1155,9 @@ int launch_split_attention(AttnParams& p, int max_ranges, cudaStream_t stream) {
 
 }  // namespace
 
-int attention_stage_launches_impl(int B, int Hkv, int with_append) {
+int attention_stage_launches_impl(int B, int Hkv, int max_blocks, int with_append) {
     if (B <= 0 || Hkv <= 0) return 0;
-    if (B <= 65535 && cluster_choice(B, Hkv).preferred) return 1;
+    if (B <= 65535 && cluster_choice(B, Hkv, max_blocks, with_append != 0, true).preferred) return 1;
     return 2 + (with_append ? 1 : 0);
 }
 
@@ -1193,7 +1216,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     if (!fast_ok) return simple();
     // small batches: one cluster per (sequence, kv head), merged on chip - no workspace, no second launch
     const int ranges = split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, q_dtype);
-    const ClusterChoice choice = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv) : ClusterChoice{0, false};
+    const ClusterChoice choice = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv, max_blocks, false, ranges > 0) : ClusterChoice{0, false};
     const int cluster = choice.preferred || ranges == 0 ? choice.size : 0;
     if (cluster > 0) {
         ClusterAttnParams c = {};
@@ -1273,8 +1296,8 @@ int rope_append_attention_impl(const void* qkv, const float* cos_table, const fl
                          group <= 8 && heads_ok(Hkv) && page_size == 16 && B <= 65535 && ((uintptr_t)qkv % 16 == 0) &&
                          ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) && ((uintptr_t)k_scales % 8 == 0) &&
                          ((uintptr_t)v_scales % 8 == 0);
-    const ClusterChoice choice = fast_ok ? cluster_choice(B, Hkv) : ClusterChoice{0, false};
     const bool two_stages = q_scratch != nullptr && split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, B200Q_F16) > 0;
+    const ClusterChoice choice = fast_ok ? cluster_choice(B, Hkv, max_blocks, true, two_stages) : ClusterChoice{0, false};
     const int cluster = choice.preferred || !two_stages ? choice.size : 0;
     if (cluster > 0) {
         int tp_in_slot = -1, tp_out_slot = -1;

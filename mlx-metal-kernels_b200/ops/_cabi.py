@@ -43,6 +43,7 @@ SIGNATURES = {
     "b200q_rope_append_paged_gqa_decode": (_i, [_vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz,
                                                 _i, _i, _i, _i, _i, _i64, _i, _i, _f, _vp]),
     "b200q_attention_stage_launches": (_i, [_i, _i, _i]),
+    "b200q_attention_launches": (_i, [_i, _i, _i, _i]),
     "b200q_quantize_kv": (_i, [_i, _vp, _vp, _vp, _i64, _i, _i, _i, _vp]),
     "b200q_quantize_kv_pair": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i, _vp]),
     "b200q_dequantize_kv_pair": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _vp]),

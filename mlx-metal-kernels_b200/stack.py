@@ -350,7 +350,7 @@ class DecodeStack:
         n = 0
         # the tcgen05 matvec splits K as the unsharded launch would: sharded rows == unsharded rows, bit for bit
         _cabi.set_tuning("ts.tp_world", self.tp_size if self.tp_size > 1 else 0)
-        attn_launches = lib.b200q_attention_stage_launches(B, self.hkv, 1)
+        attn_launches = lib.b200q_attention_launches(B, self.hkv, self.max_blocks, 1)
         normed = None if self.normed is None else self.normed.data_ptr()
         norm_launch = 0 if normed is None else 1      # the library then runs the rmsnorm as a launch of its own
         torch.index_select(self.embedding, 0, self.token_ids, out=self.h)

@@ -234,6 +234,47 @@ def test_cluster_kernel_matches_oracle(cuda, bits, lengths, Hq, Hkv, G):
 
 
 @pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("size", [1, 2, 4])
+@pytest.mark.parametrize("lengths,Hq,Hkv,G", [([129, 0, 1, 1023, 640], 32, 8, 32), ([2100], 8, 2, 64), ([16] * 9, 16, 2, 32), ([128, 100], 32, 4, 32)])
+def test_clusters_of_fewer_ctas(cuda, bits, size, lengths, Hq, Hkv, G):
+    """One, two and four CTAs per (sequence, kv head), of eight and sixteen warps: walks longer than the ring, warps without a page, empty
+    sequences."""
+    case = _case_with_lengths(lengths, Hkv, 128, 16, bits, G, seed=size)
+    q = synth.activations((len(lengths), 1, Hq, 128), 79)
+    want = opq.reference_paged_quantized_kv_gqa_decode_attention(q, _oracle_cache(case))
+    cabi.set_tuning("attn.cluster", 1)
+    cabi.set_tuning("attn.cluster_size", size)
+    try:
+        got = pq_ops.paged_quantized_kv_gqa_decode_attention(q.to(cuda), _device_cache(case, cuda), backend="cuda")
+    finally:
+        cabi.set_tuning("attn.cluster", 0)
+        cabi.set_tuning("attn.cluster_size", 0)
+    assert float((got.cpu().float() - want.float()).abs().max()) <= ATOL
+    assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("batch,Hkv,tokens", [(2, 8, 2048), (2, 8, 2064), (4, 8, 4096), (4, 8, 4112), (5, 8, 2048), (5, 8, 2064), (8, 8, 3072),
+                                              (8, 8, 3088), (16, 8, 1024), (16, 8, 1040), (17, 8, 64), (16, 2, 5120), (16, 2, 5136), (40, 2, 300)])
+def test_both_sides_of_the_cluster_rule(cuda, batch, Hkv, tokens):
+    """Lengths at which the choice between one cluster launch and split-KV with a merge changes: whichever runs agrees with the split-KV
+    kernels, also in a table with more room than the sequences need."""
+    lengths = [tokens - (i * 37) % tokens for i in range(batch)]
+    dcache = _device_cache(_case_with_lengths(lengths, Hkv, 128, 16, 4, 32, seed=tokens), cuda)
+    q = synth.activations((batch, 1, Hkv * 4, 128), 80).to(cuda)
+    got = pq_ops.paged_quantized_kv_gqa_decode_attention(q, dcache, backend="cuda")
+    cabi.set_tuning("attn.cluster", -1)
+    try:
+        split = pq_ops.paged_quantized_kv_gqa_decode_attention(q, dcache, backend="cuda")
+    finally:
+        cabi.set_tuning("attn.cluster", 0)
+    assert float((got.float() - split.float()).abs().max()) <= ATOL
+    lib = cabi.load()
+    blocks = dcache.block_table.shape[1]
+    assert lib.b200q_attention_launches(batch, Hkv, blocks, 0) <= lib.b200q_attention_stage_launches(batch, Hkv, 0)
+    assert cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("block_size", [16, 32, 64, 8, 24])
 @pytest.mark.parametrize("Hq,Hkv,D,P", [(8, 2, 128, 16), (32, 8, 128, 16), (6, 3, 64, 8)])
 def test_block_sparse_decode_matches_oracle(cuda, bits, block_size, Hq, Hkv, D, P):
