@@ -452,6 +452,8 @@ struct ClusterAttnParams {
     int stages;                 // pages in flight per warp
     uint32_t slot_bytes;        // K tile, V tile, scales of K, scales of V
     uint32_t off_bars, off_q, off_cpart;      // the warps' rings come first
+    int sink, window;           // as in AttnParams (window > 0 only without the append)
+    int walk_pages;             // pages that a sequence can have to visit (host side)
     TpOut tp_out;
 };
 struct alignas(64) ClusterParams {
@@ -460,7 +462,7 @@ struct alignas(64) ClusterParams {
     ClusterAttnParams a;
 };
 constexpr int kMaxClusterRing = 8;
-constexpr int kClusterWarps = 16, kClusterThreads = kClusterWarps * 32;
+constexpr int kClusterWarps = 16;
 
 __device__ __forceinline__ uint32_t cluster_rank_x() {
     uint32_t r;
@@ -474,8 +476,9 @@ __device__ __forceinline__ uint32_t cluster_rank_x() {
 // tokens); the scales come whole, all heads of the page, which costs less than sixteen pieces of 8 bytes.  Only the page that the new
 // token goes to waits for its append.
 // SC8: scales aligned to 8 bytes only (a template parameter: asked at run time it cost the aligned form 0.3 of 9.9 us).
-template <int BITS, int LOGG, bool WIDE, bool SC8>
-__global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterParams cp) {
+// NW: warps of a CTA (with the number at run time the merge and the cut of the pages cost the shortest calls 0.5 of 5.3 us).  WIN: with a window.
+template <int BITS, int LOGG, bool WIDE, bool SC8, int NW, bool WIN>
+__global__ void __launch_bounds__(NW * 32, 1) paged_attn_cluster_kernel(const __grid_constant__ ClusterParams cp) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const ClusterAttnParams& p = cp.a;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -490,7 +493,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(
     const int b = blockIdx.z;
     const int group = p.group;
     const int S = p.S;
-    const int n_warps = (int)(blockDim.x >> 5);
     __half* qs = reinterpret_cast<__half*>(smem + p.off_q);              // [group][D] rotated query rows
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.off_bars) + warp * NS;      // this warp's ring
     uint8_t* my_ring = smem + (size_t)warp * NS * p.slot_bytes;
@@ -508,17 +510,18 @@ __global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(
     pdl_launch_dependents();
     pdl_wait();
 
-    const int L = clamp_len(p.lengths[b], p.max_blocks * p.P);
-    const int n_pages = (L + p.P - 1) / p.P;
+    const SeqPages sq = seq_pages(p.lengths[b], p.max_blocks * p.P, p.P, WIN ? p.sink : 0, WIN ? p.window : 0);
+    const int L = sq.L, n_pages = sq.n;
     const int ppc = (n_pages + S - 1) / S;                               // pages per CTA
     const int c_lo = min(n_pages, (int)rank * ppc), c_hi = min(n_pages, c_lo + ppc);
-    const int ppw = (c_hi - c_lo + n_warps - 1) / n_warps;         // pages per warp
+    const int ppw = (c_hi - c_lo + NW - 1) / NW;         // pages per warp
     const int lo = min(c_hi, c_lo + warp * ppw), hi = min(c_hi, lo + ppw);
 
     const int n_my = hi - lo;
+    auto page_at = [&](int i) { return !WIN || i < sq.sink_pages ? i : sq.first_recent + (i - sq.sink_pages); };      // of the sequence's visited pages
     auto page_ids = [&](int base) -> int {
         const int j = base + lane;
-        const int page = j < n_my ? p.block_table[(size_t)b * p.max_blocks + lo + j] : -1;
+        const int page = j < n_my ? p.block_table[(size_t)b * p.max_blocks + page_at(lo + j)] : -1;
         return page >= p.num_pages ? -1 : page;
     };
     int ids_c = page_ids(0), ids_i = ids_c;                              // page ids of 32 consecutive pages, one per lane: consumed / issued window
@@ -656,8 +659,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(
         for (int j = 0; j < n_my; ++j) {
             if (j > 0 && (j & 31) == 0) ids_c = page_ids(j);
             ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[slot], par, &g_device_status, EV_ATTN_FULL_WAIT, ok ? kAttnWaitLimit : 64u)) && ok;
-            const int valid = min(p.P, L - (lo + j) * p.P);
-            const uint32_t attended = valid >= 16 ? 0xFFFFu : ((1u << max(valid, 0)) - 1u);
+            const uint32_t attended = page_mask16(page_at(lo + j), L, WIN ? p.sink : 0, WIN ? p.window : 0);
             if (__shfl_sync(0xffffffffu, ids_c, j & 31) >= 0 && ok) {
                 const uint32_t k_tile = smem_u32(my_ring) + (uint32_t)slot * p.slot_bytes;
                 process_page<BITS, LOGG>(acc, k_tile, k_tile + TILE, k_tile + 2 * TILE, R, attended, lane);
@@ -692,10 +694,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(
         return accv;
     };
     const uint32_t cpart_u = smem_u32(cpart);
-    for (int idx = threadIdx.x; idx < group * D; idx += blockDim.x) {
+    for (int idx = threadIdx.x; idx < group * D; idx += (NW * 32)) {
         const int head = idx / D, d = idx - head * D;
         float m_tot, l_tot;
-        const float v = merge(wpart, n_warps, wstride, head, d, m_tot, l_tot);
+        const float v = merge(wpart, NW, wstride, head, d, m_tot, l_tot);
         // slot `rank` of the first CTA's table (its own slot for the first CTA itself)
         const uint32_t base = cpart_u + (uint32_t)((rank * group + head) * PW) * 4u;
         auto put = [&](uint32_t off, float val) {
@@ -709,7 +711,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) paged_attn_cluster_kernel(
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (rank == 0) {
-        for (int idx = threadIdx.x; idx < group * D; idx += blockDim.x) {
+        for (int idx = threadIdx.x; idx < group * D; idx += (NW * 32)) {
             const int head = idx / D, d = idx - head * D;
             float m_tot, l_tot;
             const float v = merge(cpart, S, group * PW, head, d, m_tot, l_tot);
@@ -998,7 +1000,7 @@ bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtens
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     // Sixteen warps where eight would have more than a page each: a page costs a warp about a microsecond, the merge of eight more partial
     // results 0.2 (one sequence, one page a warp: q8 5.4 us with eight, 5.7 with sixteen; two sequences of 2048 tokens 9.2 and 8.5).
-    int warps = p.max_blocks > p.S * 8 ? kClusterWarps : 8;
+    int warps = p.walk_pages > p.S * 8 || p.window > 0 ? kClusterWarps : 8;
     const bool g32 = p.G == 32, wide = p.group > 4, sc8 = ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     p.hs = std::min(p.Hkv, kAttnWarps);
     p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024);
@@ -1006,7 +1008,7 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     const uint32_t q_bytes = align_up_u32((uint32_t)p.group * 128 * 2, 128), c_bytes = align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
     const uint32_t cap = (uint32_t)max_smem_optin(), fixed = 1024 + 128 * 8 + q_bytes + c_bytes;
     auto depth = [&]() { return (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (warps * p.slot_bytes)); };
-    if (depth() < 2) warps = 8;
+    if (depth() < 2 && p.window == 0) warps = 8;
     p.stages = depth();
     if (p.stages < 2) return B200Q_ERR_UNSUPPORTED;
     p.off_bars = warps * p.stages * p.slot_bytes;
@@ -1023,15 +1025,20 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
                          !scale_map(p.v_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.vsmap)))
         return B200Q_ERR_LAUNCH;
     using KernelFn = void (*)(ClusterParams);
-#define B200Q_CLUSTER_PAIR(BITS, LOGG, WIDE) {paged_attn_cluster_kernel<BITS, LOGG, WIDE, false>, paged_attn_cluster_kernel<BITS, LOGG, WIDE, true>}
-    static const KernelFn kernels[2][2][2][2] = {{{B200Q_CLUSTER_PAIR(8, 6, false), B200Q_CLUSTER_PAIR(8, 6, true)},      // [q4][group 32][wide][sc8]
-                                                  {B200Q_CLUSTER_PAIR(8, 5, false), B200Q_CLUSTER_PAIR(8, 5, true)}},
-                                                 {{B200Q_CLUSTER_PAIR(4, 6, false), B200Q_CLUSTER_PAIR(4, 6, true)},
-                                                  {B200Q_CLUSTER_PAIR(4, 5, false), B200Q_CLUSTER_PAIR(4, 5, true)}}};
-#undef B200Q_CLUSTER_PAIR
-    KernelFn kernel = kernels[p.bits == 4][g32][wide][sc8];
-    static bool configured[16][64] = {};
-    const int slot = (p.bits == 4) * 8 + g32 * 4 + wide * 2 + sc8;
+    // [form]: eight warps, dense, scales aligned to 16 bytes or to 8; sixteen warps, dense; sixteen warps, any call, aligned or not
+#define B200Q_CLUSTER_FORMS(BITS, LOGG, WIDE)                                                                                         \
+    {paged_attn_cluster_kernel<BITS, LOGG, WIDE, false, 8, false>, paged_attn_cluster_kernel<BITS, LOGG, WIDE, true, 8, false>,         \
+     paged_attn_cluster_kernel<BITS, LOGG, WIDE, false, 16, false>, paged_attn_cluster_kernel<BITS, LOGG, WIDE, false, 16, true>,       \
+     paged_attn_cluster_kernel<BITS, LOGG, WIDE, true, 16, true>}
+    static const KernelFn kernels[2][2][2][5] = {{{B200Q_CLUSTER_FORMS(8, 6, false), B200Q_CLUSTER_FORMS(8, 6, true)},      // [q4][group 32][wide][form]
+                                                  {B200Q_CLUSTER_FORMS(8, 5, false), B200Q_CLUSTER_FORMS(8, 5, true)}},
+                                                 {{B200Q_CLUSTER_FORMS(4, 6, false), B200Q_CLUSTER_FORMS(4, 6, true)},
+                                                  {B200Q_CLUSTER_FORMS(4, 5, false), B200Q_CLUSTER_FORMS(4, 5, true)}}};
+#undef B200Q_CLUSTER_FORMS
+    const int form = warps == 8 ? (sc8 ? 1 : 0) : sc8 ? 4 : p.window > 0 ? 3 : 2;
+    KernelFn kernel = kernels[p.bits == 4][g32][wide][form];
+    static bool configured[40][64] = {};
+    const int slot = ((p.bits == 4) * 4 + g32 * 2 + wide) * 5 + form;
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured[slot][dev & 63]) {
@@ -1216,7 +1223,12 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     if (!fast_ok) return simple();
     // small batches: one cluster per (sequence, kv head), merged on chip - no workspace, no second launch
     const int ranges = split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, q_dtype);
-    const ClusterChoice choice = window_size == 0 && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv, max_blocks, false, ranges > 0) : ClusterChoice{0, false};
+    // A window bounds the walk whatever the length.  Windows as long as the table stay with the split-KV kernels, whose dense result they
+    // reproduce bit for bit; without a workspace only dense calls are served.
+    const int64_t visited = ((int64_t)window_size + 15) / 16 + 1 + ((int64_t)sink_tokens + 15) / 16;
+    const int walk_pages = window_size > 0 ? (int)std::min<int64_t>(max_blocks, visited) : max_blocks;
+    const bool may = window_size == 0 || (ranges > 0 && window_size < (int64_t)max_blocks * page_size);
+    const ClusterChoice choice = may && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv, walk_pages, false, ranges > 0) : ClusterChoice{0, false};
     const int cluster = choice.preferred || ranges == 0 ? choice.size : 0;
     if (cluster > 0) {
         ClusterAttnParams c = {};
@@ -1228,6 +1240,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
         c.B = B; c.Hq = Hq; c.Hkv = Hkv; c.P = page_size; c.max_blocks = max_blocks; c.G = group_size; c.Gd = Gd;
         c.group = group; c.bits = bits; c.S = cluster; c.num_pages = num_pages; c.scale = scale;
         c.row_bytes = Hkv * dp; c.scale_row_halves = Hkv * Gd;
+        c.sink = sink_tokens; c.window = window_size; c.walk_pages = walk_pages;
         const int rc = launch_cluster_attention(c, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
     }
@@ -1312,6 +1325,7 @@ int rope_append_attention_impl(const void* qkv, const float* cos_table, const fl
         c.B = B; c.Hq = Hq; c.Hkv = Hkv; c.P = page_size; c.max_blocks = max_blocks; c.G = group_size; c.Gd = Gd;
         c.group = group; c.bits = bits; c.S = cluster; c.num_pages = num_pages; c.scale = scale;
         c.row_bytes = Hkv * dp; c.scale_row_halves = Hkv * Gd;
+        c.walk_pages = max_blocks;
         const int rc = launch_cluster_attention(c, stream);
         if (rc != B200Q_ERR_UNSUPPORTED) return rc;
         if (q_scratch == nullptr) return B200Q_ERR_WORKSPACE;

@@ -253,6 +253,29 @@ def test_clusters_of_fewer_ctas(cuda, bits, size, lengths, Hq, Hkv, G):
     assert cabi.device_status() == 0
 
 
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("size", [1, 4, 8])
+@pytest.mark.parametrize("sink,window", [(0, 16), (4, 32), (20, 5), (3, 1), (40, 100), (600, 64), (16, 640)])
+def test_windows_in_the_cluster_kernel(cuda, bits, size, sink, window):
+    """Only pages with an attended position are walked: windows and sinks that straddle pages, sequences shorter than either, walks cut over
+    more warps than they have pages."""
+    sparse_ops = importlib.import_module("mlx_metal_kernels_b200.ops.sparse_attention_ops")
+    lengths = [1, 15, 16, 17, 37, 200, 333, 700]
+    case = _case_with_lengths(lengths, 2, 128, 16, bits, 32, seed=sink + window)
+    q = synth.activations((len(lengths), 1, 8, 128), 81)
+    want = opq.reference_paged_quantized_kv_gqa_decode_attention(q, _oracle_cache(case), window=(sink, window))
+    pattern = sparse_ops.SparseAttentionPattern("sliding_window_sink" if sink else "sliding_window", window_size=window, sink_tokens=sink)
+    cabi.set_tuning("attn.cluster", 1)
+    cabi.set_tuning("attn.cluster_size", size)
+    try:
+        got = pq_ops.sparse_paged_quantized_kv_gqa_decode_attention(q.to(cuda), _device_cache(case, cuda), pattern)
+    finally:
+        cabi.set_tuning("attn.cluster", 0)
+        cabi.set_tuning("attn.cluster_size", 0)
+    assert float((got.cpu().float() - want.float()).abs().max()) <= ATOL
+    assert cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("batch,Hkv,tokens", [(2, 8, 2048), (2, 8, 2064), (4, 8, 4096), (4, 8, 4112), (5, 8, 2048), (5, 8, 2064), (8, 8, 3072),
                                               (8, 8, 3088), (16, 8, 1024), (16, 8, 1040), (17, 8, 64), (16, 2, 5120), (16, 2, 5136), (40, 2, 300)])
 def test_both_sides_of_the_cluster_rule(cuda, batch, Hkv, tokens):
