@@ -422,8 +422,8 @@ __global__ void __launch_bounds__(kSplitThreads, TWO ? B200Q_ATTN_CTAS : 1) page
 }
 
 // ------------------------------------------------------------------------------------------------
-// Cluster kernel for small batches: one thread-block cluster per (sequence, kv head), no partials in global memory
-// and no merge launch.  The CTAs of the cluster cut the sequence's pages into equal ranges, the 8 warps of a CTA cut
+// Cluster kernel for small batches and short walks: one thread-block cluster per (sequence, kv head), no partials in global memory
+// and no merge launch.  The CTAs of the cluster cut the sequence's pages into equal ranges, the 8 or 16 warps of a CTA cut
 // their range again; a warp walks its pages exactly as in the split-KV kernel.  The warps' partial (max, sum,
 // accumulator) triples are merged in shared memory, the CTAs' through distributed shared memory by the cluster's
 // first CTA, always in the same order (bitwise repeatable, and independent of how many kv heads a tensor-parallel
@@ -454,6 +454,7 @@ struct ClusterAttnParams {
     uint32_t off_bars, off_q, off_cpart;      // the warps' rings come first
     int sink, window;           // as in AttnParams (window > 0 only without the append)
     int walk_pages;             // pages that a sequence can have to visit (host side)
+    int32_t* verdict;           // as in AttnParams
     TpOut tp_out;
 };
 struct alignas(64) ClusterParams {
@@ -512,6 +513,12 @@ __global__ void __launch_bounds__(NW * 32, 1) paged_attn_cluster_kernel(const __
 
     const SeqPages sq = seq_pages(p.lengths[b], p.max_blocks * p.P, p.P, WIN ? p.sink : 0, WIN ? p.window : 0);
     const int L = sq.L, n_pages = sq.n;
+    if (BITS == 16 && p.verdict != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && warp == 0) {
+        bool good = true;
+        for (int i = lane; i < p.B; i += 32) good = good && p.lengths[i] >= 0 && p.lengths[i] <= p.max_blocks * p.P;
+        good = __all_sync(0xffffffffu, good);
+        if (lane == 0) *reinterpret_cast<volatile int32_t*>(p.verdict) = good ? 1 : 2;
+    }
     const int ppc = (n_pages + S - 1) / S;                               // pages per CTA
     const int c_lo = min(n_pages, (int)rank * ppc), c_hi = min(n_pages, c_lo + ppc);
     const int ppw = (c_hi - c_lo + NW - 1) / NW;         // pages per warp
@@ -546,10 +553,11 @@ __global__ void __launch_bounds__(NW * 32, 1) paged_attn_cluster_kernel(const __
                 mbar_arrive(bar);                                        // a missing page: nothing to copy, skipped where it is used
             } else {
                 uint8_t* dst = my_ring + (size_t)(j % NS) * p.slot_bytes;
-                mbar_arrive_expect_tx(bar, 2 * TILE + (SC8 ? 0u : 2 * sc_bytes));
-                tma_load_3d(smem_u32(dst), &cp.kmap, 0, page * 16, h, bar);
-                tma_load_3d(smem_u32(dst + TILE), &cp.vmap, 0, page * 16, h, bar);
-                if (SC8) {
+                const int z = BITS == 16 ? 2 * h : h;                    // a plain row is two tiles of 128 bytes
+                mbar_arrive_expect_tx(bar, 2 * TILE + (SC8 || BITS == 16 ? 0u : 2 * sc_bytes));
+                tma_load_3d(smem_u32(dst), &cp.kmap, 0, page * 16, z, bar);
+                tma_load_3d(smem_u32(dst + TILE), &cp.vmap, 0, page * 16, z, bar);
+                if (SC8 || BITS == 16) {
                 } else if (p.Hkv == p.hs) {
                     const size_t at = (size_t)page * 16 * p.scale_row_halves;
                     bulk_g2s(dst + 2 * TILE, p.k_scales + at, sc_bytes, bar);
@@ -567,7 +575,7 @@ __global__ void __launch_bounds__(NW * 32, 1) paged_attn_cluster_kernel(const __
     for (int j = 0; j < min(NS, n_my); ++j)
         if (j != j_app) issue(j);
 
-    if (p.fused) {
+    if constexpr (BITS != 16) if (p.fused) {
         const int heads = p.Hq + 2 * p.Hkv;
         const int pos = p.positions[b];
         const bool pos_ok = pos >= 0 && pos < p.table_len;
@@ -675,7 +683,7 @@ __global__ void __launch_bounds__(NW * 32, 1) paged_attn_cluster_kernel(const __
              [&](int head, float m, float l) { dst[head * PW + D] = m; dst[head * PW + D + 1] = l; });
     }
     __syncthreads();
-    // ---- merge the 8 warps (fixed order) into this CTA's partial; thread -> (head, d) ----
+    // ---- merge the warps (fixed order) into this CTA's partial; thread -> (head, d) ----
     auto merge = [&](const float* src, int n, int stride, int head, int d, float& m_tot, float& l_tot) -> float {
         src += head * PW;
         m_tot = -INFINITY;
@@ -939,7 +947,7 @@ inline bool heads_ok(int Hkv) { return Hkv <= kAttnWarps || Hkv % kAttnWarps == 
 struct ClusterChoice { int size; bool preferred; };      // size 0: not possible
 // fused: the launch also stands for the append (three launches against one).  split: the split-KV kernels could take the call; without them
 // (no workspace) the rule is the one for tables of any length, so a call is not refused or served by its length.
-ClusterChoice cluster_choice(int B, int Hkv, int max_blocks, bool fused, bool split) {
+ClusterChoice cluster_choice(int B, int Hkv, int max_blocks, bool fused, bool split, bool plain = false) {
     const int mode = tuning_get("attn.cluster");      // 1: whenever possible, -1: never, 0: by the rule below
     if (mode < 0 || (mode > 0 && B * Hkv > 65535)) return {0, false};
     // the choice follows the kv heads of the UNSHARDED cache ("ts.tp_world" equal head shards), so that a
@@ -962,7 +970,8 @@ ClusterChoice cluster_choice(int B, int Hkv, int max_blocks, bool fused, bool sp
     const int kv_full = Hkv * std::max(1, tuning_get("ts.tp_world"));
     for (int size = 4; split && size >= 1; size /= 2) {
         if (heads * size * 8 > 7 * (int64_t)sm_count()) continue;
-        const int walk = (max_blocks + size * kClusterWarps - 1) / (size * kClusterWarps);
+        const int warps = size * (plain ? 8 : kClusterWarps);      // plain pages: no room for more rings
+        const int walk = (max_blocks + warps - 1) / warps;
         int longest = 4;
         if (size == 4 && heads < 24) longest = kv_full >= kAttnWarps ? 2 : 3;
         if (size == 4 && kv_full < 4) longest = 5;
@@ -998,12 +1007,12 @@ bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtens
 }
 
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
+    const bool plain = p.bits == 16, bf = p.q_dtype == B200Q_BF16, g32 = p.G == 32, wide = p.group > 4, sc8 = !plain && ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     // Sixteen warps where eight would have more than a page each: a page costs a warp about a microsecond, the merge of eight more partial
     // results 0.2 (one sequence, one page a warp: q8 5.4 us with eight, 5.7 with sixteen; two sequences of 2048 tokens 9.2 and 8.5).
-    int warps = p.walk_pages > p.S * 8 || p.window > 0 ? kClusterWarps : 8;
-    const bool g32 = p.G == 32, wide = p.group > 4, sc8 = ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
+    int warps = !plain && (p.walk_pages > p.S * 8 || p.window > 0) ? kClusterWarps : 8;
     p.hs = std::min(p.Hkv, kAttnWarps);
-    p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024);
+    p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + (plain ? 0u : align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024));
     // shared memory: [1 KB alignment] rings, barriers, query rows, the CTAs' partials
     const uint32_t q_bytes = align_up_u32((uint32_t)p.group * 128 * 2, 128), c_bytes = align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
     const uint32_t cap = (uint32_t)max_smem_optin(), fixed = 1024 + 128 * 8 + q_bytes + c_bytes;
@@ -1017,11 +1026,11 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     const uint32_t off = 1024 + p.off_cpart + c_bytes;
     ClusterParams cp = {};
     cp.a = p;
-    const uint32_t row = p.bits == 4 ? 64 : 128;
-    if (!page_map(p.k_codes, row, p.num_pages * 16, p.Hkv, p.row_bytes, 1, &cp.kmap) ||
-        !page_map(p.v_codes, row, p.num_pages * 16, p.Hkv, p.row_bytes, 1, &cp.vmap))
+    const uint32_t row = p.bits == 4 ? 64 : 128, tiles = plain ? 2 : 1;
+    if (!page_map(p.k_codes, row, p.num_pages * 16, p.Hkv * tiles, p.row_bytes, tiles, &cp.kmap) ||
+        !page_map(p.v_codes, row, p.num_pages * 16, p.Hkv * tiles, p.row_bytes, tiles, &cp.vmap))
         return B200Q_ERR_LAUNCH;
-    if (p.Hkv > p.hs && !sc8 && (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.ksmap) ||
+    if (!plain && p.Hkv > p.hs && !sc8 && (!scale_map(p.k_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.ksmap) ||
                          !scale_map(p.v_scales, p.scale_row_halves * 2, p.num_pages * 16, p.hs * p.Gd * 2, &cp.vsmap)))
         return B200Q_ERR_LAUNCH;
     using KernelFn = void (*)(ClusterParams);
@@ -1035,10 +1044,13 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
                                                  {{B200Q_CLUSTER_FORMS(4, 6, false), B200Q_CLUSTER_FORMS(4, 6, true)},
                                                   {B200Q_CLUSTER_FORMS(4, 5, false), B200Q_CLUSTER_FORMS(4, 5, true)}}};
 #undef B200Q_CLUSTER_FORMS
+    static const KernelFn plain_kernels[2][2] = {      // [bf16][wide]
+        {paged_attn_cluster_kernel<16, 0, false, false, 8, false>, paged_attn_cluster_kernel<16, 0, true, false, 8, false>},
+        {paged_attn_cluster_kernel<16, 1, false, false, 8, false>, paged_attn_cluster_kernel<16, 1, true, false, 8, false>}};
     const int form = warps == 8 ? (sc8 ? 1 : 0) : sc8 ? 4 : p.window > 0 ? 3 : 2;
-    KernelFn kernel = kernels[p.bits == 4][g32][wide][form];
-    static bool configured[40][64] = {};
-    const int slot = ((p.bits == 4) * 4 + g32 * 2 + wide) * 5 + form;
+    KernelFn kernel = plain ? plain_kernels[bf][wide] : kernels[p.bits == 4][g32][wide][form];
+    static bool configured[44][64] = {};
+    const int slot = plain ? 40 + bf * 2 + wide : ((p.bits == 4) * 4 + g32 * 2 + wide) * 5 + form;
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured[slot][dev & 63]) {
@@ -1261,7 +1273,8 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     return rc == B200Q_ERR_UNSUPPORTED && tp_out_slot < 0 ? simple() : rc;      // scales of very many kv heads do not fit a ring
 }
 
-// Plain fp16 / bf16 pages on the split-KV kernels; B200Q_ERR_UNSUPPORTED outside their shapes.  `verdict`: see AttnParams.
+// Plain fp16 / bf16 pages on the cluster and the split-KV kernels (bf16, 8 kv heads, split-KV / cluster, us: 8 sequences of 128 tokens 12.0 / 5.1,
+// of 1024 14.8 / 11.3; 2 kv heads, 32 of 512 17.4 / 8.1); B200Q_ERR_UNSUPPORTED outside their shapes.  `verdict`: see AttnParams.
 int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v_pages, const int32_t* block_table, const int32_t* lengths,
                                void* out, void* workspace, size_t workspace_bytes, int B, int Hq, int Hkv, int D, int page_size,
                                int64_t num_pages, int max_blocks, float scale, int dtype, int32_t* verdict, cudaStream_t stream) {
@@ -1276,6 +1289,18 @@ int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v
     p.group = Hq / Hkv; p.num_pages = num_pages; p.scale = scale; p.q_dtype = dtype; p.bits = 16;
     p.row_bytes = Hkv * kHeadDim * 2;
     p.verdict = verdict;
+    const ClusterChoice choice = B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv, max_blocks, false, true, true) : ClusterChoice{0, false};
+    if (choice.preferred && choice.size > 0) {
+        ClusterAttnParams c = {};
+        c.q = q; c.q_dtype = dtype;
+        c.k_codes = const_cast<uint8_t*>(p.k_codes); c.v_codes = const_cast<uint8_t*>(p.v_codes);
+        c.block_table = block_table; c.lengths = lengths; c.out = out;
+        c.B = B; c.Hq = Hq; c.Hkv = Hkv; c.P = page_size; c.max_blocks = c.walk_pages = max_blocks;
+        c.group = p.group; c.bits = 16; c.S = choice.size; c.num_pages = num_pages; c.scale = scale;
+        c.row_bytes = p.row_bytes; c.verdict = verdict;
+        const int rc = launch_cluster_attention(c, stream);
+        if (rc != B200Q_ERR_UNSUPPORTED) return rc;
+    }
     return launch_split_attention(p, kMaxRanges, stream);
 }
 

@@ -94,6 +94,27 @@ def test_plain_pages(cuda, dtype, Hq, Hkv, lengths):
         gqa_ops.paged_gqa_decode_attention(*args[:4], bad)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("cluster,size", [(-1, 0), (1, 1), (1, 2), (1, 4), (1, 8)])
+@pytest.mark.parametrize("Hq,Hkv,lengths", [(8, 8, [1, 300, 17]), (4, 1, [700, 0]), (40, 8, [513]), (64, 16, [31] * 5)])
+def test_plain_pages_by_both_kernels(cuda, dtype, cluster, size, Hq, Hkv, lengths):
+    """Split-KV with a merge, and clusters of one to eight CTAs: walks longer than a warp's ring, warps without a page, an empty sequence."""
+    pages = sum((n + 15) // 16 for n in lengths) + 3
+    table, ln = _table(lengths, pages, 2), torch.tensor(lengths, dtype=torch.int32)
+    k, v = (synth.activations((pages, 16, Hkv, 128), s, "cpu", dtype) for s in (21, 22))
+    q = synth.activations((len(lengths), 1, Hq, 128), 23, "cpu", dtype)
+    want = _expected(q, k, v, table, ln)
+    cabi.set_tuning("attn.cluster", cluster)
+    cabi.set_tuning("attn.cluster_size", size)
+    try:
+        got = gqa_ops.paged_gqa_decode_attention(*(t.to(cuda) for t in (q, k, v, table, ln))).cpu().double()
+    finally:
+        cabi.set_tuning("attn.cluster", 0)
+        cabi.set_tuning("attn.cluster_size", 0)
+    assert (got - want).abs().max() <= (2e-3 if dtype == torch.float16 else 1.6e-2)
+    assert cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("bits,G", [(4, 32), (8, 64)])
 @pytest.mark.parametrize("Hq,Hkv,lengths", [(8, 1, [1, 300, 17]), (6, 3, [129, 5]), (32, 8, [700, 0, 40]), (32, 16, [40, 0, 250])])
 @pytest.mark.parametrize("shifted", ["k_scales", "v_scales", "both"])
