@@ -222,7 +222,7 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-// A probe that suspends the warp for up to a microsecond.  Probes that come back at once are repeated, and those of the waiting warps
+// A probe that suspends the warp for up to a microsecond, for every probe of a wait but the first.  Probes that come back at once are repeated, and those of the waiting warps
 // took a third of the issue slots of a busy SM from the dequantising ones (537 instructions per chunk and scheduler, 340 of them the
 // dequantisation's): 6144 x 4096 q4 for 32 rows 11.2 -> 10.4 us, gate and up of 11008 x 4096 for 256 rows 65.5 -> 60.8.
 __device__ __forceinline__ bool probe_bar(uint32_t addr, uint32_t parity) {
@@ -240,7 +240,7 @@ __device__ __forceinline__ bool probe_bar(uint32_t addr, uint32_t parity) {
 }
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int event, bool& ok) {
     const uint32_t addr = smem_u32(bar);
-    if (probe_bar(addr, parity)) return true;      // mostly it is there
+    if (mbar_try_wait(bar, parity)) return true;      // mostly it is there
     const uint32_t limit = ok ? kTsWaitLimit : 64u;
 #pragma unroll 1
     for (uint32_t i = 0; i < limit; ++i)
@@ -251,13 +251,25 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int eve
 }
 
 // One wait of a warp for several barriers: lane i polls its own (address and parity per lane; lanes without one pass `need` false).
-// For the operands of two chunks at once (gate and up, few columns): polled together 25.4 us, in turn 25.7 (14336 x 4096 q4, 32 rows).  The two
-// barriers of a single chunk are waited for in turn: together 66.2 us, in turn 62.4 (gate and up of 11008 x 4096, 256 rows).
+// For the operands of two chunks at once (gate and up, few columns): polled together 25.4 us, in turn 25.7 (14336 x 4096 q4, 32 rows), and
+// without suspending (bf16 rows 41.6 us, suspending 42.1).  The two
+// barriers of a single chunk are waited for in turn: together 66.2 us, in turn 62.4 (gate and up of 11008 x 4096, 256 rows).  One loop for
+// both cases: 60.9 us there instead of 57.0.
 __device__ __forceinline__ void wait_bars(uint32_t addr, uint32_t parity, bool need, int event, bool& ok) {
     const uint32_t limit = ok ? kTsWaitLimit : 64u;
     for (uint32_t i = 0; i < limit; ++i) {
-        const bool got = !need || probe_bar(addr, parity);
-        if (__all_sync(0xffffffffu, got)) return;
+        uint32_t got = 1;
+        if (need)
+            asm volatile(
+                "{\n"
+                ".reg .pred p;\n"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                "selp.b32 %0, 1, 0, p;\n"
+                "}\n"
+                : "=r"(got)
+                : "r"(addr), "r"(parity)
+                : "memory");
+        if (__all_sync(0xffffffffu, got != 0)) return;
     }
     atomicMax(&g_device_status, event);
     ok = false;
@@ -478,24 +490,29 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
         for (int it = 0; it < my_items; ++it) {
             if (it > 0) wait_bar(d_free, (uint32_t)(it - 1) & 1u, EV_GEMV_EMPTY_WAIT, ok);
             tc_fence_after();
+            if (MATS == 2 && per == 2) {
 #pragma unroll 1
-            for (int ch = first; ch < n_ch;) {
-                at.to(it * n_ch + ch, XS, NA);
-                const RingPos x = at.x, a = at.a;
-                const bool two = per == 2 && ch + 1 < n_ch;
-                if (two) at.to(it * n_ch + ch + 1, XS, NA);
-                if (two) {
+                for (int ch = 0; ch < n_ch; ch += 2) {
+                    at.to(it * n_ch + ch, XS, NA);
+                    const RingPos x = at.x, a = at.a;
+                    const bool two = ch + 1 < n_ch;
+                    if (two) at.to(it * n_ch + ch + 1, XS, NA);
                     // lanes 0, 1: the first chunk's operands; lanes 2, 3: the second's
                     const uint32_t bar = lane == 0 ? smem_u32(&full_x[x.slot]) : lane == 1 ? smem_u32(&a_full[a.slot]) : lane == 2 ? smem_u32(&full_x[at.x.slot]) : smem_u32(&a_full[at.a.slot]);
-                    wait_bars(bar, lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par, lane < 4, EV_GEMV_FULL_WAIT, ok);
-                } else {
-                    wait_bar(&full_x[x.slot], x.par, EV_GEMV_FULL_WAIT, ok);
-                    wait_bar(&a_full[a.slot], a.par, EV_GEMV_FULL_WAIT, ok);
+                    wait_bars(bar, lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
+                    tc_fence_after();
+                    chunk(x.slot, a.slot, ch == 0);
+                    if (two) chunk(at.x.slot, at.a.slot, false);
                 }
-                tc_fence_after();
-                chunk(x.slot, a.slot, ch == first);
-                if (two) chunk(at.x.slot, at.a.slot, false);
-                ch += (two ? 2 : 1) + ChunkWalk<MATS>::kSkip;
+            } else {
+#pragma unroll 1
+                for (int ch = first; ch < n_ch; ch += 1 + ChunkWalk<MATS>::kSkip) {
+                    at.to(it * n_ch + ch, XS, NA);
+                    wait_bar(&full_x[at.x.slot], at.x.par, EV_GEMV_FULL_WAIT, ok);
+                    wait_bar(&a_full[at.a.slot], at.a.par, EV_GEMV_FULL_WAIT, ok);
+                    tc_fence_after();
+                    chunk(at.x.slot, at.a.slot, ch == first);
+                }
             }
             tc_commit(d_full);
         }
@@ -877,14 +894,18 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
         configured[dev & 63] = true;
     }
     // Column blocks and K split by estimated time, in clocks: rounds of items over the SMs, each a chain of chunks whose cost is the
-    // dequantisation's or the tensor pipe's (measured: 22 clocks per MMA up to 32 columns, then half a clock per column; 64 k in two
-    // terms take 540 to 600 clocks beside the other groups, so wide blocks cost them nothing: gate and up of 14336 x 4096 q4 for
-    // 128 bf16 rows 72.6 us with 300 here, 64.8 with 540).  The choice
+    // dequantisation's (450; 64 k in two terms 540) or the tensor pipe's: 22 clocks per MMA up to 32 columns, then half a clock per column,
+    // and 260 a chunk in which the next chunk's way into tensor memory keeps it waiting (no arithmetic at all: 530 clocks at 64
+    // columns, 650 at 96).  The first CTA of a cluster takes about 35 clocks per column and part for the partial sums.  (Splits were once
+    // left out where the sums exceed 48 KB, from 33 rows on: 4096 x 14336 q4 48 rows 24.3 -> 16.6 us, 64 rows 24.6 -> 18.4; 4096 x
+    // 11008, groups of 32, 256 rows 35.2 -> 31.4.)  The choice
     // must not depend on how many rows THIS launch holds: a tensor-parallel shard of the rows has to reproduce the unsharded result
     // bit for bit, so the tile count of the unsharded matrix decides ("ts.tp_world" = number of equal row shards).
     const int tiles_full = tiles * std::max(1, tuning_get("ts.tp_world"));
     const int forced = tuning_get("ts.split");
-    constexpr uint32_t kRedCap = 48u * 1024u;              // bytes of the dedicated buffer for partial sums
+    // bytes of partial sums: in a dedicated buffer (96 KB of it leave too little for the rings: 64 rows of 4096 x 14336 19.8 us, through the
+    // rings 18.7; 72 KB 17.0 and 17.7), and at all
+    constexpr uint32_t kRedCap = 80u * 1024u, kRedMax = 128u * 1024u;
     double best = 0.0;
     int cols = 0, split = 1;
     const int nb0 = (p.B + kMaxCols - 1) / kMaxCols;
@@ -892,15 +913,15 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
         const int c = ((p.B + nb - 1) / nb + 15) / 16 * 16;
         const int blocks = (p.B + c - 1) / c;
         if (blocks != nb) continue;                        // the same blocks as a smaller nb
-        const double chunk = std::max(SPLIT ? 540.0 : 360.0, 8.0 * std::max(22.2, c * 0.5 + 0.8));
+        const double chunk = std::max(SPLIT ? 540.0 : 450.0, 8.0 * std::max(22.2, c * 0.5 + 0.8) + 260.0);
         for (int sp = 1; sp <= 8; sp *= 2) {
             if (forced > 0 ? sp != std::min(forced, std::max(1, p.n_stage_total)) : sp > 1 && sp > p.n_stage_total / 2) continue;
-            if (forced <= 0 && sp > 1 && (uint32_t)(sp - 1) * MATS * std::min(c, p.B) * kRows * 4 > kRedCap) continue;
+            if (forced <= 0 && sp > 1 && (uint32_t)(sp - 1) * MATS * c * kRows * 4 > kRedMax) continue;
             const int64_t items = (int64_t)tiles_full * blocks;
             const int slots = sp == 1 ? sms : max_clusters(kernel, sp, cap - 2048u);
             if (forced <= 0 && sp > 1 && items > slots) continue;
             const double rounds = (double)((items + slots - 1) / slots);
-            const double t = rounds * ((double)((p.n_stage_total + sp - 1) / sp * SC * MATS) * chunk + 1500.0 + c * MATS * 10.0) + (sp > 1 ? 1500.0 : 0.0);
+            const double t = rounds * ((double)((p.n_stage_total + sp - 1) / sp * SC * MATS) * chunk + 1500.0 + c * MATS * 10.0) + (sp > 1 ? 1500.0 + 35.0 * (sp - 1) * MATS * std::min(c, p.B) : 0.0);
             if (cols == 0 || t < best) { best = t; cols = c; split = sp; }
         }
     }

@@ -79,6 +79,26 @@ def test_symmetric_codes_without_zero_points(tcgen05, bits):
     assert rel_l2(got, want) <= TOL
 
 
+@pytest.mark.parametrize("bits,B,N,K,G", [(4, 48, 4096, 2048, 64), (4, 64, 4096, 4096, 64), (8, 48, 3000, 1024, 64), (4, 200, 900, 2816, 32), (4, 250, 4096, 1024, 64)])
+def test_large_partial_sums(cuda, bits, B, N, K, G):
+    """Splits that the launch plan chooses from 33 rows on: partial sums of 64 to 96 KB, through the buffer or the rings; half of the rows as a
+    shard gives the same bits."""
+    w, s, z = (t.to(cuda) for t in synth.quantized_weight(N, K, bits, G, seed=N + B))
+    x = synth.activations((B, K), 8, cuda)
+    got = _fn(bits)(x, w, s, z, group_size=G)
+    assert rel_l2(got, _ref(bits)(x.cpu(), w.cpu(), s.cpu(), z.cpu(), group_size=G)) <= TOL
+    assert torch.equal(_fn(bits)(x, w, s, z, group_size=G), got)
+    half = N // 2
+    cabi.set_tuning("ts.tp_world", 2)
+    try:
+        part = _fn(bits)(x, w[:half].contiguous(), s[:half].contiguous(), z[:half].contiguous(), group_size=G)
+    finally:
+        cabi.set_tuning("ts.tp_world", 0)
+    if (N + 127) // 128 == 2 * ((half + 127) // 128):          # the shard's row tiles are half of the unsharded matrix's
+        assert torch.equal(part, got[:, :half])
+    assert cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("around", [0.0, 511.5, -511.5, 900.0, -900.0, 1023.5])
 def test_zero_points_up_to_the_limit(tcgen05, bits, around):
