@@ -20,10 +20,10 @@
 //   epilogue (dequantise warps)   tcgen05.ld of D, clamp, round, residual add or SwiGLU, store
 //
 // What bounds it: a chunk (128 x 128 weights) costs the dequantisation 4 x 260 warp instructions, i.e. about 340 clocks on the SM's four
-// schedulers, and the tensor pipe 8 x 22 clocks up to 32 columns, 8 x 65 at 128; a chunk takes about 600, since every barrier
-// costs a waiting warp 150-200 clocks beside the others.  Fewer, longer pieces per wait are therefore better: eight warps per chunk
-// instead of four measured 54 against 48 us on an MLP block of 32 rows.  One block of up to 128 columns shares each dequantised
-// weight.  Measured (q4, 4096 -> 14336 -> 4096, start -> now): 32 rows 84 -> 48 us; 256 rows of 4096 -> 11008 -> 4096 528 -> 125 us.
+// schedulers, and the tensor pipe 8 x 22 clocks up to 32 columns, 8 x 65 at 128; a chunk takes about 480, since stores into tensor
+// memory and MMAs hold each other up and every barrier costs a waiting warp some time beside the others.  Fewer, longer pieces per wait are therefore better: eight warps per chunk
+// instead of four measured 54 against 48 us on an MLP block of 32 rows (at 600 clocks a chunk).  One block of up to 128 columns shares each dequantised
+// weight.  Measured (q4): block 4096 -> 14336 -> 4096, 32 rows 48 -> 45.9 us; 4096 -> 11008 -> 4096, 256 rows 119 -> 104 us.
 // Codes are unpacked in k order (one byte permute per pair): the activations need no rearrangement, and nothing but TMA touches
 // them.  (The form before this one permuted the rows in shared memory with four warps, recomputed the group constants per 32 k and
 // kept 32 columns per launch: 1800 warp instructions per chunk; a 256-row prompt chunk re-streamed its weights eight times.)
