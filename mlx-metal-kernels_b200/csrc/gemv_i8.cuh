@@ -85,12 +85,13 @@ struct I8Params {
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-template <int BYTES>
-__device__ __forceinline__ void cp_small(uint32_t dst, const void* src) {      // 4 or 8 bytes
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
-}
 __device__ __forceinline__ void cp16_part(uint32_t dst, const void* src, uint32_t bytes) {      // the rest is zero-filled
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+template <int BYTES>
+__device__ __forceinline__ void cp_piece(uint32_t dst, const void* src, bool live) {      // 4, 8 or 16 bytes, or as many zeros
+    if constexpr (BYTES == 16) cp16_part(dst, src, live ? 16u : 0u);
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(live ? BYTES : 0) : "memory");
 }
 __device__ __forceinline__ float i8_warp_sum(float v) {
 #pragma unroll
@@ -241,13 +242,15 @@ template <int BITS, int LOGG> struct I8Shape {
     static constexpr int XU = GU * 96 * NM;                  // digit bytes of a unit: 1536 (q4) or 768 (q8)
 };
 
-// VEC: the groups of a row fill whole units, so the scales of a unit are aligned pieces.  (One kernel with a run-time switch: gate and up of
-// 14336 x 4096 13.7 us instead of 13.3.)
-template <int BITS, int LOGG, int NB, bool PACKETS, bool VEC>
+// PB: bytes of a piece of scales, 16, 8 or 4, where rows of scales (and the units in them) start at multiples of it: pieces then lie in
+// shared memory as the affine step wants them, eight groups to a load.  0: rows that start anywhere; an aligned window is copied and read
+// one value at a time.  (One kernel with a run-time switch: gate and up of 14336 x 4096 13.7 us instead of 13.3.)
+template <int BITS, int LOGG, int NB, bool PACKETS, int PB>
 __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
     using S = I8Shape<BITS, LOGG>;
     constexpr int G = S::G, GB = S::GB, NM = S::NM, GU = S::GU, CP = S::CP, CH = S::CH, CG = S::CG, MB = S::MB, WIN = S::WIN;
+    constexpr bool VEC = PB != 0;
     constexpr int NT = NB <= 2 ? 1 : NB / 2;          // 8-column tiles: one batch row takes 4 columns (3 digits)
 
     const int warp = threadIdx.x >> 5;
@@ -295,8 +298,8 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
             if (m_row < rows) {
                 const int64_t first = (int64_t)(row0 + m_row) * Gn;
                 const int64_t at = (first + nu.i * GU) * 2;
-                leftM = MB;
-                if (!VEC) leftM = (int)min((int64_t)(WIN * 16), (first + Gn) * 2 - (at & ~(int64_t)15));
+                if (VEC) leftM = (Gn - nu.i * GU) * 2;
+                else leftM = (int)min((int64_t)(WIN * 16), (first + Gn) * 2 - (at & ~(int64_t)15));
                 srcM = reinterpret_cast<const uint8_t*>(mb) + (VEC ? at : at & ~(int64_t)15);
                 if (mb == nullptr) leftM = -1;
             }
@@ -306,9 +309,9 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
         if (c == 0 && leftM > 0) {
             if (VEC) {
                 const uint32_t dst = meta + (uint32_t)(t * 8 + g) * MB;
-                if constexpr (MB == 32) { cp16(dst, srcM); cp16(dst + 16, srcM + 16); }
-                else if constexpr (MB == 16) cp16(dst, srcM);
-                else cp_small<MB>(dst, srcM);
+                constexpr int SP = VEC ? PB : 16;
+#pragma unroll
+                for (int q = 0; q < MB / SP; ++q) cp_piece<SP>(dst + q * SP, srcM + (leftM > q * SP ? q * SP : 0), leftM > q * SP);
             } else {
                 // the aligned window that holds the row's values, zeros past the end of the row
                 const uint32_t dst = meta + (uint32_t)(t * 8 + g) * (WIN * 16);
@@ -652,8 +655,16 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
     p.eps = q.eps; p.B = q.B; p.N = q.N; p.K = q.K; p.Gn = q.Gn; p.act_dtype = q.act_dtype; p.norm_w_dtype = q.norm_w_dtype;
     p.row_bytes = q.row_bytes; p.tp_out = q.tp_out; p.tp_in = q.tp_in;
     p.units = (p.row_bytes + kI8UnitBytes - 1) / kI8UnitBytes;
-    const bool vec = p.Gn % S::GU == 0;
-    p.meta_slot = 32u * (vec ? S::MB : S::WIN * 16);
+    // The largest piece of scales that rows and units are multiples of.  Before -> after (window or whole units only): gate and up of
+    // q4 11008 x 2816 groups of 128, two pieces of 4 bytes, one row 9.5 -> 8.0 us, four rows 13.4 -> 11.8; 9000 x 2816 groups of 64, two of 8,
+    // 8.9 -> 7.9 and 12.6 -> 11.4; 6000 x 2688 groups of 32, four of 8, 8.4 -> 8.2 and 12.8 -> 12.1; q8 8192 x 3008 groups of 32, four of 4,
+    // four rows 18.3 -> 17.7.  More copies than that cost more than the window: one row of the last 12.74 -> 12.78, eight pieces of 4
+    // bytes (q4 5003 x 2624 groups of 32) one row 8.2 -> 8.6.
+    constexpr int P4 = S::MB <= (NB == 1 ? 8 : 16) ? 4 : 0, P8 = S::MB >= 8 ? 8 : P4, P16 = S::MB >= 16 ? 16 : P8;
+    int pb = P16;
+    while (pb > 0 && p.Gn * 2 % pb != 0) pb = pb == 16 ? P8 : pb == 8 ? P4 : 0;
+    const int form = pb == 16 ? 3 : pb == 8 ? 2 : pb == 4 ? 1 : 0;
+    p.meta_slot = 32u * (form ? S::MB : S::WIN * 16);
     // a CTA per SM, fewer only when a CTA would own less than four rows
     const int grid = std::max(1, std::min(sm_count(), (p.N + 3) / 4));
     p.rows_lo = p.N / grid;
@@ -685,16 +696,19 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
 
     const bool packets = p.tp_in.world > 0 && p.tp_in.packets;
     using KernelFn = void (*)(I8Params);
-    static const KernelFn kernels[2][2] = {{qgemv_i8_kernel<BITS, LOGG, NB, false, false>, qgemv_i8_kernel<BITS, LOGG, NB, false, true>},
-                                           {qgemv_i8_kernel<BITS, LOGG, NB, true, false>, qgemv_i8_kernel<BITS, LOGG, NB, true, true>}};
-    KernelFn kernel = kernels[packets][vec];
-    static bool configured[4][64] = {};   // per instantiation and device; a race only repeats the call
+    static const KernelFn kernels[2][4] = {
+        {qgemv_i8_kernel<BITS, LOGG, NB, false, 0>, qgemv_i8_kernel<BITS, LOGG, NB, false, P4>, qgemv_i8_kernel<BITS, LOGG, NB, false, P8>,
+         qgemv_i8_kernel<BITS, LOGG, NB, false, P16>},
+        {qgemv_i8_kernel<BITS, LOGG, NB, true, 0>, qgemv_i8_kernel<BITS, LOGG, NB, true, P4>, qgemv_i8_kernel<BITS, LOGG, NB, true, P8>,
+         qgemv_i8_kernel<BITS, LOGG, NB, true, P16>}};
+    KernelFn kernel = kernels[packets][form];
+    static bool configured[8][64] = {};   // per instantiation and device; a race only repeats the call
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!configured[packets * 2 + vec][dev & 63]) {
+    if (!configured[packets * 4 + form][dev & 63]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()) != cudaSuccess)
             return B200Q_ERR_LAUNCH;
-        configured[packets * 2 + vec][dev & 63] = true;
+        configured[packets * 4 + form][dev & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);

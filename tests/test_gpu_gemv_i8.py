@@ -55,6 +55,26 @@ def test_largest_digit_sums(cuda, bits, G, rows):
         assert rel_l2(got, want) <= 2.0 ** -11
 
 
+@pytest.mark.parametrize("bits,G", [(4, 32), (4, 64), (4, 128), (8, 32), (8, 64), (8, 128)])
+@pytest.mark.parametrize("units,tail", [(1, 1), (1, 2), (2, 4), (2, 8), (3, 4), (7, 6), (22, 2), (22, 7)])
+def test_rows_that_end_inside_a_unit(cuda, bits, G, units, tail):
+    """Rows of scales that start at multiples of 2, 4, 8 or 16 bytes: the same bits as rows that are padded to whole units, whose added
+    activations are zero and whose codes and scales are anything."""
+    per_unit = 2048 // bits // G
+    groups = (units - 1) * per_unit + min(tail, per_unit - 1)
+    K, Kp, N = groups * G, units * per_unit * G, 148 * 34 + 11 if units <= 7 else 148 * 20 + 5
+    w, s, z = (t.to(cuda) for t in synth.quantized_weight(N, Kp, bits, G, seed=units + G))
+    x = torch.zeros((4, Kp), dtype=torch.float16, device=cuda)
+    x[:, :K] = synth.activations((4, K), 3, cuda)
+    for rows in (1, 2, 4) if units <= 7 else (1, 2):      # (four rows of 22 units can exceed an SM's shared memory: another kernel)
+        for zeros in (z, None):
+            want = quant_ops.matvec_rows(bits, x[:rows].contiguous(), w, s, zeros, G)
+            got = quant_ops.matvec_rows(bits, x[:rows, :K].contiguous(), w[:, :K * bits // 8].contiguous(), s[:, :groups].contiguous(),
+                                        None if zeros is None else zeros[:, :groups].contiguous(), G)
+            assert torch.equal(got, want)
+    assert cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("power", [120, 100, -60, -100])
 def test_bf16_rows_near_both_ends_of_the_range(cuda, power):
     """bf16 rows times a power of two give the same results times that power, bit for bit, as long as these are in range."""
