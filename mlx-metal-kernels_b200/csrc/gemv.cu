@@ -196,7 +196,7 @@ int rows_to_fp16(const void* x, void* out, float* scale, int rows, int K, cudaSt
 int dispatch_fast(int bits, GemvParams& p, bool gate_up, cudaStream_t stream) {
     if (p.B <= 4 && tuning_get("gemv.i8") >= 0) {
         const int rc = bits == 4 ? gemv_i8_q4(p, gate_up, stream) : gemv_i8_q8(p, gate_up, stream);
-        if (rc != B200Q_ERR_UNSUPPORTED) return rc;      // three or four long rows do not fit into its shared memory
+        if (rc != B200Q_ERR_UNSUPPORTED) return rc;      // rows that do not fit into its shared memory
     }
     if (p.B > 16) return B200Q_ERR_UNSUPPORTED;
     return bits == 4 ? gemv_fast_q4(p, gate_up, stream) : gemv_fast_q8(p, gate_up, stream);

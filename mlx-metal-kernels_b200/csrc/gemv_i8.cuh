@@ -33,12 +33,19 @@
 // The units' sums meet in shared memory and are added in k order: the order does not depend on the CTA, the tile or the
 // number of rows, so a tensor-parallel shard reproduces the unsharded rows bit for bit.
 //
+// Long rows (several rounds of 512 threads into fixed point, or more digits than fit into an SM's shared memory): a pair of CTAs owns twice
+// the rows and each of them half of every row (KS = 2), so each prepares half of the digits.  The second CTA's sums go straight into the
+// first one's shared memory, unit by unit, and are added there in the same order: the same bits.  Before -> after: q4 4096 x 14336 one row
+// 10.0 -> 9.5 us, two 13.1 -> 11.6, four 22.5 -> 15.6 (those had to take the older kernel); 4096 x 11008 three rows 14.7 -> 12.7, four
+// 24.9 -> 13.5; q8 4096 x 14336 four rows 26.5 -> 20.1; 4096 x 4096 four rows 7.6 -> 7.2, but one row 4.8 -> 5.2: not split.
+//
 // Compiled into one translation unit per code width.
 #pragma once
 
 #include "gemv_params.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 namespace b200q {
@@ -194,6 +201,15 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, 
     }
 }
 
+// All threads of the KS CTAs of a cluster.
+template <int KS> __device__ __forceinline__ void i8_sync() {
+    if constexpr (KS == 1) __syncthreads();
+    else asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void st_first_cta(uint32_t addr, float v) {      // the same place in the cluster's first CTA
+    asm volatile("{ .reg .b32 a; mapa.shared::cluster.u32 a, %0, 0; st.shared::cluster.f32 [a], %1; }" ::"r"(addr), "f"(v) : "memory");
+}
+
 // This lane's A operands of one group of 16 rows, rows g and g + 8 at `a_addr` (+ 512): mma i of the group.
 template <int BITS, int LOGG> struct I8Words {
     static constexpr int GB = (1 << LOGG) * BITS / 8;
@@ -244,8 +260,8 @@ template <int BITS, int LOGG> struct I8Shape {
 
 // PB: bytes of a piece of scales, 16, 8 or 4, where rows of scales (and the units in them) start at multiples of it: pieces then lie in
 // shared memory as the affine step wants them, eight groups to a load.  0: rows that start anywhere; an aligned window is copied and read
-// one value at a time.  (One kernel with a run-time switch: gate and up of 14336 x 4096 13.7 us instead of 13.3.)
-template <int BITS, int LOGG, int NB, bool PACKETS, int PB>
+// one value at a time.  KS: CTAs per row, 1 or 2.  (One kernel with a run-time switch: gate and up of 14336 x 4096 13.7 us instead of 13.3.)
+template <int BITS, int LOGG, int NB, bool PACKETS, int PB, int KS>
 __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
     using S = I8Shape<BITS, LOGG>;
@@ -262,12 +278,16 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
     float* part = reinterpret_cast<float*>(smem + p.off_part);     // [tiles of a batch][mats][units][16 rows][NB]
     uint16_t* resid = reinterpret_cast<uint16_t*>(smem + p.off_res);
 
-    const int cta = blockIdx.x;
+    const int rank = KS == 1 ? 0 : blockIdx.x % KS;
+    const int cta = blockIdx.x / KS;
     const int r_lo = cta * p.rows_lo + min(cta, p.rem);
     const int r_cnt = p.rows_lo + (cta < p.rem ? 1 : 0);
     const int n_tiles = (r_cnt + 15) >> 4;
     const int tile_rows = (r_cnt + n_tiles - 1) / n_tiles;
-    const int U = p.units, mats = p.mats, B = p.B, Gn = p.Gn;
+    const int u_lo = KS == 1 ? 0 : rank * ((p.units + 1) / 2);                        // this CTA's units of a row
+    const int U = KS == 1 ? p.units : rank == 0 ? (p.units + 1) / 2 : p.units / 2;
+    const int mats = p.mats, B = p.B, Gn = p.Gn;
+    if (KS > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (waited for before the first access to the other's memory)
 
     if (threadIdx.x < (S::XU + 128) / 16) *reinterpret_cast<uint4*>(smem + p.off_zero + threadIdx.x * 16) = make_uint4(0u, 0u, 0u, 0u);
     pdl_launch_dependents();
@@ -290,15 +310,16 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
         if (nu.tile < n_tiles) {
             const int row0 = r_lo + nu.tile * tile_rows;
             const int rows = min(tile_rows, r_lo + r_cnt - row0);
-            const int left = p.row_bytes - nu.i * kI8UnitBytes - t * 16;
-            srcA = p.w[nu.m] + ((int64_t)row0 * p.row_bytes + (nu.i * kI8UnitBytes + lane_w));
+            const int u = nu.i + u_lo;
+            const int left = p.row_bytes - u * kI8UnitBytes - t * 16;
+            srcA = p.w[nu.m] + ((int64_t)row0 * p.row_bytes + (u * kI8UnitBytes + lane_w));
             leftA = g < rows ? left : 0;
             leftB = g + 8 < rows ? left : 0;
             const __half* mb = t < 2 ? p.s[nu.m] : p.z[nu.m];
             if (m_row < rows) {
                 const int64_t first = (int64_t)(row0 + m_row) * Gn;
-                const int64_t at = (first + nu.i * GU) * 2;
-                if (VEC) leftM = (Gn - nu.i * GU) * 2;
+                const int64_t at = (first + u * GU) * 2;
+                if (VEC) leftM = (Gn - u * GU) * 2;
                 else leftM = (int)min((int64_t)(WIN * 16), (first + Gn) * 2 - (at & ~(int64_t)15));
                 srcM = reinterpret_cast<const uint8_t*>(mb) + (VEC ? at : at & ~(int64_t)15);
                 if (mb == nullptr) leftM = -1;
@@ -356,7 +377,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
     const int total = B * pieces;
     auto row_of = [&](int it) { return NB == 1 ? 0 : it / pieces; };
     auto load_item = [&](int it, uint32_t (&w)[4]) -> bool {
-        const int b = row_of(it), k = (it - b * pieces) * 8;
+        const int b = row_of(it), k = (it - b * pieces) * 8 + u_lo * (GU * G);
         w[0] = w[1] = w[2] = w[3] = 0u;
         if (k < p.K) i8_load_z<PACKETS>(p, (int64_t)b * p.K + k, xsrc, w);
         return k < p.K;
@@ -379,7 +400,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
 #pragma unroll 1
     for (int it = threadIdx.x; it < total; it += kI8Threads) {      // whole warps (shuffles below)
         const int b = row_of(it), pc = it - b * pieces;
-        const int k = pc * 8;
+        const int k = pc * 8 + u_lo * (GU * G);
         const int64_t idx = (int64_t)b * p.K + k;
         uint32_t w[4];
         const bool live = load_item(it, w);
@@ -442,6 +463,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
         }
     }
     __syncthreads();
+    if (KS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
     // ---------------- per-lane constants of the consumer ----------------
     const int col_b = g >> 2;                          // batch row of this lane's B column inside a tile; one batch row: parity of the group
@@ -471,7 +493,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
         while (cu.tile < t1) {
             uint32_t m_s0 = meta0 + cmeta + m_lane, m_s1 = m_s0 + 8 * m_stride;
             if (!VEC) {
-                const uint32_t e = (uint32_t)(r_lo + cu.tile * tile_rows + g) * (uint32_t)Gn + cu.i * GU;      // low bits are enough
+                const uint32_t e = (uint32_t)(r_lo + cu.tile * tile_rows + g) * (uint32_t)Gn + (cu.i + u_lo) * GU;      // low bits are enough
                 m_s0 += (e * 2) & 15u;
                 m_s1 += ((e + 8u * Gn) * 2) & 15u;
             }
@@ -571,7 +593,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                 issue(c, meta0 + (cmeta ^ p.meta_slot));
             }
             // ---- the unit's sums into their place ----
-            float* dst = part + ((size_t)((cu.tile - t0) * mats + cu.m) * U + cu.i) * (16 * NB);
+            float* dst = part + ((size_t)((cu.tile - t0) * mats + cu.m) * p.units + cu.i + u_lo) * (16 * NB);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -579,24 +601,28 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                     float v = y[nt][h] * (float)(1 << kI8Shift);
                     v += __shfl_xor_sync(0xffffffffu, v, 1);
                     if (NB == 1) v += __shfl_xor_sync(0xffffffffu, v, 2);
-                    if ((NB == 1 ? t == 0 : (t & 1) == 0)) dst[(g + 8 * h) * NB + (NB == 1 ? 0 : 2 * nt + (t >> 1))] = v;
+                    if ((NB == 1 ? t == 0 : (t & 1) == 0)) {
+                        float* at = dst + (g + 8 * h) * NB + (NB == 1 ? 0 : 2 * nt + (t >> 1));
+                        if constexpr (KS == 1) *at = v;
+                        else st_first_cta(smem_u32(at), v);
+                    }
                 }
             cu = nu;
             cmeta ^= p.meta_slot;
         }
-        __syncthreads();
+        i8_sync<KS>();
         // ---- rows of these tiles: units added in k order, clamp, round, residual add or SwiGLU, store ----
         const float fmax_act = p.act_dtype == B200Q_F16 ? 65504.0f : 3.3895313892515355e38f;
         const int rb0 = t0 * tile_rows, n_rows = min(r_cnt, t1 * tile_rows) - rb0;
-        for (int it = threadIdx.x; it < n_rows * B; it += kI8Threads) {
+        for (int it = threadIdx.x; it < (rank == 0 ? n_rows * B : 0); it += kI8Threads) {
             const int b = NB == 1 ? 0 : it / n_rows, rr = it - b * n_rows;
             const int tl = rr / tile_rows, r = rr - tl * tile_rows;
-            const float* src = part + (size_t)tl * mats * U * (16 * NB) + r * NB + b;
+            const float* src = part + (size_t)tl * mats * p.units * (16 * NB) + r * NB + b;
             float val[2] = {0.0f, 0.0f};
             for (int m = 0; m < mats; ++m) {
                 float sum = 0.0f;
 #pragma unroll 8
-                for (int i = 0; i < U; ++i) sum += src[(m * U + i) * (16 * NB)];
+                for (int i = 0; i < p.units; ++i) sum += src[(m * p.units + i) * (16 * NB)];
                 val[m] = i8_round_act(fminf(fmaxf(sum, -fmax_act), fmax_act), p.act_dtype);
             }
             const int row = r_lo + rb0 + rr;
@@ -629,7 +655,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                 }
             }
         }
-        if (t1 < n_tiles || p.tp_out.world > 0) __syncthreads();      // the sums have been read / all peer stores are issued
+        if (t1 < n_tiles || p.tp_out.world > 0) i8_sync<KS>();      // the sums have been read / all peer stores are issued
     }
     if (p.tp_out.world > 0 && warp == 0) {
         if (p.tp_out.packets) tp_finish_writer_packets(p.tp_out, lane);
@@ -665,16 +691,19 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
     while (pb > 0 && p.Gn * 2 % pb != 0) pb = pb == 16 ? P8 : pb == 8 ? P4 : 0;
     const int form = pb == 16 ? 3 : pb == 8 ? 2 : pb == 4 ? 1 : 0;
     p.meta_slot = 32u * (form ? S::MB : S::WIN * 16);
-    // a CTA per SM, fewer only when a CTA would own less than four rows
-    const int grid = std::max(1, std::min(sm_count(), (p.N + 3) / 4));
-    p.rows_lo = p.N / grid;
-    p.rem = p.N % grid;
-    const int r_max = p.rows_lo + (p.rem ? 1 : 0);
+    const bool packets = p.tp_in.world > 0 && p.tp_in.packets;
+    int ks = 1;
     const int tile_bytes = p.mats * p.units * 16 * NB * 4;
-    p.batch = std::min((r_max + 15) / 16, std::max(1, 24 * 1024 / tile_bytes));
-    p.xstride = (uint32_t)p.units * S::XU;
-    p.cstride = (uint32_t)p.units * S::GU * 16 + (q.B > 1 ? 32 : 0);      // + 32: two batch rows are read together, from different banks
+    int grid = 1;
     auto plan = [&]() -> uint32_t {
+        // a CTA (or half a pair) per SM, fewer only when it would own less than four rows
+        grid = std::max(1, std::min(sm_count() / ks, (p.N + 3) / 4));
+        p.rows_lo = p.N / grid;
+        p.rem = p.N % grid;
+        const int r_max = p.rows_lo + (p.rem ? 1 : 0), units = (p.units + ks - 1) / ks;
+        p.batch = std::min({(r_max + 15) / 16, std::max(1, (ks == 1 ? 24 : 64) * 1024 / tile_bytes), p.batch});
+        p.xstride = (uint32_t)units * S::XU;
+        p.cstride = (uint32_t)units * S::GU * 16 + (q.B > 1 ? 32 : 0);      // + 32: two batch rows are read together, from different banks
         uint32_t off = i8_align((uint32_t)q.B * p.units * S::GU * (S::G / 8) / 32 * 4, 128);
         p.off_zero = off;  off += S::XU + 128;
         p.off_xd = off;    off += i8_align((uint32_t)q.B * p.xstride, 128);
@@ -687,39 +716,72 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
         p.off_ring = off;
         return std::max<uint32_t>(off + kI8Warps * 4096, kI8OnePerSm);
     };
-    uint32_t off = plan();
-    while (off > (uint32_t)max_smem_optin() && p.batch > 1) {      // long rows: fewer tiles whose sums lie in shared memory together
-        --p.batch;
-        off = plan();
+    auto fit = [&](int parts) -> uint32_t {
+        ks = parts;
+        p.batch = INT_MAX;
+        uint32_t off = plan();
+        while (off > (uint32_t)max_smem_optin() && p.batch > 1) {      // long rows: fewer tiles whose sums lie in shared memory together
+            --p.batch;
+            off = plan();
+        }
+        return off;
+    };
+    // Rounds of the three phases in a CTA: rows into fixed point, units, results.  A pair of CTAs costs a launch about as much as one round
+    // of the first (0.45 us), so two rounds less are asked for.  (A fused norm needs the whole row in each CTA.)
+    auto rounds = [&]() -> int {
+        const int units = (p.units + ks - 1) / ks, r_max = p.rows_lo + (p.rem ? 1 : 0), tiles = (r_max + 15) / 16;
+        auto per = [](int n, int by) { return (n + by - 1) / by; };
+        return per(q.B * units * S::GU * (S::G / 8), kI8Threads) + per(tiles * p.mats * units, kI8Warps) + per(r_max * q.B, kI8Threads);
+    };
+    uint32_t off = fit(1);
+    if (p.norm_w == nullptr && p.units >= 4) {
+        const bool fits = off <= (uint32_t)max_smem_optin();
+        const int one = rounds();
+        const uint32_t off2 = fit(2);
+        if (off2 <= (uint32_t)max_smem_optin() && (!fits || one - rounds() >= 2)) off = off2;
+        else off = fit(1);
     }
     if (off > (uint32_t)max_smem_optin()) return B200Q_ERR_UNSUPPORTED;
 
-    const bool packets = p.tp_in.world > 0 && p.tp_in.packets;
     using KernelFn = void (*)(I8Params);
-    static const KernelFn kernels[2][4] = {
-        {qgemv_i8_kernel<BITS, LOGG, NB, false, 0>, qgemv_i8_kernel<BITS, LOGG, NB, false, P4>, qgemv_i8_kernel<BITS, LOGG, NB, false, P8>,
-         qgemv_i8_kernel<BITS, LOGG, NB, false, P16>},
-        {qgemv_i8_kernel<BITS, LOGG, NB, true, 0>, qgemv_i8_kernel<BITS, LOGG, NB, true, P4>, qgemv_i8_kernel<BITS, LOGG, NB, true, P8>,
-         qgemv_i8_kernel<BITS, LOGG, NB, true, P16>}};
-    KernelFn kernel = kernels[packets][form];
-    static bool configured[8][64] = {};   // per instantiation and device; a race only repeats the call
+    static const KernelFn kernels[4][4] = {
+        {qgemv_i8_kernel<BITS, LOGG, NB, false, 0, 1>, qgemv_i8_kernel<BITS, LOGG, NB, false, P4, 1>,
+         qgemv_i8_kernel<BITS, LOGG, NB, false, P8, 1>, qgemv_i8_kernel<BITS, LOGG, NB, false, P16, 1>},
+        {qgemv_i8_kernel<BITS, LOGG, NB, true, 0, 1>, qgemv_i8_kernel<BITS, LOGG, NB, true, P4, 1>,
+         qgemv_i8_kernel<BITS, LOGG, NB, true, P8, 1>, qgemv_i8_kernel<BITS, LOGG, NB, true, P16, 1>},
+        {qgemv_i8_kernel<BITS, LOGG, NB, false, 0, 2>, qgemv_i8_kernel<BITS, LOGG, NB, false, P4, 2>,
+         qgemv_i8_kernel<BITS, LOGG, NB, false, P8, 2>, qgemv_i8_kernel<BITS, LOGG, NB, false, P16, 2>},
+        {qgemv_i8_kernel<BITS, LOGG, NB, true, 0, 2>, qgemv_i8_kernel<BITS, LOGG, NB, true, P4, 2>,
+         qgemv_i8_kernel<BITS, LOGG, NB, true, P8, 2>, qgemv_i8_kernel<BITS, LOGG, NB, true, P16, 2>}};
+    const int kind = (ks - 1) * 2 + packets;
+    KernelFn kernel = kernels[kind][form];
+    static bool configured[16][64] = {};   // per instantiation and device; a race only repeats the call
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!configured[packets * 4 + form][dev & 63]) {
+    if (!configured[kind * 4 + form][dev & 63]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()) != cudaSuccess)
             return B200Q_ERR_LAUNCH;
-        configured[packets * 4 + form][dev & 63] = true;
+        configured[kind * 4 + form][dev & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(grid * ks);
     cfg.blockDim = dim3(kI8Threads);
     cfg.dynamicSmemBytes = off;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (ks > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim = {(unsigned)ks, 1, 1};
+        ++na;
+    }
+    if (!tuning_get("no_pdl")) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = tuning_get("no_pdl") ? 0 : 1;
+    cfg.numAttrs = na;
     if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return B200Q_ERR_LAUNCH;
     return finish_launch();
 }

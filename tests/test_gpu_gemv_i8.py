@@ -75,6 +75,23 @@ def test_rows_that_end_inside_a_unit(cuda, bits, G, units, tail):
     assert cabi.device_status() == 0
 
 
+@pytest.mark.parametrize("bits,K,G,N", [(4, 14336, 64, 1000), (4, 14336, 32, 5), (8, 7200, 32, 4101), (4, 11008, 128, 700), (8, 14336, 64, 9)])
+def test_long_rows_by_pairs_of_ctas(cuda, bits, K, G, N):
+    """Rows that two CTAs share, also for gate/up; two and three rows, which may have a CTA to themselves, give the same bits as among four,
+    whose digits do not fit one CTA (but for the rows of 7200).  Against the oracle: fp32 sums rounded to fp16, below 2^-11."""
+    w, s, z = synth.quantized_weight(N, K, bits, G, seed=K + N)
+    x = synth.activations((4, K), 2, "cpu")
+    dev = to_dev(cuda, x, w, s, z)
+    got = quant_ops.matvec_rows(bits, *dev, G)
+    assert rel_l2(got, _ref(bits)(x, w, s, z, group_size=G)) <= 1e-3
+    for rows in (2, 3):
+        assert torch.equal(quant_ops.matvec_rows(bits, dev[0][:rows].contiguous(), *dev[1:], G), got[:rows])
+    assert rel_l2(quant_ops.matvec_rows(bits, dev[0][:1].contiguous(), *dev[1:], G), got[:1]) <= 2.0 ** -10
+    both = quant_ops.gate_up_rows(bits, dev[0], dev[1], dev[1], dev[2], dev[2], dev[3], dev[3], G, want_gate_up=True, want_act=False)
+    assert torch.equal(both["gate"], got) and torch.equal(both["up"], got)
+    assert cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("power", [120, 100, -60, -100])
 def test_bf16_rows_near_both_ends_of_the_range(cuda, power):
     """bf16 rows times a power of two give the same results times that power, bit for bit, as long as these are in range."""
