@@ -1010,16 +1010,20 @@ int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
     const bool plain = p.bits == 16, bf = p.q_dtype == B200Q_BF16, g32 = p.G == 32, wide = p.group > 4, sc8 = !plain && ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     // Sixteen warps where eight would have more than a page each: a page costs a warp about a microsecond, the merge of eight more partial
     // results 0.2 (one sequence, one page a warp: q8 5.4 us with eight, 5.7 with sixteen; two sequences of 2048 tokens 9.2 and 8.5).
+    // Whether their rings fit is asked of the UNSHARDED cache's scales, like the choice of the kernel: the number of warps is part of the
+    // summation order, and a shard's narrower scale rows would let it have sixteen where the unsharded call has eight.
     int warps = !plain && (p.walk_pages > p.S * 8 || p.window > 0) ? kClusterWarps : 8;
+    auto slot_for = [&](int hs) { return split_slot_bytes(p.bits, 1, 0) + (plain ? 0u : align_up_u32(2 * split_scale_bytes(hs, p.Gd), p.bits == 4 ? 512 : 1024)); };
     p.hs = std::min(p.Hkv, kAttnWarps);
-    p.slot_bytes = split_slot_bytes(p.bits, 1, 0) + (plain ? 0u : align_up_u32(2 * split_scale_bytes(p.hs, p.Gd), p.bits == 4 ? 512 : 1024));
+    p.slot_bytes = slot_for(p.hs);
+    const uint32_t slot_full = slot_for((int)std::min<int64_t>((int64_t)p.Hkv * std::max(1, tuning_get("ts.tp_world")), kAttnWarps));
     // shared memory: [1 KB alignment] rings, barriers, query rows, the CTAs' partials
     const uint32_t q_bytes = align_up_u32((uint32_t)p.group * 128 * 2, 128), c_bytes = align_up_u32((uint32_t)p.S * p.group * 130 * 4, 128);
     const uint32_t cap = (uint32_t)max_smem_optin(), fixed = 1024 + 128 * 8 + q_bytes + c_bytes;
-    auto depth = [&]() { return (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (warps * p.slot_bytes)); };
-    if (depth() < 2 && p.window == 0) warps = 8;
-    p.stages = depth();
-    if (p.stages < 2) return B200Q_ERR_UNSUPPORTED;
+    auto depth = [&](uint32_t slot_bytes) { return (int)std::min<uint32_t>(kMaxClusterRing, (cap - std::min(cap, fixed)) / (warps * slot_bytes)); };
+    if (depth(slot_full) < 2 && p.window == 0) warps = 8;
+    if (depth(slot_full) < 2) return B200Q_ERR_UNSUPPORTED;
+    p.stages = depth(p.slot_bytes);
     p.off_bars = warps * p.stages * p.slot_bytes;
     p.off_q = p.off_bars + 128 * 8;
     p.off_cpart = p.off_q + q_bytes;

@@ -297,6 +297,37 @@ def test_both_sides_of_the_cluster_rule(cuda, batch, Hkv, tokens):
     assert cabi.device_status() == 0
 
 
+@pytest.mark.parametrize("bits,G,Hq,Hkv,world", [(8, 32, 64, 8, 2), (8, 32, 64, 8, 8), (8, 64, 64, 8, 2), (4, 32, 64, 8, 4), (8, 32, 32, 8, 2), (8, 32, 64, 16, 2)])
+@pytest.mark.parametrize("tokens,window", [(800, 0), (1500, 0), (4096, 0), (1500, 600), (3000, 1024)])
+def test_head_shards_reproduce_the_unsharded_rows(cuda, bits, G, Hq, Hkv, world, tokens, window):
+    """One rank's kv heads give the unsharded call's rows bit for bit, whatever its narrower scale rows leave room for: dense calls with
+    walks of one page and more a warp, and with a window."""
+    sparse_ops = importlib.import_module("mlx_metal_kernels_b200.ops.sparse_attention_ops")
+    case = _case_with_lengths([tokens], Hkv, 128, 16, bits, G, seed=tokens + world)
+    q = synth.activations((1, 1, Hq, 128), 83).to(cuda)
+
+    def call(case, q):
+        cache = _device_cache(case, cuda)
+        if window:
+            pattern = sparse_ops.SparseAttentionPattern("sliding_window_sink", window_size=window, sink_tokens=4)
+            return pq_ops.sparse_paged_quantized_kv_gqa_decode_attention(q, cache, pattern)
+        return pq_ops.paged_quantized_kv_gqa_decode_attention(q, cache, backend="cuda")
+
+    want = call(case, q)
+    local, rows = Hkv // world, Hq // world
+    cabi.set_tuning("ts.tp_world", world)
+    try:
+        for rank in (0, world - 1):
+            shard = dict(case, original_page_shape=(*case["original_page_shape"][:2], local, 128))
+            for name in ("k_pages_q", "v_pages_q", "k_scales", "v_scales"):
+                shard[name] = case[name][:, :, rank * local:(rank + 1) * local].contiguous()
+            got = call(shard, q[:, :, rank * rows:(rank + 1) * rows].contiguous())
+            assert torch.equal(got, want[:, :, rank * rows:(rank + 1) * rows])
+    finally:
+        cabi.set_tuning("ts.tp_world", 0)
+    assert cabi.device_status() == 0
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("block_size", [16, 32, 64, 8, 24])
 @pytest.mark.parametrize("Hq,Hkv,D,P", [(8, 2, 128, 16), (32, 8, 128, 16), (6, 3, 64, 8)])
