@@ -60,8 +60,9 @@ constexpr int kI8MaxRes = 1024;               // residual values kept in shared 
 // and no conversion is needed.
 constexpr uint32_t kI8MagicBits = 0x4B400000u;
 constexpr float kI8Magic = 12582912.0f;       // 1.5 * 2^23
-// Digit sums are taken times 2^-kI8Shift until the end of a unit, so that kI8Magic times a digit's weight stays finite for every finite row.
-constexpr int kI8Shift = 20;
+// Sums are taken times 2^-kI8Shift until the end of a unit: codes times values of up to 2^123, whose sums per group are still finite, stay below
+// 2^138.  More would cost the smallest results: the sums' steps are 2^(kI8Shift - 149), and bf16 results have steps of 2^-133.
+constexpr int kI8Shift = 10;
 
 struct I8Params {
     const void* x;          // [B, K]
@@ -544,14 +545,16 @@ __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_co
                 const float s0 = scale_of(sw0, m_s0, f), s1 = scale_of(sw1, m_s1, f), z0 = scale_of(zw0, m_z0, f), z1 = scale_of(zw1, m_z1, f);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    if (f % CV == 0) s_ldw<2 * CV>(cc[nt] + f * 8, cw[nt]);
-                    const float w0 = __uint_as_float(cw[nt][f % CV * 2]), xf = __uint_as_float(cw[nt][f % CV * 2 + 1]), w1 = w0 * k_mid, off = w0 * k_off;
+                    if (NB != 4 && f % CV == 0) s_ldw<2 * CV>(cc[nt] + f * 8, cw[nt]);
                     float c[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) c[e] = __int_as_float(NB == 1 ? (t >> 1 ? acc[AC - 1][e] : acc[0][e]) : acc[nt % AC][e]);
-                    const float f0 = fmaf(c[1], w1, fmaf(c[0], w0, off)), f1 = fmaf(c[3], w1, fmaf(c[2], w0, off));
-                    y[nt][0] = fmaf(s0, fmaf(-z0, xf, f0), y[nt][0]);
-                    y[nt][1] = fmaf(s1, fmaf(-z1, xf, f1), y[nt][1]);
+                    // the magic number goes first: times the weight of a large row it would not be finite
+                    const float f0 = fmaf(c[1], k_mid, c[0] + k_off), f1 = fmaf(c[3], k_mid, c[2] + k_off);
+                    if (NB == 4 && f % CV == 0) s_ldw<2 * CV>(cc[nt] + f * 8, cw[nt]);
+                    const float w0 = __uint_as_float(cw[nt][f % CV * 2]), xf = __uint_as_float(cw[nt][f % CV * 2 + 1]);
+                    y[nt][0] = fmaf(s0, fmaf(-z0, xf, f0 * w0), y[nt][0]);
+                    y[nt][1] = fmaf(s1, fmaf(-z1, xf, f1 * w0), y[nt][1]);
                 }
             };
             // Digits of two mma per load.  One batch row: the lanes of columns 0-3 hold the even group's, those of columns 4-7 the odd group's,

@@ -103,6 +103,47 @@ def test_bf16_rows_near_both_ends_of_the_range(cuda, power):
     assert torch.equal(far.float() * 2.0 ** -power, near.float())
 
 
+def _exact(x, w, s, z, bits, G):
+    N, K = w.shape[0], x.shape[1]
+    codes = (torch.stack((w & 15, w >> 4), -1).reshape(N, K) if bits == 4 else w).double()
+    dense = (codes.reshape(N, K // G, G) - z.double()[..., None]) * s.double()[..., None]
+    return x.double() @ dense.reshape(N, K).T
+
+
+@pytest.mark.parametrize("bits,K", [(4, 256), (8, 14336)])
+@pytest.mark.parametrize("powers", [(-104, -23), (-110, -17), (-90, -24)])
+def test_small_bf16_rows_with_small_scales(cuda, bits, K, powers):
+    """Results near the lower end of bf16's normal range are right to their own rounding (2^-9) and that of the rows to fixed point (steps of
+    2^-120, 2^-10 of the smallest rows' values here, independent of one another: 2^-11 of the result)."""
+    w, s, z = synth.quantized_weight(70, K, bits, 64, seed=8)
+    s = torch.full_like(s, 2.0 ** powers[1], dtype=torch.float16)
+    x = (synth.activations((4, K), 9, "cpu", torch.bfloat16).double() * 2.0 ** powers[0]).to(torch.bfloat16)
+    for rows in (1, 2, 4):
+        got = quant_ops.matvec_rows(bits, *to_dev(cuda, x[:rows].contiguous(), w, s, z), 64)
+        assert rel_l2(got, _exact(x[:rows], w, s, z, bits, 64)) <= 2.0 ** -9 + 2.0 ** -11
+
+
+@pytest.mark.parametrize("bits,K", [(4, 256), (4, 14336), (8, 14336)])
+def test_large_and_small_bf16_rows_together(cuda, bits, K):
+    """Rows near both ends of bf16's range, and one whose values lie near both, in one call: each is right to its own rounding, and the
+    same bits as by itself."""
+    w, s, z = synth.quantized_weight(70, K, bits, 64, seed=11)
+    s = torch.full_like(s, 2.0 ** -20, dtype=torch.float16)
+    x = synth.activations((4, K), 12, "cpu", torch.bfloat16).double()
+    x[0] *= 2.0 ** 120                        # the sum of a group (at most 64 values of 2^123) stays finite in fp32
+    x[1] *= 2.0 ** -104
+    x[2, :K - 64] *= 2.0 ** 60
+    x[2, K - 64:] *= 2.0 ** 110
+    x = x.to(torch.bfloat16)
+    dev = to_dev(cuda, x, w, s, z)
+    got = quant_ops.matvec_rows(bits, *dev, 64)
+    want = _exact(x, w, s, z, bits, 64)
+    for row in range(4):
+        assert rel_l2(got[row], want[row]) <= 2.0 ** -9 + 2.0 ** -11
+        pair = quant_ops.matvec_rows(bits, dev[0][[row, row]].contiguous(), *dev[1:], 64)
+        assert torch.equal(pair[0], got[row]) and torch.equal(pair[1], got[row])
+
+
 @pytest.mark.parametrize("rows", [1, 2, 4])
 @pytest.mark.parametrize("lo,hi", [(0, 96), (96, 333), (5, 6)])
 def test_row_shards_reproduce_the_unsharded_rows(cuda, rows, lo, hi):
