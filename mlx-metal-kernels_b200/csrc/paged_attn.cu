@@ -16,6 +16,7 @@
 //
 // Everything else (other head dims, other group sizes) runs the simple kernel: one
 // warp per (sequence, query head), the reference's streaming-softmax loop.
+#include "attn_route.h"
 #include "paged_attn_page.cuh"
 #include "tensor_map.cuh"
 
@@ -613,8 +614,8 @@ __global__ void __launch_bounds__(NW * 32, 1) paged_attn_cluster_kernel(const __
         // append k (rotated) and v of kv head h to the page of `pos`: the CTA whose range holds that page
         const int blk = pos >= 0 ? pos / p.P : -1;
         const int owner = (ppc > 0 && blk >= 0) ? min(S - 1, blk / ppc) : 0;
-        if ((int)rank == owner && warp >= 6) {
-            const bool is_v = warp == 7;
+        if ((int)rank == owner && append_role(warp, NW) != kAppendNothing) {
+            const bool is_v = append_role(warp, NW) == kAppendV;
             int page = (blk >= 0 && blk < p.max_blocks) ? p.block_table[(size_t)b * p.max_blocks + blk] : -1;
             if (page < 0 || page >= p.num_pages) {
                 if (lane == 0) atomicMax(&g_device_status, (int)EV_KV_PAGE_UNASSIGNED);

@@ -198,7 +198,7 @@ def test_full_shape_layer_matches_oracle(cuda, batch):
 
 
 @pytest.mark.parametrize("bits,B,Hq,Hkv,poss", [(8, 1, 32, 8, [4096]), (4, 2, 32, 8, [16, 700]), (8, 3, 8, 2, [0, 31, 95]),
-                                               (8, 1, 4, 4, [47]), (4, 5, 16, 8, [3, 200, 15, 16, 1023])])
+                                               (8, 1, 4, 4, [47]), (4, 5, 16, 8, [3, 200, 15, 16, 1023]), (4, 1, 64, 8, [2500])])
 @pytest.mark.parametrize("cluster", [1, -1])
 def test_rope_append_attention_one_call(cuda, bits, B, Hq, Hkv, poss, cluster):
     """b200q_rope_append_paged_gqa_decode (one cluster kernel at small batch, else append + split-KV attention) against
