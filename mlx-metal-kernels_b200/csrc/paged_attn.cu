@@ -945,43 +945,14 @@ inline int subs_for(int hc) { return kAttnWarps % hc == 0 ? kAttnWarps / hc : 1;
 inline bool heads_ok(int Hkv) { return Hkv <= kAttnWarps || Hkv % kAttnWarps == 0; }
 
 // ---- cluster kernel: host side ----
-struct ClusterChoice { int size; bool preferred; };      // size 0: not possible
-// fused: the launch also stands for the append (three launches against one).  split: the split-KV kernels could take the call; without them
-// (no workspace) the rule is the one for tables of any length, so a call is not refused or served by its length.
-ClusterChoice cluster_choice(int B, int Hkv, int max_blocks, bool fused, bool split, bool plain = false) {
-    const int mode = tuning_get("attn.cluster");      // 1: whenever possible, -1: never, 0: by the rule below
-    if (mode < 0 || (mode > 0 && B * Hkv > 65535)) return {0, false};
-    // the choice follows the kv heads of the UNSHARDED cache ("ts.tp_world" equal head shards), so that a
-    // tensor-parallel rank runs the same kernel, and the same summation order, as the unsharded call
-    const int64_t heads = (int64_t)B * Hkv * std::max(1, tuning_get("ts.tp_world"));
-    const int forced = tuning_get("attn.cluster_size");
-    if (forced == 1 || forced == 2 || forced == 4 || forced == 8 || forced == 16) return {mode == 0 && heads * forced > 2 * sm_count() ? 0 : forced, mode > 0 || heads * forced * 4 <= 3 * sm_count()};
-    // Eight CTAs per cluster while the clusters fill at most three quarters of the SMs, whatever the length (the opt-in size 16 is slower at
-    // every length: one sequence of q8, 8 kv heads, sizes 4 / 8 / 16: 1024 tokens 14.3 / 12.3 / 18.4 us, 8192 26.6 / 20.5 / 24.6).
-    if (mode > 0 || heads * 8 * 4 <= 3 * sm_count()) return {8, true};
-    // More heads: as many CTAs per cluster as leave all clusters resident at once, if a warp's walk is short.  A page costs a warp about
-    // one microsecond (it walks alone), the launch 5 us; the split-KV kernel balances ragged batches over all SMs, but with its partial
-    // results and the merge launch takes 9 to 17 us for the shortest ones.  The block table's capacity bounds the walk (the lengths
-    // live on the device).  Split-KV / cluster, us, q4, 8 kv heads, equal lengths and ragged ones down to an eighth: 2 sequences of 2048
-    // tokens 11.1 / 8.2 and 9.1 / 8.1 (of 4096 in q8 13.0 / 12.1 and 11.1 / 11.5: not taken); 7 of 1024 15.7 / 8.2 and 14.4 / 8.0, of 3072
-    // 20.2 / 15.6 and 16.5 / 14.6; 16 of 128 10.5 / 5.8, of 1024 15.1 / 12.6 and 13.4 / 11.1.  Fewer than 8 kv heads cost the split-KV
-    // kernel more: 2 heads, 16 sequences of 4096 tokens 18.7 / 13.1 and 14.5 / 11.4 (of 8192, 7 sequences, 19.3 / 17.8 and 15.4 / 16.8).  With
-    // the append in the same launch the cluster wins 1 to 3 us more (a layer of 2 sequences of 4000 tokens 65.2 / 63.8, 8 of 3000
-    // 91.4 / 86.8, 16 of 1000 89.5 / 87.9).
-    const int kv_full = Hkv * std::max(1, tuning_get("ts.tp_world"));
-    for (int size = 4; split && size >= 1; size /= 2) {
-        if (heads * size * 8 > 7 * (int64_t)sm_count()) continue;
-        const int warps = size * (plain ? 8 : kClusterWarps);      // plain pages: no room for more rings
-        const int walk = (max_blocks + warps - 1) / warps;
-        int longest = 4;
-        if (size == 4 && heads < 24) longest = kv_full >= kAttnWarps ? 2 : 3;
-        if (size == 4 && kv_full < 4) longest = 5;
-        if (size == 2) longest = (int)heads / 10;
-        if (walk <= longest + (fused ? 2 : 0)) return {size, true};
-        break;
-    }
-    // up to two waves of clusters stay possible for callers without a workspace
-    return {heads * 8 <= 2 * sm_count() ? 8 : 0, false};
+ClusterChoice choose_cluster(int B, int Hkv, int group, int max_blocks, AttnUse use, bool split) {
+    ClusterQuery c = {};
+    c.B = B; c.Hkv = Hkv; c.group = group; c.walk_pages = max_blocks; c.use = use; c.split = split;
+    c.tp_world = std::max(1, tuning_get("ts.tp_world"));
+    c.mode = tuning_get("attn.cluster");
+    c.forced_size = tuning_get("attn.cluster_size");
+    c.sms = sm_count();
+    return cluster_choice(c);
 }
 
 // Byte tensor [heads][tokens][row] of a page pool whose token rows are `pitch` bytes apart; box = heads of a CTA x 16 tokens x row.
@@ -1181,7 +1152,7 @@ int launch_split_attention(AttnParams& p, int max_ranges, cudaStream_t stream) {
 
 int attention_stage_launches_impl(int B, int Hkv, int max_blocks, int with_append) {
     if (B <= 0 || Hkv <= 0) return 0;
-    if (B <= 65535 && cluster_choice(B, Hkv, max_blocks, with_append != 0, true).preferred) return 1;
+    if (B <= 65535 && choose_cluster(B, Hkv, 1, max_blocks, with_append != 0 ? AttnUse::kAppend : AttnUse::kDense, true).preferred) return 1;
     return 2 + (with_append ? 1 : 0);
 }
 
@@ -1245,7 +1216,7 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     const int64_t visited = ((int64_t)window_size + 15) / 16 + 1 + ((int64_t)sink_tokens + 15) / 16;
     const int walk_pages = window_size > 0 ? (int)std::min<int64_t>(max_blocks, visited) : max_blocks;
     const bool may = window_size == 0 || (ranges > 0 && window_size < (int64_t)max_blocks * page_size);
-    const ClusterChoice choice = may && B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv, walk_pages, false, ranges > 0) : ClusterChoice{0, false};
+    const ClusterChoice choice = may && B <= 65535 && Hkv <= 65535 ? choose_cluster(B, Hkv, group, walk_pages, window_size > 0 ? AttnUse::kWindow : AttnUse::kDense, ranges > 0) : ClusterChoice{0, false};
     const int cluster = choice.preferred || ranges == 0 ? choice.size : 0;
     if (cluster > 0) {
         ClusterAttnParams c = {};
@@ -1294,7 +1265,7 @@ int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v
     p.group = Hq / Hkv; p.num_pages = num_pages; p.scale = scale; p.q_dtype = dtype; p.bits = 16;
     p.row_bytes = Hkv * kHeadDim * 2;
     p.verdict = verdict;
-    const ClusterChoice choice = B <= 65535 && Hkv <= 65535 ? cluster_choice(B, Hkv, max_blocks, false, true, true) : ClusterChoice{0, false};
+    const ClusterChoice choice = B <= 65535 && Hkv <= 65535 ? choose_cluster(B, Hkv, Hq / Hkv, max_blocks, AttnUse::kPlain, true) : ClusterChoice{0, false};
     if (choice.preferred && choice.size > 0) {
         ClusterAttnParams c = {};
         c.q = q; c.q_dtype = dtype;
@@ -1340,7 +1311,7 @@ int rope_append_attention_impl(const void* qkv, const float* cos_table, const fl
                          ((uintptr_t)k_codes % 16 == 0) && ((uintptr_t)v_codes % 16 == 0) && ((uintptr_t)k_scales % 8 == 0) &&
                          ((uintptr_t)v_scales % 8 == 0);
     const bool two_stages = q_scratch != nullptr && split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, B200Q_F16) > 0;
-    const ClusterChoice choice = fast_ok ? cluster_choice(B, Hkv, max_blocks, true, two_stages) : ClusterChoice{0, false};
+    const ClusterChoice choice = fast_ok ? choose_cluster(B, Hkv, group, max_blocks, AttnUse::kAppend, two_stages) : ClusterChoice{0, false};
     const int cluster = choice.preferred || !two_stages ? choice.size : 0;
     if (cluster > 0) {
         int tp_in_slot = -1, tp_out_slot = -1;
