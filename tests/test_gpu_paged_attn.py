@@ -276,11 +276,13 @@ def test_windows_in_the_cluster_kernel(cuda, bits, size, sink, window):
     assert cabi.device_status() == 0
 
 
-@pytest.mark.parametrize("batch,Hkv,tokens", [(2, 8, 2048), (2, 8, 2064), (4, 8, 4096), (4, 8, 4112), (5, 8, 2048), (5, 8, 2064), (8, 8, 3072),
-                                              (8, 8, 3088), (16, 8, 1024), (16, 8, 1040), (17, 8, 64), (16, 2, 5120), (16, 2, 5136), (40, 2, 300)])
-def test_both_sides_of_the_cluster_rule(cuda, batch, Hkv, tokens):
-    """Lengths at which the choice between one cluster launch and split-KV with a merge changes: whichever runs agrees with the split-KV
-    kernels, also in a table with more room than the sequences need."""
+@pytest.mark.parametrize("batch,Hkv,tokens,launches", [(2, 8, 2032, 1), (2, 8, 2048, 2), (2, 8, 2064, 2), (4, 8, 4080, 1), (4, 8, 4096, 2), (4, 8, 4112, 2),
+                                                       (5, 8, 2032, 1), (5, 8, 2048, 2), (5, 8, 2064, 2), (8, 8, 3056, 1), (8, 8, 3072, 2), (8, 8, 3088, 2),
+                                                       (16, 8, 1008, 1), (16, 8, 1024, 2), (16, 8, 1040, 2), (17, 8, 64, 2), (16, 2, 5104, 1), (16, 2, 5120, 2),
+                                                       (16, 2, 5136, 2), (40, 2, 300, 1)])
+def test_both_sides_of_the_cluster_rule(cuda, batch, Hkv, tokens, launches):
+    """Lengths at which the choice between one cluster launch and split-KV with a merge changes on 148 SMs (the table has one page more than the
+    longest sequence): each side has the number of launches that its kernel takes, and agrees with the split-KV kernels."""
     lengths = [tokens - (i * 37) % tokens for i in range(batch)]
     dcache = _device_cache(_case_with_lengths(lengths, Hkv, 128, 16, 4, 32, seed=tokens), cuda)
     q = synth.activations((batch, 1, Hkv * 4, 128), 80).to(cuda)
@@ -291,9 +293,9 @@ def test_both_sides_of_the_cluster_rule(cuda, batch, Hkv, tokens):
     finally:
         cabi.set_tuning("attn.cluster", 0)
     assert float((got.float() - split.float()).abs().max()) <= ATOL
-    lib = cabi.load()
-    blocks = dcache.block_table.shape[1]
-    assert lib.b200q_attention_launches(batch, Hkv, blocks, 0) <= lib.b200q_attention_stage_launches(batch, Hkv, 0)
+    if torch.cuda.get_device_properties(cuda).multi_processor_count == 148:
+        assert cabi.load().b200q_attention_launches(batch, Hkv, dcache.block_table.shape[1], 0) == launches
+    assert torch.equal(got, split) or launches == 1
     assert cabi.device_status() == 0
 
 

@@ -79,15 +79,24 @@ def test_symmetric_codes_without_zero_points(tcgen05, bits):
     assert rel_l2(got, want) <= TOL
 
 
-@pytest.mark.parametrize("bits,B,N,K,G", [(4, 48, 4096, 2048, 64), (4, 64, 4096, 4096, 64), (8, 48, 3000, 1024, 64), (4, 200, 900, 2816, 32), (4, 250, 4096, 1024, 64)])
-def test_large_partial_sums(cuda, bits, B, N, K, G):
-    """Splits that the launch plan chooses from 33 rows on: partial sums of 64 to 96 KB, through the buffer or the rings; half of the rows as a
-    shard gives the same bits."""
+@pytest.mark.parametrize("bits,B,N,K,G,split", [(4, 48, 4096, 2048, 64, 2), (4, 64, 4096, 4096, 64, 2), (8, 48, 3000, 1024, 64, 1), (4, 200, 900, 2816, 32, 2),
+                                                (4, 250, 4096, 1024, 64, 1), (4, 33, 4096, 8192, 64, 4), (8, 48, 4096, 8192, 64, 4), (4, 64, 4096, 8192, 64, 4)])
+def test_large_partial_sums(cuda, bits, B, N, K, G, split):
+    """Splits that the launch plan chooses from 33 rows on (on 148 SMs): none, two parts, and four with partial sums of 50 and 72 KB in the buffer
+    and 96 KB through the rings.  The plan's result is that of the same split by request, and differs from the one without; half of the
+    rows as a shard gives the same bits."""
     w, s, z = (t.to(cuda) for t in synth.quantized_weight(N, K, bits, G, seed=N + B))
     x = synth.activations((B, K), 8, cuda)
     got = _fn(bits)(x, w, s, z, group_size=G)
     assert rel_l2(got, _ref(bits)(x.cpu(), w.cpu(), s.cpu(), z.cpu(), group_size=G)) <= TOL
     assert torch.equal(_fn(bits)(x, w, s, z, group_size=G), got)
+    if torch.cuda.get_device_properties(cuda).multi_processor_count == 148:
+        for parts in {1, split}:
+            cabi.set_tuning("ts.split", parts)
+            try:
+                assert torch.equal(_fn(bits)(x, w, s, z, group_size=G), got) == (parts == split)
+            finally:
+                cabi.set_tuning("ts.split", 0)
     half = N // 2
     cabi.set_tuning("ts.tp_world", 2)
     try:

@@ -10,23 +10,32 @@ DRIVER = r"""
 #include <cstdio>
 using namespace b200q;
 
-// the loops of the MMA issuers in qgemm_ts.cu
+// the two loops of the MMA issuers in qgemm_ts.cu: two chunks per round of waits (two matrices), and one
 template <int MATS> int replay(int j, int per, int items, int n_ch, int xs, int na) {
     ChunkWalk<MATS> w(j);
-    int bad = 0;
+    int bad = 0, seen = 0, want = 0;
     auto look = [&](int g) {
         const int a = MATS * g + (MATS == 2 ? j : 0);
         bad += w.x.slot != g % xs || w.x.par != ((uint32_t)(g / xs) & 1u) || w.a.slot != a % na || w.a.par != ((uint32_t)(a / na) & 1u);
+        ++seen;
     };
-    for (int it = 0; it < items; ++it)
-        for (int ch = ChunkWalk<MATS>::first(j); ch < n_ch;) {
-            w.to(it * n_ch + ch, xs, na);
-            look(it * n_ch + ch);
-            const bool two = per == 2 && ch + 1 < n_ch;
-            if (two) { w.to(it * n_ch + ch + 1, xs, na); look(it * n_ch + ch + 1); }
-            ch += (two ? 2 : 1) + ChunkWalk<MATS>::kSkip;
+    for (int it = 0; it < items; ++it) {
+        if (MATS == 2 && per == 2) {
+            for (int ch = 0; ch < n_ch; ch += 2) {
+                w.to(it * n_ch + ch, xs, na);
+                look(it * n_ch + ch);
+                const bool two = ch + 1 < n_ch;
+                if (two) { w.to(it * n_ch + ch + 1, xs, na); look(it * n_ch + ch + 1); }
+            }
+        } else {
+            for (int ch = ChunkWalk<MATS>::first(j); ch < n_ch; ch += 1 + ChunkWalk<MATS>::kSkip) {
+                w.to(it * n_ch + ch, xs, na);
+                look(it * n_ch + ch);
+            }
         }
-    return bad;
+        want += MATS == 2 ? n_ch : (n_ch + 1 - j) / 2;
+    }
+    return bad + (seen != want);
 }
 int main() {
     int bad = 0, runs = 0;
