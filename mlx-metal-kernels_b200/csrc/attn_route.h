@@ -21,7 +21,7 @@ enum class AttnUse {
 };
 struct ClusterQuery {
     int B, Hkv, group;          // sequences, kv heads of this process, query heads per kv head
-    int walk_pages;             // pages that a sequence can have to visit: the block table's capacity, or the window's (the lengths live on the device)
+    int walk_pages;             // pages that a sequence can have to visit: the block table's capacity or the window's (lengths live on the device)
     AttnUse use;
     bool split;                 // the split-KV kernels could take the call; without them (no workspace) the rule is the one for tables of any
                                 // length, so a call is not refused or served by its length
@@ -45,12 +45,12 @@ inline ClusterChoice cluster_choice(const ClusterQuery& c) {
     if (heads * 8 * 4 <= 3 * c.sms) {
         // Plain pages and windows only up to the walk at which the split-KV kernels, which use all SMs, become the faster ones: the cluster
         // takes 0.85 us per 1024 tokens whatever the heads, split-KV 0.3 to 0.6 per sequence but starts 2 to 11 us later.
-        // Split-KV / cluster, us, plain pages of one sequence of 8192, 16384 and 65536 tokens: 8 kv heads 12.6 / 12.4, 18.2 / 19.3, 46.4 / 56.7; 4 heads
-        // 11.4 / 11.2, 13.4 / 18.2, 30.0 / 55.8; one head 18.5 / 10.8, 20.2 / 17.0, 31.8 / 55.4; four sequences of 2 heads 17.4 / 12.9, 22.7 / 19.1,
-        // 53.4 / 57.8; eight of one head 28.2 / 15.3, 37.4 / 23.5, 95.5 / 69.5.  q8 windows of 8192 and 16384, one sequence: 8 heads 14.0 / 13.5
-        // and 17.4 / 20.5, 4 heads 12.3 / 13.1 and 17.0 / 19.8, one head 20.1 / 12.8 and 22.7 / 19.1.  More than four query heads per kv head cost the
-        // cluster a quarter more per page; with a number of kv heads that does not divide 8 split-KV starts sooner.  (Dense quantised
-        // calls and the append have this form at any length.)
+        // Split-KV / cluster, us, plain pages of 8192, 16384 and 65536 tokens: one sequence of 8 kv heads 12.6 / 12.4, 18.2 / 19.3, 46.4 / 56.7,
+        // of 4 heads 11.4 / 11.2, 13.4 / 18.2, 30.0 / 55.8, of one 18.5 / 10.8, 20.2 / 17.0, 31.8 / 55.4; four sequences of 2 heads
+        // 17.4 / 12.9, 22.7 / 19.1, 53.4 / 57.8; eight of one head 28.2 / 15.3, 37.4 / 23.5, 95.5 / 69.5.  q8 windows of 8192 and 16384, one
+        // sequence: 8 heads 14.0 / 13.5 and 17.4 / 20.5, 4 heads 12.3 / 13.1 and 17.0 / 19.8, one head 20.1 / 12.8 and 22.7 / 19.1.  More than
+        // four query heads per kv head cost the cluster a quarter more per page; with a number of kv heads that does not divide 8
+        // split-KV starts sooner.  (Dense quantised calls and the append have this form at any length.)
         const bool bounded = c.split && (c.use == AttnUse::kPlain || c.use == AttnUse::kWindow) && c.B < 6;
         if (!bounded) return {8, true};
         const int64_t one = kv >= 8 ? 544 : 8 % kv != 0 ? 288 : std::max(416, 1408 / kv);      // pages, for one sequence

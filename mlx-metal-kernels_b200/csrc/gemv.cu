@@ -128,11 +128,12 @@ bool fast_path_ok(const GemvParams& p) {
 
 // Which kernel takes a launch: "gemv.ts" = 1 sends everything the tcgen05 kernel supports to it, -1 nothing, 0 (default) the batches
 // of gemv.ts_min_batch rows and more.  Default 5: the integer kernel has no instance above four rows, and against the fp16 mma.sync
-// kernel tcgen05 wins from there on (fp16 rows, 14336 x 4096 q4: 15.6 against 19.1 us at five rows; 4096 x 14336: 16.4 against 26.4).
+// kernel tcgen05 wins from there on (fp16 rows, 14336 x 4096 q4: 14.2 against 18.9 us at five rows; 4096 x 14336: 15.0 against 26.2).
 // One region of bf16 rows goes the other way: their weights take two terms there, which doubles the chain of chunks, and with a
-// row tile for more than half of the SMs no K split can shorten it; up to eight rows are one launch of the mma.sync kernel
-// (11008 x 4096 q4, eight rows: 20.4 against 25.4 us, gate and up 28.9 against 42.4; 2048 or 8192 long rows: 18.0 against 15.1,
-// 56.7 against 46.0).
+// row tile for more than half of the SMs no K split can shorten it; up to eight rows are one launch of the mma.sync kernel.
+// mma.sync / tcgen05, us, eight rows of q4, groups of 64: 11008 x 4096 20.4 / 22.2, gate and up 28.6 / 39.5; 11008 x 7168 32.8 / 35.3;
+// outside: 11008 x 2048 15.0 / 13.1, 9344 x 4096 18.7 / 15.7, 2048 x 8192 22.3 / 13.4.  The region is coarse: q8 (14336 x 4096 26.5 / 22.0)
+// and groups of 32 (11008 x 4096 26.0 / 22.7) would be faster with tcgen05 inside it, 11008 x 8192 (34.4 / 39.9) with mma.sync outside.
 bool prefer_ts(const GemvParams& p) {
     const int mode = tuning_get("gemv.ts");
     if (mode < 0) return false;

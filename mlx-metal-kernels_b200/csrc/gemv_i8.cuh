@@ -5,12 +5,11 @@
 // What bounds it: HBM.  At 6.5 TB/s an SM receives 23 bytes, i.e. 46 q4 codes, per clock, so the code path has to stay
 // well below 4 issue slots per 46 codes.  The kernel it replaces for these batches (gemv_fast.cuh) turns every code pair into
 // fp16 (5 logic instructions and 2 mma.sync per 512 codes and row half) and needed 2.2 slots per clock at 0.49 of the
-// copy rate (2 x 14336 x 4096 q4, one row: 20.7 us; here 12.5 us, 0.82).
-// Beside HBM it was loads from shared memory: 13 of them per 1 KB of codes and warp held up the rest (stall "MIO throttle" first, by the
-// counters; without the five of the affine step the same launch ran at the copy rate).  Hence digits in the order of the
-// mma, two mma per 16-byte load, scales eight groups per load, constants two steps per load, 6.5 loads in all, and no conversions in the
-// affine step.  Cold weights, passes back to back, before -> after: q4 2 x 14336 x 4096 one row 14.3 -> 12.5 us, four rows 24.6 -> 20.0;
-// 4096 x 14336 11.2 -> 10.1; 4096 x 4096 5.1 -> 4.8; q8 8192 x 3008 groups of 32 8.9 -> 8.4.
+// copy rate (2 x 14336 x 4096 q4, one row: 20.7 us; here 12.2 us, 0.84).
+// Beside HBM it is loads from shared memory: with 13 of them per 1 KB of codes and warp "MIO throttle" was the first stall.  Hence digits in
+// the order of the mma, two mma per 16-byte load, scales eight groups per load, constants two steps per load, 6.5 loads in all, and no
+// conversions in the affine step.  Cold weights, passes back to back, 13 loads -> now: q4 2 x 14336 x 4096 one row 14.3 -> 12.2 us, four rows
+// 24.6 -> 20.0; 4096 x 4096 one row 5.1 -> 4.8; q8 8192 x 3008 groups of 32 one row 8.9 -> 8.5.
 //   * mma.sync.m16n8k32 u8 x s8: a q4 word gives its even codes with one mask and its odd ones with a shift and a mask, a
 //     q8 word is the operand as it lies.  512 codes per instruction, exact in int32.
 //   * the activations become integers.  Per quantisation group they are scaled by a power of two to 22-bit fixed point
@@ -27,7 +26,7 @@
 // with cp.async into a private ring (4 KB of codes per warp in flight, 64 KB per SM, started before griddepcontrol.wait since
 // weights do not depend on the previous kernel): no producer warps and no barriers in the stream.  While piece c of a unit is
 // consumed, piece c of the warp's next unit takes its place, so all shared-memory addresses are constants.  (Twice the
-// ring in flight gained nothing: 2 x 14336 x 4096 15.7 against 14.9 us, the decode step 1.80 against 1.73 ms.)
+// ring in flight gained nothing: 2 x 14336 x 4096 13.8 against 12.5 us.)
 // One CTA per SM, by its shared memory: with room for two, the CTAs of the next kernel of a dependent chain start beside this
 // one's, and later ones then share an SM while another SM has none (gate/up and down of one row in turn: 36 us against 26.8).
 // The units' sums meet in shared memory and are added in k order: the order does not depend on the CTA, the tile or the
@@ -35,9 +34,9 @@
 //
 // Long rows (several rounds of 512 threads into fixed point, or more digits than fit into an SM's shared memory): a pair of CTAs owns twice
 // the rows and each of them half of every row (KS = 2), so each prepares half of the digits.  The second CTA's sums go straight into the
-// first one's shared memory, unit by unit, and are added there in the same order: the same bits.  Before -> after: q4 4096 x 14336 one row
-// 10.0 -> 9.5 us, two 13.1 -> 11.6, four 22.5 -> 15.6 (those had to take the older kernel); 4096 x 11008 three rows 14.7 -> 12.7, four
-// 24.9 -> 13.5; q8 4096 x 14336 four rows 26.5 -> 20.1; 4096 x 4096 four rows 7.6 -> 7.2, but one row 4.8 -> 5.2: not split.
+// first one's shared memory, unit by unit, and are added there in the same order: the same bits.  One CTA -> a pair: q4 4096 x 14336 one row
+// 10.0 -> 9.5 us, two 13.1 -> 11.5, four 22.5 -> 15.4 (whose digits do not fit one CTA: the older kernel); 4096 x 11008 three rows
+// 14.7 -> 12.9, four 24.9 -> 13.7; q8 4096 x 14336 four rows 26.5 -> 20.2; 4096 x 4096 four rows 7.6 -> 7.1, but one row 4.8 -> 5.2: not split.
 //
 // Compiled into one translation unit per code width.
 #pragma once
@@ -261,7 +260,7 @@ template <int BITS, int LOGG> struct I8Shape {
 
 // PB: bytes of a piece of scales, 16, 8 or 4, where rows of scales (and the units in them) start at multiples of it: pieces then lie in
 // shared memory as the affine step wants them, eight groups to a load.  0: rows that start anywhere; an aligned window is copied and read
-// one value at a time.  KS: CTAs per row, 1 or 2.  (One kernel with a run-time switch: gate and up of 14336 x 4096 13.7 us instead of 13.3.)
+// one value at a time.  KS: CTAs per row, 1 or 2.  (PB at run time: 3 % slower.)
 template <int BITS, int LOGG, int NB, bool PACKETS, int PB, int KS>
 __global__ void __launch_bounds__(kI8Threads, 1) qgemv_i8_kernel(const __grid_constant__ I8Params p) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -684,11 +683,10 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
     p.eps = q.eps; p.B = q.B; p.N = q.N; p.K = q.K; p.Gn = q.Gn; p.act_dtype = q.act_dtype; p.norm_w_dtype = q.norm_w_dtype;
     p.row_bytes = q.row_bytes; p.tp_out = q.tp_out; p.tp_in = q.tp_in;
     p.units = (p.row_bytes + kI8UnitBytes - 1) / kI8UnitBytes;
-    // The largest piece of scales that rows and units are multiples of.  Before -> after (window or whole units only): gate and up of
-    // q4 11008 x 2816 groups of 128, two pieces of 4 bytes, one row 9.5 -> 8.0 us, four rows 13.4 -> 11.8; 9000 x 2816 groups of 64, two of 8,
-    // 8.9 -> 7.9 and 12.6 -> 11.4; 6000 x 2688 groups of 32, four of 8, 8.4 -> 8.2 and 12.8 -> 12.1; q8 8192 x 3008 groups of 32, four of 4,
-    // four rows 18.3 -> 17.7.  More copies than that cost more than the window: one row of the last 12.74 -> 12.78, eight pieces of 4
-    // bytes (q4 5003 x 2624 groups of 32) one row 8.2 -> 8.6.
+    // The largest piece of scales that rows and units are multiples of.  Window -> pieces, gate and up, one and four rows: q4 11008 x 2816
+    // groups of 128, two pieces of 4 bytes, 9.5 -> 8.0 us and 13.4 -> 11.9; 9000 x 2816 groups of 64, two of 8, 8.9 -> 7.9 and 12.6 -> 11.4;
+    // 6000 x 2688 groups of 32, four of 8, 8.4 -> 8.2 and 12.8 -> 12.1.  More pieces cost more than the window: one row of q8 8192 x 3008 groups
+    // of 32, four of 4, 12.74 -> 12.78; q4 5003 x 2624 groups of 32, eight of 4, 8.2 -> 8.6.
     constexpr int P4 = S::MB <= (NB == 1 ? 8 : 16) ? 4 : 0, P8 = S::MB >= 8 ? 8 : P4, P16 = S::MB >= 16 ? 16 : P8;
     int pb = P16;
     while (pb > 0 && p.Gn * 2 % pb != 0) pb = pb == 16 ? P8 : pb == 8 ? P4 : 0;
@@ -729,8 +727,9 @@ int launch_i8(const GemvParams& q, bool gate_up, cudaStream_t stream) {
         }
         return off;
     };
-    // Rounds of the three phases in a CTA: rows into fixed point, units, results.  A pair of CTAs costs a launch about as much as one round
-    // of the first (0.45 us), so two rounds less are asked for.  (A fused norm needs the whole row in each CTA.)
+    // Rounds of the three phases in a CTA: rows into fixed point, units, results.  A pair costs a launch 0.4 us (4096 x 4096 one row, which it
+    // saves nothing, 4.8 -> 5.2), a round of the first phase 0.6 us by the SM's clock, so two rounds less, of whichever phase, are asked
+    // for.  (A fused norm needs the whole row in each CTA.)
     auto rounds = [&]() -> int {
         const int units = (p.units + ks - 1) / ks, r_max = p.rows_lo + (p.rem ? 1 : 0), tiles = (r_max + 15) / 16;
         auto per = [](int n, int by) { return (n + by - 1) / by; };

@@ -979,13 +979,16 @@ bool scale_map(const void* ptr, int pitch, int64_t tokens, int box_bytes, CUtens
 }
 
 int launch_cluster_attention(ClusterAttnParams& p, cudaStream_t stream) {
-    const bool plain = p.bits == 16, bf = p.q_dtype == B200Q_BF16, g32 = p.G == 32, wide = p.group > 4, sc8 = !plain && ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
+    const bool plain = p.bits == 16, bf = p.q_dtype == B200Q_BF16, g32 = p.G == 32, wide = p.group > 4;
+    const bool sc8 = !plain && ((uintptr_t)p.k_scales | (uintptr_t)p.v_scales) % 16 != 0;
     // Sixteen warps where eight would have more than a page each: a page costs a warp about a microsecond, the merge of eight more partial
     // results 0.2 (one sequence, one page a warp: q8 5.4 us with eight, 5.7 with sixteen; two sequences of 2048 tokens 9.2 and 8.5).
     // Whether their rings fit is asked of the UNSHARDED cache's scales, like the choice of the kernel: the number of warps is part of the
     // summation order, and a shard's narrower scale rows would let it have sixteen where the unsharded call has eight.
     int warps = !plain && (p.walk_pages > p.S * 8 || p.window > 0) ? kClusterWarps : 8;
-    auto slot_for = [&](int hs) { return split_slot_bytes(p.bits, 1, 0) + (plain ? 0u : align_up_u32(2 * split_scale_bytes(hs, p.Gd), p.bits == 4 ? 512 : 1024)); };
+    auto slot_for = [&](int hs) {
+        return split_slot_bytes(p.bits, 1, 0) + (plain ? 0u : align_up_u32(2 * split_scale_bytes(hs, p.Gd), p.bits == 4 ? 512 : 1024));
+    };
     p.hs = std::min(p.Hkv, kAttnWarps);
     p.slot_bytes = slot_for(p.hs);
     const uint32_t slot_full = slot_for((int)std::min<int64_t>((int64_t)p.Hkv * std::max(1, tuning_get("ts.tp_world")), kAttnWarps));
@@ -1211,12 +1214,13 @@ int paged_gqa_decode_impl(int bits, const void* q, const uint8_t* k_codes, const
     if (!fast_ok) return simple();
     // small batches: one cluster per (sequence, kv head), merged on chip - no workspace, no second launch
     const int ranges = split_ranges(workspace, workspace_bytes, B, Hq, Hkv, D, q_dtype);
-    // A window bounds the walk whatever the length.  Windows as long as the table stay with the split-KV kernels, whose dense result they
+    // A window bounds the walk whatever the length of the sequence.  Windows as long as the table stay with the split-KV kernels, whose dense result they
     // reproduce bit for bit; without a workspace only dense calls are served.
     const int64_t visited = ((int64_t)window_size + 15) / 16 + 1 + ((int64_t)sink_tokens + 15) / 16;
     const int walk_pages = window_size > 0 ? (int)std::min<int64_t>(max_blocks, visited) : max_blocks;
     const bool may = window_size == 0 || (ranges > 0 && window_size < (int64_t)max_blocks * page_size);
-    const ClusterChoice choice = may && B <= 65535 && Hkv <= 65535 ? choose_cluster(B, Hkv, group, walk_pages, window_size > 0 ? AttnUse::kWindow : AttnUse::kDense, ranges > 0) : ClusterChoice{0, false};
+    const AttnUse use = window_size > 0 ? AttnUse::kWindow : AttnUse::kDense;
+    const ClusterChoice choice = may && B <= 65535 && Hkv <= 65535 ? choose_cluster(B, Hkv, group, walk_pages, use, ranges > 0) : ClusterChoice{0, false};
     const int cluster = choice.preferred || ranges == 0 ? choice.size : 0;
     if (cluster > 0) {
         ClusterAttnParams c = {};
@@ -1265,7 +1269,8 @@ int paged_plain_attention_impl(const void* q, const void* k_pages, const void* v
     p.group = Hq / Hkv; p.num_pages = num_pages; p.scale = scale; p.q_dtype = dtype; p.bits = 16;
     p.row_bytes = Hkv * kHeadDim * 2;
     p.verdict = verdict;
-    const ClusterChoice choice = B <= 65535 && Hkv <= 65535 ? choose_cluster(B, Hkv, Hq / Hkv, max_blocks, AttnUse::kPlain, true) : ClusterChoice{0, false};
+    const ClusterChoice choice =
+        B <= 65535 && Hkv <= 65535 ? choose_cluster(B, Hkv, Hq / Hkv, max_blocks, AttnUse::kPlain, true) : ClusterChoice{0, false};
     if (choice.preferred && choice.size > 0) {
         ClusterAttnParams c = {};
         c.q = q; c.q_dtype = dtype;

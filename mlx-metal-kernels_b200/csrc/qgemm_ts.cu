@@ -21,9 +21,9 @@
 //
 // What bounds it: a chunk (128 x 128 weights) costs the dequantisation 4 x 260 warp instructions, i.e. about 340 clocks on the SM's four
 // schedulers, and the tensor pipe 8 x 22 clocks up to 32 columns, 8 x 65 at 128; a chunk takes about 480, since stores into tensor
-// memory and MMAs hold each other up and every barrier costs a waiting warp some time beside the others.  Fewer, longer pieces per wait are therefore better: eight warps per chunk
-// instead of four measured 54 against 48 us on an MLP block of 32 rows (at 600 clocks a chunk).  One block of up to 128 columns shares each dequantised
-// weight.  Measured (q4): block 4096 -> 14336 -> 4096, 32 rows 48 -> 45.9 us; 4096 -> 11008 -> 4096, 256 rows 119 -> 104 us.
+// memory and MMAs hold each other up and every barrier costs a waiting warp some time beside the others.  Fewer, longer pieces per wait are
+// therefore better: eight warps per chunk instead of four were 12 % slower on an MLP block of 32 rows.  One block of up to 128 columns
+// shares each dequantised weight.  q4 MLP blocks: 4096 -> 14336 -> 4096, 32 rows 45.9 us; 4096 -> 11008 -> 4096, 256 rows 104 us.
 // Codes are unpacked in k order (one byte permute per pair): the activations need no rearrangement, and nothing but TMA touches
 // them.  (The form before this one permuted the rows in shared memory with four warps, recomputed the group constants per 32 k and
 // kept 32 columns per launch: 1800 warp instructions per chunk; a 256-row prompt chunk re-streamed its weights eight times.)
@@ -222,9 +222,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-// A probe that suspends the warp for up to a microsecond, for every probe of a wait but the first.  Probes that come back at once are repeated, and those of the waiting warps
-// took a third of the issue slots of a busy SM from the dequantising ones (537 instructions per chunk and scheduler, 340 of them the
-// dequantisation's): 6144 x 4096 q4 for 32 rows 11.2 -> 10.4 us, gate and up of 11008 x 4096 for 256 rows 65.5 -> 60.8.
+// A probe that suspends the warp for up to a microsecond.  The first probe of a wait is a plain one, all others are this: plain ones come back
+// at once, and repeated by the waiting warps they took a third of a busy SM's issue slots from the dequantising ones (537 instructions
+// per chunk and scheduler, 340 of them the dequantisation's).  Without -> with: 6144 x 4096 q4 for 32 rows 11.2 -> 10.4 us.
 __device__ __forceinline__ bool probe_bar(uint32_t addr, uint32_t parity) {
     uint32_t got;
     asm volatile(
@@ -251,10 +251,9 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int eve
 }
 
 // One wait of a warp for several barriers: lane i polls its own (address and parity per lane; lanes without one pass `need` false).
-// For the operands of two chunks at once (gate and up, few columns): polled together 25.4 us, in turn 25.7 (14336 x 4096 q4, 32 rows), and
-// without suspending (bf16 rows 41.6 us, suspending 42.1).  The two
-// barriers of a single chunk are waited for in turn: together 66.2 us, in turn 62.4 (gate and up of 11008 x 4096, 256 rows).  One loop for
-// both cases: 60.9 us there instead of 57.0.
+// For the operands of two chunks at once (gate and up, few columns): in turn is 1 % slower there, and so is suspending (14336 x 4096 q4, 32 rows).
+// The two barriers of a single chunk are waited for in turn: together is 6 % slower, and one loop for both cases 7 % (gate and up of
+// 11008 x 4096, 256 rows, 57 us).
 __device__ __forceinline__ void wait_bars(uint32_t addr, uint32_t parity, bool need, int event, bool& ok) {
     const uint32_t limit = ok ? kTsWaitLimit : 64u;
     for (uint32_t i = 0; i < limit; ++i) {
@@ -498,8 +497,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) qgemm_ts_kernel(const __grid_co
                     const bool two = ch + 1 < n_ch;
                     if (two) at.to(it * n_ch + ch + 1, XS, NA);
                     // lanes 0, 1: the first chunk's operands; lanes 2, 3: the second's
-                    const uint32_t bar = lane == 0 ? smem_u32(&full_x[x.slot]) : lane == 1 ? smem_u32(&a_full[a.slot]) : lane == 2 ? smem_u32(&full_x[at.x.slot]) : smem_u32(&a_full[at.a.slot]);
-                    wait_bars(bar, lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
+                    const uint32_t bar = lane == 0   ? smem_u32(&full_x[x.slot])
+                                         : lane == 1 ? smem_u32(&a_full[a.slot])
+                                         : lane == 2 ? smem_u32(&full_x[at.x.slot])
+                                                     : smem_u32(&a_full[at.a.slot]);
+                    const uint32_t par = lane == 0 ? x.par : lane == 1 ? a.par : lane == 2 ? at.x.par : at.a.par;
+                    wait_bars(bar, par, lane < (two ? 4 : 2), EV_GEMV_FULL_WAIT, ok);
                     tc_fence_after();
                     chunk(x.slot, a.slot, ch == 0);
                     if (two) chunk(at.x.slot, at.a.slot, false);
@@ -896,15 +899,13 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     // Column blocks and K split by estimated time, in clocks: rounds of items over the SMs, each a chain of chunks whose cost is the
     // dequantisation's (450; 64 k in two terms 540) or the tensor pipe's: 22 clocks per MMA up to 32 columns, then half a clock per column,
     // and 260 a chunk in which the next chunk's way into tensor memory keeps it waiting (no arithmetic at all: 530 clocks at 64
-    // columns, 650 at 96).  The first CTA of a cluster takes about 35 clocks per column and part for the partial sums.  (Splits were once
-    // left out where the sums exceed 48 KB, from 33 rows on: 4096 x 14336 q4 48 rows 24.3 -> 16.6 us, 64 rows 24.6 -> 18.4; 4096 x
-    // 11008, groups of 32, 256 rows 35.2 -> 31.4.)  The choice
+    // columns, 650 at 96).  The first CTA of a cluster takes about 35 clocks per column and part for the partial sums.  The choice
     // must not depend on how many rows THIS launch holds: a tensor-parallel shard of the rows has to reproduce the unsharded result
     // bit for bit, so the tile count of the unsharded matrix decides ("ts.tp_world" = number of equal row shards).
     const int tiles_full = tiles * std::max(1, tuning_get("ts.tp_world"));
     const int forced = tuning_get("ts.split");
-    // bytes of partial sums: in a dedicated buffer (96 KB of it leave too little for the rings: 64 rows of 4096 x 14336 19.8 us, through the
-    // rings 18.7; 72 KB 17.0 and 17.7), and at all
+    // bytes of partial sums: in a dedicated buffer (4096 x 14336 q4: 72 KB, 48 rows, 17.0 us, through the rings 17.7; 96 KB, 64 rows, which leave
+    // the rings too little, 19.8 and 18.7), and at all (not beyond 48 KB, and so fewer parts: 24.3 and 24.6)
     constexpr uint32_t kRedCap = 80u * 1024u, kRedMax = 128u * 1024u;
     double best = 0.0;
     int cols = 0, split = 1;
@@ -921,7 +922,8 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
             const int slots = sp == 1 ? sms : max_clusters(kernel, sp, cap - 2048u);
             if (forced <= 0 && sp > 1 && items > slots) continue;
             const double rounds = (double)((items + slots - 1) / slots);
-            const double t = rounds * ((double)((p.n_stage_total + sp - 1) / sp * SC * MATS) * chunk + 1500.0 + c * MATS * 10.0) + (sp > 1 ? 1500.0 + 35.0 * (sp - 1) * MATS * std::min(c, p.B) : 0.0);
+            const double item = (double)((p.n_stage_total + sp - 1) / sp * SC * MATS) * chunk + 1500.0 + c * MATS * 10.0;
+            const double t = rounds * item + (sp > 1 ? 1500.0 + 35.0 * (sp - 1) * MATS * std::min(c, p.B) : 0.0);
             if (cols == 0 || t < best) { best = t; cols = c; split = sp; }
         }
     }
@@ -970,7 +972,8 @@ int launch_ts(TsParams& p, int K, cudaStream_t stream) {
     p.off_meta = p.off_x + (uint32_t)xs * p.x_bytes;
     const uint32_t rings_end = p.off_meta + (uint32_t)p.meta_bufs * kMetaBuf;
     p.off_red = fast_red ? rings_end : 0u;
-    if (split > 1 && !fast_red && (uint64_t)(split - 1) * MATS * cols * kRows * 4 > (uint64_t)rings_end - 1024u) return B200Q_ERR_UNSUPPORTED;      // only with a forced split
+    // only with a split or few stages by request ("ts.split", "ts.stages")
+    if (split > 1 && !fast_red && (uint64_t)(split - 1) * MATS * cols * kRows * 4 > (uint64_t)rings_end - 1024u) return B200Q_ERR_UNSUPPORTED;
 
     if (!tensor_map_2d(p.x, (uint64_t)K * 2, (uint64_t)p.B, 128, (uint32_t)cols, CU_TENSOR_MAP_SWIZZLE_128B, &p.xmap)) return B200Q_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg = {};
